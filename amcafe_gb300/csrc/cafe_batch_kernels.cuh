@@ -15,12 +15,11 @@
 // path this time) leave their blocks idle.
 
 enum {
-  BK_RESET_A = 0,  // CTR_HOT = 0 (before the melt pass)
+  BK_RESET = 0,    // CTR_HOT = 0 (before the melt pass)
   BK_MELT,
   BK_PBOX0,
   BK_PBOX1,
   BK_LIST,
-  BK_RESET_B,      // CTR_NLIQ = 0 (after the liquid-list pass used it)
   BK_ACOUNT,
   BK_SCAN,
   BK_ASCATTER,
@@ -28,15 +27,16 @@ enum {
   BK_LCOUNT,
   BK_SCANP,
   BK_LSCATTER,
-  BK_RESET_C,      // CTR_SLOW = CTR_NPAIRS = 0
   BK_PREP,
   BK_GEO,
   BK_ORDER,
+  BK_CHILD0,       // one per generation of foreseen captures
+  BK_CHILD1,
+  BK_CHILD2,
   BK_LOOP,
   BK_FINAL,
   BK_WB,
-  BK_M2S,
-  BK_REPORT,       // CTR_HOT and the error word into the host-visible report
+  BK_M2S,          // also CTR_HOT and the error word into the host-visible report
   BK_COUNT
 };
 
@@ -80,8 +80,8 @@ __device__ __forceinline__ bool cafe_batch_slot(const CafeBatchArgs &B, int kind
   if (!cafe_batch_slot(B, kind, r, b, nb)) return;    \
   const CafeBatchReal &R = B.R[r]
 
-__global__ void kb_reset_a(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_RESET_A);
+__global__ void kb_reset(CafeBatchArgs B) {
+  CAFE_BATCH_BLOCK(BK_RESET);
   if (threadIdx.x == 0) R.D.ctr[CTR_HOT] = 0;
 }
 __global__ void kb_melt(CafeBatchArgs B) {
@@ -99,10 +99,6 @@ __global__ void kb_solid2mushy_pbox1(CafeBatchArgs B) {
 __global__ void kb_solid2mushy_list(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_LIST);
   d_solid2mushy_list(R.D, R.K, b, nb);
-}
-__global__ void kb_reset_b(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_RESET_B);
-  if (threadIdx.x == 0) R.D.ctr[CTR_NLIQ] = 0;
 }
 __global__ void kb_active_count(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_ACOUNT);
@@ -132,15 +128,6 @@ __global__ void kb_lists_scatter(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_LSCATTER);
   d_lists_scatter(R.D, b, nb);
 }
-__global__ void kb_reset_c(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_RESET_C);
-  if (threadIdx.x == 0) {
-    R.D.ctr[CTR_SLOW] = 0;
-    R.D.ctr[CTR_NPAIRS] = 0;
-    R.D.fill_seq[0] = 0;  // the event loop's fill hand-off (two blocks per realisation)
-    R.D.fill_seq[1] = 0;
-  }
-}
 __global__ void kb_rows_prep(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_PREP);
   d_rows_prep(R.D, R.K, b, nb);
@@ -153,13 +140,18 @@ __global__ void kb_rows_order(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_ORDER);
   d_rows_order(R.D, R.K, b, nb);
 }
+static_assert(CAFE_CHILD_DEPTH == 3, "one batched launch per generation");
+__global__ void __launch_bounds__(CAFE_QUAD_THREADS) kb_children(CafeBatchArgs B, int depth) {
+  CAFE_BATCH_BLOCK(BK_CHILD0 + depth);
+  d_children(R.D, R.K, depth, b, nb);
+}
 __global__ void __launch_bounds__(CAFE_LOOP_THREADS, 1) kb_event_loop(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_LOOP);
   d_event_loop(R.D, R.K, R.D.Pd, R.D.act_cap + 1, R.allow_fast, b, nb);
 }
 __global__ void kb_rows_finalize(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_FINAL);
-  d_rows_finalize(R.D, b, nb);
+  d_rows_finalize(R.D, R.K, b, nb);
 }
 __global__ void kb_writeback(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_WB);
@@ -168,10 +160,7 @@ __global__ void kb_writeback(CafeBatchArgs B) {
 __global__ void kb_mushy2solid(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_M2S);
   d_mushy2solid(R.D, R.K, b, nb);
-}
-__global__ void kb_report(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_REPORT);
-  if (threadIdx.x == 0) {
+  if (b == 0 && threadIdx.x == 0) {  // nothing sets either after the event loop
     B.report[2 * r] = R.D.ctr[CTR_HOT];
     B.report[2 * r + 1] = *R.D.err;
   }

@@ -19,6 +19,10 @@
 #include "cafe_rng.h"
 
 #define CAFE_NSLOT 26
+// Generations of foreseen captures whose rows are made ahead of the event loop,
+// and how far past the step's end (in time steps) a capture is foreseen.
+#define CAFE_CHILD_DEPTH 3
+#define CAFE_CHILD_REACH 1.1
 
 // Error bits written to CafeDev::err by device code.
 enum {
@@ -27,17 +31,16 @@ enum {
   CAFE_ERR_GRAIN_CAP = 4,
   CAFE_ERR_MUSHY_CAP = 8,
   CAFE_ERR_ITER_CAP = 16,
-  CAFE_ERR_SYNC = 32,  // a bounded wait between the event loop's two blocks ran out
 };
 
-// The new-row fill that the event loop's main block hands to its helper
-// block (k_event_loop with two blocks): the row, the captured cell's active
-// position, the event, the cell's grain, centre and extent, the time, and
-// the helper's result (the order key of the row's largest |g|).
-struct CafeFillReq {
-  int r, p, e, gid;
-  double c[3], ext, T;
-  unsigned long long gk;
+// One slot of a frontier row's record: numerator g, neighbour position q (-1
+// when absent) and, in the low five bits of m, the neighbour direction; above
+// them the number, plus one, of the row made ahead for a capture through it (0
+// when none).
+struct __align__(16) CafeSlot {
+  double g;
+  int q;
+  uint32_t m;
 };
 
 // Scalars that change every step (computed on the host from Grid/TempField).
@@ -147,46 +150,52 @@ struct CafeDev {
   // active list and per-position copies
   int32_t *act;
   long long act_cap;
-  uint8_t *a_state, *a_cls, *a_nn, *a_cold;
+  uint8_t *a_state, *a_cls, *a_cold;
+  // a_nbr: 26 neighbour positions by direction (ascending cell index; direction
+  // s and 25 - s are opposite), -1 = not active or outside the grid
   int32_t *a_gid, *a_liq, *a_frow, *a_nbr;
   double *a_ext, *a_cx, *a_cy, *a_cz, *a_ruq;
+  double *a_nuc;  // nucleation probability per position (Gaussian undercooling only)
   // mushy list (vs2ind) and frontier rows
   int32_t *vs2;
   long long vs2_cap;
   int32_t *row_pos, *row_j;
-  uint8_t *row_alive, *row_ord;
+  // a row's record: its slots by g (row_slot, CAFE_NSLOT entries), the place
+  // of each direction in it (row_rank, 32 entries) and the live places
+  // (row_live)
+  CafeSlot *row_slot;
+  uint8_t *row_rank;
   uint32_t *row_live;
-  double *row_g;
-  // per (row, slot): extent and centre (x, y, z) given to the neighbour when
-  // this slot captures it, 4 doubles
+  // per (row, direction): extent and centre (x, y, z) given to the neighbour
+  // when this slot captures it, 4 doubles
   double *row_geo;
+  // rows 0 .. row_cap - 1 are the step's frontier rows; rows row_cap ..
+  // row_cap + ch_cap - 1 are made ahead for captures foreseen within the step:
+  // the slot (row * CAFE_NSLOT + direction), grain and time of each capture.
+  // row_new: the rows that captures created, in their order
   long long row_cap;
+  int ch_cap;
+  int32_t *ch_src, *ch_gid, *row_new;
+  double *ch_T;
   // (row, slot) pairs whose capture geometry the row set-up evaluates, as
   // row * 32 + slot, row_cap * CAFE_NSLOT entries
   int32_t *row_pairs;
   // rows during the event loop: row_E is the row cell's extent (ExtA)
   // including the growth of events 1..row_m, copied back to a_ext afterwards;
-  // a row grows at the events (birth, row_death]; row_key orders the rows by
-  // estimated absolute capture time; row_b* hold the exact best candidate of
-  // the iteration row_stamp (row_bq: the position that slot captures);
-  // row_key2 is the key of the row's smallest candidate time apart from slot
-  // row_bslot at that evaluation, the row's key once that slot is captured
-  // by another row
+  // a row grows at the events (birth, row_death]; row_key bounds the row's
+  // absolute capture time from below; row_res is its place in the resident set
+  // (-1 none); row_mag: order keys of the largest |g|, the largest extent, the
+  // smallest and the largest velocity of the step's rows
   double *row_E;
-  int32_t *row_m, *row_death, *row_stamp, *row_bslot, *row_bq;
-  unsigned long long *row_key, *row_key2;
-  double *row_bt, *row_bruq;
-  // per-event growth: ev_vd[e] = fl(v * DtMin_e) (+0 for a nucleation),
-  // ev_vs[e] = running sum of ev_vd
+  int32_t *row_m, *row_death, *row_res;
+  unsigned long long *row_key, *row_mag;
+  // the logged growth of each event (CTR_EVLOG: fl(v * DtMin), or DtMin) and
+  // its running sum
   double *ev_vd, *ev_vs;
   long long ev_cap;
   // scan scratch
   int32_t *blk;       // per-block counts / offsets
   long long blk_cap;
-  // the event loop's fill hand-off: the request, and two sequence numbers
-  // (posted by the main block, done by the helper; zeroed before each launch)
-  CafeFillReq *fill;
-  int *fill_seq;
   // device scalars
   int *ctr;           // see CTR_* below
   int *err;
@@ -203,7 +212,7 @@ enum {
   CTR_NNUC,        // nucleations this step
   CTR_NVS2_END,    // mushy-list length after the event loop
   CTR_NLIQ,        // liquid cells listed by the last write-back
-  CTR_SLOW,        // 1: this step's rows do not share one growth velocity
+  CTR_SLOW,        // this step's rows: bit 0 not one growth velocity, bit 1 full scan only
   CTR_NROWS_END,   // frontier rows after the event loop
   CTR_NPAIRS,      // (row, slot) pairs listed for the row set-up
   CTR_EASM_BOX,    // 6 slots: box of the cells at or above the liquidus (EASM)
@@ -213,13 +222,16 @@ enum {
   CTR_EASM_QHEAD,                       // next queued cell to take
   CTR_GLOG_N,                           // growth-log entries written
   CTR_GLOG_OVER,                        // 1: the growth log ran out of room
+  CTR_EVLOG,                            // 1: ev_vd holds DtMin, 0: fl(v * DtMin)
+  CTR_NCHILD,                           // foreseen captures listed, one count per generation
+  CTR_NCHILD_LAST = CTR_NCHILD + CAFE_CHILD_DEPTH - 1,
   CTR_ZLO, CTR_ZHI,                     // z range of the mushy and liquid cells after the last step
   CTR_COUNT
 };
 static_assert(CTR_EASM_CURSOR % 2 == 0, "64-bit cursor needs an 8-byte aligned slot");
 enum { STAT_EVENTS = 0, STAT_NUC, STAT_MAXNA, STAT_MAXROWS, STAT_STEPS, STAT_NEGDT, STAT_SUMNA, STAT_SUMROWS,
        STAT_SLOWSTEPS, STAT_EVALS, STAT_CYC_SELECT, STAT_CYC_APPLY, STAT_CYC_FILL, STAT_CYC_OTHER,
-       STAT_EASM_INTEGRALS, STAT_DETAIL, STAT_COUNT = STAT_DETAIL + 32 };
+       STAT_EASM_INTEGRALS, STAT_COUNT };
 
 // --------------------------------------------------------------- temperature
 // TempField::AnalyticTempCurr (TempField.C:155-190) for one cell; returns the

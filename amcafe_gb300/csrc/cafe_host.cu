@@ -422,7 +422,7 @@ struct cafe_sim {
   int prev_lo[3] = {0, 0, 0}, prev_hi[3] = {0, 0, 0};
   bool full_k2 = false;   // next solid->mushy pass must scan the whole box
   int event_scan = 0;     // 1: evaluate every frontier row at every event
-  bool event_helper = false;  // the event loop's new-row fills run in a second block
+  bool event_helper = false;  // cafe_options::event_fill_helper (batched launches: two event-loop blocks)
   std::vector<void *> owned;
   int *h_pinned = nullptr;  // pinned host mirror of ctr + err
   // staging for host transfers (allocated on first use)
@@ -521,8 +521,7 @@ int sim_sync(cafe_sim *s) {
   if (err) {
     return fail(CAFE_E_CAPACITY,
                 "device capacity exceeded (flags 0x%x: 1 active list, 2 frontier rows, 4 grain "
-                "table, 8 mushy list, 16 event cap; 32: the event loop's two blocks timed out "
-                "waiting for each other); recreate with larger capacities",
+                "table, 8 mushy list, 16 event cap); recreate with larger capacities",
                 err);
   }
   return CAFE_OK;
@@ -831,34 +830,6 @@ int end_of_scan(cafe_sim *s, const int *hot_known = nullptr) {
   return CAFE_OK;
 }
 
-// The event loop: one block, or with the fill helper two blocks launched
-// cooperatively (both resident at once, which the hand-off between them
-// needs). The hand-off's sequence words start at zero.
-int launch_event_loop(cafe_sim *s, const CafeStepParams *Pp) {
-  cudaStream_t st = s->stream;
-  const CafeDev &D = s->D;
-  const long long max_ev = D.act_cap + 1;
-  const int allow_fast = s->event_scan ? 0 : 1;
-  if (!s->event_helper) {
-    k_event_loop<<<1, CAFE_LOOP_THREADS, 0, st>>>(s->D, s->K, Pp, max_ev, allow_fast);
-    CUDA_TRY(cudaGetLastError());
-    return CAFE_OK;
-  }
-  CUDA_TRY(cudaMemsetAsync(D.fill_seq, 0, 2 * sizeof(int), st));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2);
-  cfg.blockDim = dim3(CAFE_LOOP_THREADS);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, k_event_loop, s->D, s->K, Pp, max_ev, allow_fast));
-  return CAFE_OK;
-}
-
 // VoxelsCA::UpdateVoxels on the device (no host synchronisation). In a graph
 // the box kernels get fixed grids and read their boxes from the parameters.
 int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
@@ -885,7 +856,6 @@ int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
       k_solid2mushy_list<<<s->gsm * 4, 256, 0, st>>>(D, K);
       LAUNCHED(CAFE_PH_CLASSIFY, 1);
     }
-    CUDA_TRY(cudaMemsetAsync(D.ctr + CTR_NLIQ, 0, sizeof(int), st));
     const int ab = (int)std::min<long long>(s->nblk_act, (long long)s->gsm * 8);  // persistent grid
     k_active_count<<<ab, CAFE_DENSE_THREADS, 0, st>>>(D, K, Pp, s->act_chunks, s->nblk_act);
     k_scan_blocks<<<1, 1024, 0, st>>>(D.blk, s->nblk_act, D.ctr + CTR_NA);
@@ -900,25 +870,21 @@ int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
     k_lists_count<<<nbp, CAFE_DENSE_THREADS, 0, st>>>(D);
     k_scan_pairs<<<1, 1024, 0, st>>>(D.blk, s->nblk_pos, D.ctr + CTR_NA, D.ctr + CTR_NVS2, D.ctr + CTR_NROWS);
     k_lists_scatter<<<nbp, CAFE_DENSE_THREADS, 0, st>>>(D);
-    if (K.easm)  // rows grow with per-cell velocities: the exact per-event scan
-      k_set_int<<<1, 1, 0, st>>>(D.ctr + CTR_SLOW, 1);
-    else
-      CUDA_TRY(cudaMemsetAsync(D.ctr + CTR_SLOW, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(D.ctr + CTR_NPAIRS, 0, sizeof(int), st));
     k_rows_prep<<<s->gsm * 4, 256, 0, st>>>(D, K);
     k_rows_geo<<<s->gsm * 8, 256, 0, st>>>(D, K);
     k_rows_order<<<s->gsm * 4, 256, 0, st>>>(D, K);
-    LAUNCHED(CAFE_PH_GATHER, 7);
+    for (int d = 0; d < CAFE_CHILD_DEPTH; ++d)
+      k_children<<<s->gsm * CAFE_CHILD_BLOCKS_PER_SM, CAFE_QUAD_THREADS, 0, st>>>(D, K, d);
+    LAUNCHED(CAFE_PH_GATHER, 7 + CAFE_CHILD_DEPTH);
   }
   {
     PhaseScope ps(s, CAFE_PH_EVENTS);
-    int rc = launch_event_loop(s, Pp);
-    if (rc) return rc;
+    k_event_loop<<<1, CAFE_LOOP_THREADS, 0, st>>>(D, K, Pp, D.act_cap + 1, s->event_scan ? 0 : 1);
     if (D.glog_cell) {
       k_glog_begin<<<s->gsm * 4, 256, 0, st>>>(D, Pp);
       LAUNCHED(CAFE_PH_EVENTS, 1);
     }
-    k_rows_finalize<<<s->gsm * 4, 256, 0, st>>>(D);
+    k_rows_finalize<<<s->gsm * 4, 256, 0, st>>>(D, K);
     LAUNCHED(CAFE_PH_EVENTS, 2);
     if (D.glog_cell) {
       k_glog_end<<<s->gsm * 4, 256, 0, st>>>(D, K);
@@ -1060,11 +1026,6 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
     return fail(CAFE_E_CUDA, "cudaSetDevice(%d): %s", opt ? opt->device : 0, cudaGetErrorString(ce));
   }
   cudaDeviceGetAttribute(&s->nsm, cudaDevAttrMultiProcessorCount, s->device);
-  {
-    int coop = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device);
-    if (!coop || s->nsm < 2) s->event_helper = false;
-  }
   s->gsm = s->nsm;
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete s;
@@ -1190,6 +1151,10 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
   // the pool, far smaller than the active list; an explicit active capacity
   // raises this limit with it
   D.row_cap = std::min<long long>(acap, opt && opt->active_capacity > 0 ? (1LL << 22) : (1LL << 20));
+  // rows made ahead for foreseen captures (a step has some hundred; those that
+  // do not fit are filled by the event loop)
+  D.ch_cap = (int)std::min<long long>(acap, 1 << 14);
+  const size_t nrow = (size_t)D.row_cap + D.ch_cap;
   D.ev_cap = acap + 2;  // an event captures or nucleates one active cell
   double est = g.mu * (g.dX[0] * 1e6) * (g.dX[1] * 1e6) * g.nX[0] * g.nX[1] * (s->Nzh * g.dX[2] * 1e6) +
                (s->nlayerTot + 1) * g.lrate * (g.dX[0] * 1e6) * (g.dX[1] * 1e6) * g.nX[0] * g.nX[1] * (g.layerT * 1e6);
@@ -1223,26 +1188,23 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
       (rc = dalloc(&D.buildj, N, o)) || (rc = dalloc(&D.build, N, o)) || (rc = dalloc(&D.pos_of, N, o)) || (rc = dalloc(&D.liq, acap, o)) ||
       (rc = dalloc(&D.cth, 4 * (size_t)D.grain_cap, o)) || (rc = dalloc(&D.rot, 9 * (size_t)D.grain_cap, o)) ||
       (rc = dalloc(&D.act, acap, o)) || (rc = dalloc(&D.a_state, acap, o)) || (rc = dalloc(&D.a_cls, acap, o)) ||
-      (rc = dalloc(&D.a_nn, acap, o)) || (rc = dalloc(&D.a_cold, acap, o)) || (rc = dalloc(&D.a_gid, acap, o)) ||
+      (rc = dalloc(&D.a_cold, acap, o)) || (rc = dalloc(&D.a_gid, acap, o)) ||
       (rc = dalloc(&D.a_liq, acap, o)) || (rc = dalloc(&D.a_frow, acap, o)) ||
       (rc = dalloc(&D.a_nbr, (size_t)acap * CAFE_NSLOT, o)) || (rc = dalloc(&D.a_ext, acap, o)) ||
       (rc = dalloc(&D.a_cx, acap, o)) || (rc = dalloc(&D.a_cy, acap, o)) || (rc = dalloc(&D.a_cz, acap, o)) ||
-      (rc = dalloc(&D.a_ruq, acap, o)) || (rc = dalloc(&D.vs2, acap, o)) || (rc = dalloc(&D.row_pos, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_j, D.row_cap, o)) || (rc = dalloc(&D.row_alive, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_ord, (size_t)D.row_cap * CAFE_NSLOT, o)) || (rc = dalloc(&D.row_live, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_g, (size_t)D.row_cap * CAFE_NSLOT, o)) ||
-      (rc = dalloc(&D.row_geo, (size_t)D.row_cap * CAFE_NSLOT * 4, o)) ||
+      (rc = dalloc(&D.a_ruq, acap, o)) || (rc = dalloc(&D.vs2, acap, o)) || (rc = dalloc(&D.row_pos, nrow, o)) ||
+      (rc = dalloc(&D.row_j, nrow, o)) || (rc = dalloc(&D.row_live, nrow, o)) ||
+      (rc = dalloc(&D.row_slot, nrow * CAFE_NSLOT, o)) || (rc = dalloc(&D.row_rank, nrow * 32, o)) ||
+      (rc = dalloc(&D.row_geo, nrow * CAFE_NSLOT * 4, o)) ||
+      (rc = dalloc(&D.row_new, D.row_cap, o)) || (rc = dalloc(&D.ch_src, D.ch_cap, o)) ||
+      (rc = dalloc(&D.ch_gid, D.ch_cap, o)) || (rc = dalloc(&D.ch_T, D.ch_cap, o)) ||
       (rc = dalloc(&D.row_pairs, (size_t)D.row_cap * CAFE_NSLOT, o)) || (rc = dalloc(&D.blk, D.blk_cap, o)) ||
-      (rc = dalloc(&D.row_E, D.row_cap, o)) || (rc = dalloc(&D.row_death, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_m, D.row_cap, o)) || (rc = dalloc(&D.ev_vd, D.ev_cap, o)) ||
-      (rc = dalloc(&D.ev_vs, D.ev_cap, o)) ||
-      (rc = dalloc(&D.row_stamp, D.row_cap, o)) || (rc = dalloc(&D.row_bslot, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_bq, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_key, D.row_cap, o)) || (rc = dalloc(&D.row_key2, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_bt, D.row_cap, o)) ||
-      (rc = dalloc(&D.row_bruq, D.row_cap, o)) ||
+      (rc = dalloc(&D.row_E, nrow, o)) || (rc = dalloc(&D.row_death, nrow, o)) ||
+      (rc = dalloc(&D.row_m, nrow, o)) || (rc = dalloc(&D.row_res, nrow, o)) ||
+      (rc = dalloc(&D.row_key, nrow, o)) || (rc = dalloc(&D.row_mag, 4, o)) ||
+      (rc = dalloc(&D.ev_vd, D.ev_cap, o)) || (rc = dalloc(&D.ev_vs, D.ev_cap, o)) || (K.nuc_gauss && (rc = dalloc(&D.a_nuc, acap, o))) ||
       (rc = dalloc(&D.ctr, CTR_COUNT, o)) || (rc = dalloc(&D.err, 1, o)) || (rc = dalloc(&D.stat, STAT_COUNT, o)) ||
-      (rc = dalloc(&D.Pd, 1, o)) || (rc = dalloc(&D.fill, 1, o)) || (rc = dalloc(&D.fill_seq, 2, o)) ||
+      (rc = dalloc(&D.Pd, 1, o)) ||
       (rc = dalloc(&D.act_flags, (size_t)((N + CAFE_CELLS_PER_BLOCK - 1) / CAFE_CELLS_PER_BLOCK) * CAFE_DENSE_THREADS, o)) || (rc = dalloc(&D.tcls, std::max<long long>(D.tcls_cap, 1), o)) ||
       (K.easm && ((rc = dalloc(&D.temp, N, o)) || (rc = dalloc(&D.a_vh, acap, o)) ||
                   (rc = dalloc(&D.easm_q, (size_t)(D.easm_qcap = std::min<long long>(N, 1LL << 21)), o))))) {
@@ -2356,7 +2318,7 @@ struct CafeBatchEngine {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> ev_plain;
   int share = 4, chunks = 1;      // launch shape in use
-  bool loop_pairs = false;        // two event-loop blocks per realisation (fill helper)
+  int loop_blocks = 1;            // event-loop blocks per realisation (2 with the fill helper; the second is idle)
   bool tuned = false;
   int tune_steps = 6;             // batch steps timed per candidate
   std::vector<std::pair<std::pair<int, int>, double>> trials;  // ((share, chunks), ms per batch step)
@@ -2369,22 +2331,24 @@ struct CafeBatchEngine {
 
 namespace {
 
-const int kBatchThreads[BK_COUNT] = {32, 256, 256, 256, 256, 32, CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256,
-                                     CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 32, 256, 256, 256,
-                                     CAFE_LOOP_THREADS, 256, 256, 256, 32};
+const int kBatchThreads[BK_COUNT] = {32, 256, 256, 256, 256, CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256,
+                                     CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256, 256, 256,
+                                     CAFE_QUAD_THREADS, CAFE_QUAD_THREADS, CAFE_QUAD_THREADS,
+                                     CAFE_LOOP_THREADS, 256, 256, 256};
 
 // blocks of realisation s in a batched launch of `kind` (its plain graphed
 // step's grid, cafe_sim launch_melt / launch_voxels)
-long long batch_blocks(const cafe_sim *s, int kind, bool loop_pairs) {
+long long batch_blocks(const cafe_sim *s, int kind, int loop_blocks) {
   const long long g = s->gsm;
   switch (kind) {
-    case BK_LOOP: return loop_pairs ? 2 : 1;
+    case BK_LOOP: return loop_blocks;
     case BK_MELT: case BK_PBOX0: case BK_PBOX1: return g * 16;
+    case BK_CHILD0: case BK_CHILD1: case BK_CHILD2: return g * CAFE_CHILD_BLOCKS_PER_SM;
     case BK_LIST: case BK_PREP: case BK_ORDER: case BK_FINAL: return g * 4;
     case BK_ACOUNT: case BK_ASCATTER: return std::max<long long>(1, std::min<long long>(s->nblk_act, g * 8));
     case BK_GATHER: case BK_GEO: case BK_WB: case BK_M2S: return g * 8;
     case BK_LCOUNT: case BK_LSCATTER: return std::max<long long>(1, s->nblk_pos);
-    default: return 1;  // resets, scans, the event loop, the report
+    default: return 1;  // the reset, scans
   }
 }
 
@@ -2411,7 +2375,7 @@ int batch_capture(CafeBatchEngine *E) {
     long long acc = 0;
     for (int r = 0; r < n; ++r) {
       start[(size_t)k * (n + 1) + r] = (int)acc;
-      acc += batch_blocks(E->sims[r], k, E->loop_pairs);
+      acc += batch_blocks(E->sims[r], k, E->loop_blocks);
     }
     if (acc > 0x7fffffffLL) return fail(CAFE_E_CAPACITY, "batch: too many blocks in one launch");
     start[(size_t)k * (n + 1) + n] = (int)acc;
@@ -2428,12 +2392,11 @@ int batch_capture(CafeBatchEngine *E) {
   cudaStream_t st = E->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
   CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  kb_reset_a<<<E->total[BK_RESET_A], T[BK_RESET_A], 0, st>>>(A);
+  kb_reset<<<E->total[BK_RESET], T[BK_RESET], 0, st>>>(A);
   kb_melt<<<E->total[BK_MELT], T[BK_MELT], 0, st>>>(A);
   kb_solid2mushy_pbox0<<<E->total[BK_PBOX0], T[BK_PBOX0], 0, st>>>(A);
   kb_solid2mushy_pbox1<<<E->total[BK_PBOX1], T[BK_PBOX1], 0, st>>>(A);
   kb_solid2mushy_list<<<E->total[BK_LIST], T[BK_LIST], 0, st>>>(A);
-  kb_reset_b<<<E->total[BK_RESET_B], T[BK_RESET_B], 0, st>>>(A);
   kb_active_count<<<E->total[BK_ACOUNT], T[BK_ACOUNT], 0, st>>>(A);
   kb_scan_blocks<<<E->total[BK_SCAN], T[BK_SCAN], 0, st>>>(A);
   kb_active_scatter<<<E->total[BK_ASCATTER], T[BK_ASCATTER], 0, st>>>(A);
@@ -2441,29 +2404,15 @@ int batch_capture(CafeBatchEngine *E) {
   kb_lists_count<<<E->total[BK_LCOUNT], T[BK_LCOUNT], 0, st>>>(A);
   kb_scan_pairs<<<E->total[BK_SCANP], T[BK_SCANP], 0, st>>>(A);
   kb_lists_scatter<<<E->total[BK_LSCATTER], T[BK_LSCATTER], 0, st>>>(A);
-  kb_reset_c<<<E->total[BK_RESET_C], T[BK_RESET_C], 0, st>>>(A);
   kb_rows_prep<<<E->total[BK_PREP], T[BK_PREP], 0, st>>>(A);
   kb_rows_geo<<<E->total[BK_GEO], T[BK_GEO], 0, st>>>(A);
   kb_rows_order<<<E->total[BK_ORDER], T[BK_ORDER], 0, st>>>(A);
-  if (E->loop_pairs) {
-    // every pair must be resident at once: a cooperative launch
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(E->total[BK_LOOP]);
-    cfg.blockDim = dim3(T[BK_LOOP]);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kb_event_loop, A);
-  } else {
-    kb_event_loop<<<E->total[BK_LOOP], T[BK_LOOP], 0, st>>>(A);
-  }
+  for (int d = 0; d < CAFE_CHILD_DEPTH; ++d)
+    kb_children<<<E->total[BK_CHILD0 + d], T[BK_CHILD0 + d], 0, st>>>(A, d);
+  kb_event_loop<<<E->total[BK_LOOP], T[BK_LOOP], 0, st>>>(A);
   kb_rows_finalize<<<E->total[BK_FINAL], T[BK_FINAL], 0, st>>>(A);
   kb_writeback<<<E->total[BK_WB], T[BK_WB], 0, st>>>(A);
   kb_mushy2solid<<<E->total[BK_M2S], T[BK_M2S], 0, st>>>(A);
-  kb_report<<<E->total[BK_REPORT], T[BK_REPORT], 0, st>>>(A);
   cudaMemcpyAsync(E->hReport, E->dReport, 2 * (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st);
   cudaGraph_t g = nullptr;
   cudaError_t le = cudaGetLastError();
@@ -2508,7 +2457,7 @@ int batch_tune_next(CafeBatchEngine *E, double ms) {
   snprintf(buf, sizeof buf,
            "], \"chosen\": {\"grid_share_sms\": %d, \"compaction_chunks\": %d}, \"steps_each\": %d, "
            "\"event_loop_blocks\": %d}",
-           E->trials[best].first.first, E->trials[best].first.second, E->tune_steps, E->loop_pairs ? 2 : 1);
+           E->trials[best].first.first, E->trials[best].first.second, E->tune_steps, E->loop_blocks);
   s += buf;
   E->log = s;
   E->tuned = true;
@@ -2558,16 +2507,7 @@ CafeBatchEngine *cafe_internal_batch_engine_create(cafe_sim *const *sims, int n,
   }
   E->hR.resize(n);
   E->hR_valid.assign(n, 0);
-  {
-    // event-loop pairs when every realisation has its helper on and all the
-    // pairs fit on the GPU at once
-    int per_sm = 0, coop = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, E->device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kb_event_loop, CAFE_LOOP_THREADS, 0);
-    bool all = true;
-    for (int r = 0; r < n; ++r) all = all && sims[r]->event_helper;
-    E->loop_pairs = all && coop && (long long)per_sm * E->nsm >= 2LL * n;
-  }
+  E->loop_blocks = std::all_of(sims, sims + n, [](const cafe_sim *s) { return s->event_helper; }) ? 2 : 1;
   // every realisation reads its step parameters from its slot of dP
   for (int r = 0; r < n; ++r) {
     cafe_sim *s = sims[r];

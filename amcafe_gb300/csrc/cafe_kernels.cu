@@ -65,6 +65,11 @@ __device__ __forceinline__ double cafe_nuc_rate(const CafeDev &D, const CafeCons
   return K.rX * crm_exp(-.5 * (x1 * x1));
 }
 
+// ... as k_gather stored it for the step
+__device__ __forceinline__ double cafe_nuc_rate_at(const CafeDev &D, const CafeConsts &K, int icap) {
+  return K.nuc_gauss ? D.a_nuc[icap] : K.rX;
+}
+
 __device__ __forceinline__ int cafe_hot(const CafeDev &D, const CafeConsts &K, const CafeStepParams &P,
                                         int i, int j, int k) {
   return K.hot_cls[cafe_cls(D, P, i, j, k)];
@@ -569,7 +574,8 @@ __global__ void k_active_scatter(CafeDev D, CafeConsts K, const CafeStepParams *
 
 // ------------------------------------------------------------------ gather
 // Per active position: copies of the cell data, temperature class, neighbour
-// positions in ascending index order (-1 = not active), liquid-neighbour count,
+// positions by direction (CAFE_NSLOT, in ascending index order; -1 = not active
+// or outside the grid), liquid-neighbour count,
 // all-neighbours-below-liquidus flag and the ruq offset (VoxelsCA.C:380:
 // ruq[p] = (U_p - .5) dX / 100, U_p the p-th uniform of minstd(30 tInd + seed1)).
 __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, const int cafe_bid, const int cafe_nblk) {
@@ -580,6 +586,14 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
   if (cafe_bid == 0 && threadIdx.x == 0) {  // rebuilt by k_writeback for the next step
     D.ctr[CTR_ZLO] = 0x7fffffff;
     D.ctr[CTR_ZHI] = -1;
+    D.row_mag[0] = D.row_mag[1] = 0ULL;  // formed by k_rows_order and k_children
+    D.row_mag[2] = ~0ULL;
+    D.row_mag[3] = 0ULL;
+    // the row set-up's counters; a per-cell field grows rows with their own velocities
+    D.ctr[CTR_SLOW] = K.easm ? 1 : 0;
+    D.ctr[CTR_NPAIRS] = 0;
+    for (int d = 0; d < CAFE_CHILD_DEPTH; ++d) D.ctr[CTR_NCHILD + d] = 0;
+    D.ctr[CTR_NLIQ] = 0;  // listed again by k_writeback (k_solid2mushy_list has read it)
   }
   for (int p = cafe_bid * blockDim.x + threadIdx.x; p < na; p += cafe_nblk * blockDim.x) {
     long long idx = D.act[p];
@@ -597,23 +611,30 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
       double T = D.temp[idx];
       D.a_vh[p] = T >= K.tL ? 0.0 : K.Avel * crm_pow_int(K.tL - T, K.nvel_i);
     }
-    long long nb[26];
-    int n = cafe_moore(K, i, j, k, nb);
-    int m = 0, liq = 0, cold = 1;
-    for (int a = 0; a < n; ++a) {
-      int q = D.pos_of[nb[a]];
-      if (q < 0) continue;
-      D.a_nbr[(long long)p * CAFE_NSLOT + m] = q;
-      ++m;
-      if (D.state[nb[a]] == 1) ++liq;
-      int ni, nj, nk;
-      cafe_cell_xyz(K, nb[a], ni, nj, nk);
-      if (cafe_hot(D, K, P, ni, nj, nk)) cold = 0;
-    }
-    D.a_nn[p] = (uint8_t)m;
+    int liq = 0, cold = 1;
+#pragma unroll 1
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+      for (int dyx = 0; dyx < 9; ++dyx) {
+        const int dy = dyx / 3 - 1, dx = dyx % 3 - 1;
+        if (dz == 0 && dyx == 4) continue;
+        const int d27 = (dz + 1) * 9 + dyx, a = d27 - (d27 > 13 ? 1 : 0);
+        const int x = i + dx, y = j + dy, z = k + dz;
+        int q = -1;
+        if (x >= 0 && x < K.nx && y >= 0 && y < K.ny && z >= 0 && z < K.nz) {
+          const long long nb = (long long)K.nxy * z + (long long)K.nx * y + x;
+          q = D.pos_of[nb];
+          if (q >= 0) {
+            if (D.state[nb] == 1) ++liq;
+            if (cafe_hot(D, K, P, x, y, z)) cold = 0;
+          }
+        }
+        D.a_nbr[(long long)p * CAFE_NSLOT + a] = q;
+      }
     D.a_liq[p] = liq;
     D.a_cold[p] = (uint8_t)cold;
     D.a_frow[p] = -1;
+    if (K.nuc_gauss) D.a_nuc[p] = cafe_nuc_rate(D, K, p);
     double U = cafe_uniform_at(seed, (uint64_t)p);
     D.a_ruq[p] = (U - .5) * K.ruq_dx / 100.;
   }
@@ -764,7 +785,7 @@ __device__ __forceinline__ void d_lists_scatter(const CafeDev &D, const int cafe
       if (jf < D.row_cap) {
         D.row_pos[jf] = (int32_t)p;
         D.row_j[jf] = (int32_t)j2;
-        D.row_alive[jf] = 1;
+        D.row_res[jf] = -1;
         D.a_frow[p] = (int32_t)jf;
       } else {
         atomicOr(D.err, CAFE_ERR_ROW_CAP);
@@ -819,1719 +840,25 @@ __device__ __forceinline__ int cafe_exp_lb(double x) {
   return f == 0 ? -4096 : f - 1023;
 }
 
-// Row order, exact best candidate and largest |g| of row r (position p) once
-// every lane of the calling warp holds its slot: liv (the neighbour is liquid),
-// gv (its numerator g) and q (its position). The live slots are ordered by g
-// (NaN last, ties by slot) into row_ord, followed by the other slots. With
-// `eval`, the row's exact best candidate at iteration `ev` and time T is stored
-// (what cafe_row_best computes, one slot per lane). Returns, in every lane, the
-// order key of the largest finite |g| of the live slots, or 0 when none.
-// `parts` selects the row order (CAFE_FIN_ORDER) and the rest (CAFE_FIN_BEST:
-// row_live, the best candidate, the largest |g|), so that two warps holding
-// the same slots can share the work.
-#define CAFE_FIN_ORDER 1
-#define CAFE_FIN_BEST 2
-__device__ unsigned long long cafe_row_finish_warp(const CafeDev &D, const CafeConsts &K, long long r, int p,
-                                                   int nn, bool liv, double gv, int q, bool eval, int ev,
-                                                   double T, bool have_t = false, double t_pre = 0.0,
-                                                   double ruqs_pre = 0.0,
-                                                   int parts = CAFE_FIN_ORDER | CAFE_FIN_BEST) {
-  const unsigned FULL = 0xffffffffu;
-  int lane = threadIdx.x & 31;
-  uint32_t live = __ballot_sync(FULL, liv);
-  // rank of this slot in the row order
-#ifdef CAFE_DETAIL_CYCLES
-  long long fz0 = clock64();
-#endif
-  const bool gfin = !cafe_is_nan(gv);
-  if (parts & CAFE_FIN_ORDER) {
-    unsigned long long key = (liv && gfin) ? cafe_key_canon(gv) : CAFE_KEY_NONE;
-    int rank = liv ? 0 : __popc(live);
-    // (every slot position, so that the shuffles are independent; the bits of
-    // live above nn are clear)
-#pragma unroll
-    for (int t = 0; t < CAFE_NSLOT; ++t) {
-      unsigned long long kt = cafe_shfl_u64(key, t);
-      bool lt = (live >> t) & 1u;
-      if (liv)
-        rank += lt && (kt < key || (kt == key && t < lane));
-      else
-        rank += !lt && t < nn && t < lane;
-    }
-    if (lane < nn) D.row_ord[r * CAFE_NSLOT + rank] = (uint8_t)lane;
-  }
-  if (!(parts & CAFE_FIN_BEST)) return 0ULL;
-  if (lane == 0) D.row_live[r] = live;
-#ifdef CAFE_DETAIL_CYCLES
-  long long fz1 = clock64();
-#endif
-  if (eval) {
-    // t and ruqs of each live slot (given by the caller when have_t)
-    double t = 0.0, ruqs = 0.0;
-    bool cand = false;
-    if (liv) {
-      if (have_t) {
-        t = t_pre;
-        ruqs = ruqs_pre;
-      } else {
-        double E = D.a_ext[p];
-        double v = cafe_vh(D, K, p);
-        double dr = gv - E;
-        t = dr / v;
-        ruqs = .5 * (D.a_ruq[p] + D.a_ruq[q]);
-      }
-      cand = !cafe_is_nan(t);
-    }
-    // lexicographic (t, ruqs, slot) minimum over the warp (VoxelsCA.C:427-440)
-    const unsigned long long tk0 = cand ? cafe_key_canon(t) : CAFE_KEY_NONE;
-    unsigned long long tk = tk0;
-    unsigned long long rk = cand ? cafe_key_canon(ruqs) : CAFE_KEY_NONE;
-    int sl = cand ? lane : 255;
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long tk2 = (unsigned long long)__shfl_xor_sync(FULL, (long long)tk, o);
-      unsigned long long rk2 = (unsigned long long)__shfl_xor_sync(FULL, (long long)rk, o);
-      int sl2 = __shfl_xor_sync(FULL, sl, o);
-      if (tk2 < tk || (tk2 == tk && (rk2 < rk || (rk2 == rk && sl2 < sl)))) {
-        tk = tk2;
-        rk = rk2;
-        sl = sl2;
-      }
-    }
-    // the smallest time of the other candidates (the row's time once slot sl
-    // is captured by another row)
-    unsigned long long k2 = lane == sl ? CAFE_KEY_NONE : tk0;
-    for (int o = 16; o > 0; o >>= 1) k2 = min(k2, cafe_shfl_u64_xor(k2, o));
-    double bt = __shfl_sync(FULL, t, sl & 31);
-    double bruq = __shfl_sync(FULL, ruqs, sl & 31);
-    int bq = __shfl_sync(FULL, q, sl & 31);
-    if (lane == 0) {
-      D.row_stamp[r] = ev + 1;
-      if (sl == 255) {
-        D.row_key[r] = CAFE_KEY_NONE;
-      } else {
-        D.row_bt[r] = bt;
-        D.row_bruq[r] = bruq;
-        D.row_bslot[r] = sl;
-        D.row_bq[r] = bq;
-        const unsigned long long key = cafe_key(T + bt);
-        D.row_key[r] = key;
-        D.row_key2[r] = k2 == CAFE_KEY_NONE ? key : cafe_key(T + cafe_unkey(k2));
-      }
-    }
-  }
-#ifdef CAFE_DETAIL_CYCLES
-  long long fz2 = clock64();
-#endif
-  unsigned long long ak = (liv && gfin) ? cafe_key(fabs(gv)) : 0ULL;
-  for (int o = 16; o > 0; o >>= 1) ak = max(ak, (unsigned long long)__shfl_xor_sync(FULL, (long long)ak, o));
-  __syncwarp();
-#ifdef CAFE_DETAIL_CYCLES
-  if (gridDim.x == 1 && lane == 0) {
-    long long fz3 = clock64();
-    atomicAdd(&D.stat[STAT_DETAIL + 24], (unsigned long long)(fz1 - fz0));
-    atomicAdd(&D.stat[STAT_DETAIL + 25], (unsigned long long)(fz2 - fz1));
-    atomicAdd(&D.stat[STAT_DETAIL + 26], (unsigned long long)(fz3 - fz2));
-  }
-#endif
-  return ak;
-}
-
-// The captured cell's grain, centre and extent as the capture section just
-// stored them, handed to the fill through shared memory.
-struct CafeNewCell {
-  double c[3], ext;
-  int gid;
-};
-// Per-slot partial results passed between the four warps of cafe_row_fill_quad.
-struct CafeQuadScratch {
-  double cth[32], sph[32], l[32], d1I[32], dI2[32], d1J[32], dJ3[32], dr[32], ruqs[32];
-};
-#define CAFE_QUAD_THREADS 128
-__device__ __forceinline__ void cafe_bar_quad() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-// Fills row r for position p, the cell just captured, with warps 0-3 of the
-// block together (all 128 threads must call it): every liquid neighbour slot
-// gets its numerator g and capture result (extent, centre), the slots are
-// ordered and, with `eval`, the row's exact best candidate at iteration `ev`
-// and time T is stored. A warp issues one FP64 instruction at a time whatever its
-// active lanes, so the independent chains of each slot's geometry run in
-// different warps, lane s of each warp on slot s. First stage:
-//   warp 0: cos th and the cell distance l; warp 1: sin ph;
-//   warp 2: |R^T dn|_1 and the projection on edge p0-p1;
-//   warp 3: the projection on edge p0-p2 and the tie-break ruqs.
-// Second stage, after one barrier: warps 0 and 1 form g; warp 0 the capture
-// time t = (g - ExtA)/v (with eval) and the row's best candidate, warp 1 the
-// slot order; warp 2 the extent and warp 3 the centre a capture from this row
-// gives. The return value is valid in warp 0.
-__device__ unsigned long long cafe_row_fill_quad(const CafeDev &D, const CafeConsts &K, long long r, int p,
-                                                 bool eval, int ev, double T, CafeQuadScratch &S,
-                                                 const CafeNewCell *nc = nullptr) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#ifdef CAFE_DETAIL_CYCLES
-  long long fq0 = clock64();
-#endif
-  int nn = D.a_nn[p];
-  int gp = nc ? nc->gid : D.a_gid[p];
-  bool grain_ok = gp >= 1 && gp <= D.grain_cap;
-  bool liv = false;
-  int q = 0;
-  double dn[3] = {0.0, 0.0, 0.0}, cs[3] = {0.0, 0.0, 0.0};
-  int ci = 0, cj = 0, ck = 0, si = 0, sj = 0, sk = 0;
-  if (lane < nn) {
-    q = D.a_nbr[(long long)p * CAFE_NSLOT + lane];
-    liv = D.a_state[q] == 1;
-  }
-  const bool work = liv && grain_ok;
-  double R[9], loc[3], dr = 0.0, pk[3][3];
-  double E0 = 0.0, v0 = 1.0;  // warp 0: the row's extent and velocity for t
-  int s0i = 0;
-  if (work) {
-    cafe_cell_xyz(K, D.act[q], ci, cj, ck);
-    cafe_cell_xyz(K, D.act[p], si, sj, sk);
-    cs[0] = nc ? nc->c[0] : D.a_cx[p];
-    cs[1] = nc ? nc->c[1] : D.a_cy[p];
-    cs[2] = nc ? nc->c[2] : D.a_cz[p];
-    cafe_geo_dn(K, ci, cj, ck, cs, dn);
-    if (w == 0) {
-      if (eval) {
-        E0 = nc ? nc->ext : D.a_ext[p];
-        v0 = cafe_vh(D, K, p);
-      }
-      S.cth[lane] = cafe_geo_costh(dn);
-      S.l[lane] = cafe_geo_l(K, ci, cj, ck, si, sj, sk);
-    } else if (w == 1) {
-      S.sph[lane] = cafe_geo_sinph(dn);
-    } else {
-      const double *Rg = D.rot + 9LL * (gp - 1);
-      for (int a = 0; a < 9; ++a) R[a] = Rg[a];
-      dr = cafe_geo_loc(R, dn, loc);
-      s0i = cafe_geo_corners(loc, dr, pk);
-      if (w == 2) {
-        S.dr[lane] = dr;
-        cafe_geo_edge(loc, pk[0], pk[1], &S.d1I[lane], &S.dI2[lane]);
-      } else {
-        cafe_geo_edge(loc, pk[0], pk[2], &S.d1J[lane], &S.dJ3[lane]);
-        if (eval) S.ruqs[lane] = .5 * (D.a_ruq[p] + D.a_ruq[q]);
-      }
-    }
-  }
-#ifdef CAFE_DETAIL_CYCLES
-  long long fq1 = clock64();
-#endif
-  cafe_bar_quad();
-#ifdef CAFE_DETAIL_CYCLES
-  long long fq2 = clock64();
-#endif
-  // second stage, no barrier after it: warp 0 forms g and the capture time
-  // and takes the row's best candidate, warp 1 forms g and orders the slots,
-  // warps 2 and 3 finish the capture geometry (extent, centre), which only a
-  // later capture by this row reads
-  double gv = liv ? NAN : 0.0;  // a capturing cell without a grain never captures
-  unsigned long long ak = 0ULL;
-#ifdef CAFE_DETAIL_CYCLES
-  long long fq3 = clock64();
-#endif
-  if (w <= 1) {
-    double f = 0.0;
-    if (work) {
-      f = crm_pow_half(S.cth[lane] * S.sph[lane]);
-      gv = f * S.dr[lane];
-    }
-    if (w == 0) {
-      double t = NAN;
-      if (work && eval) {
-        double dr2 = gv - E0;
-        t = dr2 / v0;
-      }
-      if (liv) D.row_g[r * CAFE_NSLOT + lane] = gv;
-      ak = cafe_row_finish_warp(D, K, r, p, nn, liv, gv, q, eval, ev, T, true, t, work ? S.ruqs[lane] : 0.0,
-                                CAFE_FIN_BEST);
-    } else {
-      // the slot order (read only by later evaluations)
-      cafe_row_finish_warp(D, K, r, p, nn, liv, gv, q, false, ev, T, false, 0.0, 0.0, CAFE_FIN_ORDER);
-    }
-  } else if (work) {
-    double Lmud = cafe_geo_lmud(K, S.l[lane], S.d1I[lane], S.dI2[lane], S.d1J[lane], S.dJ3[lane]);
-    double *o = D.row_geo + (r * CAFE_NSLOT + lane) * 4;
-    if (w == 2) {
-      double f = crm_pow_half(S.cth[lane] * S.sph[lane]);
-      o[0] = f * Lmud * 1.0;
-    } else {
-      double cn[3];
-      cafe_geo_centre(R, cs, pk[0], s0i, Lmud, cn);
-      o[1] = cn[0];
-      o[2] = cn[1];
-      o[3] = cn[2];
-    }
-  }
-#ifdef CAFE_DETAIL_CYCLES
-  if (lane == 0) {
-    long long fq4 = clock64();
-    atomicAdd(&D.stat[STAT_DETAIL + 16 + w], (unsigned long long)(fq1 - fq0));
-    if (w >= 2) atomicAdd(&D.stat[STAT_DETAIL + 18 + w], (unsigned long long)(fq4 - fq3));
-    if (w == 0) {
-      atomicAdd(&D.stat[STAT_DETAIL + 22], (unsigned long long)(fq4 - fq3));
-      atomicAdd(&D.stat[STAT_DETAIL + 23], 1ULL);
-    }
-  }
-#endif
-  return ak;
-}
-
-// ------------------------------------------------------------------ event loop
-// A capture candidate: time t and tie-break ruqs, compared through their
-// order keys (equal doubles give equal keys; NaN times are never candidates).
-struct CafeCand {
-  unsigned long long tk, rk;
-  double t, ruqs;
-  int j, s;  // vs2 index and neighbour slot of the capturing cell; j < 0 = none
-  int r, p, q;  // (not compared) its row, its active position and the captured position
-};
-__device__ __forceinline__ CafeCand cafe_cand_none() {
-  CafeCand c;
-  c.tk = c.rk = CAFE_KEY_NONE;
-  c.t = c.ruqs = 0.0;
-  c.j = -1;
-  c.s = 0;
-  c.r = c.p = c.q = 0;
-  return c;
-}
-__device__ __forceinline__ bool cafe_cand_better(const CafeCand &a, const CafeCand &b) {
-  // lexicographic (t, ruqs, scan position): VoxelsCA.C:427-440 keeps the first
-  // scanned candidate among full ties
-  if (a.j < 0) return false;
-  if (b.j < 0) return true;
-  if (a.tk != b.tk) return a.tk < b.tk;
-  if (a.rk != b.rk) return a.rk < b.rk;
-  if (a.j != b.j) return a.j < b.j;
-  return a.s < b.s;
-}
-__device__ __forceinline__ CafeCand cafe_shfl_cand(const CafeCand &c, int o) {
-  CafeCand r;
-  r.tk = cafe_shfl_u64_xor(c.tk, o);
-  r.rk = cafe_shfl_u64_xor(c.rk, o);
-  r.t = __shfl_xor_sync(0xffffffffu, c.t, o);
-  r.ruqs = __shfl_xor_sync(0xffffffffu, c.ruqs, o);
-  r.j = __shfl_xor_sync(0xffffffffu, c.j, o);
-  r.s = __shfl_xor_sync(0xffffffffu, c.s, o);
-  r.r = __shfl_xor_sync(0xffffffffu, c.r, o);
-  r.p = __shfl_xor_sync(0xffffffffu, c.p, o);
-  r.q = __shfl_xor_sync(0xffffffffu, c.q, o);
-  return r;
-}
-// Best candidate of the warp, in every lane.
-__device__ __forceinline__ CafeCand cafe_warp_best(CafeCand best) {
-  for (int o = 16; o > 0; o >>= 1) {
-    CafeCand c = cafe_shfl_cand(best, o);
-    if (cafe_cand_better(c, best)) best = c;
-  }
-  return best;
-}
-#define CAFE_KEY_1E6 0xc12e848000000000ULL  // cafe_key(1e6)
-
-// Best candidate of frontier row r (VoxelsCA.C:386-445 restricted to one cell)
-// with the row cell's current extent. For a positive finite growth velocity the
-// capture time fl(fl(g - E)/v) is non-decreasing in g, so the live slots are
-// visited in g order and the visit stops at the first time above the row's
-// minimum; otherwise every live slot is evaluated. `bounded` applies the
-// reference's acceptance limit t <= 1e6 (VoxelsCA.C:383, 427).
-__device__ __forceinline__ void cafe_row_best_live(const CafeDev &D, const CafeConsts &K, long long r,
-                                                   uint32_t live, CafeCand &best, bool bounded,
-                                                   unsigned long long *k2out = nullptr) {
-  int p = D.row_pos[r];
-  if (!live) return;
-  double E = D.row_E[r];
-  double v = cafe_vh(D, K, p);
-  long long vb = crm_bits(v);
-  bool mono = vb > 0 && vb < CRM_BITS_INF;  // 0 < v < inf
-  const double *g = D.row_g + r * CAFE_NSLOT;
-  const uint8_t *ord = D.row_ord + r * CAFE_NSLOT;
-  const int32_t *nbr = D.a_nbr + (long long)p * CAFE_NSLOT;
-  int nn = D.a_nn[p];
-  int jrow = D.row_j[r];
-  double ruq_p = D.a_ruq[p];
-  bool have = false;
-  unsigned long long tfirst = 0;
-  // with k2out (best enters empty): the smallest time key of the candidates
-  // other than the best one; in g order the slot that ends the visit has it
-  unsigned long long k2 = CAFE_KEY_NONE;
-  // visits slot s of order position k with numerator gs and neighbour q:
-  // 0 go on, 1 the visit ends
-  auto visit = [&](int k, int s, double gs, int q) -> int {
-    if (!(live >> s & 1u)) return 0;
-    double dr = gs - E;
-    double t = dr / v;
-    if (cafe_is_nan(t)) return 0;
-    unsigned long long tk = cafe_key_canon(t);
-    if (bounded && !(tk <= CAFE_KEY_1E6)) return mono ? 1 : 0;
-    if (mono && have && tk > tfirst) {
-      k2 = min(k2, tk);
-      return 1;
-    }
-    CafeCand c;
-    c.t = t;
-    c.tk = tk;
-    c.ruqs = .5 * (ruq_p + D.a_ruq[q]);
-    c.rk = cafe_key_canon(c.ruqs);
-    c.j = jrow;
-    c.s = s;
-    c.r = (int)r;
-    c.p = p;
-    c.q = q;
-    if (cafe_cand_better(c, best)) {
-      if (have) k2 = min(k2, best.tk);
-      best = c;
-    } else {
-      k2 = min(k2, tk);
-    }
-    if (!have) {
-      have = true;
-      tfirst = tk;
-    }
-    return 0;
-  };
-  // the first four slots of the visiting order with their numerators and
-  // neighbours, loaded together (a visit usually ends within them)
-  int s4[4], q4[4];
-  double g4[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) s4[i] = i < nn ? (mono ? (int)ord[i] : i) : 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    g4[i] = i < nn ? g[s4[i]] : 0.0;
-    q4[i] = i < nn ? nbr[s4[i]] : 0;
-  }
-  bool ended = false;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (!ended && i < nn) ended = visit(i, s4[i], g4[i], q4[i]) != 0;
-  for (int k = 4; k < nn && !ended; ++k) {
-    int s = mono ? ord[k] : k;
-    ended = visit(k, s, g[s], nbr[s]) != 0;
-  }
-  if (k2out) *k2out = k2;
-}
-__device__ __forceinline__ void cafe_row_best(const CafeDev &D, const CafeConsts &K, long long r,
-                                              CafeCand &best, bool bounded = true) {
-  cafe_row_best_live(D, K, r, D.row_live[r], best, bounded);
-}
-
-// Slot of `target` in q's neighbour list, -1 if absent. All CAFE_NSLOT entries
-// are loaded at once (the list storage is always that long) and masked by nn.
-__device__ __forceinline__ int cafe_find_slot(const CafeDev &D, int q, int target) {
-  int nn = D.a_nn[q];
-  const int32_t *nb = D.a_nbr + (long long)q * CAFE_NSLOT;
-  int found = -1;
-#pragma unroll
-  for (int s = CAFE_NSLOT - 1; s >= 0; --s) {
-    int v = nb[s];
-    if (s < nn && v == target) found = s;
-  }
-  return found;
-}
-
-// ---- keyed rows -------------------------------------------------------------
-// Every frontier cell of a step grows by the same fl(v * DtMin) at every capture
-// event while it has a liquid neighbour (VoxelsCA.C:511-516), and a row's
-// candidate times all fall by about DtMin per event. A row therefore carries a
-// key: the absolute time T + t_best of its best candidate when it was last
-// evaluated exactly. Between evaluations the key is within a small rounding
-// bound of the row's exact current value (or below it once a candidate was
-// captured by someone else), so the event needs exact times only for the rows
-// whose key lies within twice that bound of the smallest key. When the row's
-// best candidate is the one captured elsewhere, the key becomes row_key2, the
-// key of the row's next candidate at the same evaluation, which bounds the
-// row's exact value the same way. An extent that a
-// negative event may clamp at zero (VoxelsCA.C:515) breaks the bound; such rows
-// are stamped -1 and evaluated again. The growth is logged once per event and
-// replayed per row when the row is evaluated, and for every row at the end of
-// the step (k_rows_finalize).
-#define CAFE_ALIVE 0x7fffffff   // row_death of a row that is still alive
-#define CAFE_M_DONE 0x7fffffff  // row_m of a row whose extent is kept current
-#ifndef CAFE_CATCHUP
-#define CAFE_CATCHUP 2  // logged events a selecting thread replays per event for its second row
-#endif
-
-// Applies the logged growth of events row_m+1 .. min(upto, row_death). A
-// nucleation logs +0, which leaves an extent unchanged (extents are never -0).
-__device__ __forceinline__ void cafe_row_replay(const CafeDev &D, int r, int upto) {
-  int m = D.row_m[r];
-  int stop = min(upto, D.row_death[r]);
-  if (stop <= m) return;
-  double E = D.row_E[r];
-  for (int k = m + 1; k <= stop; ++k) {
-    E = E + D.ev_vd[k];
-    E = cafe_is_neg(E) ? 0.0 : E;  // (E < 0.0) ? 0.0 : E
-  }
-  D.row_E[r] = E;
-  D.row_m[r] = stop;
-}
-
-// Exact evaluation of row r (live slots `live`) for the iteration after `ev`
-// events at time T.
-__device__ __forceinline__ void cafe_row_eval_live(const CafeDev &D, const CafeConsts &K, int r, int ev,
-                                                   double T, uint32_t live) {
-#ifdef CAFE_DETAIL_CYCLES
-  long long rp0 = clock64();
-  int rm0 = D.row_m[r];
-#endif
-  cafe_row_replay(D, r, ev);
-#ifdef CAFE_DETAIL_CYCLES
-  atomicAdd(&D.stat[STAT_DETAIL + 27], (unsigned long long)(D.row_m[r] - rm0 > 0 ? D.row_m[r] - rm0 : 0));
-  atomicAdd(&D.stat[STAT_DETAIL + 28], 1ULL);
-  atomicAdd(&D.stat[STAT_DETAIL + 29], (unsigned long long)(clock64() - rp0));
-#endif
-  CafeCand b = cafe_cand_none();
-#ifdef CAFE_DETAIL_CYCLES
-  long long be0 = clock64();
-#endif
-  unsigned long long k2;
-  cafe_row_best_live(D, K, r, live, b, false, &k2);
-#ifdef CAFE_DETAIL_CYCLES
-  atomicAdd(&D.stat[STAT_DETAIL + 30], (unsigned long long)(clock64() - be0));
-  atomicAdd(&D.stat[STAT_DETAIL + 31], 1ULL);
-#endif
-  D.row_stamp[r] = ev + 1;
-  if (b.j < 0) {
-    D.row_key[r] = CAFE_KEY_NONE;
-    return;
-  }
-  D.row_bt[r] = b.t;
-  D.row_bruq[r] = b.ruqs;
-  D.row_bslot[r] = b.s;
-  D.row_bq[r] = b.q;
-  const unsigned long long key = cafe_key(T + b.t);
-  D.row_key[r] = key;
-  D.row_key2[r] = k2 == CAFE_KEY_NONE ? key : cafe_key(T + cafe_unkey(k2));
-}
-__device__ __forceinline__ void cafe_row_eval(const CafeDev &D, const CafeConsts &K, int r, int ev,
-                                              double T) {
-  cafe_row_eval_live(D, K, r, ev, T, D.row_live[r]);
-}
-
-// Frontier rows of the step, in three passes so that the capture geometry,
-// the expensive part, runs with one (row, slot) pair per lane:
-// k_rows_prep (one warp per row) finds each row's liquid neighbours, sets the
-// row's extent and growth watermark, and lists the pairs that need geometry;
-// k_rows_geo evaluates the listed pairs; k_rows_order (one warp per row)
-// orders each row's slots and, when every row grows with the same velocity,
-// takes its exact best candidate and key.
-__device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
-  int nrows = D.ctr[CTR_NROWS];
-  if (nrows > D.row_cap) nrows = (int)D.row_cap;
-  const int warps = (cafe_nblk * blockDim.x) >> 5;
-  const int w = (cafe_bid * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const unsigned FULL = 0xffffffffu;
-  const double V = K.vhat_cls[1];
-  for (int r = w; r < nrows; r += warps) {
-    int p = D.row_pos[r];
-    int nn = D.a_nn[p];
-    int gp = D.a_gid[p];
-    bool grain_ok = gp >= 1 && gp <= D.grain_cap;
-    bool liv = false;
-    if (lane < nn) liv = D.a_state[D.a_nbr[(long long)p * CAFE_NSLOT + lane]] == 1;
-    if (liv && !grain_ok) D.row_g[(long long)r * CAFE_NSLOT + lane] = NAN;  // never captures
-    uint32_t work = __ballot_sync(FULL, liv && grain_ok);
-    int base = 0;
-    if (lane == 0 && work) base = atomicAdd(&D.ctr[CTR_NPAIRS], __popc(work));
-    base = __shfl_sync(FULL, base, 0);
-    if (work >> lane & 1u) D.row_pairs[base + __popc(work & ((1u << lane) - 1u))] = r * 32 + lane;
-    if (lane == 0) {
-      D.row_E[r] = D.a_ext[p];
-      D.row_m[r] = 0;
-      D.row_death[r] = CAFE_ALIVE;
-      if (D.a_cls[p] != 1 || !(V > 0.0 && V < INFINITY)) atomicOr(&D.ctr[CTR_SLOW], 1);
-    }
-  }
-}
-__global__ void k_rows_prep(CafeDev D, CafeConsts K) {
-  d_rows_prep(D, K, blockIdx.x, gridDim.x);
-}
-
-__device__ __forceinline__ void d_rows_geo(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
-  int n = D.ctr[CTR_NPAIRS];
-  const long long cap = D.row_cap * CAFE_NSLOT;
-  if (n > cap) n = (int)cap;
-  for (int i = cafe_bid * blockDim.x + threadIdx.x; i < n; i += cafe_nblk * blockDim.x) {
-    int v = D.row_pairs[i];
-    int r = v >> 5, sl = v & 31;
-    int p = D.row_pos[r];
-    int q = D.a_nbr[(long long)p * CAFE_NSLOT + sl];
-    const double *Rg = D.rot + 9LL * (D.a_gid[p] - 1);
-    double Rm[9];
-    for (int a = 0; a < 9; ++a) Rm[a] = Rg[a];
-    int i0, j0, k0, si, sj, sk;
-    cafe_cell_xyz(K, D.act[q], i0, j0, k0);
-    cafe_cell_xyz(K, D.act[p], si, sj, sk);
-    double cs[3] = {D.a_cx[p], D.a_cy[p], D.a_cz[p]};
-    double g, e, cn[3];
-    cafe_capture_geometry(K, i0, j0, k0, si, sj, sk, cs, Rm, &g, &e, cn);
-    long long o = (long long)r * CAFE_NSLOT + sl;
-    D.row_g[o] = g;
-    double *og = D.row_geo + o * 4;
-    og[0] = e;
-    og[1] = cn[0];
-    og[2] = cn[1];
-    og[3] = cn[2];
-  }
-}
-__global__ void k_rows_geo(CafeDev D, CafeConsts K) {
-  d_rows_geo(D, K, blockIdx.x, gridDim.x);
-}
-
-__device__ __forceinline__ void d_rows_order(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
-  int nrows = D.ctr[CTR_NROWS];
-  if (nrows > D.row_cap) nrows = (int)D.row_cap;
-  const int warps = (cafe_nblk * blockDim.x) >> 5;
-  const int w = (cafe_bid * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  for (int r = w; r < nrows; r += warps) {
-    int p = D.row_pos[r];
-    int nn = D.a_nn[p];
-    int q = 0;
-    bool liv = false;
-    double gv = 0.0;
-    if (lane < nn) {
-      q = D.a_nbr[(long long)p * CAFE_NSLOT + lane];
-      liv = D.a_state[q] == 1;
-      if (liv) gv = D.row_g[(long long)r * CAFE_NSLOT + lane];
-    }
-    cafe_row_finish_warp(D, K, r, p, nn, liv, gv, q, true, 0, 0.0);
-  }
-}
-__global__ void k_rows_order(CafeDev D, CafeConsts K) {
-  d_rows_order(D, K, blockIdx.x, gridDim.x);
-}
-
-// ---- event selection by a group of warps ------------------------------------
-// Shared scratch of one selecting group (up to 16 warps).
-struct CafeSelShared {
-  unsigned long long redk[16];
-  CafeCand red[16];
-  unsigned long long kthr;
-  long long evals;  // selection rounds that evaluated rows exactly
-#ifdef CAFE_DETAIL_CYCLES
-  long long cyc[4], rounds;
-#endif
-};
-// bar.sync on a named barrier, with an OR reduction of v over the n threads.
-__device__ __forceinline__ int cafe_bar_or(int id, int n, int v) {
-  int r;
-  asm volatile(
-      "{ .reg .pred p, q;\n\t"
-      "setp.ne.s32 q, %1, 0;\n\t"
-      "bar.red.or.pred p, %2, %3, q;\n\t"
-      "selp.s32 %0, 1, 0, p; }"
-      : "=r"(r)
-      : "r"(v), "r"(id), "r"(n)
-      : "memory");
-  return r;
-}
-__device__ __forceinline__ void cafe_bar_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-
-// Smallest and second smallest key (and rows) of a sequence of rows: row r
-// with key k enters.
-__device__ __forceinline__ void cafe_top2(unsigned long long k, int r, unsigned long long &m, int &mr,
-                                          unsigned long long &m2, int &r2) {
-  if (k < m) {
-    m2 = m;
-    r2 = mr;
-    m = k;
-    mr = r;
-  } else if (k < m2) {
-    m2 = k;
-    r2 = r;
-  }
-}
-
-// Keyed selection of the best capture among rows [0, nrows) for the iteration
-// after `ev` events at time T (VoxelsCA.C:386-480 restricted to the rows that
-// can hold the minimum), by the group of gn threads (gtid = 0..gn-1) that
-// shares named barrier `bar`. Thread gtid owns rows r = gtid (mod gn) and keeps
-// the smallest key among them in my_min, with its row in my_hot, and the
-// smallest key of its other rows in my_u2, with its row in my_r2 (-1 none; -2
-// not known), all rescanned when dirty[gtid] is set; a forced[gtid] flag makes
-// it evaluate its rows stamped -1. Every key change made elsewhere (a row's
-// key raised, a row's death, a new row) sets dirty, so between rescans the
-// thread's own evaluations are the only changes. The result is left
-// in S.red[0] (valid after the group's next barrier; every group thread has
-// passed the last barrier when this returns).
-__device__ void cafe_select_keyed(const CafeDev &D, const CafeConsts &K, int ev, double T, int nrows, int gtid,
-                                  int gn, int bar, unsigned long long &my_min, int &my_hot,
-                                  unsigned long long &my_u2, int &my_r2, bool &my_forced, unsigned char *dirty,
-                                  unsigned char *forced, CafeSelShared &S, double gmax, double emax, double dsum,
-                                  double V) {
-  const int lane = gtid & 31, gw = gtid >> 5, ngw = gn >> 5;
-#ifdef CAFE_DETAIL_CYCLES
-  long long sc0 = cafe_clock_ordered();
-#endif
-  if (forced[gtid]) {
-    forced[gtid] = 0;
-    my_forced = true;
-  }
-  if (dirty[gtid]) {
-    dirty[gtid] = 0;
-    unsigned long long m = CAFE_KEY_NONE, m2 = CAFE_KEY_NONE;
-    int mr = -1, r2 = -1;
-    // batches of eight loads in flight together
-    for (int r0 = gtid; r0 < nrows; r0 += 8 * gn) {
-      unsigned long long kk[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = r0 + i * gn;
-        kk[i] = r < nrows ? D.row_key[r] : CAFE_KEY_NONE;
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) cafe_top2(kk[i], r0 + i * gn, m, mr, m2, r2);
-    }
-    my_min = m;
-    my_hot = mr;
-    my_u2 = m2;
-    my_r2 = r2;
-  }
-  CafeCand best;
-  // this thread's last scan in this selection: marked rows, the two smallest
-  // keys of the others
-  bool sc_have = false;
-  uint32_t sc_mark = 0;
-  unsigned long long sc_u = CAFE_KEY_NONE, sc_u2 = CAFE_KEY_NONE;
-  int sc_ur = -1, sc_r2 = -1;
-#ifdef CAFE_DETAIL_CYCLES
-  long long sc1 = cafe_clock_ordered();
-  if (gtid == 0) S.cyc[0] += sc1 - sc0;  // dirty rescan
-#endif
-  while (true) {
-#ifdef CAFE_DETAIL_CYCLES
-    long long sr0 = cafe_clock_ordered();
-#endif
-    unsigned long long km = my_min;
-    for (int o = 16; o > 0; o >>= 1) km = min(km, cafe_shfl_u64_xor(km, o));
-    if (lane == 0) S.redk[gw] = km;
-    cafe_bar_n(bar, gn);
-    if (gw == 0) {
-      km = lane < ngw ? S.redk[lane] : CAFE_KEY_NONE;
-      for (int o = 16; o > 0; o >>= 1) km = min(km, cafe_shfl_u64_xor(km, o));
-      if (lane == 0) {
-        unsigned long long kt = CAFE_KEY_NONE;
-        if (km != CAFE_KEY_NONE) {
-          // rows whose exact value may be the minimum: keys within twice the
-          // rounding bound delta = (ev+16) 2^-48 (|K*| + |T| + (gmax+emax)/v
-          // + 2 sum|dt| + 1e-300); the magnitude is bounded by a power of
-          // two from the exponents of its terms (below 8 times the largest)
-          double kd = cafe_unkey(km);
-          int eg = max(cafe_exp_ub(gmax), cafe_exp_ub(emax)) + 1 - cafe_exp_lb(V);
-          int em = max(max(cafe_exp_ub(kd), cafe_exp_ub(T)), max(eg, cafe_exp_ub(dsum) + 1)) + 3;
-          int ed = em - 47;  // 2 delta < (ev+16) 2^ed
-          if (ed > -126 && ed < 100 && ev < (1 << 24)) {
-            float delta2 = (float)(ev + 16) * __int_as_float((ed + 127) << 23);
-            double thr = kd + (double)delta2;
-            kt = cafe_is_nan(thr) ? CAFE_KEY_NONE : cafe_key(thr);
-          } else {
-            double magd = fabs(kd) + fabs(T) + (gmax + emax) / V + 2.0 * dsum + 1e-300;
-            double thr = kd + 2.0 * ((double)(ev + 16) * 0x1p-48 * magd);
-            kt = cafe_is_nan(thr) ? CAFE_KEY_NONE : cafe_key(thr);
-          }
-        }
-        S.kthr = kt;
-      }
-    }
-    cafe_bar_n(bar, gn);
-#ifdef CAFE_DETAIL_CYCLES
-    long long sr1 = cafe_clock_ordered();
-    if (gtid == 0) S.cyc[1] += sr1 - sr0;  // minimum and threshold
-#endif
-    const unsigned long long kthr = S.kthr;
-    int again = 0;
-#ifdef CAFE_DETAIL_CYCLES
-    long long eval_cyc = 0, phase_a = 0;
-    int n_mark = 0;
-#endif
-    best = cafe_cand_none();
-    if (kthr != CAFE_KEY_NONE && (my_min <= kthr || my_forced)) {
-      // visits row r: evaluates it when its key may be the minimum and was not
-      // evaluated for this iteration (or when it is forced), takes its best
-      // candidate when its key is at or below the threshold, returns the key
-      auto visit = [&](int r) -> unsigned long long {
-        unsigned long long k = D.row_key[r];
-        int stamp = D.row_stamp[r];
-        // stamp -1: forced after a possible clamp of the row's extent
-        if ((k <= kthr && stamp != ev + 1) || (stamp == -1 && D.row_alive[r])) {
-#ifdef CAFE_DETAIL_CYCLES
-          long long ev0 = cafe_clock_ordered();
-#endif
-          cafe_row_eval(D, K, r, ev, T);
-#ifdef CAFE_DETAIL_CYCLES
-          eval_cyc += cafe_clock_ordered() - ev0;
-#endif
-          k = D.row_key[r];
-          again = 1;
-        }
-        if (k <= kthr) {
-          CafeCand c;
-          c.t = D.row_bt[r];
-          c.ruqs = D.row_bruq[r];
-          c.tk = cafe_key_canon(c.t);
-          c.rk = cafe_key_canon(c.ruqs);
-          c.j = D.row_j[r];
-          c.s = D.row_bslot[r];
-          c.r = r;
-          c.p = D.row_pos[r];
-          c.q = D.row_bq[r];
-          if (cafe_cand_better(c, best)) best = c;
-        }
-        return k;
-      };
-      if (!my_forced && my_r2 != -2 && my_u2 > kthr && my_hot >= 0) {
-        // every other row of this thread has a key above the threshold: only
-        // the smallest-key row is visited and no other key is loaded
-#ifdef CAFE_DETAIL_CYCLES
-        n_mark += 1;
-#endif
-        const unsigned long long k = visit(my_hot);
-        if (k <= my_u2) {
-          my_min = k;
-        } else {
-          // the second row is now the smallest; the next one is not known
-          my_min = my_u2;
-          my_hot = my_r2;
-          my_r2 = -2;
-        }
-      } else {
-        unsigned long long m = CAFE_KEY_NONE, m2 = CAFE_KEY_NONE;
-        int mr = -1, r2 = -1;
-        // this thread's rows r = r0 + i gn, 32 at a time: first their keys,
-        // loaded together, mark the rows at or below the threshold (and, when
-        // forced, the rows stamped -1); then only the marked rows are visited.
-        // Within one selection only this thread changes its rows, and only
-        // marked ones: with its rows in one chunk, a later round whose
-        // threshold lies below the smallest unmarked key of the last scan
-        // visits the same marked rows again without loading the other keys.
-        const bool one_chunk = nrows <= 32 * gn;
-        for (int r0 = gtid; r0 < nrows; r0 += 32 * gn) {
-          uint32_t mark = 0;
-          if (one_chunk && sc_have && !my_forced && sc_u > kthr) {
-            mark = sc_mark;
-            m = sc_u;
-            mr = sc_ur;
-            m2 = sc_u2;
-            r2 = sc_r2;
-          } else {
-#ifdef CAFE_DETAIL_CYCLES
-            long long pa0 = cafe_clock_ordered();
-#endif
-            // (branch-free batches of eight loads, so that they are in flight
-            // together)
-#pragma unroll
-            for (int b = 0; b < 32; b += 8) {
-              if (r0 + b * gn >= nrows) break;
-              unsigned long long kk[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const int r = r0 + (b + i) * gn;
-                kk[i] = r < nrows ? D.row_key[r] : CAFE_KEY_NONE;
-              }
-              uint32_t fm = 0;  // rows stamped -1, visited whatever their key
-              if (my_forced) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const int r = r0 + (b + i) * gn;
-                  fm |= (r < nrows && D.row_stamp[r] == -1) ? 1u << i : 0u;
-                }
-              }
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                // a visited row's key enters the two smallest after its visit
-                if (kk[i] <= kthr || (fm >> i & 1u))
-                  mark |= 1u << (b + i);
-                else
-                  cafe_top2(kk[i], r0 + (b + i) * gn, m, mr, m2, r2);
-              }
-            }
-#ifdef CAFE_DETAIL_CYCLES
-            phase_a += cafe_clock_ordered() - pa0;
-            n_mark += __popc(mark);
-#endif
-            if (one_chunk) {
-              sc_have = true;
-              sc_mark = mark;
-              sc_u = m;
-              sc_ur = mr;
-              sc_u2 = m2;
-              sc_r2 = r2;
-            }
-          }
-          while (mark) {
-            const int r = r0 + (__ffs(mark) - 1) * gn;
-            mark &= mark - 1;
-            cafe_top2(visit(r), r, m, mr, m2, r2);
-          }
-        }
-        my_min = m;
-        my_hot = mr;
-        my_u2 = m2;
-        my_r2 = r2;
-        my_forced = false;
-      }
-    }
-#ifdef CAFE_DETAIL_CYCLES
-    if (again) {
-      // scan time of the evaluating threads apart from their evaluations
-      atomicAdd(&D.stat[STAT_DETAIL + 10], (unsigned long long)(cafe_clock_ordered() - sr1 - eval_cyc));
-      atomicAdd(&D.stat[STAT_DETAIL + 11], 1ULL);
-      atomicAdd(&D.stat[STAT_DETAIL + 12], (unsigned long long)eval_cyc);
-      atomicAdd(&D.stat[STAT_DETAIL + 14], (unsigned long long)phase_a);
-      atomicAdd(&D.stat[STAT_DETAIL + 15], (unsigned long long)n_mark);
-    }
-#endif
-#ifdef CAFE_DETAIL_CYCLES
-    long long sr2 = cafe_clock_ordered();
-    if (gtid == 0) S.cyc[2] += sr2 - sr1;  // scan and evaluations (this thread)
-#endif
-    again = cafe_bar_or(bar, gn, again);
-#ifdef CAFE_DETAIL_CYCLES
-    if (gtid == 0) {
-      S.cyc[3] += cafe_clock_ordered() - sr2;  // waiting for the slowest thread's evaluations
-      S.rounds++;
-    }
-#endif
-    if (gtid == 0 && again) S.evals++;
-    if (!again) break;
-  }
-  best = cafe_warp_best(best);
-  if (lane == 0) S.red[gw] = best;
-  cafe_bar_n(bar, gn);
-  if (gw == 0) {
-    CafeCand b = lane < ngw ? S.red[lane] : cafe_cand_none();
-    b = cafe_warp_best(b);
-    if (lane == 0) S.red[0] = b;
-  }
-}
-
-// The capture/nucleation loop of one step (VoxelsCA.C:381-610), one block.
-//
-// Keyed mode (every frontier row grows with one velocity) pipelines two events:
-// after the winner of event e is applied and the captured cell's neighbours are
-// updated, warps 0-3 fill the row of the newly captured cell while warps 4-15
-// select the best capture of event e+1 among the other rows. The winner of
-// e+1 is the better of that selection and the new row's own exact best
-// candidate: a row not evaluated by the selection has a key above the
-// threshold, so its exact time is above the selected one. Per event: (1)
-// thread 0 settles the winner (its candidate carries the row and both cells)
-// with the draw made one event ahead and logs the growth; (2) thread 0 applies
-// the capture or nucleation, warp 1 updates the captured cell's neighbours and
-// their rows (row deaths, second-key promotions), thread 64 draws the next
-// event's uniform, and on a negative event the selecting threads flag the rows
-// whose extent may clamp; (3) the new-row fill beside the next selection; (4)
-// thread 0 merges the two. Exact mode (the reference's per-event scan of every
-// row, also the fallback when the rows stop sharing one velocity) evaluates
-// every row at every event.
-// ---- the fill helper: a second block of the event loop -----------------------
-// A warp issues one FP64 instruction per ~64 cycles and each SM sub-partition
-// completes one FP64 warp-instruction per ~64 cycles, so the new row's fill
-// (its four warps' chains, ~20k cycles) saturates the FP64 pipes of the SM it
-// runs on and slows the next event's selection there. With two blocks
-// (cooperative launch: both resident), the main block posts the fill of each
-// new row as soon as the event's winner is known, and the helper block, on
-// another SM, fills the row while the main block applies the capture and
-// selects the next event; the main block takes the result at the merge.
-// Both sides wait with a wall-clock limit; a wait that runs out sets
-// CAFE_ERR_SYNC and ends the step.
-#define CAFE_SYNC_WAIT_NS 2000000000ULL
-__device__ __forceinline__ unsigned long long cafe_globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ int cafe_ld_acquire(const int *p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void cafe_st_release(int *p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-// Thread 0: waits until *p != last (or == want when want >= 0); returns the
-// value seen, or INT_MIN when the wait ran out (error bit set).
-__device__ __forceinline__ int cafe_wait_seq(const CafeDev &D, const int *p, int last, int want) {
-  const unsigned long long t0 = cafe_globaltimer();
-  unsigned int spins = 0;
-  while (true) {
-    int v = cafe_ld_acquire(p);
-    if (want >= 0 ? v == want : v != last) return v;
-    if ((++spins & 255u) == 0 && cafe_globaltimer() - t0 > CAFE_SYNC_WAIT_NS) {
-      atomicOr(D.err, CAFE_ERR_SYNC);
-      return (int)0x80000000;
-    }
-  }
-}
-
-__device__ __noinline__ void cafe_fill_helper(const CafeDev &D, const CafeConsts &K, CafeQuadScratch &S) {
-  __shared__ int s_cmd;
-  __shared__ CafeFillReq s_req;
-  const int tid = threadIdx.x;
-  int last = 0;
-  while (true) {
-    if (tid == 0) {
-      const int v = cafe_wait_seq(D, D.fill_seq, last, -1);
-      s_cmd = v;
-      if (v > 0) s_req = *D.fill;  // after the acquire: the main block's request
-    }
-    __syncthreads();
-    const int v = s_cmd;
-    if (v <= 0) return;  // -1: the main block left the keyed loop; INT_MIN: time-out
-    last = v;
-    if (tid < CAFE_QUAD_THREADS) {
-      CafeNewCell nc;
-      nc.c[0] = s_req.c[0];
-      nc.c[1] = s_req.c[1];
-      nc.c[2] = s_req.c[2];
-      nc.ext = s_req.ext;
-      nc.gid = s_req.gid;
-      unsigned long long gk = cafe_row_fill_quad(D, K, s_req.r, s_req.p, true, s_req.e, s_req.T, S, &nc);
-      if (tid == 0) D.fill->gk = gk;
-    }
-    __syncthreads();
-    if (tid == 0) cafe_st_release(D.fill_seq + 1, v);  // orders the row's stores before it
-  }
-}
-
-__device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, long long max_events, int allow_fast, const int cafe_bid, const int cafe_nblk) {
-  const CafeStepParams P = *Pp;
-  constexpr int NSEL = CAFE_LOOP_THREADS - CAFE_QUAD_THREADS;  // threads of the selecting warps
-  __shared__ CafeCand red[CAFE_LOOP_THREADS / 32];
-  __shared__ CafeSelShared s_sel;
-  __shared__ CafeCand s_best;  // winner of the next event (keyed mode)
-  __shared__ double s_tinc, s_dt, s_dsum, s_gmax, s_emax, s_vd, s_vs;
-  __shared__ int s_nvs2, s_countS, s_nrows, s_ngrain, s_done, s_nuc, s_icap, s_jspos, s_bslot, s_brow, s_na,
-      s_slow, s_ev, s_switch, s_newrow;
-  __shared__ unsigned char s_dirty[NSEL];   // a row of selecting thread i changed its key elsewhere
-  __shared__ unsigned char s_forced[NSEL];  // a row of selecting thread i was stamped -1
-  __shared__ uint32_t s_rng, s_rng_next;  // stream state after the consumed draws, after the next one
-  __shared__ double s_unext;               // the next event's draw (VoxelsCA.C:483)
-  __shared__ CafeNewCell s_nc;
-  __shared__ unsigned int s_sdloc;
-  __shared__ long long s_nnuc, s_negdt;
-  __shared__ long long s_cyc[4];  // winner, capture + bookkeeping, new row || selection, merge
-  __shared__ long long s_t0;
-  __shared__ CafeQuadScratch s_quad;
-#ifdef CAFE_DETAIL_CYCLES
-  // finer event-loop sections, thread 0's clock (profiling builds only)
-  __shared__ long long s_dcyc[16], s_dt0;
-#define CAFE_DCYC(slot)                          \
-  do {                                           \
-    if (threadIdx.x == 0) {                      \
-      long long _t = cafe_clock_ordered();       \
-      s_dcyc[slot] += _t - s_dt0;                \
-      s_dt0 = _t;                                \
-    }                                            \
-  } while (0)
-  if (threadIdx.x < 16) s_dcyc[threadIdx.x] = 0;
-  __shared__ unsigned long long s_fb0, s_sp0;
-  if (threadIdx.x == 0) {
-    s_dt0 = cafe_clock_ordered();
-    s_fb0 = *(volatile unsigned long long *)&crm_fallback_calls;
-    s_sp0 = *(volatile unsigned long long *)&crm_special_calls;
-  }
-#else
-#define CAFE_DCYC(slot) \
-  do {                  \
-  } while (0)
-#endif
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nthr = blockDim.x, nwarp = blockDim.x >> 5;
-  const int hid = tid - CAFE_QUAD_THREADS;  // index among the selecting warps (>= 0 there)
-  if (cafe_bid == 1) {  // the fill helper (two-block launch)
-    cafe_fill_helper(D, K, s_quad);
-    return;
-  }
-  const bool use_helper = cafe_nblk == 2;
-  __shared__ int s_post, s_seq;  // this event's fill went to the helper; requests posted
-  const double V = K.vhat_cls[1];
-  unsigned long long my_min = CAFE_KEY_NONE;  // smallest key of this selecting thread's rows
-  int my_hot = -1;                            // ... and its row
-  unsigned long long my_u2 = CAFE_KEY_NONE;   // smallest key of its other rows
-  int my_r2 = -2;                             // ... and its row (-1 none, -2 not known)
-  int hot_r = -1;                             // the row whose extent this thread keeps current
-  bool hot_ok = false;                        // hot_E is its extent after event e - 1
-  double hot_E = 0.0;
-  int sec_r = -1;                             // likewise its second-smallest-key row
-  bool sec_ok = false;
-  double sec_E = 0.0;
-  bool my_forced = false;                     // one of them is stamped -1
-  if (hid >= 0) {
-    s_dirty[hid] = 1;
-    s_forced[hid] = 0;
-  }
-  if (tid == 0) {
-    s_na = D.ctr[CTR_NA];
-    s_nvs2 = D.ctr[CTR_NVS2];
-    s_nrows = D.ctr[CTR_NROWS];
-    s_ngrain = D.ctr[CTR_NGRAIN];
-    uint32_t seed = cafe_minstd_seed((uint64_t)(uint32_t)(30 * P.tInd + (int)K.seed1));
-    s_rng = cafe_minstd_skip(seed, 2ULL * (uint64_t)s_na);
-    {
-      // the first event's draw; later draws are made one event ahead
-      cafe_uniform_stream st;
-      st.x = s_rng;
-      s_unext = cafe_uniform_next(&st);
-      s_rng_next = st.x;
-    }
-    s_sdloc = K.seed0 + 32u * (unsigned int)P.tInd + 64u * (unsigned int)s_ngrain;
-    s_tinc = 0.0;
-    s_dsum = 0.0;
-    s_vd = 0.0;
-    s_vs = 0.0;
-    s_countS = s_na;
-    s_nnuc = 0;
-    s_negdt = 0;
-    s_sel.evals = 0;
-#ifdef CAFE_DETAIL_CYCLES
-    s_sel.cyc[0] = s_sel.cyc[1] = s_sel.cyc[2] = s_sel.cyc[3] = s_sel.rounds = 0;
-#endif
-    s_ev = 0;
-    s_switch = 0;
-    s_newrow = -1;
-    s_post = 0;
-    s_seq = 0;
-    s_cyc[0] = s_cyc[1] = s_cyc[2] = s_cyc[3] = 0;
-    D.ev_vd[0] = 0.0;
-    D.ev_vs[0] = 0.0;
-    s_slow = !allow_fast || D.ctr[CTR_SLOW] != 0;
-    s_done = (*D.err != 0) || (s_na > D.act_cap) || (s_nvs2 > D.vs2_cap) || (s_nrows > D.row_cap);
-    if (s_na + 2 > D.ev_cap) {
-      atomicOr(D.err, CAFE_ERR_ITER_CAP);
-      s_done = 1;
-    }
-  }
-  __syncthreads();
-  // ======================================================== keyed, pipelined
-  if (!s_slow && !s_done) {
-    // magnitudes for the key rounding bound: largest numerator and extent
-    {
-      unsigned long long gk = 0, ek = 0;
-      for (int r = tid; r < s_nrows; r += nthr) {
-        int p = D.row_pos[r];
-        uint32_t live = D.row_live[r];
-        int nn = D.a_nn[p];
-        for (int k = 0; k < nn; ++k)
-          if (live >> k & 1u) {
-            double gv = fabs(D.row_g[(long long)r * CAFE_NSLOT + k]);
-            if (!cafe_is_nan(gv)) gk = max(gk, cafe_key(gv));
-          }
-        const double er = D.row_E[r];  // NaN extents occur (the reference's 0/0) and are left out
-        if (!cafe_is_nan(er)) ek = max(ek, cafe_key(fabs(er)));
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        gk = max(gk, cafe_shfl_u64_xor(gk, o));
-        ek = max(ek, cafe_shfl_u64_xor(ek, o));
-      }
-      if (lane == 0) {
-        red[warp].tk = gk;
-        red[warp].rk = ek;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        unsigned long long g2 = 0, e2 = 0;
-        for (int w = 0; w < nwarp; ++w) {
-          g2 = max(g2, red[w].tk);
-          e2 = max(e2, red[w].rk);
-        }
-        s_gmax = g2 ? cafe_unkey(g2) : 0.0;
-        s_emax = e2 ? cafe_unkey(e2) : 0.0;
-      }
-      __syncthreads();
-    }
-    // selection of the first event
-    if (hid >= 0)
-      cafe_select_keyed(D, K, 0, 0.0, s_nrows, hid, NSEL, 2, my_min, my_hot, my_u2, my_r2, my_forced, s_dirty,
-                        s_forced, s_sel, s_gmax, s_emax, s_dsum, V);
-    __syncthreads();
-    if (tid == 0) s_best = s_sel.red[0];
-    __syncthreads();
-    while (true) {
-      // ---- (1) the winner of this event (VoxelsCA.C:427-505), thread 0
-      if (tid == 0) {
-        s_t0 = clock64();
-        // while (vSind2 != countS && tinc < DelT)
-        const bool tin = !cafe_is_nan(s_tinc) && cafe_key(s_tinc) < cafe_key(K.DelT);
-        if (!(s_nvs2 != s_countS && tin)) s_done = 1;
-        s_countS = s_nvs2;
-        CafeCand b = s_best;
-        if (!s_done) {
-          if (b.j < 0 || !(b.tk < CAFE_KEY_1E6) || s_ev >= max_events) {
-            if (b.j >= 0 && b.tk < CAFE_KEY_1E6) atomicOr(D.err, CAFE_ERR_ITER_CAP);
-            s_done = 1;
-          } else {
-            // the draw made one event ahead from the current stream state
-            const double U = s_unext;
-            s_rng = s_rng_next;
-            // (the candidate carries vs2[j], its row and the captured
-            // position a_nbr[vs2[j], s])
-            s_jspos = b.p;
-            s_bslot = b.s;
-            s_brow = b.r;
-            s_icap = b.q;
-            s_nuc = U < cafe_nuc_rate(D, K, s_icap);
-            s_dt = s_nuc ? 0.0 : b.t;
-            if (cafe_is_neg(s_dt)) s_negdt++;
-            s_ev += 1;
-            // log this event's growth of the rows (VoxelsCA.C:514)
-            s_vd = s_nuc ? 0.0 : V * s_dt;
-            D.ev_vd[s_ev] = s_vd;
-            s_vs = s_vs + s_vd;
-            D.ev_vs[s_ev] = s_vs;
-            s_dsum += fabs(s_dt);
-            s_tinc += s_dt;
-            // hand the new row's fill to the helper block now when the
-            // captured cell will start a row of the shared velocity class
-            // (the condition phase 3 tests; the capture changes neither the
-            // cell's liquid count nor its neighbours' states)
-            s_post = 0;
-            const int icp = s_icap;
-            if (use_helper && !s_nuc && s_nrows < D.row_cap && D.a_liq[icp] > 0 && D.a_cold[icp] &&
-                D.a_cls[icp] == 1) {
-              CafeFillReq *F = D.fill;
-              const double *gq = D.row_geo + ((long long)s_brow * CAFE_NSLOT + s_bslot) * 4;
-              F->r = s_nrows;
-              F->p = icp;
-              F->e = s_ev;
-              F->gid = D.a_gid[s_jspos];
-              F->ext = gq[0];
-              F->c[0] = gq[1];
-              F->c[1] = gq[2];
-              F->c[2] = gq[3];
-              F->T = s_tinc;
-              s_seq += 1;
-              cafe_st_release(D.fill_seq, s_seq);
-              s_post = 1;
-            }
-          }
-        }
-        long long tn = clock64();
-        s_cyc[0] += tn - s_t0;
-        s_t0 = tn;
-      }
-      __syncthreads();
-      if (s_done) break;
-      CAFE_DCYC(0);
-      const int e = s_ev, icap = s_icap;
-      const int nrows_ev = s_nrows;  // rows before this event's new row
-      // ---- (2) the captured cell, its neighbours' rows, clamp flags
-      if (tid == 0) {
-        // the captured cell (VoxelsCA.C:483-505 and 518-605)
-        const int js = s_jspos;
-        D.a_state[icap] = 2;
-        if (s_nvs2 < D.vs2_cap) {
-          D.vs2[s_nvs2] = icap;
-        } else {
-          atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
-          s_done = 1;
-        }
-        s_nvs2 += 1;
-        if (s_nuc) {
-          int ci, cj, ck;
-          cafe_cell_xyz(K, D.act[icap], ci, cj, ck);
-          if (s_ngrain < D.grain_cap) {
-            double q4[4];
-            cafe_sample_orientation(K, s_sdloc, q4);
-            double *c = D.cth + 4LL * s_ngrain;
-            for (int a = 0; a < 4; ++a) c[a] = q4[a];
-            cafe_rot_from_cth(c, D.rot + 9LL * s_ngrain);
-          } else {
-            atomicOr(D.err, CAFE_ERR_GRAIN_CAP);
-            s_done = 1;
-          }
-          s_ngrain += 1;
-          D.a_gid[icap] = s_ngrain;
-          s_nc.gid = s_ngrain;
-          D.a_cx[icap] = s_nc.c[0] = ((double)ci + .5) * K.dx[0];
-          D.a_cy[icap] = s_nc.c[1] = ((double)cj + .5) * K.dx[1];
-          D.a_cz[icap] = s_nc.c[2] = ((double)ck + .5) * K.dx[2];
-          s_sdloc += 10u;
-          D.a_ext[icap] = s_nc.ext = 0.0;
-          s_nnuc++;
-        } else {
-          // the capture result of this slot, computed when the row was filled
-          const int gcap = D.a_gid[js];
-          if (gcap >= 1 && gcap <= D.grain_cap) {
-            // the grain's rotation, read by the new row's fill
-            cafe_prefetch_l1(D.rot + 9LL * (gcap - 1));
-            cafe_prefetch_l1(D.rot + 9LL * (gcap - 1) + 8);
-          }
-          cafe_prefetch_l1(D.act + icap);
-          D.a_gid[icap] = s_nc.gid = gcap;
-          const double *gq = D.row_geo + ((long long)s_brow * CAFE_NSLOT + s_bslot) * 4;
-          D.a_ext[icap] = s_nc.ext = gq[0];
-          D.a_cx[icap] = s_nc.c[0] = gq[1];
-          D.a_cy[icap] = s_nc.c[1] = gq[2];
-          D.a_cz[icap] = s_nc.c[2] = gq[3];
-        }
-      } else if (warp == 1) {
-        // neighbours of the captured cell lose one liquid neighbour
-        const int nn = D.a_nn[icap];
-        if (lane < nn) {
-          int q = D.a_nbr[(long long)icap * CAFE_NSLOT + lane];
-          // the new row's fill reads these next (nothing writes them here)
-          cafe_prefetch_l1(D.a_state + q);
-          cafe_prefetch_l1(D.act + q);
-          // every load before the stores, so that the loads of one chain
-          // level are in flight together
-          const int liq = D.a_liq[q];
-          const int r = D.a_frow[q];
-          const int sl = cafe_find_slot(D, q, icap);
-          const int rr = r >= 0 ? r : 0;
-          const bool alive = r >= 0 && D.row_alive[rr];
-          const uint32_t lv = D.row_live[rr];
-          const int bs = D.row_bslot[rr];
-          const unsigned long long k1 = D.row_key[rr], k2 = D.row_key2[rr];
-          const int left = liq - 1;
-          D.a_liq[q] = left;
-          if (alive) {
-            if (sl >= 0) D.row_live[r] = lv & ~(1u << sl);
-            if (left <= 0) {
-              D.row_alive[r] = 0;
-              D.row_death[r] = e;  // it grew at this event too
-              D.row_key[r] = CAFE_KEY_NONE;
-              s_dirty[r % NSEL] = 1;
-            } else if (sl >= 0 && sl == bs && k2 > k1) {
-              // the row's best candidate is gone: its key rises to that of
-              // its next candidate at the same evaluation, which bounds the
-              // row's exact value from below as the old key did
-              D.row_key[r] = k2;
-              s_dirty[r % NSEL] = 1;
-            }
-          }
-        }
-      } else if (tid == 64) {
-        // the next event's draw, off the winner section's chain (the stream
-        // advances by two engine outputs per event whatever the event)
-        cafe_uniform_stream st;
-        st.x = s_rng;
-        s_unext = cafe_uniform_next(&st);
-        s_rng_next = st.x;
-      } else if (hid >= 0) {
-        if (!s_nuc && cafe_is_neg(s_dt)) {
-          // a negative event may clamp a small extent at zero (VoxelsCA.C:515),
-          // which breaks the key bound of that row: mark the rows whose
-          // extrapolated extent comes near zero for re-evaluation
-          const double vd = s_vd;
-          const double margin = (double)(e + 16) * 0x1p-48 * (s_emax + s_gmax + V * s_dsum + 1e-300);
-          const double vs_prev = D.ev_vs[e - 1];
-          for (int r = hid; r < nrows_ev; r += NSEL) {
-            if (D.row_death[r] < e) continue;
-            int m = D.row_m[r];
-            if (m >= e) continue;
-            double elb = D.row_E[r] + (vs_prev - D.ev_vs[m]);
-            if (elb + vd < margin) {
-              D.row_stamp[r] = -1;
-              s_forced[r % NSEL] = 1;
-            }
-          }
-        }
-        // this thread's smallest-key row is the one an exact evaluation of
-        // the next selection most likely needs. Once its extent is current
-        // (after that evaluation's replay) it is kept current, one addition
-        // per event with the logged growth, held in registers and written
-        // through, so that the next evaluation replays nothing: the same
-        // additions in the same order as the lazy replay, only earlier (and
-        // after the clamp check above, which reads the state before this
-        // event). Only this thread writes its rows' extents in the keyed loop;
-        // a row that dies marks its owner dirty, whose rescan moves my_hot.
-        if (my_hot >= 0 && my_hot < nrows_ev) {
-          if (hot_r != my_hot) {
-            hot_r = my_hot;
-            hot_ok = false;
-          }
-          if (!hot_ok && D.row_m[hot_r] == e - 1 && D.row_death[hot_r] >= e) {
-            hot_E = D.row_E[hot_r];
-            hot_ok = true;
-          }
-          if (hot_ok) {
-            hot_E = hot_E + s_vd;
-            hot_E = cafe_is_neg(hot_E) ? 0.0 : hot_E;  // (E < 0.0) ? 0.0 : E
-            D.row_E[hot_r] = hot_E;
-            D.row_m[hot_r] = e;
-          }
-        } else {
-          hot_r = -1;
-          hot_ok = false;
-        }
-        // The second-smallest-key row becomes the smallest when the smallest
-        // one's key rises (its best candidate captured elsewhere). It is kept
-        // current the same way; as it is rarely evaluated, it is first brought
-        // up to date by a replay of at most CAFE_CATCHUP logged events per
-        // event, in this section where the selecting threads are otherwise
-        // idle. A row of this thread that dies marks it dirty, whose rescan
-        // moves my_r2.
-        if (my_r2 >= 0 && my_r2 < nrows_ev && my_r2 != hot_r) {
-          if (sec_r != my_r2) {
-            sec_r = my_r2;
-            sec_ok = false;
-          }
-          if (!sec_ok) {
-            // one level of loads: the row's death, watermark and extent, then
-            // the logged growths (independent of the running extent)
-            const int death = D.row_death[sec_r], m0 = D.row_m[sec_r];
-            double E = D.row_E[sec_r];
-            if (death >= e && m0 <= e - 1) {
-              const int stop = min(e - 1, m0 + CAFE_CATCHUP);
-#pragma unroll
-              for (int i = 1; i <= CAFE_CATCHUP; ++i) {
-                const int k = m0 + i;
-                if (k <= stop) {
-                  E = E + D.ev_vd[k];
-                  E = cafe_is_neg(E) ? 0.0 : E;  // (E < 0.0) ? 0.0 : E
-                }
-              }
-              if (stop == e - 1) {
-                sec_E = E;
-                sec_ok = true;
-              } else {
-                D.row_E[sec_r] = E;
-                D.row_m[sec_r] = stop;
-              }
-            }
-          }
-          if (sec_ok) {
-            sec_E = sec_E + s_vd;
-            sec_E = cafe_is_neg(sec_E) ? 0.0 : sec_E;  // (E < 0.0) ? 0.0 : E
-            D.row_E[sec_r] = sec_E;
-            D.row_m[sec_r] = e;
-          }
-        } else {
-          sec_r = -1;
-          sec_ok = false;
-        }
-      }
-      __syncthreads();
-      CAFE_DCYC(1);
-      if (tid == 0) {
-        long long tn = clock64();
-        s_cyc[1] += tn - s_t0;
-        s_t0 = tn;
-      }
-      // ---- (3) the new row (warps 0-3) || selection of the next event (the rest)
-      if (warp < CAFE_QUAD_THREADS / 32) {
-        if (s_post) {
-          // the helper fills this row: its bookkeeping here, its result at (4)
-          if (tid == 0) {
-            const int r = nrows_ev;
-            D.row_pos[r] = icap;
-            D.row_j[r] = s_nvs2 - 1;
-            D.row_alive[r] = 1;
-            D.a_frow[icap] = r;
-            D.row_death[r] = CAFE_ALIVE;
-            D.row_E[r] = D.a_ext[icap];
-            D.row_m[r] = e;
-          }
-        } else if (D.a_liq[icap] > 0 && D.a_cold[icap] && !s_done) {
-          int r = nrows_ev;
-          if (r < D.row_cap) {
-            if (tid == 0) {
-              D.row_pos[r] = icap;
-              D.row_j[r] = s_nvs2 - 1;
-              D.row_alive[r] = 1;
-              D.a_frow[icap] = r;
-              D.row_death[r] = CAFE_ALIVE;
-              D.row_E[r] = D.a_ext[icap];
-              D.row_m[r] = e;
-            }
-            const bool same_v = D.a_cls[icap] == 1;
-            unsigned long long gk = cafe_row_fill_quad(D, K, r, icap, same_v, e, s_tinc, s_quad, &s_nc);
-            if (tid == 0) {
-              if (!same_v) {
-                s_switch = 1;
-              } else {
-                if (gk != 0ULL) {
-                  double gm = cafe_unkey(gk);
-                  if (gm > s_gmax) s_gmax = gm;
-                }
-                double ea = fabs(D.a_ext[icap]);
-                if (ea > s_emax) s_emax = ea;
-              }
-              s_nrows = r + 1;
-              s_newrow = r;
-            }
-          } else if (tid == 0) {
-            atomicOr(D.err, CAFE_ERR_ROW_CAP);
-            s_done = 1;
-          }
-        }
-      } else {
-        cafe_select_keyed(D, K, e, s_tinc, nrows_ev, hid, NSEL, 2, my_min, my_hot, my_u2, my_r2, my_forced, s_dirty,
-                          s_forced, s_sel, s_gmax, s_emax, s_dsum, V);
-      }
-      __syncthreads();
-      CAFE_DCYC(2);
-      // ---- (4) the winner of the next event: selection or the new row
-      if (tid == 0) {
-        long long tn = clock64();
-        s_cyc[2] += tn - s_t0;
-        s_t0 = tn;
-        if (s_post) {
-          // the helper's fill of this event's new row (bounded wait)
-          const int got = cafe_wait_seq(D, D.fill_seq + 1, 0, s_seq);
-          if (got != s_seq) {
-            s_done = 1;
-          } else {
-            const int r = nrows_ev;
-            const unsigned long long gk = D.fill->gk;
-            if (gk != 0ULL) {
-              double gm = cafe_unkey(gk);
-              if (gm > s_gmax) s_gmax = gm;
-            }
-            double ea = fabs(D.a_ext[icap]);
-            if (ea > s_emax) s_emax = ea;
-            s_nrows = r + 1;
-            s_newrow = r;
-          }
-          s_post = 0;
-        }
-        CafeCand b = s_sel.red[0];
-        const int r = s_newrow;
-        if (r >= 0) {
-          s_newrow = -1;
-          s_dirty[r % NSEL] = 1;  // the row joins its owner's set
-          if (D.row_key[r] != CAFE_KEY_NONE) {
-            CafeCand c;
-            c.t = D.row_bt[r];
-            c.ruqs = D.row_bruq[r];
-            c.tk = cafe_key_canon(c.t);
-            c.rk = cafe_key_canon(c.ruqs);
-            c.j = D.row_j[r];
-            c.s = D.row_bslot[r];
-            c.r = r;
-            c.p = D.row_pos[r];
-            c.q = D.row_bq[r];
-            if (cafe_cand_better(c, b)) b = c;
-          }
-        }
-        s_best = b;
-        tn = clock64();
-        s_cyc[3] += tn - s_t0;
-        s_t0 = tn;
-      }
-      __syncthreads();
-      CAFE_DCYC(3);
-      if (s_switch) break;
-    }
-    if (s_switch && !s_done) {
-      // a capturing cell with another growth velocity: bring every row up to
-      // date and continue with the exact per-event scan
-      for (int r = tid; r < s_nrows; r += nthr) {
-        cafe_row_replay(D, r, s_ev);
-        D.row_m[r] = CAFE_M_DONE;
-      }
-      __syncthreads();
-      if (tid == 0) s_slow = 1;
-      __syncthreads();
-    }
-  } else if (s_slow && !s_done) {
-    // exact per-event scan with eager growth: extents are kept current
-    for (int r = tid; r < s_nrows; r += nthr) D.row_m[r] = CAFE_M_DONE;
-    __syncthreads();
-  }
-  // the helper block leaves (no request is outstanding here: every posted
-  // fill is taken at (4) of its own event)
-  if (use_helper && tid == 0) cafe_st_release(D.fill_seq, -1);
-  // ======================================================== exact scan
-  while (s_slow && !s_done) {
-    if (tid == 0) {
-      // while (vSind2 != countS && tinc < DelT)
-      if (!(s_nvs2 != s_countS && s_tinc < K.DelT)) s_done = 1;
-      s_countS = s_nvs2;
-    }
-    __syncthreads();
-    if (s_done) break;
-    // ---- every row's best candidate (VoxelsCA.C:386-445)
-    CafeCand best = cafe_cand_none();
-    for (int r = tid; r < s_nrows; r += nthr)
-      if (D.row_alive[r]) cafe_row_best(D, K, r, best);
-    best = cafe_warp_best(best);
-    if (lane == 0) red[warp] = best;
-    __syncthreads();
-    if (warp == 0) {
-      CafeCand b = lane < nwarp ? red[lane] : cafe_cand_none();
-      b = cafe_warp_best(b);
-      if (lane == 0) {
-        if (b.j < 0 || !(b.tk < CAFE_KEY_1E6) || s_ev >= max_events) {
-          if (b.j >= 0 && b.tk < CAFE_KEY_1E6) atomicOr(D.err, CAFE_ERR_ITER_CAP);
-          s_done = 1;
-        } else {
-          cafe_uniform_stream st;
-          st.x = s_rng;
-          double U = cafe_uniform_next(&st);
-          s_rng = st.x;
-          int jspos = D.vs2[b.j];
-          s_jspos = jspos;
-          s_bslot = b.s;
-          s_icap = D.a_nbr[(long long)jspos * CAFE_NSLOT + b.s];
-          s_nuc = U < cafe_nuc_rate(D, K, s_icap);
-          s_dt = s_nuc ? 0.0 : b.t;
-          if (s_dt < 0.0) s_negdt++;
-          s_ev += 1;
-        }
-      }
-    }
-    __syncthreads();
-    if (s_done) break;
-    // ---- growth of every mushy cell of the list (VoxelsCA.C:511-516)
-    if (!s_nuc) {
-      double d = s_dt;
-      if (isfinite(d)) {
-        for (int r = tid; r < s_nrows; r += nthr) {
-          if (!D.row_alive[r]) continue;
-          int p = D.row_pos[r];
-          double e = D.row_E[r] + cafe_vh(D, K, p) * d;
-          D.row_E[r] = (e < 0.0) ? 0.0 : e;
-        }
-      } else {
-        // a non-finite DtMin also reaches the cells that have no liquid
-        // neighbour (0 * inf)
-        for (int j = tid; j < s_countS; j += nthr) {
-          int p = D.vs2[j];
-          int r = D.a_frow[p];
-          double v = (r >= 0 && D.row_alive[r]) ? cafe_vh(D, K, p) : 0.0;
-          double *ep = r >= 0 ? &D.row_E[r] : &D.a_ext[p];
-          double e = *ep + v * d;
-          *ep = (e < 0.0) ? 0.0 : e;
-        }
-      }
-    }
-    __syncthreads();
-    const int icap = s_icap;
-    // ---- the captured cell (VoxelsCA.C:483-505 and 518-605)
-    if (tid == 0) {
-      const int js = s_jspos;
-      D.a_state[icap] = 2;
-      if (s_nvs2 < D.vs2_cap) {
-        D.vs2[s_nvs2] = icap;
-      } else {
-        atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
-        s_done = 1;
-      }
-      s_nvs2 += 1;
-      if (s_nuc) {
-        int ci, cj, ck;
-        cafe_cell_xyz(K, D.act[icap], ci, cj, ck);
-        if (s_ngrain < D.grain_cap) {
-          double q4[4];
-          cafe_sample_orientation(K, s_sdloc, q4);
-          double *c = D.cth + 4LL * s_ngrain;
-          for (int a = 0; a < 4; ++a) c[a] = q4[a];
-          cafe_rot_from_cth(c, D.rot + 9LL * s_ngrain);
-        } else {
-          atomicOr(D.err, CAFE_ERR_GRAIN_CAP);
-          s_done = 1;
-        }
-        s_ngrain += 1;
-        D.a_gid[icap] = s_ngrain;
-        D.a_cx[icap] = ((double)ci + .5) * K.dx[0];
-        D.a_cy[icap] = ((double)cj + .5) * K.dx[1];
-        D.a_cz[icap] = ((double)ck + .5) * K.dx[2];
-        s_sdloc += 10u;
-        D.a_ext[icap] = 0.0;
-        s_nnuc++;
-      } else {
-        D.a_gid[icap] = D.a_gid[js];
-        const double *gq = D.row_geo + ((long long)D.a_frow[js] * CAFE_NSLOT + s_bslot) * 4;
-        D.a_ext[icap] = gq[0];
-        D.a_cx[icap] = gq[1];
-        D.a_cy[icap] = gq[2];
-        D.a_cz[icap] = gq[3];
-      }
-      s_tinc += s_dt;
-    } else if (warp == 1) {
-      // ---- neighbours of the captured cell lose one liquid neighbour
-      const int nn = D.a_nn[icap];
-      if (lane < nn) {
-        int q = D.a_nbr[(long long)icap * CAFE_NSLOT + lane];
-        int left = --D.a_liq[q];
-        int r = D.a_frow[q];
-        if (r >= 0 && D.row_alive[r]) {
-          int sl = cafe_find_slot(D, q, icap);
-          if (sl >= 0) D.row_live[r] &= ~(1u << sl);
-          if (left <= 0) {
-            D.row_alive[r] = 0;
-            D.row_death[r] = s_ev;
-            D.row_key[r] = CAFE_KEY_NONE;
-          }
-        }
-      }
-    }
-    __syncthreads();
-    // ---- the captured cell becomes a capturing cell if it qualifies
-    if (warp < CAFE_QUAD_THREADS / 32) {
-      if (D.a_liq[icap] > 0 && D.a_cold[icap] && !s_done) {
-        int r = s_nrows;
-        if (r < D.row_cap) {
-          if (tid == 0) {
-            D.row_pos[r] = icap;
-            D.row_j[r] = s_nvs2 - 1;
-            D.row_alive[r] = 1;
-            D.a_frow[icap] = r;
-            D.row_death[r] = CAFE_ALIVE;
-            D.row_E[r] = D.a_ext[icap];
-            D.row_m[r] = CAFE_M_DONE;
-          }
-          cafe_row_fill_quad(D, K, r, icap, false, s_ev, s_tinc, s_quad);
-          if (tid == 0) s_nrows = r + 1;
-        } else if (tid == 0) {
-          atomicOr(D.err, CAFE_ERR_ROW_CAP);
-          s_done = 1;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    D.ctr[CTR_NGRAIN] = s_ngrain;
-    D.ctr[CTR_NVS2_END] = s_nvs2;
-    D.ctr[CTR_NROWS_END] = s_nrows;
-    D.ctr[CTR_NEV] = s_ev;
-    D.ctr[CTR_NNUC] = (int)s_nnuc;
-    atomicAdd(&D.stat[STAT_EVENTS], (unsigned long long)s_ev);
-    atomicAdd(&D.stat[STAT_NUC], (unsigned long long)s_nnuc);
-    atomicAdd(&D.stat[STAT_NEGDT], (unsigned long long)s_negdt);
-    atomicMax(&D.stat[STAT_MAXNA], (unsigned long long)s_na);
-    atomicMax(&D.stat[STAT_MAXROWS], (unsigned long long)s_nrows);
-    atomicAdd(&D.stat[STAT_STEPS], 1ULL);
-    atomicAdd(&D.stat[STAT_SUMNA], (unsigned long long)s_na);
-    atomicAdd(&D.stat[STAT_SUMROWS], (unsigned long long)s_nrows);
-    atomicAdd(&D.stat[STAT_EVALS], (unsigned long long)s_sel.evals);
-    if (s_slow) atomicAdd(&D.stat[STAT_SLOWSTEPS], 1ULL);
-    for (int c = 0; c < 4; ++c) atomicAdd(&D.stat[STAT_CYC_SELECT + c], (unsigned long long)s_cyc[c]);
-#ifdef CAFE_DETAIL_CYCLES
-    for (int c = 0; c < 16; ++c)
-      if (c != 9 && c != 13 && c != 14) atomicAdd(&D.stat[STAT_DETAIL + c], (unsigned long long)s_dcyc[c]);
-    atomicAdd(&D.stat[STAT_DETAIL + 9], *(volatile unsigned long long *)&crm_fallback_calls - s_fb0);
-    atomicAdd(&D.stat[STAT_DETAIL + 13], *(volatile unsigned long long *)&crm_special_calls - s_sp0);
-    for (int c = 0; c < 4; ++c) atomicAdd(&D.stat[STAT_DETAIL + 4 + c], (unsigned long long)s_sel.cyc[c]);
-    atomicAdd(&D.stat[STAT_DETAIL + 8], (unsigned long long)s_sel.rounds);
-#endif
-  }
-#undef CAFE_DCYC
-}
-__global__ void __launch_bounds__(CAFE_LOOP_THREADS, 1)
-    k_event_loop(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, long long max_events, int allow_fast) {
-  d_event_loop(D, K, Pp, max_events, allow_fast, blockIdx.x, gridDim.x);
-}
+#include "cafe_events.cuh"
 
 // Brings every row's extent up to the end of the step (the lazily applied
 // growth of VoxelsCA.C:511-516), spread over the whole GPU, and copies it back
 // to the row cell's active-list position.
-__device__ __forceinline__ void d_rows_finalize(const CafeDev &D, const int cafe_bid, const int cafe_nblk) {
+__device__ __forceinline__ void d_rows_finalize(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
   int nrows = D.ctr[CTR_NROWS_END];
   if (nrows > D.row_cap) nrows = (int)D.row_cap;
   int nev = D.ctr[CTR_NEV];
-  for (int r = cafe_bid * blockDim.x + threadIdx.x; r < nrows; r += cafe_nblk * blockDim.x) {
-    cafe_row_replay(D, r, nev);
+  const bool pr = D.ctr[CTR_EVLOG] != 0;
+  const int nrows0 = D.ctr[CTR_NROWS];
+  for (int k = cafe_bid * blockDim.x + threadIdx.x; k < nrows; k += cafe_nblk * blockDim.x) {
+    const int r = cafe_row_at(D, nrows0, k);
+    cafe_row_replay(D, K, r, nev, pr);
     D.a_ext[D.row_pos[r]] = D.row_E[r];
   }
 }
-__global__ void k_rows_finalize(CafeDev D) {
-  d_rows_finalize(D, blockIdx.x, gridDim.x);
+__global__ void k_rows_finalize(CafeDev D, CafeConsts K) {
+  d_rows_finalize(D, K, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------------ write back
@@ -3372,12 +1699,12 @@ __global__ void k_glog_begin(CafeDev D, const CafeStepParams *__restrict__ Pp) {
     if (blockIdx.x == 0 && threadIdx.x == 0) D.ctr[CTR_GLOG_OVER] = 1;
     return;
   }
-  const int tind = Pp->tInd;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x) {
-    int p = D.row_pos[r];
-    D.glog_cell[base + r] = (int32_t)D.act[p];
-    D.glog_step[base + r] = tind;
-    D.glog_tau[base + r] = D.a_ext[p];
+  const int tind = Pp->tInd, nrows0 = D.ctr[CTR_NROWS];
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nrows; k += gridDim.x * blockDim.x) {
+    int p = D.row_pos[cafe_row_at(D, nrows0, k)];
+    D.glog_cell[base + k] = (int32_t)D.act[p];
+    D.glog_step[base + k] = tind;
+    D.glog_tau[base + k] = D.a_ext[p];
   }
 }
 // After k_rows_finalize: growth time = (final extent - extent before) / v
@@ -3387,11 +1714,12 @@ __global__ void k_glog_end(CafeDev D, CafeConsts K) {
   if (nrows > D.row_cap) nrows = (int)D.row_cap;
   long long base = D.ctr[CTR_GLOG_N];
   if (base + nrows > D.glog_cap) return;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x) {
-    int p = D.row_pos[r];
+  const int nrows0 = D.ctr[CTR_NROWS];
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nrows; k += gridDim.x * blockDim.x) {
+    int p = D.row_pos[cafe_row_at(D, nrows0, k)];
     double v = cafe_vh(D, K, p);
-    double e0 = D.glog_tau[base + r];
-    D.glog_tau[base + r] = v > 0.0 ? (D.a_ext[p] - e0) / v : 0.0;
+    double e0 = D.glog_tau[base + k];
+    D.glog_tau[base + k] = v > 0.0 ? (D.a_ext[p] - e0) / v : 0.0;
   }
 }
 __global__ void k_glog_advance(CafeDev D) {

@@ -36,10 +36,9 @@ typedef struct {
   long long grain_capacity;    /* initial grain-table capacity; 0 = automatic */
   int event_scan;              /* 0: keyed event selection (default); 1: evaluate every
                                   frontier cell at every event (the reference's scan) */
-  int event_fill_helper;       /* 1: the event loop hands each new frontier row's set-up to a
-                                  second thread block on another SM (same results; measured
-                                  slower on this GPU: the selection, not the set-up, bounds an
-                                  event); 0 (default): one block does everything */
+  int event_fill_helper;       /* 1: batched launches give the event loop of each realisation a
+                                  second thread block. It is idle: new frontier rows are set up
+                                  ahead of the loop. Same results as 0 (default) */
 } cafe_options;
 
 typedef struct {
@@ -72,15 +71,15 @@ typedef struct {
   unsigned long long sum_active;   /* sum over steps of the active-list length */
   unsigned long long sum_rows;     /* sum over steps of the frontier size */
   unsigned long long launches;     /* kernels launched by this handle since the last phase reset */
-  unsigned long long exact_scan_steps; /* steps run with the full per-event scan */
-  unsigned long long row_evaluations;  /* keyed-selection rounds that evaluated rows exactly */
-  unsigned long long cycles_select;    /* event-loop SM cycles taking this event's winner */
-  unsigned long long cycles_apply;     /* ... applying the capture/nucleation */
-  unsigned long long cycles_fill;      /* ... new frontier row and next selection, side by side */
+  unsigned long long exact_scan_steps; /* steps whose rows do not share one growth velocity, or that
+                                          ran the full per-event scan */
+  unsigned long long row_evaluations;  /* windows of resident rows the event loop opened */
+  unsigned long long cycles_select;    /* event-loop SM cycles selecting the events' winners */
+  unsigned long long cycles_apply;     /* ... applying the capture/nucleation, growth */
+  unsigned long long cycles_fill;      /* ... filling new frontier rows that were not foreseen */
   unsigned long long graph_captures;   /* step graphs captured (one per handle unless buffers move) */
   unsigned long long easm_integrals;   /* EASM: Utilities::Integral evaluations (25 nodes each) */
-  unsigned long long cycles_merge;     /* ... taking the next event's winner (the new row's
-                                          result included) */
+  unsigned long long cycles_merge;     /* ... opening windows */
 } cafe_stats;
 
 /* Grid::Grid (Grid.C:15-109, deck parse Grid.C:165-318) + Partition::

@@ -1,0 +1,77 @@
+"""The event loop's resident window against the full per-event scan
+(event_scan=1), which evaluates every frontier row at every event: identical
+states (NaN extents included), grains and event counts."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+DECKS = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "decks")
+
+# one voxel of beam travel and several hundred captures per step: more frontier
+# rows than a window holds, windows opened again within a step, rows of captures
+# two and more generations deep, negative-time events
+WIDE = """dx 2.5e-6
+nX %d %d %d
+bmV 1.0
+bmP 200.0
+bmDelT 2.5e-6
+r 2e-3
+lT 30e-6
+bpH 12.5e-6
+tL 1609
+tS 1531.5
+meltparam 10e-6 %g %g 20e-6
+bhatch 40e-6
+mu 4e-4
+lrate 4e-4
+patternID 2
+outint 1000000
+offset 0.0 0.0 0.0
+gridsize 1.2e-4 1.0e-4
+gridtheta %g
+dendritegrowth2 %g 2.0
+%s
+"""
+
+
+def _run(deck, steps, **kw):
+    from amcafe_gb300 import Simulation
+
+    with Simulation(deck, **kw) as sim:
+        sim.InitializeVoxels()
+        sim.begin()
+        sim.run(steps)
+        st = sim.state()
+        st["ctheta"] = sim.ctheta()
+        s = sim.stats()
+    return st, s
+
+
+def _same(deck, steps):
+    a, sa = _run(deck, steps)
+    b, sb = _run(deck, steps, event_scan=1)
+    for k in a:
+        assert np.array_equal(a[k], b[k], equal_nan=a[k].dtype.kind == "f"), k
+    for k in ("events", "nucleations", "negative_dt", "max_rows", "sum_rows"):
+        assert sa[k] == sb[k], k
+    return sa
+
+
+@pytest.mark.parametrize("deck,steps", [("layers_rot.in", 90), ("odd_dims.in", 12), ("track_easm60.in", 0),
+                                        ("track_ros.in", 0)])
+def test_window_equals_full_scan(deck, steps):
+    _same(os.path.join(DECKS, deck), steps)
+
+
+@pytest.mark.parametrize("nx,ny,nz,rear,half,turn,growth,extra,steps", [
+    (48, 40, 17, 40e-6, 40e-6, 0.0, 1e-5, "", 40),
+    (47, 41, 19, 40e-6, 40e-6, 0.6, 1e-4, "", 24),   # six voxels of growth a step: captures many generations deep
+    (45, 33, 18, 30e-6, 30e-6, 0.0, 1e-5, "rosenthal 0.35 20.0 5e-6", 60),
+])
+def test_wide_fronts(tmp_path, nx, ny, nz, rear, half, turn, growth, extra, steps):
+    path = tmp_path / "wide.in"
+    path.write_text(WIDE % (nx, ny, nz, rear, half, turn, growth, extra))
+    s = _same(str(path), steps)
+    assert s["events"] > 0
