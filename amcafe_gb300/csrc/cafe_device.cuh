@@ -23,6 +23,8 @@
 // and how far past the step's end (in time steps) a capture is foreseen.
 #define CAFE_CHILD_DEPTH 3
 #define CAFE_CHILD_REACH 1.1
+// Rows listed for the event loop's first window.
+#define CAFE_DUE_MAX 4096
 
 // Error bits written to CafeDev::err by device code.
 enum {
@@ -33,12 +35,13 @@ enum {
   CAFE_ERR_ITER_CAP = 16,
 };
 
-// One slot of a frontier row's record: numerator g, neighbour position q (-1
-// when absent) and, in the low five bits of m, the neighbour direction; above
+// One slot of a frontier row's record: numerator g, order key of the tie-break
+// ruqs (VoxelsCA.C:436), neighbour position q and, in the low five bits of m, the neighbour direction; above
 // them the number, plus one, of the row made ahead for a capture through it (0
 // when none).
-struct __align__(16) CafeSlot {
+struct CafeSlot {
   double g;
+  unsigned long long rk;
   int q;
   uint32_t m;
 };
@@ -160,12 +163,13 @@ struct CafeDev {
   int32_t *vs2;
   long long vs2_cap;
   int32_t *row_pos, *row_j;
-  // a row's record: its slots by g (row_slot, CAFE_NSLOT entries), the place
-  // of each direction in it (row_rank, 32 entries) and the live places
-  // (row_live)
+  // a row's record: the slots that held a liquid neighbour when it was made, by
+  // g (row_slot, row_n of CAFE_NSLOT entries); row_k: the place from which on a
+  // slot may not be captured yet
   CafeSlot *row_slot;
-  uint8_t *row_rank;
-  uint32_t *row_live;
+  uint8_t *row_n, *row_k;
+  // event that captured a position this step (0: none)
+  int32_t *a_ev;
   // per (row, direction): extent and centre (x, y, z) given to the neighbour
   // when this slot captures it, 4 doubles
   double *row_geo;
@@ -182,12 +186,11 @@ struct CafeDev {
   int32_t *row_pairs;
   // rows during the event loop: row_E is the row cell's extent (ExtA)
   // including the growth of events 1..row_m, copied back to a_ext afterwards;
-  // a row grows at the events (birth, row_death]; row_key bounds the row's
-  // absolute capture time from below; row_res is its place in the resident set
-  // (-1 none); row_mag: order keys of the largest |g|, the largest extent, the
-  // smallest and the largest velocity of the step's rows
+  // row_key bounds the row's absolute capture time from below; row_mag: order
+  // keys of the largest |g|, the largest extent, the smallest and the largest
+  // velocity of the step's rows
   double *row_E;
-  int32_t *row_m, *row_death, *row_res;
+  int32_t *row_m, *row_due;  // row_due: CAFE_DUE_MAX rows that can capture soon
   unsigned long long *row_key, *row_mag;
   // the logged growth of each event (CTR_EVLOG: fl(v * DtMin), or DtMin) and
   // its running sum
@@ -222,6 +225,8 @@ enum {
   CTR_EASM_QHEAD,                       // next queued cell to take
   CTR_GLOG_N,                           // growth-log entries written
   CTR_GLOG_OVER,                        // 1: the growth log ran out of room
+  CTR_NDUE,                             // rows listed for the event loop's first window
+  CTR_NKEY,                             // rows with a capture candidate at the step's start
   CTR_EVLOG,                            // 1: ev_vd holds DtMin, 0: fl(v * DtMin)
   CTR_NCHILD,                           // foreseen captures listed, one count per generation
   CTR_NCHILD_LAST = CTR_NCHILD + CAFE_CHILD_DEPTH - 1,

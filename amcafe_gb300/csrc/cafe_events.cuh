@@ -4,9 +4,11 @@
 // A frontier row is a mushy cell with a liquid neighbour. Its slots are the 26
 // neighbour directions; those that hold a liquid neighbour are candidates with
 // capture time t = fl(fl(g - E)/v), g the slot's numerator, E the row cell's
-// extent and v its growth velocity. A row's record lists its slots by g
-// (CafeSlot row_slot[26]), so that its earliest candidate is the first one
-// still live; row_live is the mask of live slots in that order.
+// extent and v its growth velocity. A row's record lists the slots that held a
+// liquid neighbour when it was made by g (CafeSlot row_slot[26], row_n of
+// them), so that its earliest candidate is the first one whose neighbour has not
+// been captured since (a_ev, the event that captured a position, 0 for none);
+// row_k is the place to look from.
 
 // ------------------------------------------------------------------ row set-up
 // Captures that can happen within the step are foreseen: when a record is
@@ -22,29 +24,26 @@ struct CafeChildList {
 };
 __device__ __forceinline__ int cafe_slot_child(uint32_t m) { return (int)(m >> 5) - 1; }
 
+#define CAFE_DUE_REACH 4.0  // time steps
+
 // Sorts the slots of row r (one per lane: liv, numerator gv, neighbour position
-// q) by g (NaN last among the live ones, ties by slot, the other slots after
-// them) into the row's record, and forms the row's key: the order key of T + t
+// q) by g (NaN last, ties by slot) into the row's record, and forms the row's key: the order key of T + t
 // for its first candidate, a lower bound of the row's absolute capture time
-// (CAFE_KEY_NONE without a candidate). E and v are the row's. Returns, in every
+// (CAFE_KEY_NONE without a candidate). E, v and ruq are the row's. Returns, in every
 // lane, the order key of the largest |g| of the live slots (0 when none).
 __device__ __forceinline__ unsigned long long cafe_row_sort_warp(const CafeDev &D, long long r, bool liv, double gv,
-                                                                 int q, double E, double v, double T, int gid,
-                                                                 const CafeChildList &C) {
+                                                                 int q, double E, double v, double T, int gid, double ruq,
+                                                                 const CafeChildList &C, bool fill) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const uint32_t live = __ballot_sync(FULL, liv);
   const bool gfin = !cafe_is_nan(gv);
   const unsigned long long key = (liv && gfin) ? cafe_key_canon(gv) : CAFE_KEY_NONE;
-  int rank = liv ? 0 : __popc(live);
+  int rank = 0;
 #pragma unroll
   for (int t = 0; t < CAFE_NSLOT; ++t) {
     unsigned long long kt = cafe_shfl_u64(key, t);
-    bool lt = (live >> t) & 1u;
-    if (liv)
-      rank += lt && (kt < key || (kt == key && t < lane));
-    else
-      rank += !lt && t < lane;
+    rank += ((live >> t) & 1u) && (kt < key || (kt == key && t < lane));
   }
   // the slot's capture time and, when it comes due within the step, its child
   double t = NAN;
@@ -62,14 +61,25 @@ __device__ __forceinline__ unsigned long long cafe_row_sort_warp(const CafeDev &
       }
     }
   }
-  if (lane < CAFE_NSLOT) {
+  if (liv) {
     CafeSlot s;
-    s.g = liv ? gv : NAN;
+    s.g = gv;
     s.q = q;
     s.m = (uint32_t)lane | child;
+    s.rk = cafe_key_canon(.5 * (ruq + D.a_ruq[q]));
     D.row_slot[r * CAFE_NSLOT + rank] = s;
-    D.row_rank[r * 32 + lane] = (uint8_t)rank;
-    if (lane == 0) D.row_live[r] = (1u << __popc(live)) - 1u;
+  } else if (fill && lane < CAFE_NSLOT) {
+    // (the rest of the record is read along with it: keep it in cache)
+    CafeSlot s;
+    s.g = NAN;
+    s.rk = CAFE_KEY_NONE;
+    s.q = 0;
+    s.m = 0;
+    D.row_slot[r * CAFE_NSLOT + __popc(live) + __popc(~live & ((1u << lane) - 1u))] = s;
+  }
+  if (lane == 0) {
+    D.row_n[r] = (uint8_t)__popc(live);
+    D.row_k[r] = 0;
   }
   if (liv && rank == 0) {
     D.row_key[r] = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(T + t);
@@ -152,7 +162,7 @@ __device__ __noinline__ unsigned long long cafe_row_fill_quad(const CafeDev &D, 
   if (w == 0) {
     double gv = liv ? NAN : 0.0;  // a capturing cell without a grain never captures
     if (work) gv = crm_pow_half(S.cth[lane] * S.sph[lane]) * S.dr[lane];
-    ak = cafe_row_sort_warp(D, r, liv, gv, q, nc.ext, cafe_vh(D, K, p), T, gp, C);
+    ak = cafe_row_sort_warp(D, r, liv, gv, q, nc.ext, cafe_vh(D, K, p), T, gp, D.a_ruq[p], C, true);
   } else if (w >= 2 && work) {
     double Lmud = cafe_geo_lmud(K, S.l[lane], S.d1I[lane], S.dI2[lane], S.d1J[lane], S.dJ3[lane]);
     double *o = D.row_geo + (r * CAFE_NSLOT + lane) * 4;
@@ -177,7 +187,8 @@ struct CafeCand {
   unsigned long long tk, rk;
   double t;
   int j, s;     // vs2 index and neighbour slot of the capturing cell; j < 0 = none
-  int r, q, child;  // (not compared) its row, the captured position and that cell's foreseen row
+  int r, q;     // (not compared) its row and the captured position
+  uint32_t m;   // ... and the slot's CafeSlot::m
 };
 __device__ __forceinline__ CafeCand cafe_cand_none() {
   CafeCand c;
@@ -186,7 +197,7 @@ __device__ __forceinline__ CafeCand cafe_cand_none() {
   c.j = -1;
   c.s = 0;
   c.r = c.q = 0;
-  c.child = -1;
+  c.m = 0;
   return c;
 }
 __device__ __forceinline__ bool cafe_cand_better(const CafeCand &a, const CafeCand &b) {
@@ -210,28 +221,50 @@ __device__ __forceinline__ CafeCand cafe_warp_best(CafeCand best) {
     c.s = __shfl_xor_sync(0xffffffffu, best.s, o);
     c.r = __shfl_xor_sync(0xffffffffu, best.r, o);
     c.q = __shfl_xor_sync(0xffffffffu, best.q, o);
-    c.child = __shfl_xor_sync(0xffffffffu, best.child, o);
+    c.m = __shfl_xor_sync(0xffffffffu, best.m, o);
     if (cafe_cand_better(c, best)) best = c;
   }
   return best;
 }
 #define CAFE_KEY_1E6 0xc12e848000000000ULL  // cafe_key(1e6)
 
+// First place from k on in row r's record whose neighbour is not captured;
+// row_n[r] when none is left.
+__device__ __forceinline__ int cafe_row_next(const CafeDev &D, int r, int k) {
+  const int n = D.row_n[r];
+  const CafeSlot *rec = D.row_slot + (long long)r * CAFE_NSLOT;
+  while (k < n && D.a_ev[rec[k].q] != 0) ++k;
+  return k;
+}
+// Event at which row r lost its last liquid neighbour (it grew at that event
+// too), CAFE_ALIVE when one is left. The slots of largest g are captured last,
+// so the first look nearly always ends it.
+#define CAFE_ALIVE 0x7fffffff
+__device__ __forceinline__ int cafe_row_death(const CafeDev &D, int r) {
+  const CafeSlot *rec = D.row_slot + (long long)r * CAFE_NSLOT;
+  int d = 0;
+  for (int k = (int)D.row_n[r] - 1; k >= 0; --k) {
+    const int e = D.a_ev[rec[k].q];
+    if (e == 0) return CAFE_ALIVE;
+    d = max(d, e);
+  }
+  return d;
+}
+
 // Best candidate of frontier row r (VoxelsCA.C:386-445 restricted to one cell)
-// with extent E, velocity v and live slots `live`. For a
+// with extent E and velocity v, looking from place k of its record on. For a
 // positive finite velocity the capture time is non-decreasing in g, so the
 // visit in g order stops at the first time above the row's minimum; otherwise
 // every live slot is evaluated. The reference's acceptance limit t <= 1e6
 // (VoxelsCA.C:383, 427) applies.
-__device__ __noinline__ void cafe_row_best(const CafeDev &D, int r, double E, double v, uint32_t live,
-                                           CafeCand &best) {
-  const int p = D.row_pos[r];
+__device__ __noinline__ void cafe_row_best(const CafeDev &D, int r, double E, double v, int k, CafeCand &best) {
   const long long vb = crm_bits(v);
   const bool mono = vb > 0 && vb < CRM_BITS_INF;  // 0 < v < inf
   bool have = false;
   unsigned long long tfirst = 0;
-  for (; live; live &= live - 1) {
-    const CafeSlot s = D.row_slot[(long long)r * CAFE_NSLOT + __ffs(live) - 1];
+  for (const int n = D.row_n[r]; k < n; ++k) {
+    const CafeSlot s = D.row_slot[(long long)r * CAFE_NSLOT + k];
+    if (D.a_ev[s.q] != 0) continue;
     double dr = s.g - E;
     double t = dr / v;
     if (cafe_is_nan(t)) continue;
@@ -244,12 +277,12 @@ __device__ __noinline__ void cafe_row_best(const CafeDev &D, int r, double E, do
     CafeCand c;
     c.t = t;
     c.tk = tk;
-    c.rk = cafe_key_canon(.5 * (D.a_ruq[p] + D.a_ruq[s.q]));
+    c.rk = s.rk;
     c.j = D.row_j[r];
     c.s = (int)(s.m & 31u);
     c.r = r;
     c.q = s.q;
-    c.child = cafe_slot_child(s.m);
+    c.m = s.m;
     if (cafe_cand_better(c, best)) best = c;
     if (!have) {
       have = true;
@@ -263,21 +296,33 @@ __device__ __noinline__ void cafe_row_best(const CafeDev &D, int r, double E, do
 // only when the row is needed or at the end of the step (k_rows_finalize). The
 // log holds fl(v * DtMin) when the step's rows share one velocity (v NaN here),
 // else DtMin, which each row multiplies by its own velocity.
-#define CAFE_ALIVE 0x7fffffff   // row_death of a row that is still alive
-#define CAFE_M_DONE 0x7fffffff  // row_m of a row whose extent is kept current
+#define CAFE_M_DONE 0x7fffffff  // row_m of a row whose extent is kept current elsewhere
+
+// a / v for 0 < v normal, y = 1/v correctly rounded: two corrections of a * y by
+// the exact remainder (Markstein, IBM J. Res. Dev. 34(1), 1990: with a correctly
+// rounded reciprocal the last one rounds the quotient correctly from a faithful
+// one). Operands near the ends of the exponent range take the division.
+__device__ __forceinline__ double cafe_div_by(double a, double v, double y) {
+  const int ea = (int)((crm_bits(a) >> 52) & 0x7ff), ev = (int)((crm_bits(v) >> 52) & 0x7ff);
+  if (ea < 200 || ea > 1800 || ev < 800 || ev > 1200 || (crm_bits(v) & 0xfffffffffffffLL) == 0xfffffffffffffLL)
+    return a / v;
+  double q = a * y;
+  q = fma(fma(-q, v, a), y, q);
+  return fma(fma(-q, v, a), y, q);
+}
 
 // One event's growth of an extent (VoxelsCA.C:511-516).
 __device__ __forceinline__ double cafe_grow(double E, double vd) {
   E = E + vd;
   return cafe_is_neg(E) ? 0.0 : E;  // (E < 0.0) ? 0.0 : E
 }
-// Extent of row r after the logged growth of events row_m+1 .. min(upto,
-// row_death). A nucleation logs +0, which leaves an extent unchanged (extents
+// Extent of row r after the logged growth of events row_m+1 .. min(upto, its
+// last). A nucleation logs +0, which leaves an extent unchanged (extents
 // are never -0).
 template <bool PR>
 __device__ __forceinline__ double cafe_row_replayed(const CafeDev &D, int r, int upto, double v, int &stop) {
   const int m = D.row_m[r];
-  stop = min(upto, D.row_death[r]);
+  stop = m < upto ? min(upto, cafe_row_death(D, r)) : m;
   double E = D.row_E[r];
   if (stop <= m) {
     stop = m;
@@ -331,7 +376,6 @@ __device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &
       const double E = D.a_ext[p];
       D.row_E[r] = E;
       D.row_m[r] = 0;
-      D.row_death[r] = CAFE_ALIVE;
       const double v = cafe_vh(D, K, p);
       const int bad = (cafe_v_ordinary(v) && fabs(E) != INFINITY) ? 0 : 2;
       const int slow = bad | (D.a_cls[p] != 1 ? 1 : 0);
@@ -384,6 +428,8 @@ __device__ __forceinline__ void d_rows_order(const CafeDev &D, const CafeConsts 
   const int lane = threadIdx.x & 31;
   unsigned long long gk = 0ULL, ek = 0ULL, vk = CAFE_KEY_NONE, xk = 0ULL;
   const CafeChildList C = {&D.ctr[CTR_NCHILD], 0, D.ch_cap, K.DelT * CAFE_CHILD_REACH};
+  const unsigned long long due = cafe_key(K.DelT * CAFE_DUE_REACH);
+  int nkey = 0;  // (lane 0) rows with a candidate
   for (int r = w; r < nrows; r += warps) {
     int p = D.row_pos[r];
     int q = -1;
@@ -396,8 +442,19 @@ __device__ __forceinline__ void d_rows_order(const CafeDev &D, const CafeConsts 
     }
     __syncwarp();  // the record is read before it is written in order
     const double E = D.row_E[r], v = cafe_vh(D, K, p);
-    gk = max(gk, cafe_row_sort_warp(D, r, liv, gv, q, E, v, 0.0, D.a_gid[p], C));
+    const unsigned long long ak = cafe_row_sort_warp(D, r, liv, gv, q, E, v, 0.0, D.a_gid[p], D.a_ruq[p], C, false);
+    gk = max(gk, ak);
+    __syncwarp();
     if (!cafe_is_nan(E)) ek = max(ek, cafe_key(fabs(E)));  // NaN extents occur (the reference's 0/0)
+    // rows that can capture soon are listed for the event loop's first window
+    if (lane == 0) {
+      const unsigned long long key = D.row_key[r];
+      if (key != CAFE_KEY_NONE) ++nkey;
+      if (key <= due) {
+        const int i = atomicAdd(&D.ctr[CTR_NDUE], 1);
+        if (i < CAFE_DUE_MAX) D.row_due[i] = r;
+      }
+    }
     vk = min(vk, cafe_key(v));
     xk = max(xk, cafe_key(v));
   }
@@ -406,6 +463,7 @@ __device__ __forceinline__ void d_rows_order(const CafeDev &D, const CafeConsts 
     atomicMax(&D.row_mag[1], ek);
     atomicMin(&D.row_mag[2], vk);
     atomicMax(&D.row_mag[3], xk);
+    if (nkey) atomicAdd(&D.ctr[CTR_NKEY], nkey);
   }
 }
 __global__ void k_rows_order(CafeDev D, CafeConsts K) {
@@ -441,6 +499,7 @@ __device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K
     const unsigned long long gk = cafe_row_fill_quad(D, K, id, p, D.ch_T[i], Q, nc, C);
     if (threadIdx.x == 0) {
       D.row_key[id] = CAFE_KEY_NONE;  // until the row exists
+      D.row_m[id] = CAFE_M_DONE;  // (set when it leaves the resident set)
       atomicMax(&D.row_mag[0], gk);
       if (!cafe_is_nan(nc.ext)) atomicMax(&D.row_mag[1], cafe_key(fabs(nc.ext)));
       const double v = cafe_vh(D, K, p);
@@ -465,16 +524,20 @@ __global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_children(const __grid_con
 // set: the rows whose key (lower bound of the absolute capture time T + t when
 // last evaluated) lies at or below a window bound W, and the rows created by
 // captures (made ahead by k_children when the capture was foreseen, filled in
-// the loop otherwise). A resident row has its extent in a register of the thread that owns
-// its index and its first live slot in shared memory. Per event:
-//   select   every resident's g - E, the minimum over the block by integer order
-//            keys (two redux per warp and level), and a test that no other
-//            candidate lies within the rounding of the division by v. A tie (or
-//            a near one) is resolved by evaluating the close rows exactly in the
-//            reference's order (time, ruqs, vs2 index, slot);
-//   apply    one warp updates the captured cell and its neighbours' rows while
-//            one thread divides out the capture time and advances the clock and
-//            another draws the next event's uniform;
+// the loop otherwise). A resident row's extent and first live slot are in shared
+// memory; one thread owns it. What an event costs is instructions on its chain
+// (~11 SM cycles each, against ~700 for a load that misses L1), so rows keep no
+// live masks: a row looks for its next slot when its first one is captured. Per event:
+//   select   every resident's g - E, its minimum over the block by 32-bit order
+//            keys (the high word; with PR a single-precision time). When no other
+//            candidate's key is within the keys' resolution the minimum stands;
+//            else the close ones are compared in full: equal g - E by ruqs, and
+//            what only exact times decide in the reference's order (time, ruqs,
+//            vs2 index, slot);
+//   apply    the owner of a row whose first slot was captured moves it on; one
+//            warp updates the captured cell and brings in its row, one thread
+//            divides out the capture time and advances the clock, another draws
+//            the next event's uniform;
 //   grow     every resident's extent by the logged growth, in the reference's
 //            order of additions (the rows outside the set replay the log when
 //            they enter it or at the step's end).
@@ -485,14 +548,15 @@ __global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_children(const __grid_con
 // window. Rows with another velocity than the step's class-1 velocity switch the
 // step to per-row velocities (PR); a velocity that is not positive and finite,
 // or a window that does not fit, to the full scan of every row per event.
-#define CAFE_RES_PER 2  // resident rows per thread
-#define CAFE_RES_MAX (CAFE_RES_PER * CAFE_LOOP_THREADS)
+#define CAFE_RES_MAX 768  // resident rows
 #define CAFE_RES_TARGET 320  // rows an opened window aims at: one per thread with room for the step's new rows
 #define CAFE_OPEN_TRIES 48   // windows in a row without an event before the step takes the full scan
+#define CAFE_WARPS (CAFE_LOOP_THREADS / 32)
 #define CAFE_CAP_WARP (CAFE_LOOP_THREADS / 32 - 1)     // captures
 #define CAFE_CLOCK_WARP (CAFE_LOOP_THREADS / 32 - 2)   // capture time and clock
 #define CAFE_DRAW_WARP (CAFE_LOOP_THREADS / 32 - 3)    // nucleation draws
-static_assert(CAFE_CAP_WARP >= 6, "warps 0-3 fill rows");
+#define CAFE_AHEAD_WARP (CAFE_LOOP_THREADS / 32 - 4)   // loads the likely next events' data ahead
+static_assert(CAFE_CAP_WARP >= 8, "warps 0-3 fill rows");
 // Row of the k-th frontier row of the step: the rows present at its start, then
 // the rows that captures created, in their order (row_new).
 __device__ __forceinline__ int cafe_row_at(const CafeDev &D, int nrows0, int k) {
@@ -501,7 +565,7 @@ __device__ __forceinline__ int cafe_row_at(const CafeDev &D, int nrows0, int k) 
 
 struct CafeLoop {
   // the loop's scalars (VoxelsCA.C:381-610)
-  double tinc, dt, vd, vs, vneg, vmin, vmax, dsum, gmax, emax;
+  double tinc, dt, vd, vs, vmin, vmax, dsum, gmax, emax;
   double unext[2];  // unext[e & 1]: event e's draw
   int fill, nvs2, countS, nrows0, nrows, ngrain, done, nuc, ev, sw, na, newrow, slow;
   uint32_t rng;
@@ -511,25 +575,30 @@ struct CafeLoop {
 };
 struct CafeResident {
   double g[CAFE_RES_MAX];      // numerator of the first live slot, NaN when none
+  double E[CAFE_RES_MAX];      // extent
   double v[CAFE_RES_MAX];      // growth velocity (PR)
+  float rv[CAFE_RES_MAX];      // ... and its reciprocal
+  unsigned long long rk[CAFE_RES_MAX];  // the first live slot's tie-break ruqs (order key)
   int r[CAFE_RES_MAX];         // row, -1 when free
-  int q[CAFE_RES_MAX];         // the first live slot's neighbour position
-  uint32_t m[CAFE_RES_MAX];    // ... and its slot
-  uint32_t live[CAFE_RES_MAX];  // live slots in g order
+  int q[CAFE_RES_MAX];         // the first live slot's neighbour position, -1 when none
+  uint32_t m[CAFE_RES_MAX];    // ... and its CafeSlot::m
+  unsigned char k[CAFE_RES_MAX];     // ... and its place in the record
   unsigned char flag[CAFE_RES_MAX];  // CAFE_RF_*
   unsigned short free[CAFE_RES_MAX];
-  unsigned long long wk[CAFE_LOOP_THREADS / 32], thr[32];
-  double wd[CAFE_LOOP_THREADS / 32];
-  int wi[CAFE_LOOP_THREADS / 32], hist[32];
-  int top, nfree, newslot, overflow;
-  double newE;              // extent of the row that enters at newslot
-  unsigned long long klim;  // a smallest key below it needs no further test
+  // each warp's smallest candidate: key, index, row, position, slot, g - E
+  uint32_t wh[CAFE_WARPS], wm[CAFE_WARPS];
+  int wi[CAFE_WARPS], wr[CAFE_WARPS], wq[CAFE_WARPS], wf[CAFE_WARPS];
+  double wd[CAFE_WARPS];
+  unsigned long long wk[CAFE_WARPS], wrk[CAFE_WARPS], thr[32];  // full keys of the close ones
+  int hist[32];
+  int top, nfree, newslot, overflow, sink[32];
+  uint32_t klim[2];  // [e & 1]: a smallest key below it needs no further test at event e
   unsigned long long kw;    // rows with keys at or below it are resident
   double wlim, dsum_cap;    // latest safe T + t; the window holds while dsum <= dsum_cap and ev <= ev_cap
   int ev_cap, all;          // all: every row with a candidate is resident
-  CafeCand red[CAFE_LOOP_THREADS / 32];
+  CafeCand red[CAFE_WARPS];
 };
-#define CAFE_RF_NEAR 1   // the next live slot's g is within a relative 2^-19
+#define CAFE_RF_NEAR 1   // the next slot's g is within a relative 2^-19
 #define CAFE_RF_DYING 2  // no live slot is left: the row grew at this event for the last time
 
 // (smallest key, its lane's index) of a warp, in every lane: two redux steps
@@ -541,281 +610,526 @@ __device__ __forceinline__ unsigned long long cafe_warp_min_key(unsigned long lo
   src = __ffs(__ballot_sync(0xffffffffu, hi == mh && lo == ml)) - 1;
   return ((unsigned long long)mh << 32) | ml;
 }
+// Order key of the high word of a double, or of a float (exponent mask xm);
+// 0xffffffff for inf and NaN.
+__device__ __forceinline__ uint32_t cafe_key32(int hi, int xm) {
+  return (hi & xm) == xm ? 0xffffffffu : (uint32_t)(hi ^ ((hi >> 31) | (int)0x80000000));
+}
 
-// The first live slot of a row's record and whether the next one is close.
-__device__ __forceinline__ void cafe_res_first(const CafeDev &D, CafeResident &S, int i, int r, uint32_t live) {
+// Place k of the record of row r, resident index i, becomes its first slot;
+// place n: none is left.
+__device__ __forceinline__ void cafe_res_first(const CafeDev &D, CafeResident &S, int i, int r, int k) {
+  const int n = D.row_n[r];
   const CafeSlot *rec = D.row_slot + (long long)r * CAFE_NSLOT;
-  if (!live) {
+  // the slots from k on with their capture state, two at a time
+  CafeSlot a;
+  a.q = -1;
+  while (k < n) {
+    const CafeSlot x = rec[k], y = rec[min(k + 1, n - 1)];
+    const int ex = D.a_ev[x.q], ey = D.a_ev[y.q];
+    a = x;
+    if (ex == 0) break;
+    a = y;
+    ++k;
+    if (k < n && ey == 0) break;
+    ++k;
+  }
+  if (k >= n) {
     S.g[i] = NAN;
-    S.flag[i] = 0;
+    S.q[i] = -1;
+    S.flag[i] = CAFE_RF_DYING;
     return;
   }
-  const uint32_t rest = live & (live - 1);
-  const CafeSlot a = rec[__ffs(live) - 1];
-  const double g2 = rest ? rec[__ffs(rest) - 1].g : NAN;
+  // (a captured next slot may leave the flag set: that only costs a comparison)
+  const unsigned long long k1 = cafe_key_canon(a.g);
+  const unsigned long long k2 = k + 1 < n ? cafe_key_canon(rec[k + 1].g) : CAFE_KEY_NONE;
   S.g[i] = a.g;
   S.q[i] = a.q;
   S.m[i] = a.m;
-  const unsigned long long k1 = cafe_key_canon(a.g), k2 = cafe_key_canon(g2);
-  S.flag[i] = (rest && !cafe_is_nan(g2) && k2 - k1 < (1ULL << 33)) ? CAFE_RF_NEAR : 0;
+  S.rk[i] = a.rk;
+  S.k[i] = (unsigned char)k;
+  S.flag[i] = k2 - k1 < (1ULL << 33) ? CAFE_RF_NEAR : 0;
+}
+
+// A nucleation takes position icap (VoxelsCA.C:483-505).
+__device__ __noinline__ void cafe_nucleate(const CafeDev &D, const CafeConsts &K, CafeLoop &L, int icap) {
+  int ci, cj, ck;
+  cafe_cell_xyz(K, D.act[icap], ci, cj, ck);
+  if (L.ngrain < D.grain_cap) {
+    double q4[4];
+    cafe_sample_orientation(K, L.sdloc, q4);
+    double *c = D.cth + 4LL * L.ngrain;
+    for (int a = 0; a < 4; ++a) c[a] = q4[a];
+    cafe_rot_from_cth(c, D.rot + 9LL * L.ngrain);
+  } else {
+    atomicOr(D.err, CAFE_ERR_GRAIN_CAP);
+    L.done = 1;
+  }
+  L.ngrain += 1;
+  D.a_gid[icap] = L.nc.gid = L.ngrain;
+  D.a_cx[icap] = L.nc.c[0] = ((double)ci + .5) * K.dx[0];
+  D.a_cy[icap] = L.nc.c[1] = ((double)cj + .5) * K.dx[1];
+  D.a_cz[icap] = L.nc.c[2] = ((double)ck + .5) * K.dx[2];
+  L.sdloc += 10u;
+  D.a_ext[icap] = L.nc.ext = 0.0;
+  L.nnuc++;
+}
+
+// Keys within KC of each other may belong to equal times, or be out of order:
+// the high word resolves 2^-20; a single-precision time is good to 2^-22. Keys of
+// magnitudes at or below KTINY (2^-900, 2^-100) are all close to each other.
+template <bool PR>
+constexpr __host__ __device__ uint32_t cafe_kc() { return PR ? 16u : 2u; }
+template <bool PR>
+constexpr __host__ __device__ uint32_t cafe_ktiny() { return 0x80000000u | (PR ? 0x0d800000u : (1023u - 900u) << 20); }
+template <bool PR>
+constexpr __host__ __device__ int cafe_xm() { return PR ? 0x7f800000 : 0x7ff00000; }
+
+// The largest key that a winner at clock T may have and be the global one.
+template <bool PR>
+__device__ __forceinline__ uint32_t cafe_window_limit(const CafeResident &S, double V, double DelT, int ev, double T, double dsum) {
+    if (!S.all && !(ev < S.ev_cap && dsum <= S.dsum_cap)) return 0u;
+    double lim = fmin(S.wlim - T, 0x1.e847fp19) * (PR ? 1.0 : V);  // 0x1.e847fp19 < 1e6
+    lim = lim - fabs(lim) * 0x1p-18;
+    return PR ? cafe_key32(__float_as_int((float)lim), cafe_xm<PR>()) : cafe_key32(__double2hiint(lim), cafe_xm<PR>());
+}
+
+// The loop's rare parts, out of line: an event's chain pays for every
+// instruction line that the loop spreads over. They read the device state
+// from a copy in shared memory, so that the loop's own stays in constant memory.
+
+// Every resident's extent, place and (keys) key back to the row arrays.
+template <bool PR>
+__device__ __noinline__ void cafe_res_flush(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev, bool keys) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
+  const unsigned FULL = 0xffffffffu;
+  const double V = K.vhat_cls[1];
+  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
+  for (int i = tid; i < S.top; i += NT) {
+    const int r = S.r[i];
+    if (r < 0) continue;
+    D.row_E[r] = S.E[i];
+    D.row_m[r] = ev;
+    D.row_k[r] = S.k[i];
+    if (keys) {
+      const double t = (S.g[i] - S.E[i]) / (PR ? S.v[i] : V);
+      D.row_key[r] = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
+    }
+  }
+}
+
+// Row S.r[i] enters: its growth so far, its first live slot.
+template <bool PR>
+__device__ __noinline__ void cafe_load_resident(const CafeDev &D, const CafeConsts &K, CafeResident &S, int i, int ev) {
+  const int r = S.r[i];
+  double v = 0.0;
+  if (PR) {
+    v = cafe_vh(D, K, D.row_pos[r]);
+    S.v[i] = v;
+    S.rv[i] = 1.0f / (float)v;
+  }
+  int stop;
+  const double E = cafe_row_replayed<PR>(D, r, ev, v, stop);
+  S.E[i] = E;
+  cafe_res_first(D, S, i, r, D.row_k[r]);
+  if (S.flag[i] & CAFE_RF_DYING) {  // every neighbour is captured: not a candidate any more
+    D.row_E[r] = E;
+    D.row_m[r] = stop;
+    D.row_key[r] = CAFE_KEY_NONE;
+    S.flag[i] = 0;
+    S.r[i] = -1;
+    S.free[atomicAdd(&S.nfree, 1)] = (unsigned short)i;
+  } else {
+    D.row_m[r] = CAFE_M_DONE;  // until it is written back
+  }
+}
+
+// Opens the window: the earliest rows by key become resident.
+template <bool PR>
+__device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev, int tries) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
+  const unsigned FULL = 0xffffffffu;
+  const double V = K.vhat_cls[1];
+  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
+  cafe_res_flush<PR>(D, K, L, S, ev, true);
+  __syncthreads();
+  // the first window takes its rows from the list of those that are due
+  // soon (k_rows_order), later ones from all rows of the step
+  const bool first = ev == 0 && tries == 1 && D.ctr[CTR_NDUE] <= CAFE_DUE_MAX;
+  const int nrows0 = L.nrows0, nrows = first ? D.ctr[CTR_NDUE] : L.nrows;
+  auto row_at = [&](int k) -> int { return first ? D.row_due[k] : cafe_row_at(D, nrows0, k); };
+  unsigned long long mn = CAFE_KEY_NONE;
+  int cnt = 0;
+  for (int r0 = tid; r0 < nrows; r0 += 8 * NT) {
+    unsigned long long kk[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) kk[u] = r0 + u * NT < nrows ? D.row_key[row_at(r0 + u * NT)] : CAFE_KEY_NONE;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      mn = min(mn, kk[u]);
+      cnt += kk[u] != CAFE_KEY_NONE;
+    }
+  }
+  int src;
+  mn = cafe_warp_min_key(mn, src);
+  cnt = __reduce_add_sync(FULL, cnt);
+  if (lane == 0) {
+    S.wk[warp] = mn;
+    S.wi[warp] = cnt;
+  }
+  if (tid < 32) S.hist[tid] = 0;
+  for (int i = tid; i < CAFE_RES_MAX; i += NT) {
+    S.g[i] = NAN;
+    S.q[i] = S.r[i] = -1;
+    S.flag[i] = 0;
+  }
+  __syncthreads();
+  mn = cafe_warp_min_key(lane < NW ? S.wk[lane] : CAFE_KEY_NONE, src);
+  cnt = __reduce_add_sync(FULL, lane < NW ? S.wi[lane] : 0);
+  // the rows that are not listed have keys above this bound
+  const unsigned long long kdue = first && D.ctr[CTR_NKEY] > cnt ? cafe_key(K.DelT * CAFE_DUE_REACH) : CAFE_KEY_NONE - 1;
+  const bool all = cnt <= CAFE_RES_TARGET;
+  // rounding bound of the keys for the next 4096 events and 64 DelT of growth
+  const double dcap = L.dsum + 64.0 * K.DelT;
+  const double base = (mn == CAFE_KEY_NONE ? 0.0 : cafe_unkey(mn));
+  const double slack = (double)(ev + 4096 + 16) * 0x1p-47 *
+                       (fabs(base) + 64.0 * K.DelT + fabs(L.tinc) + 2.0 * dcap +
+                        (L.gmax + L.emax) / (PR ? L.vmin : V) + 1e-300);
+  int pick = 31;
+  if (!all) {
+    if (tid < 32) {
+      // thresholds in steps of a factor sqrt(2), DelT/1024 .. 45 DelT beyond the smallest key
+      const double f = (tid & 1) ? 1.4142135623730951 : 1.0;
+      const double wj = base + 4.0 * slack + K.DelT * (f * crm_from_bits((long long)(1023 - 10 + (tid >> 1)) << 52));
+      S.thr[tid] = cafe_is_nan(wj) ? CAFE_KEY_NONE - 1 : cafe_key(wj);
+    }
+    __syncthreads();
+    const unsigned long long last = S.thr[31];
+    for (int r = tid; r < nrows; r += NT) {
+      const unsigned long long k = D.row_key[row_at(r)];
+      if (k > last) continue;
+      int lo = 0, hi = 31;  // first threshold at or above the key
+      while (lo < hi) {
+        const int md = (lo + hi) >> 1;
+        if (k <= S.thr[md]) hi = md; else lo = md + 1;
+      }
+      atomicAdd(&S.hist[lo], 1);
+    }
+    __syncthreads();
+    int h = S.hist[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(FULL, h, o);
+      if (lane >= o) h += u;
+    }
+    const uint32_t fits = __ballot_sync(FULL, h <= CAFE_RES_TARGET);
+    // the counts ascend: the last threshold that fits the target, else the first if it fits at all
+    pick = fits ? 31 - __clz(fits) : 0;
+    const int n0 = __shfl_sync(FULL, h, 0);
+    if (tid == 0) S.overflow = !fits && n0 > CAFE_RES_MAX - 64;
+  }
+  const unsigned long long kw = min(kdue, all ? CAFE_KEY_NONE - 1 : S.thr[pick]);
+  const bool every = kw == CAFE_KEY_NONE - 1;
+  if (tid == 0) {
+    if (all) S.overflow = 0;
+    if (!every && !(cafe_unkey(kw) < 1e300)) S.overflow = 1;
+    if (!(slack < 1e300) || tries >= CAFE_OPEN_TRIES) S.overflow = 1;
+    S.kw = kw;
+    S.all = every;
+    S.top = 0;
+    S.nfree = 0;
+    S.ev_cap = ev + 4096;
+    S.dsum_cap = dcap;
+    S.wlim = every ? INFINITY : cafe_unkey(kw) - slack;
+    L.opens++;
+    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, L.dsum);
+  }
+  __syncthreads();
+  if (S.overflow) return;
+  for (int k = tid; k < nrows; k += NT) {
+    const int r = row_at(k);
+    if (D.row_key[r] <= kw) {
+      const int i = atomicAdd(&S.top, 1);
+      if (i < CAFE_RES_MAX) S.r[i] = r;
+    }
+  }
+  __syncthreads();
+  {
+    const int top = S.top;
+    for (int i = tid; i < top; i += NT) cafe_load_resident<PR>(D, K, S, i, ev);
+  }
+  __syncthreads();
+}
+
+// Exact candidates of the rows with keys at or below kthr, the reference's order
+// among them; the best one is left in S.red[0].
+template <bool PR>
+__device__ __noinline__ void cafe_select_exact(const CafeDev &D, const CafeConsts &K, CafeResident &S, uint32_t kthr) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
+  const unsigned FULL = 0xffffffffu;
+  const double V = K.vhat_cls[1];
+  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
+  CafeCand wc = cafe_cand_none();
+  const int top = S.top;
+  for (int i = tid; i < top; i += NT) {
+    const double d = S.g[i] - S.E[i];
+    const uint32_t k = cafe_key32(PR ? __float_as_int((float)d * S.rv[i]) : __double2hiint(d), cafe_xm<PR>());
+    if (k <= kthr && k != 0xffffffffu) cafe_row_best(D, S.r[i], S.E[i], PR ? S.v[i] : V, S.k[i], wc);
+  }
+  wc = cafe_warp_best(wc);
+  if (lane == 0) S.red[warp] = wc;
+  __syncthreads();
+  if (warp == 0) {
+    wc = cafe_warp_best(lane < NW ? S.red[lane] : cafe_cand_none());
+    __syncwarp();
+    if (lane == 0) S.red[0] = wc;
+  }
+  __syncthreads();
+}
+
+// A negative event may clamp a small extent at zero (VoxelsCA.C:515),
+// which breaks the key bound of a row outside the set: the rows whose
+// extrapolated extent comes near zero are brought up to date with a new key
+// (true: one of them may be due before the window's end).
+template <bool PR>
+__device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
+  const unsigned FULL = 0xffffffffu;
+  const double V = K.vhat_cls[1];
+  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
+  const double vd = L.vd, vsp = D.ev_vs[ev - 1], vx = PR ? L.vmax : V;
+  const double margin = (double)(ev + 16) * 0x1p-48 * (L.emax + L.gmax + vx * L.dsum + 1e-300);
+  // rows that still hold the step's first extents (row_m 0, nearly all) have
+  // grown by the whole running sum: they are decided by one threshold
+  const double g0 = vsp + vd;
+  const double need = PR ? (g0 >= 0.0 ? margin - g0 * L.vmin : margin - g0 * L.vmax) : margin - g0;
+  const long long thr0 = need > 0.0 ? crm_bits(need * (1.0 + 0x1p-40)) : 0;
+  bool again = false;
+  const int nrows = L.nrows, nrows0 = L.nrows0;
+  for (int k0 = tid; k0 < nrows; k0 += 8 * NT) {
+    int rr[8], mm[8];
+    uint32_t todo = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) rr[u] = k0 + u * NT < nrows ? cafe_row_at(D, nrows0, k0 + u * NT) : -1;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) mm[u] = rr[u] >= 0 ? D.row_m[rr[u]] : ev;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (mm[u] < ev && (mm[u] != 0 || thr0 > 0)) todo |= 1u << u;
+    if (todo) {
+      long long eb[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) eb[u] = todo >> u & 1u ? crm_bits(D.row_E[rr[u]]) : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (mm[u] == 0 && eb[u] >= thr0) todo &= ~(1u << u);  // (NaN too: it never captures)
+    }
+    for (; todo; todo &= todo - 1) {
+    int r = 0, m = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (u == __ffs(todo) - 1) {
+        r = rr[u];
+        m = mm[u];
+      }
+    const double v = PR ? cafe_vh(D, K, D.row_pos[r]) : V;
+    const double gr = (vsp - D.ev_vs[m]) + vd;
+    if (D.row_E[r] + (PR ? v * gr : gr) >= margin) continue;
+    int stop;
+    const double En = cafe_row_replayed<PR>(D, r, ev, v, stop);
+    D.row_E[r] = En;
+    D.row_m[r] = stop < ev ? CAFE_M_DONE : ev;  // (a row that stopped growing keeps its extent)
+    const int k = cafe_row_next(D, r, D.row_k[r]);
+    D.row_k[r] = (uint8_t)k;
+    if (k < D.row_n[r]) {
+      const double t = (D.row_slot[(long long)r * CAFE_NSLOT + k].g - En) / v;
+      const unsigned long long key = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
+      D.row_key[r] = key;
+      again = again || key <= S.kw;
+    }
+    }
+  }
+  return __syncthreads_or(again);
+}
+
+// The captured cell's own row when it was not foreseen, or found no room in the
+// resident set (true: open a new window).
+template <bool PR>
+__device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, CafeQuadScratch &Q, int ev, int icap) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
+  const unsigned FULL = 0xffffffffu;
+  const double V = K.vhat_cls[1];
+  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
+  const int nr = L.newrow;
+  if (!L.fill) {
+    if (tid == 0) {
+      D.row_E[nr] = L.nc.ext;
+      const int k = cafe_row_next(D, nr, 0);
+      const double t = (D.row_slot[(long long)nr * CAFE_NSLOT + k].g - L.nc.ext) / (PR ? cafe_vh(D, K, icap) : V);
+      D.row_key[nr] = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
+    }
+    __syncthreads();
+    return true;
+  }
+  __syncthreads();
+  if (warp < CAFE_QUAD_THREADS / 32) {
+    const CafeChildList none = {nullptr, 0, 0, 0.0};
+    const unsigned long long gk = cafe_row_fill_quad(D, K, nr, icap, L.tinc, Q, L.nc, none);
+    if (tid == 0) {
+      D.row_E[nr] = L.nc.ext;
+      if (gk != 0ULL) L.gmax = fmax(L.gmax, cafe_unkey(gk));
+      if (!cafe_is_nan(L.nc.ext)) L.emax = fmax(L.emax, fabs(L.nc.ext));
+      int i = -1;
+      if (S.nfree > 0) i = S.free[--S.nfree];
+      else if (S.top < CAFE_RES_MAX) i = S.top++;
+      S.newslot = i;
+      if (i >= 0) S.r[i] = nr;
+    }
+  }
+  __syncthreads();
+  const int i = S.newslot;
+  if (i >= 0 && i % NT == tid) cafe_load_resident<PR>(D, K, S, i, ev);
+  __syncthreads();
+  return i < 0;
 }
 
 // Keyed loop over the resident set; every thread of the block calls it. Leaves
 // with L.done set, or with L.sw set when the step must continue with the full
-// scan (every row's extent and live mask are then in the row arrays).
+// scan (every row's extent and place are then in the row arrays).
 template <bool PR>
 __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const CafeConsts &K, long long max_events,
-                                                     CafeLoop &L, CafeResident &S, CafeQuadScratch &Q) {
+                                                     CafeLoop &L, CafeResident &S, CafeQuadScratch &Q,
+                                                     const CafeDev &sD, const CafeConsts &sK) {
   const unsigned FULL = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_LOOP_THREADS / 32;
   const double V = K.vhat_cls[1];
-  // key distance within which two approximate values may belong to equal times:
-  // a few ulps of g - E; with PR the value is (g - E) times a reciprocal good
-  // to about 2^-44
-  const unsigned long long TOL = PR ? (1ULL << 14) : 8ULL;
-  const unsigned long long KTINY = cafe_key(0x1p-900);
-  double E[CAFE_RES_PER], rv[CAFE_RES_PER];
-#pragma unroll
-  for (int c = 0; c < CAFE_RES_PER; ++c) E[c] = rv[c] = 0.0;
+  constexpr uint32_t KC = cafe_kc<PR>(), KTINY = cafe_ktiny<PR>();
+  constexpr int XM = cafe_xm<PR>();
   int ev = 0;
   int tries = 0;  // windows opened since the last event
   bool need_open = true;
   if (tid == 0) S.top = 0;
   __syncthreads();
   long long t0 = clock64();
-  // every resident's extent, live mask and key back to the row arrays
-  auto flush = [&](bool keys) {
-#pragma unroll
-    for (int c = 0; c < CAFE_RES_PER; ++c) {
-      const int i = tid + c * NT;
-      if (i >= S.top || S.r[i] < 0) continue;
-      const int r = S.r[i];
-      D.row_E[r] = E[c];
-      D.row_m[r] = ev;
-      D.row_live[r] = S.live[i];
-      D.row_res[r] = -1;
-      if (keys) {
-        const double t = (S.g[i] - E[c]) / (PR ? S.v[i] : V);
-        D.row_key[r] = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
-      }
-    }
-  };
-  auto load_resident = [&](int c, int i) {
-    const int r = S.r[i];
-    const uint32_t live = D.row_live[r];
-    double v = 0.0;
-    if (PR) {
-      v = cafe_vh(D, K, D.row_pos[r]);
-      S.v[i] = v;
-      rv[c] = 1.0 / v;
-    }
-    int stop;
-    E[c] = cafe_row_replayed<PR>(D, r, ev, v, stop);
-    S.live[i] = live;
-    cafe_res_first(D, S, i, r, live);
-    D.row_res[r] = i;
-  };
+  const double rV = 1.0 / V;
+  int cnv = L.nvs2, cnr = L.nrows;  // (capturing warp) list and row counts
   while (true) {
     if (need_open) {
       // ---- open the window: the earliest rows by key
       need_open = false;
       ++tries;
-      flush(true);
-      __syncthreads();
-      const int nrows = L.nrows, nrows0 = L.nrows0;
-      unsigned long long mn = CAFE_KEY_NONE;
-      int cnt = 0;
-      for (int r0 = tid; r0 < nrows; r0 += 8 * NT) {
-        unsigned long long kk[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) kk[u] = r0 + u * NT < nrows ? D.row_key[cafe_row_at(D, nrows0, r0 + u * NT)] : CAFE_KEY_NONE;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          mn = min(mn, kk[u]);
-          cnt += kk[u] != CAFE_KEY_NONE;
-        }
-      }
-      int src;
-      mn = cafe_warp_min_key(mn, src);
-      cnt = __reduce_add_sync(FULL, cnt);
-      if (lane == 0) {
-        S.wk[warp] = mn;
-        S.wi[warp] = cnt;
-      }
-      if (tid < 32) S.hist[tid] = 0;
-      __syncthreads();
-      mn = cafe_warp_min_key(lane < NW ? S.wk[lane] : CAFE_KEY_NONE, src);
-      cnt = __reduce_add_sync(FULL, lane < NW ? S.wi[lane] : 0);
-      const bool all = cnt <= CAFE_RES_TARGET;
-      // rounding bound of the keys for the next 4096 events and 64 DelT of growth
-      const double dcap = L.dsum + 64.0 * K.DelT;
-      const double base = (mn == CAFE_KEY_NONE ? 0.0 : cafe_unkey(mn));
-      const double slack = (double)(ev + 4096 + 16) * 0x1p-47 *
-                           (fabs(base) + 64.0 * K.DelT + fabs(L.tinc) + 2.0 * dcap +
-                            (L.gmax + L.emax) / (PR ? L.vmin : V) + 1e-300);
-      int pick = 31;
-      if (!all) {
-        if (tid < 32) {
-          // thresholds in steps of a factor sqrt(2), DelT/1024 .. 45 DelT beyond the smallest key
-          const double f = (tid & 1) ? 1.4142135623730951 : 1.0;
-          const double wj = base + 4.0 * slack + K.DelT * (f * crm_from_bits((long long)(1023 - 10 + (tid >> 1)) << 52));
-          S.thr[tid] = cafe_is_nan(wj) ? CAFE_KEY_NONE - 1 : cafe_key(wj);
-        }
-        __syncthreads();
-        const unsigned long long last = S.thr[31];
-        for (int r = tid; r < nrows; r += NT) {
-          const unsigned long long k = D.row_key[cafe_row_at(D, nrows0, r)];
-          if (k > last) continue;
-          int lo = 0, hi = 31;  // first threshold at or above the key
-          while (lo < hi) {
-            const int md = (lo + hi) >> 1;
-            if (k <= S.thr[md]) hi = md; else lo = md + 1;
-          }
-          atomicAdd(&S.hist[lo], 1);
-        }
-        __syncthreads();
-        int h = S.hist[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(FULL, h, o);
-          if (lane >= o) h += u;
-        }
-        const uint32_t fits = __ballot_sync(FULL, h <= CAFE_RES_TARGET);
-        // the counts ascend: the last threshold that fits the target, else the first if it fits at all
-        pick = fits ? 31 - __clz(fits) : 0;
-        const int n0 = __shfl_sync(FULL, h, 0);
-        if (tid == 0) S.overflow = !fits && n0 > CAFE_RES_MAX - 64;
-      }
-      const unsigned long long kw = all ? CAFE_KEY_NONE - 1 : S.thr[pick];
-      if (tid == 0) {
-        if (all) S.overflow = 0;
-        if (!(slack < 1e300) || tries >= CAFE_OPEN_TRIES) S.overflow = 1;
-        S.kw = kw;
-        S.all = all;
-        S.top = 0;
-        S.nfree = 0;
-        S.ev_cap = ev + 4096;
-        S.dsum_cap = dcap;
-        S.wlim = all ? INFINITY : cafe_unkey(kw) - slack;
-        L.opens++;
-        // the bound of the next winner's key
-        const double v = PR ? 1.0 : V;
-        const double lim = fmin(S.wlim - L.tinc, 0x1.e847fp19) * v;  // 0x1.e847fp19 < 1e6
-        S.klim = cafe_key(lim - fabs(lim) * 0x1p-30);
-      }
-      __syncthreads();
-      if (S.overflow) {
-        if (tid == 0) L.sw = 1;
-        __syncthreads();
-        break;
-      }
-      for (int k = tid; k < nrows; k += NT) {
-        const int r = cafe_row_at(D, nrows0, k);
-        if (D.row_key[r] <= kw) {
-          const int i = atomicAdd(&S.top, 1);
-          if (i < CAFE_RES_MAX) S.r[i] = r;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < CAFE_RES_PER; ++c) {
-        const int i = tid + c * NT;
-        if (i < S.top) load_resident(c, i);
-      }
-      __syncthreads();
+      cafe_window_open<PR>(sD, sK, L, S, ev, tries);
       if (tid == 0) {
         const long long t1 = clock64();
         L.cyc[3] += t1 - t0;
         t0 = t1;
       }
+      if (S.overflow) {
+        if (tid == 0) L.sw = 1;
+        __syncthreads();
+        break;
+      }
     }
     // ---- select: the smallest (g - E) / v over the resident rows
-    unsigned long long kk[CAFE_RES_PER], bk = CAFE_KEY_NONE;
+    uint32_t bk = 0xffffffffu, b2 = 0xffffffffu;  // this thread's smallest and second smallest keys
     double bd = 0.0;
     int bi = -1;
-    const int top = S.top;
-#pragma unroll
-    for (int c = 0; c < CAFE_RES_PER; ++c) {
-      const int i = tid + c * NT;
-      kk[c] = CAFE_KEY_NONE;
-      if (i < top && S.r[i] >= 0) {
-        const double d = S.g[i] - E[c];
-        const double x = PR ? d * rv[c] : d;
-        if (!cafe_is_nan(x)) kk[c] = cafe_key_canon(x);
-        if (kk[c] < bk) {
-          bk = kk[c];
+    {
+      const int top = S.top;
+      for (int i = tid; i < top; i += NT) {  // (g is NaN where no row is)
+        const double d = S.g[i] - S.E[i];
+        const uint32_t k = cafe_key32(PR ? __float_as_int((float)d * S.rv[i]) : __double2hiint(d), XM);
+        b2 = min(b2, max(k, bk));
+        if (k < bk) {
+          bk = k;
           bd = d;
           bi = i;
         }
       }
     }
-    int src;
     {
-      const unsigned long long wm = cafe_warp_min_key(bk, src);
-      if (lane == src) {
-        S.wk[warp] = wm;
-        S.wi[warp] = bi;
-        S.wd[warp] = bd;
+      const uint32_t wmin = __reduce_min_sync(FULL, bk);
+      const uint32_t thr = wmin + KC;
+      const uint32_t cl = wmin == 0xffffffffu ? 0u : __ballot_sync(FULL, bk <= thr);
+      if (cl == 0u) {
+        if (lane == 0) S.wh[warp] = wmin;
+      } else {
+        int lead = __ffs(cl) - 1;
+        // a candidate's own next slot: g apart by 2^-19 relative cannot round
+        // together unless the extent dwarfs g
+        bool hard = false;
+        unsigned long long kf = CAFE_KEY_NONE;
+        if (bk <= thr) {
+          const int ed = (__double2hiint(bd) >> 20) & 0x7ff, eg = (__double2hiint(S.g[bi]) >> 20) & 0x7ff;
+          hard = S.flag[bi] || ed > eg + 20 || b2 <= thr;
+          kf = cafe_key_canon(bd);
+        }
+        if (cl & (cl - 1u)) {
+          // several close ones: by g - E, then by ruqs (equal g - E gives equal
+          // times); apart by less than the division's rounding, or equal in
+          // both: undecided here
+          const unsigned long long k1 = cafe_warp_min_key(kf, lead);
+          const unsigned long long rf = kf == k1 ? S.rk[bi] : CAFE_KEY_NONE;
+          const unsigned long long r1 = cafe_warp_min_key(rf, lead);
+          const uint32_t eq = __ballot_sync(FULL, kf == k1 && rf == r1);
+          hard = __any_sync(FULL, hard || (kf != k1 && kf - k1 < 8)) || (eq & (eq - 1u)) || PR;
+        }
+        if (lane == lead) {
+          S.wh[warp] = wmin;
+          S.wf[warp] = hard;
+          S.wd[warp] = bd;
+          S.wk[warp] = kf;
+          S.wrk[warp] = S.rk[bi];
+          S.wi[warp] = bi;
+          S.wr[warp] = S.r[bi];
+          S.wq[warp] = S.q[bi];
+          S.wm[warp] = S.m[bi];
+        }
       }
     }
     __syncthreads();
-    const unsigned long long kmin = cafe_warp_min_key(lane < NW ? S.wk[lane] : CAFE_KEY_NONE, src);
-    const int win = S.wi[src];
-    const double wd = S.wd[src];
-    // (read before the next barrier: the captures change them after it)
-    int wr = -1, wq = 0, ws = 0, child = -1;
-    if (kmin != CAFE_KEY_NONE) {
-      wr = S.r[win];
-      wq = S.q[win];
-      ws = (int)(S.m[win] & 31u);
-      child = cafe_slot_child(S.m[win]);
-    }
-    // another candidate within the rounding of the division?
-    bool tie = false;
-    if (kmin != CAFE_KEY_NONE) {
-      unsigned long long thr = kmin + TOL;
-      const int ex = (int)((crm_bits(cafe_unkey(kmin)) >> 52) & 0x7ff);
-      if (ex < 1023 - 900) thr = KTINY;  // zero or tiny: times may round together
-      bool close = false;
-#pragma unroll
-      for (int c = 0; c < CAFE_RES_PER; ++c) {
-        const int i = tid + c * NT;
-        if (kk[c] <= thr) {
-          if (i != win) {
-            close = true;
-          } else {
-            // its own next slot: g apart by 2^-19 relative cannot round together
-            // unless the extent dwarfs g
-            const int ed = (int)((crm_bits(wd) >> 52) & 0x7ff), eg = (int)((crm_bits(S.g[i]) >> 52) & 0x7ff);
-            close = close || (S.flag[i] & CAFE_RF_NEAR) || ed > eg + 20 || thr == KTINY;
-          }
-        }
+    const uint32_t wkey = lane < NW ? S.wh[lane] : 0xffffffffu;
+    const uint32_t kmin = __reduce_min_sync(FULL, wkey);
+    const bool inside = kmin < S.klim[(ev + 1) & 1];
+    const uint32_t wcl = __ballot_sync(FULL, wkey <= kmin + KC && wkey != 0xffffffffu);
+    const uint32_t kmag = kmin & 0x80000000u ? kmin : ~kmin;  // key of the magnitude
+    int src = __ffs(wcl | 0x80000000u) - 1;
+    bool exact = !inside || kmag <= KTINY;
+    if (!exact) {
+      if (wcl & (wcl - 1u)) {  // several warps' candidates are close: likewise among them
+        const bool c = wcl >> lane & 1u;
+        const unsigned long long kf = c ? S.wk[lane] : CAFE_KEY_NONE;
+        const unsigned long long k1 = cafe_warp_min_key(kf, src);
+        const unsigned long long rf = kf == k1 ? S.wrk[lane] : CAFE_KEY_NONE;
+        const unsigned long long r1 = cafe_warp_min_key(rf, src);
+        const uint32_t eq = __ballot_sync(FULL, kf == k1 && rf == r1);
+        exact = __any_sync(FULL, c && (S.wf[lane] || (kf != k1 && kf - k1 < 8))) || (eq & (eq - 1u)) || PR;
+      } else {
+        exact = S.wf[src];
       }
-      tie = __syncthreads_or(close);
     }
-    const bool plain = kmin != CAFE_KEY_NONE && !tie && kmin < S.klim;
+    src &= NW - 1;
+    const double wd = S.wd[src];
+    const int win = S.wi[src];
+    int wr = S.wr[src], wq = S.wq[src];
+    uint32_t wm = S.wm[src];
     CafeCand wc = cafe_cand_none();
-    if (!plain) {
-      if (!S.all && !(kmin < S.klim)) {  // beyond the window (or nothing in it)
+    if (exact) {
+      if (!S.all && !inside) {  // beyond the window (or nothing in it)
         __syncthreads();
         need_open = true;
         continue;
       }
       // exact candidates of the close rows, the reference's order among them
-      if (kmin != CAFE_KEY_NONE) {
-        const int ex = (int)((crm_bits(cafe_unkey(kmin)) >> 52) & 0x7ff);
-        const unsigned long long thr = ex < 1023 - 900 ? KTINY : kmin + TOL;
-#pragma unroll
-        for (int c = 0; c < CAFE_RES_PER; ++c) {
-          const int i = tid + c * NT;
-          if (kk[c] <= thr) cafe_row_best(D, S.r[i], E[c], PR ? S.v[i] : V, S.live[i], wc);
-        }
-        wc = cafe_warp_best(wc);
-        if (lane == 0) S.red[warp] = wc;
-        __syncthreads();
-        wc = cafe_warp_best(lane < NW ? S.red[lane] : cafe_cand_none());
-        __syncthreads();
-      }
+      const uint32_t kthr = kmag > KTINY ? kmin + KC : max(kmin + KC, KTINY);
+      if (kmin != 0xffffffffu) cafe_select_exact<PR>(sD, sK, S, kthr);
+      wc = kmin != 0xffffffffu ? S.red[0] : cafe_cand_none();
+      __syncthreads();
       if (wc.j < 0 || !(wc.tk < CAFE_KEY_1E6)) {  // no candidate is left
         if (tid == 0) L.done = 1;
         __syncthreads();
@@ -823,8 +1137,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       }
       wr = wc.r;
       wq = wc.q;
-      ws = wc.s;
-      child = wc.child;
+      wm = wc.m;
     }
     if (ev >= max_events) {
       if (tid == 0) {
@@ -842,160 +1155,115 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       t0 = t1;
     }
     // ---- apply the event
-    const int icap = wq;
+    const int icap = wq, child = cafe_slot_child(wm);
     if (warp == CAFE_CAP_WARP) {
-      const int p = D.row_pos[wr];
-      const bool cold = D.a_cold[icap] != 0;
-      const int cls = D.a_cls[icap];
-      const bool nuc = L.unext[ev & 1] < cafe_nuc_rate_at(D, K, icap);
-      // level 1: the neighbours; the capture result of this slot (lanes 26-29:
-      // extent and centre, computed when the row was filled) and the grain
-      int q = -1, gcap = 0;
+      // level 1: the foreseen row's record (lane = place); the capture result of
+      // this slot (lanes 26-29: extent and centre, computed when the row was
+      // filled) and the grain
+      int gcap = 0, cn = 0;
       double gx = 0.0;
-      if (lane < CAFE_NSLOT) q = D.a_nbr[(long long)icap * CAFE_NSLOT + lane];
-      else if (lane < 30) gx = D.row_geo[((long long)wr * CAFE_NSLOT + ws) * 4 + lane - 26];
-      else if (lane == 30) gcap = D.a_gid[p];
-      // ... and the foreseen row's record
       CafeSlot cr;
       cr.g = NAN;
+      cr.rk = CAFE_KEY_NONE;
       cr.q = -1;
       cr.m = 0;
-      int crk = 0;
+      const bool nuc = L.unext[ev & 1] < cafe_nuc_rate_at(D, K, icap);
       const bool foreseen = child >= 0 && !nuc;
-      if (foreseen && lane < CAFE_NSLOT) {
-        cr = D.row_slot[(long long)child * CAFE_NSLOT + lane];
-        crk = D.row_rank[(long long)child * 32 + lane];
+      if (foreseen) {
+        cn = D.row_n[child];
+        if (lane < CAFE_NSLOT) cr = D.row_slot[(long long)child * CAFE_NSLOT + lane];
       }
-      // level 2
-      int st = 0, fr = -1;
-      if (q >= 0) {
-        st = D.a_state[q];
-        fr = D.a_frow[q];
+      if (lane >= CAFE_NSLOT && lane < 30) gx = D.row_geo[((long long)wr * CAFE_NSLOT + (wm & 31u)) * 4 + lane - 26];
+      if (lane == 30) gcap = D.a_gid[D.row_pos[wr]];
+      const bool cold = D.a_cold[icap] != 0;
+      const int cls = D.a_cls[icap];
+      const double vq = PR ? cafe_vh(D, K, icap) : V;
+      // level 2: which of its neighbours (all but the captured ones) are left
+      bool left = false;
+      if (foreseen) {
+        left = lane < cn && D.a_ev[cr.q] == 0;
+      } else if (lane < CAFE_NSLOT) {
+        const int q = D.a_nbr[(long long)icap * CAFE_NSLOT + lane];
+        left = q >= 0 && D.a_state[q] == 1;
       }
-      const uint32_t clive = __reduce_or_sync(FULL, st == 1 ? 1u << crk : 0u);
-      const bool grows = clive != 0u && cold;
-      // a foreseen row enters the resident set at once (its neighbours that were
-      // captured meanwhile are no longer live)
+      const uint32_t clive = __ballot_sync(FULL, left);
+      const bool grows = clive != 0u && cold, room = cnr < D.row_cap;
+      const int row = foreseen ? child : cnr;
+      // the captured cell's own row: a foreseen one enters the resident set at once
       int ci = -1;
-      if (foreseen && grows) {
-        if (lane == 0) {
-          if (S.nfree > 0) ci = S.free[--S.nfree];
-          else if (S.top < CAFE_RES_MAX) ci = S.top++;
+      if (grows && foreseen && room) {
+        const int nf = S.nfree, tp = S.top;
+        __syncwarp();
+        if (nf > 0) {
+          ci = S.free[nf - 1];
+          if (lane == 0) S.nfree = nf - 1;
+        } else if (tp < CAFE_RES_MAX) {
+          ci = tp;
+          if (lane == 0) S.top = tp + 1;
         }
-        ci = __shfl_sync(FULL, ci, 0);
-        const uint32_t rest = clive & (clive - 1u);
-        const int k1 = __ffs(clive) - 1, k2 = rest ? __ffs(rest) - 1 : 31;
-        const double g2 = __shfl_sync(FULL, cr.g, k2);  // (lane 31: NaN)
+        const int k1 = __ffs(clive) - 1;
+        const double g2 = __shfl_sync(FULL, cr.g, k1 + 1);
         if (ci >= 0) {
           if (lane == k1) {
+            const unsigned long long d2 = k1 + 1 < cn ? cafe_key_canon(g2) - cafe_key_canon(cr.g) : CAFE_KEY_NONE;
             S.g[ci] = cr.g;
             S.q[ci] = cr.q;
             S.m[ci] = cr.m;
-            S.live[ci] = clive;
-            S.flag[ci] = (!cafe_is_nan(g2) && cafe_key_canon(g2) - cafe_key_canon(cr.g) < (1ULL << 33)) ? CAFE_RF_NEAR : 0;
+            S.rk[ci] = cr.rk;
+            S.k[ci] = (unsigned char)k1;
+            S.flag[ci] = d2 < (1ULL << 33) ? CAFE_RF_NEAR : 0;
             S.r[ci] = child;
-            if (PR) S.v[ci] = cafe_vh(D, K, icap);
-          }
-          if (lane == 26) S.newE = gx;
-        } else if (lane == 0) {
-          D.row_live[child] = clive;
-        }
-      }
-      if (lane == 0) S.newslot = ci;
-      // level 3: the neighbours' rows
-      if (fr >= 0) {
-        const int rs = D.row_res[fr];
-        const uint32_t lg = D.row_live[fr];
-        const int rk = D.row_rank[(long long)fr * 32 + (CAFE_NSLOT - 1 - lane)];
-        const uint32_t live = rs >= 0 ? S.live[rs] : lg;
-        const uint32_t bit = 1u << rk;
-        if (live & bit) {
-          const uint32_t nl = live & ~bit;
-          if (rs >= 0) {
-            S.live[rs] = nl;
-            if (!nl) {
-              S.g[rs] = NAN;
-              S.flag[rs] = CAFE_RF_DYING;
-              D.row_death[fr] = ev;  // it grew at this event too
-            } else if ((live & (bit - 1u)) == 0u) {
-              cafe_res_first(D, S, rs, fr, nl);
-            }
-          } else {
-            D.row_live[fr] = nl;
-            if (!nl) {
-              D.row_death[fr] = ev;
-              D.row_key[fr] = CAFE_KEY_NONE;
+            if (PR) {
+              S.v[ci] = vq;
+              S.rv[ci] = 1.0f / (float)vq;
             }
           }
+          if (lane == 26) S.E[ci] = gx;
         }
       }
       // the captured cell (VoxelsCA.C:483-505 and 518-605)
       if (nuc) {
-        if (lane == 0) {
-          int ci, cj, ck;
-          cafe_cell_xyz(K, D.act[icap], ci, cj, ck);
-          if (L.ngrain < D.grain_cap) {
-            double q4[4];
-            cafe_sample_orientation(K, L.sdloc, q4);
-            double *cc = D.cth + 4LL * L.ngrain;
-            for (int a = 0; a < 4; ++a) cc[a] = q4[a];
-            cafe_rot_from_cth(cc, D.rot + 9LL * L.ngrain);
-          } else {
-            atomicOr(D.err, CAFE_ERR_GRAIN_CAP);
-            L.done = 1;
-          }
-          L.ngrain += 1;
-          D.a_gid[icap] = L.nc.gid = L.ngrain;
-          D.a_cx[icap] = L.nc.c[0] = ((double)ci + .5) * K.dx[0];
-          D.a_cy[icap] = L.nc.c[1] = ((double)cj + .5) * K.dx[1];
-          D.a_cz[icap] = L.nc.c[2] = ((double)ck + .5) * K.dx[2];
-          L.sdloc += 10u;
-          D.a_ext[icap] = L.nc.ext = 0.0;
-          L.nnuc++;
+        if (lane == 0) cafe_nucleate(sD, sK, L, icap);
+      } else if (lane >= 26) {
+        // (one store each: the destination by lane)
+        double *gd = lane == 26 ? D.a_ext : lane == 27 ? D.a_cx : lane == 28 ? D.a_cy : D.a_cz;
+        double *sd = lane == 26 ? &L.nc.ext : &L.nc.c[(lane - 27) & 3];
+        if (lane < 30) {
+          gd[icap] = gx;
+          *sd = gx;
+          if (lane == 26 && fabs(gx) == INFINITY) L.sw = 1;  // its times need the full scan
+        } else if (lane == 30) {
+          D.a_gid[icap] = gcap;
+          L.nc.gid = gcap;
         }
-      } else if (lane == 26) {
-        D.a_ext[icap] = L.nc.ext = gx;
-        if (fabs(gx) == INFINITY) L.sw = 1;  // its times need the full scan
-      } else if (lane == 27) {
-        D.a_cx[icap] = L.nc.c[0] = gx;
-      } else if (lane == 28) {
-        D.a_cy[icap] = L.nc.c[1] = gx;
-      } else if (lane == 29) {
-        D.a_cz[icap] = L.nc.c[2] = gx;
-      } else if (lane == 30) {
-        D.a_gid[icap] = L.nc.gid = gcap;
       }
       if (lane == 31) {
         D.a_state[icap] = 2;
-        if (L.nvs2 < D.vs2_cap) {
-          D.vs2[L.nvs2] = icap;
+        D.a_ev[icap] = ev;
+        if (cnv < D.vs2_cap) {
+          D.vs2[cnv] = icap;
         } else {
           atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
           L.done = 1;
         }
-        L.countS = L.nvs2;
-        L.nvs2 += 1;
-        L.newrow = -1;
+        L.newrow = grows && room ? row : -1;
+        L.fill = !foreseen;
+        S.newslot = ci;
         if (grows) {
-          const int k = L.nrows;
-          if (k < D.row_cap) {
-            const int r = foreseen ? child : k;
-            D.row_pos[r] = icap;
-            D.row_j[r] = L.nvs2 - 1;
-            D.row_res[r] = ci;
-            D.a_frow[icap] = r;
-            D.row_death[r] = CAFE_ALIVE;
-            D.row_m[r] = ev;
-            D.row_new[k - L.nrows0] = r;
-            L.nrows = k + 1;
-            L.newrow = r;
-            L.fill = !foreseen;
+          if (room) {
+            D.row_j[row] = cnv;
+            D.a_frow[icap] = row;
+            D.row_new[cnr - L.nrows0] = row;
+            L.nrows = cnr + 1;
+            if (ci < 0) {
+              D.row_pos[row] = icap;
+              D.row_m[row] = ev;
+            }
             // a cell of another growth velocity
             if (PR) {
-              const double v = cafe_vh(D, K, icap);
-              if (!cafe_v_ordinary(v)) L.sw = 1;
-              L.vmin = fmin(L.vmin, v);
-              L.vmax = fmax(L.vmax, v);
+              if (!cafe_v_ordinary(vq)) L.sw = 1;
+              L.vmin = fmin(L.vmin, vq);
+              L.vmax = fmax(L.vmax, vq);
             } else if (cls != 1) {
               L.sw = 1;
             }
@@ -1005,145 +1273,96 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
           }
         }
       }
+      cnv += 1;
+      cnr += grows && room;
     } else if (tid == CAFE_CLOCK_WARP * 32) {
       // the capture time, the clock (VoxelsCA.C:381, 483-516) and the growth log
       const bool nuc = L.unext[ev & 1] < cafe_nuc_rate_at(D, K, icap);
-      const double t = plain ? wd / (PR ? S.v[win] : V) : wc.t;
+      const double t = exact ? wc.t : (PR ? wd / S.v[win] : cafe_div_by(wd, V, rV));
       const double dt = nuc ? 0.0 : t;
-      L.dt = dt;
       const double vd = PR ? dt : (nuc ? 0.0 : V * dt);
+      const double tinc = L.tinc + dt;
       L.vd = vd;
+      L.tinc = tinc;
+      // while (vSind2 != countS && tinc < DelT): an event always lengthens the list
+      if (cafe_is_nan(tinc) || !(cafe_key(tinc) < cafe_key(K.DelT))) L.done = 1;
       D.ev_vd[ev] = vd;
-      L.tinc += dt;
-      L.dsum += fabs(dt);
-      L.vs += vd;
-      D.ev_vs[ev] = L.vs;
-      if (cafe_is_neg(dt)) {
-        L.negdt++;
-        L.vneg += fabs(vd);
-      }
-      L.nuc = nuc;
+      const double vs = L.vs + vd, dsum = L.dsum + fabs(dt);
+      L.vs = vs;
+      L.dsum = dsum;
+      D.ev_vs[ev] = vs;
+      if (cafe_is_neg(dt)) L.negdt++;
+      S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, tinc, dsum);
     } else if (tid == CAFE_DRAW_WARP * 32) {
       // the next event's draw (VoxelsCA.C:483; two engine outputs per event)
       cafe_uniform_stream st;
       st.x = L.rng;
       L.unext[(ev + 1) & 1] = cafe_uniform_next(&st);
       L.rng = st.x;
+    } else if (warp == CAFE_AHEAD_WARP) {
+      // the event most likely to follow (the smallest candidate of the other
+      // warps that does not aim at the captured cell; right in two of three
+      // events): what its capture loads, into this SM's L1
+      const uint32_t a = lane < NW && lane != src && wkey != 0xffffffffu && S.wq[lane] != icap ? wkey : 0xffffffffu;
+      const uint32_t k2 = __reduce_min_sync(FULL, a);
+      if (k2 != 0xffffffffu) {
+        const int s2 = __ffs(__ballot_sync(FULL, a == k2)) - 1;
+        const int q2 = S.wq[s2], r2 = S.wr[s2], c2 = cafe_slot_child(S.wm[s2]);
+        int x = 0;  // (kept, so that the loads are)
+        if (lane < CAFE_NSLOT) {
+          if (c2 >= 0) {
+            const int n2 = D.row_n[c2];
+            const CafeSlot cs = D.row_slot[(long long)c2 * CAFE_NSLOT + lane];
+            x = D.a_ev[cs.q] + (int)cs.m + __double2hiint(cs.g) + (int)cs.rk + n2;
+          }
+        } else if (lane < 30) {
+          x = __double2hiint(D.row_geo[((long long)r2 * CAFE_NSLOT + (S.wm[s2] & 31u)) * 4 + lane - 26]);
+        } else if (lane == 30) {
+          x = D.a_gid[D.row_pos[r2]];
+        } else {
+          x = D.a_cold[q2] + D.a_cls[q2];
+        }
+        S.sink[lane] = x;
+      }
+    }
+    // a row whose first slot is the captured cell moves on to its next one (the
+    // captured cell itself counts as captured by then)
+    {
+      const int top = S.top;
+      for (int i = tid; i < top; i += NT)
+        if (S.q[i] == icap) cafe_res_first(D, S, i, S.r[i], S.k[i] + 1);
     }
     __syncthreads();
     // ---- grow (VoxelsCA.C:511-516); a row that lost its last slot leaves
+    const int born = S.newslot;
     {
       const double vd = L.vd;
-      const int top2 = S.top, born = S.newslot;
-#pragma unroll
-      for (int c = 0; c < CAFE_RES_PER; ++c) {
-        const int i = tid + c * NT;
-        if (i == born) {  // created by this event: grows from the next one on
-          E[c] = S.newE;
-          if (PR) {
-            const double v = S.v[i], y = (double)(1.0f / (float)v);
-            rv[c] = y * (2.0 - v * y);
-          }
-        } else if (i < top2 && S.r[i] >= 0) {
-          E[c] = cafe_grow(E[c], PR ? S.v[i] * vd : vd);
-          if (S.flag[i] & CAFE_RF_DYING) {
-            const int r = S.r[i];
-            D.row_E[r] = E[c];
-            D.row_m[r] = ev;
-            D.row_live[r] = 0u;
-            D.row_key[r] = CAFE_KEY_NONE;
-            D.row_res[r] = -1;
-            S.flag[i] = 0;
-            S.r[i] = -1;
-            S.free[atomicAdd(&S.nfree, 1)] = (unsigned short)i;
-          }
+      const int top = S.top;
+      for (int i = tid; i < top; i += NT) {
+        // (a row created by this event grows from the next one on)
+        if (i == born || S.r[i] < 0) continue;
+        const double E = cafe_grow(S.E[i], PR ? S.v[i] * vd : vd);
+        S.E[i] = E;
+        if (S.flag[i] & CAFE_RF_DYING) {
+          const int r = S.r[i];
+          D.row_E[r] = E;
+          D.row_m[r] = ev;
+          D.row_key[r] = CAFE_KEY_NONE;
+          S.flag[i] = 0;
+          S.r[i] = -1;
+          S.free[atomicAdd(&S.nfree, 1)] = (unsigned short)i;
         }
       }
     }
-    if (tid == CAFE_CLOCK_WARP * 32) {
-      // while (vSind2 != countS && tinc < DelT)
-      const bool tin = !cafe_is_nan(L.tinc) && cafe_key(L.tinc) < cafe_key(K.DelT);
-      if (!(L.nvs2 != L.countS && tin)) L.done = 1;
-      const double lim = fmin(S.wlim - L.tinc, 0x1.e847fp19) * (PR ? 1.0 : V);
-      S.klim = (ev < S.ev_cap && L.dsum <= S.dsum_cap) || S.all ? cafe_key(lim - fabs(lim) * 0x1p-30) : 0ULL;
-    }
-    __syncthreads();
     if (tid == 0) {
       const long long t1 = clock64();
       L.cyc[1] += t1 - t0;
       t0 = t1;
     }
-    // ---- a negative event may clamp a small extent at zero (VoxelsCA.C:515),
-    // which breaks the key bound of a row outside the set: the rows whose
-    // extrapolated extent comes near zero are brought up to date with a new key
-    if (cafe_is_neg(L.vd)) {
-      const double vd = L.vd, vsp = D.ev_vs[ev - 1], vx = PR ? L.vmax : V;
-      const double margin = (double)(ev + 16) * 0x1p-48 * (L.emax + L.gmax + vx * L.dsum + 1e-300);
-      // an extent above all the negative growth so far cannot have come near zero
-      const long long safe = crm_bits((PR ? L.vneg * vx : L.vneg) * (1.0 + 0x1p-20) + 2.0 * margin);
-      bool again = false;
-      const int nrows = L.nrows, nrows0 = L.nrows0;
-      for (int k = tid; k < nrows; k += NT) {
-        const int r = cafe_row_at(D, nrows0, k);
-        if (crm_bits(D.row_E[r]) >= safe) continue;  // (NaN too: it never captures)
-        if (D.row_res[r] >= 0 || D.row_death[r] < ev) continue;
-        const int m = D.row_m[r];
-        if (m >= ev) continue;
-        const double v = PR ? cafe_vh(D, K, D.row_pos[r]) : V;
-        const double gr = (vsp - D.ev_vs[m]) + vd;
-        if (D.row_E[r] + (PR ? v * gr : gr) >= margin) continue;
-        int stop;
-        const double En = cafe_row_replayed<PR>(D, r, ev, v, stop);
-        D.row_E[r] = En;
-        D.row_m[r] = stop;
-        const uint32_t live = D.row_live[r];
-        if (live) {
-          const double t = (D.row_slot[(long long)r * CAFE_NSLOT + __ffs(live) - 1].g - En) / v;
-          const unsigned long long key = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
-          D.row_key[r] = key;
-          again = again || key <= S.kw;
-        }
-      }
-      if (__syncthreads_or(again)) need_open = true;
-    }
-    // ---- the captured cell's own row
-    const int nr = L.newrow;
-    if (nr >= 0 && !L.fill) {
-      if (S.newslot < 0) {  // no room: write the set back and open a new window
-        if (tid == 0) {
-          D.row_E[nr] = L.nc.ext;
-          const double t = (D.row_slot[(long long)nr * CAFE_NSLOT + __ffs(D.row_live[nr]) - 1].g - L.nc.ext) /
-                           (PR ? cafe_vh(D, K, icap) : V);
-          D.row_key[nr] = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
-        }
-        need_open = true;
-        __syncthreads();
-      }
-    } else if (nr >= 0) {
-      if (warp < CAFE_QUAD_THREADS / 32) {
-        const CafeChildList none = {nullptr, 0, 0, 0.0};
-        const unsigned long long gk = cafe_row_fill_quad(D, K, nr, icap, L.tinc, Q, L.nc, none);
-        if (tid == 0) {
-          D.row_E[nr] = L.nc.ext;
-          if (gk != 0ULL) L.gmax = fmax(L.gmax, cafe_unkey(gk));
-          if (!cafe_is_nan(L.nc.ext)) L.emax = fmax(L.emax, fabs(L.nc.ext));
-          int i = -1;
-          if (S.nfree > 0) i = S.free[--S.nfree];
-          else if (S.top < CAFE_RES_MAX) i = S.top++;
-          S.newslot = i;
-          if (i >= 0) S.r[i] = nr;
-        }
-      }
-      __syncthreads();
-      const int i = S.newslot;
-      if (i < 0) {
-        need_open = true;  // no room: write the set back and open a new window
-      } else if (i % NT == tid) {
-#pragma unroll
-        for (int c = 0; c < CAFE_RES_PER; ++c)
-          if (i == tid + c * NT) load_resident(c, i);
-      }
-      __syncthreads();
+    // ---- events with more to do than the row that was foreseen
+    if (cafe_is_neg(L.vd) && cafe_negative_event<PR>(sD, sK, L, S, ev)) need_open = true;
+    if (L.newrow >= 0 && born < 0) {
+      if (cafe_new_row<PR>(sD, sK, L, S, Q, ev, icap)) need_open = true;
       if (tid == 0) {
         const long long t1 = clock64();
         L.cyc[2] += t1 - t0;
@@ -1152,7 +1371,11 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     }
     if (L.done || L.sw) break;
   }
-  flush(false);
+  cafe_res_flush<PR>(sD, sK, L, S, ev, false);
+  if (tid == CAFE_CAP_WARP * 32) {
+    L.nvs2 = cnv;
+    L.countS = cnv - 1;
+  }
   if (tid == 0) {
     L.ev = ev;
     D.ctr[CTR_EVLOG] = PR ? 1 : 0;
@@ -1160,58 +1383,14 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
   __syncthreads();
 }
 
-__device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, long long max_events, int allow_fast, const int cafe_bid, const int cafe_nblk) {
-  __shared__ CafeLoop L;
-  __shared__ CafeResident S;
-  __shared__ CafeQuadScratch Q;
+// The reference's scan of every row per event: from the start (mode 2), or where
+// the resident loop stopped with L.sw.
+__device__ __noinline__ void cafe_events_scan(const CafeDev &D, const CafeConsts &K, long long max_events, CafeLoop &L,
+                                              CafeResident &S, CafeQuadScratch &Q, int mode) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_LOOP_THREADS / 32;
-  if (cafe_bid != 0) return;  // event_fill_helper's second block: the loop leaves it nothing to do
-  if (tid == 0) {
-    L.na = D.ctr[CTR_NA];
-    L.nvs2 = D.ctr[CTR_NVS2];
-    L.nrows = L.nrows0 = D.ctr[CTR_NROWS];
-    L.ngrain = D.ctr[CTR_NGRAIN];
-    const int tInd = Pp->tInd;
-    uint32_t seed = cafe_minstd_seed((uint64_t)(uint32_t)(30 * tInd + (int)K.seed1));
-    cafe_uniform_stream st;
-    st.x = cafe_minstd_skip(seed, 2ULL * (uint64_t)L.na);
-    L.unext[1] = cafe_uniform_next(&st);  // the first event's draw; later draws are made one event ahead
-    L.rng = st.x;
-    L.sdloc = K.seed0 + 32u * (unsigned int)tInd + 64u * (unsigned int)L.ngrain;
-    L.tinc = L.dsum = L.vd = L.dt = L.vs = L.vneg = 0.0;
-    L.gmax = D.row_mag[0] ? cafe_unkey(D.row_mag[0]) : 0.0;
-    L.emax = D.row_mag[1] ? cafe_unkey(D.row_mag[1]) : 0.0;
-    L.vmin = D.row_mag[2] != CAFE_KEY_NONE ? cafe_unkey(D.row_mag[2]) : 1.0;
-    L.vmax = D.row_mag[3] ? cafe_unkey(D.row_mag[3]) : 1.0;
-    L.countS = L.na;
-    L.nnuc = L.negdt = L.opens = 0;
-    L.ev = L.sw = 0;
-    L.newrow = -1;
-    L.cyc[0] = L.cyc[1] = L.cyc[2] = L.cyc[3] = 0;
-    D.ev_vd[0] = D.ev_vs[0] = 0.0;
-    D.ctr[CTR_EVLOG] = 0;
-    const int slow = D.ctr[CTR_SLOW];
-    // 0: rows share one velocity; 1: per-row velocities; 2: full scan
-    L.slow = (!allow_fast || (slow & 2)) ? 2 : (slow & 1);
-    L.done = (*D.err != 0) || (L.na > D.act_cap) || (L.nvs2 > D.vs2_cap) || (L.nrows > D.row_cap);
-    if (L.na + 2 > D.ev_cap) {
-      atomicOr(D.err, CAFE_ERR_ITER_CAP);
-      L.done = 1;
-    }
-    // while (vSind2 != countS && tinc < DelT)
-    if (!(L.nvs2 != L.countS && L.tinc < K.DelT)) L.done = 1;
-  }
-  __syncthreads();
-  const int mode = L.slow;
-  if (!L.done) {
-    if (mode == 0)
-      cafe_events_resident<false>(D, K, max_events, L, S, Q);
-    else if (mode == 1)
-      cafe_events_resident<true>(D, K, max_events, L, S, Q);
-  }
-  const bool scan = mode == 2 || L.sw;
-  if (scan && !L.done) {
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
+  if (L.done || !(mode == 2 || L.sw)) return;
+  {
     // extents are kept current from here on
     const int e0 = L.ev;
     for (int k = tid; k < L.nrows; k += NT) {
@@ -1223,7 +1402,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
   }
   // ======================================================== full scan
   bool first = true;
-  while (scan && !L.done) {
+  while (!L.done) {
     if (tid == 0 && !first) {
       // while (vSind2 != countS && tinc < DelT)
       if (!(L.nvs2 != L.countS && L.tinc < K.DelT)) L.done = 1;
@@ -1235,8 +1414,9 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
     CafeCand best = cafe_cand_none();
     for (int k = tid; k < L.nrows; k += NT) {
       const int r = cafe_row_at(D, L.nrows0, k);
-      const uint32_t live = D.row_live[r];
-      if (live) cafe_row_best(D, r, D.row_E[r], cafe_vh(D, K, D.row_pos[r]), live, best);
+      const int k0 = D.row_k[r], k1 = cafe_row_next(D, r, k0);
+      if (k1 != k0) D.row_k[r] = (uint8_t)k1;
+      if (k1 < D.row_n[r]) cafe_row_best(D, r, D.row_E[r], cafe_vh(D, K, D.row_pos[r]), k1, best);
     }
     best = cafe_warp_best(best);
     if (lane == 0) S.red[warp] = best;
@@ -1272,7 +1452,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
       if (isfinite(d)) {
         for (int k = tid; k < L.nrows; k += NT) {
           const int r = cafe_row_at(D, L.nrows0, k);
-          if (!D.row_live[r]) continue;
+          if (D.row_k[r] >= D.row_n[r]) continue;  // (no liquid neighbour)
           double e = D.row_E[r] + cafe_vh(D, K, D.row_pos[r]) * d;
           D.row_E[r] = (e < 0.0) ? 0.0 : e;
         }
@@ -1282,7 +1462,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
         for (int j = tid; j < L.countS; j += NT) {
           int p = D.vs2[j];
           int r = D.a_frow[p];
-          double v = (r >= 0 && D.row_live[r]) ? cafe_vh(D, K, p) : 0.0;
+          double v = (r >= 0 && D.row_k[r] < D.row_n[r]) ? cafe_vh(D, K, p) : 0.0;
           double *ep = r >= 0 ? &D.row_E[r] : &D.a_ext[p];
           double e = *ep + v * d;
           *ep = (e < 0.0) ? 0.0 : e;
@@ -1293,6 +1473,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
     // ---- the captured cell (VoxelsCA.C:483-505 and 518-605)
     if (tid == 0) {
       D.a_state[icap] = 2;
+      D.a_ev[icap] = ev;
       if (L.nvs2 < D.vs2_cap) {
         D.vs2[L.nvs2] = icap;
       } else {
@@ -1301,57 +1482,20 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
       }
       L.nvs2 += 1;
       if (L.nuc) {
-        int ci, cj, ck;
-        cafe_cell_xyz(K, D.act[icap], ci, cj, ck);
-        if (L.ngrain < D.grain_cap) {
-          double q4[4];
-          cafe_sample_orientation(K, L.sdloc, q4);
-          double *c = D.cth + 4LL * L.ngrain;
-          for (int a = 0; a < 4; ++a) c[a] = q4[a];
-          cafe_rot_from_cth(c, D.rot + 9LL * L.ngrain);
-        } else {
-          atomicOr(D.err, CAFE_ERR_GRAIN_CAP);
-          L.done = 1;
-        }
-        L.ngrain += 1;
-        L.nc.gid = L.ngrain;
-        L.nc.c[0] = ((double)ci + .5) * K.dx[0];
-        L.nc.c[1] = ((double)cj + .5) * K.dx[1];
-        L.nc.c[2] = ((double)ck + .5) * K.dx[2];
-        L.nc.ext = 0.0;
-        L.sdloc += 10u;
-        L.nnuc++;
+        cafe_nucleate(D, K, L, icap);
       } else {
         const double *gq = D.row_geo + ((long long)wr * CAFE_NSLOT + best.s) * 4;
-        L.nc.gid = D.a_gid[D.row_pos[wr]];
-        L.nc.ext = gq[0];
-        L.nc.c[0] = gq[1];
-        L.nc.c[1] = gq[2];
-        L.nc.c[2] = gq[3];
+        D.a_gid[icap] = L.nc.gid = D.a_gid[D.row_pos[wr]];
+        D.a_ext[icap] = L.nc.ext = gq[0];
+        D.a_cx[icap] = L.nc.c[0] = gq[1];
+        D.a_cy[icap] = L.nc.c[1] = gq[2];
+        D.a_cz[icap] = L.nc.c[2] = gq[3];
       }
-      D.a_gid[icap] = L.nc.gid;
-      D.a_ext[icap] = L.nc.ext;
-      D.a_cx[icap] = L.nc.c[0];
-      D.a_cy[icap] = L.nc.c[1];
-      D.a_cz[icap] = L.nc.c[2];
       L.tinc += L.dt;
     } else if (warp == 1) {
-      // ---- neighbours of the captured cell lose one liquid neighbour
       const int q = lane < CAFE_NSLOT ? D.a_nbr[(long long)icap * CAFE_NSLOT + lane] : -1;
-      const bool liq = q >= 0 && D.a_state[q] == 1;
-      const bool any = __ballot_sync(0xffffffffu, liq) != 0u;
+      const bool any = __any_sync(0xffffffffu, q >= 0 && D.a_state[q] == 1);
       if (lane == 0) L.newrow = any && D.a_cold[icap] ? 1 : 0;
-      const int r = q >= 0 ? D.a_frow[q] : -1;
-      if (r >= 0) {
-        const uint32_t live = D.row_live[r], bit = 1u << D.row_rank[(long long)r * 32 + (CAFE_NSLOT - 1 - lane)];
-        if (live & bit) {
-          D.row_live[r] = live & ~bit;
-          if (live == bit) {
-            D.row_death[r] = ev;
-            D.row_key[r] = CAFE_KEY_NONE;
-          }
-        }
-      }
     }
     __syncthreads();
     // ---- the captured cell becomes a capturing cell if it qualifies
@@ -1361,9 +1505,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
         if (tid == 0) {
           D.row_pos[r] = icap;
           D.row_j[r] = L.nvs2 - 1;
-          D.row_res[r] = -1;
           D.a_frow[icap] = r;
-          D.row_death[r] = CAFE_ALIVE;
           D.row_E[r] = L.nc.ext;
           D.row_m[r] = CAFE_M_DONE;
           D.row_new[r - L.nrows0] = r;
@@ -1378,6 +1520,63 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
     }
     __syncthreads();
   }
+}
+
+__device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, long long max_events, int allow_fast, const int cafe_bid, const int cafe_nblk) {
+  __shared__ CafeLoop L;
+  __shared__ CafeResident S;
+  __shared__ CafeQuadScratch Q;
+  __shared__ CafeDev sD;
+  __shared__ CafeConsts sK;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_LOOP_THREADS / 32;
+  if (cafe_bid != 0) return;  // event_fill_helper's second block: the loop leaves it nothing to do
+  if (tid == 32) sD = D;
+  if (tid == 64) sK = K;
+  if (tid == 0) {
+    L.na = D.ctr[CTR_NA];
+    L.nvs2 = D.ctr[CTR_NVS2];
+    L.nrows = L.nrows0 = D.ctr[CTR_NROWS];
+    L.ngrain = D.ctr[CTR_NGRAIN];
+    const int tInd = Pp->tInd;
+    uint32_t seed = cafe_minstd_seed((uint64_t)(uint32_t)(30 * tInd + (int)K.seed1));
+    cafe_uniform_stream st;
+    st.x = cafe_minstd_skip(seed, 2ULL * (uint64_t)L.na);
+    L.unext[1] = cafe_uniform_next(&st);  // the first event's draw; later draws are made one event ahead
+    L.rng = st.x;
+    L.sdloc = K.seed0 + 32u * (unsigned int)tInd + 64u * (unsigned int)L.ngrain;
+    L.tinc = L.dsum = L.vd = L.dt = L.vs = 0.0;
+    L.gmax = D.row_mag[0] ? cafe_unkey(D.row_mag[0]) : 0.0;
+    L.emax = D.row_mag[1] ? cafe_unkey(D.row_mag[1]) : 0.0;
+    L.vmin = D.row_mag[2] != CAFE_KEY_NONE ? cafe_unkey(D.row_mag[2]) : 1.0;
+    L.vmax = D.row_mag[3] ? cafe_unkey(D.row_mag[3]) : 1.0;
+    L.countS = L.na;
+    L.nnuc = L.negdt = L.opens = 0;
+    L.ev = L.sw = 0;
+    L.newrow = -1;
+    L.cyc[0] = L.cyc[1] = L.cyc[2] = L.cyc[3] = 0;
+    D.ev_vd[0] = D.ev_vs[0] = 0.0;
+    D.ctr[CTR_EVLOG] = 0;
+    const int slow = D.ctr[CTR_SLOW];
+    // 0: rows share one velocity; 1: per-row velocities; 2: full scan
+    L.slow = (!allow_fast || (slow & 2)) ? 2 : (slow & 1);
+    L.done = (*D.err != 0) || (L.na > D.act_cap) || (L.nvs2 > D.vs2_cap) || (L.nrows > D.row_cap);
+    if (L.na + 2 > D.ev_cap) {
+      atomicOr(D.err, CAFE_ERR_ITER_CAP);
+      L.done = 1;
+    }
+    // while (vSind2 != countS && tinc < DelT)
+    if (!(L.nvs2 != L.countS && L.tinc < K.DelT)) L.done = 1;
+  }
+  __syncthreads();
+  const int mode = L.slow;
+  if (!L.done) {
+    if (mode == 0)
+      cafe_events_resident<false>(D, K, max_events, L, S, Q, sD, sK);
+    else if (mode == 1)
+      cafe_events_resident<true>(D, K, max_events, L, S, Q, sD, sK);
+  }
+  cafe_events_scan(sD, sK, max_events, L, S, Q, mode);
   if (tid == 0) {
     D.ctr[CTR_NGRAIN] = L.ngrain;
     D.ctr[CTR_NVS2_END] = L.nvs2;

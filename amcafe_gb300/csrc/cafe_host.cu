@@ -1187,20 +1187,19 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
       (rc = dalloc(&D.cx, N, o)) || (rc = dalloc(&D.cy, N, o)) || (rc = dalloc(&D.cz, N, o)) ||
       (rc = dalloc(&D.buildj, N, o)) || (rc = dalloc(&D.build, N, o)) || (rc = dalloc(&D.pos_of, N, o)) || (rc = dalloc(&D.liq, acap, o)) ||
       (rc = dalloc(&D.cth, 4 * (size_t)D.grain_cap, o)) || (rc = dalloc(&D.rot, 9 * (size_t)D.grain_cap, o)) ||
-      (rc = dalloc(&D.act, acap, o)) || (rc = dalloc(&D.a_state, acap, o)) || (rc = dalloc(&D.a_cls, acap, o)) ||
-      (rc = dalloc(&D.a_cold, acap, o)) || (rc = dalloc(&D.a_gid, acap, o)) ||
+      (rc = dalloc(&D.act, acap, o)) || (rc = dalloc(&D.a_state, acap + 4, o)) || (rc = dalloc(&D.a_cls, acap + 4, o)) ||
+      (rc = dalloc(&D.a_cold, acap + 4, o)) || (rc = dalloc(&D.a_gid, acap, o)) ||
       (rc = dalloc(&D.a_liq, acap, o)) || (rc = dalloc(&D.a_frow, acap, o)) ||
       (rc = dalloc(&D.a_nbr, (size_t)acap * CAFE_NSLOT, o)) || (rc = dalloc(&D.a_ext, acap, o)) ||
       (rc = dalloc(&D.a_cx, acap, o)) || (rc = dalloc(&D.a_cy, acap, o)) || (rc = dalloc(&D.a_cz, acap, o)) ||
       (rc = dalloc(&D.a_ruq, acap, o)) || (rc = dalloc(&D.vs2, acap, o)) || (rc = dalloc(&D.row_pos, nrow, o)) ||
-      (rc = dalloc(&D.row_j, nrow, o)) || (rc = dalloc(&D.row_live, nrow, o)) ||
-      (rc = dalloc(&D.row_slot, nrow * CAFE_NSLOT, o)) || (rc = dalloc(&D.row_rank, nrow * 32, o)) ||
+      (rc = dalloc(&D.row_j, nrow, o)) || (rc = dalloc(&D.row_n, nrow, o)) || (rc = dalloc(&D.row_k, nrow, o)) ||
+      (rc = dalloc(&D.row_slot, nrow * CAFE_NSLOT, o)) || (rc = dalloc(&D.a_ev, acap, o)) ||
       (rc = dalloc(&D.row_geo, nrow * CAFE_NSLOT * 4, o)) ||
       (rc = dalloc(&D.row_new, D.row_cap, o)) || (rc = dalloc(&D.ch_src, D.ch_cap, o)) ||
       (rc = dalloc(&D.ch_gid, D.ch_cap, o)) || (rc = dalloc(&D.ch_T, D.ch_cap, o)) ||
       (rc = dalloc(&D.row_pairs, (size_t)D.row_cap * CAFE_NSLOT, o)) || (rc = dalloc(&D.blk, D.blk_cap, o)) ||
-      (rc = dalloc(&D.row_E, nrow, o)) || (rc = dalloc(&D.row_death, nrow, o)) ||
-      (rc = dalloc(&D.row_m, nrow, o)) || (rc = dalloc(&D.row_res, nrow, o)) ||
+      (rc = dalloc(&D.row_E, nrow, o)) || (rc = dalloc(&D.row_m, nrow, o)) || (rc = dalloc(&D.row_due, CAFE_DUE_MAX, o)) ||
       (rc = dalloc(&D.row_key, nrow, o)) || (rc = dalloc(&D.row_mag, 4, o)) ||
       (rc = dalloc(&D.ev_vd, D.ev_cap, o)) || (rc = dalloc(&D.ev_vs, D.ev_cap, o)) || (K.nuc_gauss && (rc = dalloc(&D.a_nuc, acap, o))) ||
       (rc = dalloc(&D.ctr, CTR_COUNT, o)) || (rc = dalloc(&D.err, 1, o)) || (rc = dalloc(&D.stat, STAT_COUNT, o)) ||

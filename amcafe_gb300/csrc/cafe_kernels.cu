@@ -591,7 +591,7 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
     D.row_mag[3] = 0ULL;
     // the row set-up's counters; a per-cell field grows rows with their own velocities
     D.ctr[CTR_SLOW] = K.easm ? 1 : 0;
-    D.ctr[CTR_NPAIRS] = 0;
+    D.ctr[CTR_NPAIRS] = D.ctr[CTR_NDUE] = D.ctr[CTR_NKEY] = 0;
     for (int d = 0; d < CAFE_CHILD_DEPTH; ++d) D.ctr[CTR_NCHILD + d] = 0;
     D.ctr[CTR_NLIQ] = 0;  // listed again by k_writeback (k_solid2mushy_list has read it)
   }
@@ -634,6 +634,7 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
     D.a_liq[p] = liq;
     D.a_cold[p] = (uint8_t)cold;
     D.a_frow[p] = -1;
+    D.a_ev[p] = 0;
     if (K.nuc_gauss) D.a_nuc[p] = cafe_nuc_rate(D, K, p);
     double U = cafe_uniform_at(seed, (uint64_t)p);
     D.a_ruq[p] = (U - .5) * K.ruq_dx / 100.;
@@ -785,7 +786,6 @@ __device__ __forceinline__ void d_lists_scatter(const CafeDev &D, const int cafe
       if (jf < D.row_cap) {
         D.row_pos[jf] = (int32_t)p;
         D.row_j[jf] = (int32_t)j2;
-        D.row_res[jf] = -1;
         D.a_frow[p] = (int32_t)jf;
       } else {
         atomicOr(D.err, CAFE_ERR_ROW_CAP);
