@@ -17,12 +17,11 @@
 enum {
   BK_RESET = 0,    // CTR_HOT = 0 (before the melt pass)
   BK_MELT,
-  BK_PBOX0,
-  BK_PBOX1,
-  BK_LIST,
+  BK_S2M,
   BK_ACOUNT,
   BK_SCAN,
   BK_ASCATTER,
+  BK_RESET_ROWS,   // the row set-up's counters
   BK_GATHER,
   BK_LCOUNT,
   BK_SCANP,
@@ -36,7 +35,8 @@ enum {
   BK_LOOP,
   BK_FINAL,
   BK_WB,
-  BK_M2S,          // also CTR_HOT and the error word into the host-visible report
+  BK_M2S,
+  BK_REPORT,       // CTR_HOT and the error word into the host-visible report
   BK_COUNT
 };
 
@@ -45,7 +45,7 @@ struct CafeBatchReal {
   CafeConsts K;
   int act_chunks;   // cafe_sim::act_chunks
   int allow_fast;   // 0: the reference's full per-event scan
-  long long nblk_act, nblk_pos;
+  long long nblk_pos;
 };
 
 struct CafeBatchArgs {
@@ -88,29 +88,25 @@ __global__ void kb_melt(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_MELT);
   d_melt(R.D, R.K, R.D.Pd, b, nb);
 }
-__global__ void kb_solid2mushy_pbox0(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_PBOX0);
-  d_solid2mushy_pbox(R.D, R.K, R.D.Pd, 0, b, nb);
-}
-__global__ void kb_solid2mushy_pbox1(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_PBOX1);
-  d_solid2mushy_pbox(R.D, R.K, R.D.Pd, 1, b, nb);
-}
-__global__ void kb_solid2mushy_list(CafeBatchArgs B) {
-  CAFE_BATCH_BLOCK(BK_LIST);
-  d_solid2mushy_list(R.D, R.K, b, nb);
+__global__ void kb_solid2mushy(CafeBatchArgs B) {
+  CAFE_BATCH_BLOCK(BK_S2M);
+  d_solid2mushy(R.D, R.K, R.D.Pd, b, nb);
 }
 __global__ void kb_active_count(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_ACOUNT);
-  d_active_count(R.D, R.K, R.D.Pd, R.act_chunks, R.nblk_act, b, nb);
+  d_active_count(R.D, R.K, R.D.Pd, R.act_chunks, b, nb);
 }
 __global__ void __launch_bounds__(1024) kb_scan_blocks(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_SCAN);
-  d_scan_blocks(R.D.blk, R.nblk_act, R.D.ctr + CTR_NA, b, nb);
+  d_scan_blocks(R.D, R.K, R.D.Pd, R.act_chunks);
 }
 __global__ void kb_active_scatter(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_ASCATTER);
-  d_active_scatter(R.D, R.K, R.D.Pd, R.act_chunks, R.nblk_act, b, nb);
+  d_active_scatter(R.D, R.K, R.D.Pd, R.act_chunks, b, nb);
+}
+__global__ void kb_reset_rows(CafeBatchArgs B) {
+  CAFE_BATCH_BLOCK(BK_RESET_ROWS);
+  if (threadIdx.x == 0) d_reset_rows(R.D, R.K);
 }
 __global__ void kb_gather(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_GATHER);
@@ -160,7 +156,10 @@ __global__ void kb_writeback(CafeBatchArgs B) {
 __global__ void kb_mushy2solid(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_M2S);
   d_mushy2solid(R.D, R.K, b, nb);
-  if (b == 0 && threadIdx.x == 0) {  // nothing sets either after the event loop
+}
+__global__ void kb_report(CafeBatchArgs B) {
+  CAFE_BATCH_BLOCK(BK_REPORT);
+  if (threadIdx.x == 0) {
     B.report[2 * r] = R.D.ctr[CTR_HOT];
     B.report[2 * r + 1] = *R.D.err;
   }

@@ -230,7 +230,8 @@ enum {
   CTR_EVLOG,                            // 1: ev_vd holds DtMin, 0: fl(v * DtMin)
   CTR_NCHILD,                           // foreseen captures listed, one count per generation
   CTR_NCHILD_LAST = CTR_NCHILD + CAFE_CHILD_DEPTH - 1,
-  CTR_ZLO, CTR_ZHI,                     // z range of the mushy and liquid cells after the last step
+  CTR_BOX,                              // 6 slots: box of the mushy and liquid cells after the last step
+  CTR_BOX_LAST = CTR_BOX + 5,           // (x, y, z lows, then highs)
   CTR_COUNT
 };
 static_assert(CTR_EASM_CURSOR % 2 == 0, "64-bit cursor needs an 8-byte aligned slot");

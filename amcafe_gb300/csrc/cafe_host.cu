@@ -456,13 +456,18 @@ struct cafe_sim {
   long long graph_captures = 0;
 };
 
+// Most virtual blocks of the active-set compaction (8-cell chunks by row).
+static long long act_blocks(const CafeConsts &K, int chunks) {
+  const long long n = (long long)((K.nx + 7) / 8) * K.ny * K.nz, per = (long long)CAFE_DENSE_THREADS * chunks;
+  return (n + per - 1) / per;
+}
+
 void cafe_internal_set_share(cafe_sim *s, int share, int graphs) {
   if (!s || share < 1) return;
   s->use_graph = graphs != 0;
   s->gsm = std::max(4, s->nsm / share);
   s->act_chunks = CAFE_ACT_MAX_CHUNKS;
-  long long per_block = (long long)CAFE_CELLS_PER_BLOCK * s->act_chunks;
-  s->nblk_act = (s->K.N + per_block - 1) / per_block;
+  s->nblk_act = act_blocks(s->K, s->act_chunks);
 }
 
 namespace {
@@ -535,11 +540,14 @@ int read_ctr(cafe_sim *s, int which, int *out) {
   return CAFE_OK;
 }
 
-// The next step's active-set compaction scans every z plane (after a state
+// The next step's active-set compaction scans every cell (after a state
 // that no step produced: initialisation, upload, restore).
 int full_active_range(cafe_sim *s) {
-  k_set_int<<<1, 1, 0, s->stream>>>(s->D.ctr + CTR_ZLO, 0);
-  k_set_int<<<1, 1, 0, s->stream>>>(s->D.ctr + CTR_ZHI, s->K.nz - 1);
+  const int hi[3] = {s->K.nx - 1, s->K.ny - 1, s->K.nz - 1};
+  for (int a = 0; a < 3; ++a) {
+    k_set_int<<<1, 1, 0, s->stream>>>(s->D.ctr + CTR_BOX + a, 0);
+    k_set_int<<<1, 1, 0, s->stream>>>(s->D.ctr + CTR_BOX + 3 + a, hi[a]);
+  }
   CUDA_TRY(cudaGetLastError());
   return CAFE_OK;
 }
@@ -845,21 +853,13 @@ int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
       LAUNCHED(CAFE_PH_CLASSIFY, 1);
       s->full_k2 = false;
     } else {
-      long long vb = (long long)(P.hi[0] - P.lo[0] + 2) * (P.hi[1] - P.lo[1] + 2) * (P.hi[2] - P.lo[2] + 2);
-      k_solid2mushy_pbox<<<graph ? s->gsm * 16 : grid_blocks(vb, 256, s), 256, 0, st>>>(D, K, Pp, 0);
-      LAUNCHED(CAFE_PH_CLASSIFY, 1);
-      long long pb = (long long)(P.phi[0] - P.plo[0] + 2) * (P.phi[1] - P.plo[1] + 2) * (P.phi[2] - P.plo[2] + 2);
-      if (graph || (P.phi[0] > P.plo[0] && P.phi[1] > P.plo[1] && P.phi[2] > P.plo[2])) {
-        k_solid2mushy_pbox<<<graph ? s->gsm * 16 : grid_blocks(pb, 256, s), 256, 0, st>>>(D, K, Pp, 1);
-        LAUNCHED(CAFE_PH_CLASSIFY, 1);
-      }
-      k_solid2mushy_list<<<s->gsm * 4, 256, 0, st>>>(D, K);
+      k_solid2mushy<<<s->gsm * 8, 256, 0, st>>>(D, K, Pp);
       LAUNCHED(CAFE_PH_CLASSIFY, 1);
     }
     const int ab = (int)std::min<long long>(s->nblk_act, (long long)s->gsm * 8);  // persistent grid
-    k_active_count<<<ab, CAFE_DENSE_THREADS, 0, st>>>(D, K, Pp, s->act_chunks, s->nblk_act);
-    k_scan_blocks<<<1, 1024, 0, st>>>(D.blk, s->nblk_act, D.ctr + CTR_NA);
-    k_active_scatter<<<ab, CAFE_DENSE_THREADS, 0, st>>>(D, K, Pp, s->act_chunks, s->nblk_act);
+    k_active_count<<<ab, CAFE_DENSE_THREADS, 0, st>>>(D, K, Pp, s->act_chunks);
+    k_scan_blocks<<<1, 1024, 0, st>>>(D, K, Pp, s->act_chunks);
+    k_active_scatter<<<ab, CAFE_DENSE_THREADS, 0, st>>>(D, K, Pp, s->act_chunks);
     LAUNCHED(CAFE_PH_CLASSIFY, 3);
   }
   int gb = s->gsm * 8;
@@ -1161,11 +1161,8 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
   long long gcap = opt && opt->grain_capacity > 0 ? opt->grain_capacity : (long long)(2 * est) + (1 << 16);
   D.grain_cap = (int)std::min<long long>(gcap, 2000000000LL);
   s->nblk = (N + CAFE_CELLS_PER_BLOCK - 1) / CAFE_CELLS_PER_BLOCK;
-  s->act_chunks = N >= (1LL << 26) ? CAFE_ACT_MAX_CHUNKS : 1;
-  {
-    long long per_block = (long long)CAFE_CELLS_PER_BLOCK * s->act_chunks;
-    s->nblk_act = (N + per_block - 1) / per_block;
-  }
+  s->act_chunks = 1;
+  s->nblk_act = act_blocks(K, s->act_chunks);
   s->nblk_pos = (acap + CAFE_CELLS_PER_BLOCK - 1) / CAFE_CELLS_PER_BLOCK;
   // the class map covers the pool box of a step; with the analytic field its
   // size is bounded by the pool extents (make_step_params), so it is sized
@@ -1181,9 +1178,9 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
     }
     D.tcls_cap = std::min<long long>(std::max<long long>(box, 1), N);
   }
-  D.blk_cap = std::max(s->nblk, 2 * s->nblk_pos);
+  D.blk_cap = std::max(act_blocks(K, 1), 2 * s->nblk_pos);
   auto &o = s->owned;
-  if ((rc = dalloc(&D.state, N, o)) || (rc = dalloc(&D.gid, N, o)) || (rc = dalloc(&D.ext, N, o)) ||
+  if ((rc = dalloc(&D.state, N + 16, o)) || (rc = dalloc(&D.gid, N, o)) || (rc = dalloc(&D.ext, N, o)) ||
       (rc = dalloc(&D.cx, N, o)) || (rc = dalloc(&D.cy, N, o)) || (rc = dalloc(&D.cz, N, o)) ||
       (rc = dalloc(&D.buildj, N, o)) || (rc = dalloc(&D.build, N, o)) || (rc = dalloc(&D.pos_of, N, o)) || (rc = dalloc(&D.liq, acap, o)) ||
       (rc = dalloc(&D.cth, 4 * (size_t)D.grain_cap, o)) || (rc = dalloc(&D.rot, 9 * (size_t)D.grain_cap, o)) ||
@@ -1204,7 +1201,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
       (rc = dalloc(&D.ev_vd, D.ev_cap, o)) || (rc = dalloc(&D.ev_vs, D.ev_cap, o)) || (K.nuc_gauss && (rc = dalloc(&D.a_nuc, acap, o))) ||
       (rc = dalloc(&D.ctr, CTR_COUNT, o)) || (rc = dalloc(&D.err, 1, o)) || (rc = dalloc(&D.stat, STAT_COUNT, o)) ||
       (rc = dalloc(&D.Pd, 1, o)) ||
-      (rc = dalloc(&D.act_flags, (size_t)((N + CAFE_CELLS_PER_BLOCK - 1) / CAFE_CELLS_PER_BLOCK) * CAFE_DENSE_THREADS, o)) || (rc = dalloc(&D.tcls, std::max<long long>(D.tcls_cap, 1), o)) ||
+      (rc = dalloc(&D.act_flags, (size_t)act_blocks(K, 1) * CAFE_DENSE_THREADS, o)) || (rc = dalloc(&D.tcls, std::max<long long>(D.tcls_cap, 1), o)) ||
       (K.easm && ((rc = dalloc(&D.temp, N, o)) || (rc = dalloc(&D.a_vh, acap, o)) ||
                   (rc = dalloc(&D.easm_q, (size_t)(D.easm_qcap = std::min<long long>(N, 1LL << 21)), o))))) {
     cafe_sim_destroy(s);
@@ -1214,7 +1211,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
     cafe_sim_destroy(s);
     return fail(CAFE_E_CUDA, "cudaMallocHost failed");
   }
-  cudaMemsetAsync(D.state, 0, N, s->stream);
+  cudaMemsetAsync(D.state, 0, N + 16, s->stream);
   cudaMemsetAsync(D.gid, 0, N * sizeof(int32_t), s->stream);
   cudaMemsetAsync(D.ext, 0, N * sizeof(double), s->stream);
   cudaMemsetAsync(D.cx, 0, N * sizeof(double), s->stream);
@@ -2330,10 +2327,10 @@ struct CafeBatchEngine {
 
 namespace {
 
-const int kBatchThreads[BK_COUNT] = {32, 256, 256, 256, 256, CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256,
+const int kBatchThreads[BK_COUNT] = {32, 256, 256, CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 32, 256,
                                      CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256, 256, 256,
                                      CAFE_QUAD_THREADS, CAFE_QUAD_THREADS, CAFE_QUAD_THREADS,
-                                     CAFE_LOOP_THREADS, 256, 256, 256};
+                                     CAFE_LOOP_THREADS, 256, 256, 256, 32};
 
 // blocks of realisation s in a batched launch of `kind` (its plain graphed
 // step's grid, cafe_sim launch_melt / launch_voxels)
@@ -2341,13 +2338,14 @@ long long batch_blocks(const cafe_sim *s, int kind, int loop_blocks) {
   const long long g = s->gsm;
   switch (kind) {
     case BK_LOOP: return loop_blocks;
-    case BK_MELT: case BK_PBOX0: case BK_PBOX1: return g * 16;
+    case BK_MELT: return g * 16;
+    case BK_S2M: return g * 8;
     case BK_CHILD0: case BK_CHILD1: case BK_CHILD2: return g * CAFE_CHILD_BLOCKS_PER_SM;
-    case BK_LIST: case BK_PREP: case BK_ORDER: case BK_FINAL: return g * 4;
+    case BK_PREP: case BK_ORDER: case BK_FINAL: return g * 4;
     case BK_ACOUNT: case BK_ASCATTER: return std::max<long long>(1, std::min<long long>(s->nblk_act, g * 8));
     case BK_GATHER: case BK_GEO: case BK_WB: case BK_M2S: return g * 8;
     case BK_LCOUNT: case BK_LSCATTER: return std::max<long long>(1, s->nblk_pos);
-    default: return 1;  // the reset, scans
+    default: return 1;  // resets, scans, the report
   }
 }
 
@@ -2357,8 +2355,7 @@ void batch_set_shape(CafeBatchEngine *E, int gsm, int chunks) {
   for (cafe_sim *s : E->sims) {
     s->gsm = gsm;
     s->act_chunks = chunks;
-    long long per_block = (long long)CAFE_CELLS_PER_BLOCK * chunks;
-    s->nblk_act = (s->K.N + per_block - 1) / per_block;
+    s->nblk_act = act_blocks(s->K, chunks);
   }
   std::fill(E->hR_valid.begin(), E->hR_valid.end(), 0);
 }
@@ -2393,12 +2390,11 @@ int batch_capture(CafeBatchEngine *E) {
   CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   kb_reset<<<E->total[BK_RESET], T[BK_RESET], 0, st>>>(A);
   kb_melt<<<E->total[BK_MELT], T[BK_MELT], 0, st>>>(A);
-  kb_solid2mushy_pbox0<<<E->total[BK_PBOX0], T[BK_PBOX0], 0, st>>>(A);
-  kb_solid2mushy_pbox1<<<E->total[BK_PBOX1], T[BK_PBOX1], 0, st>>>(A);
-  kb_solid2mushy_list<<<E->total[BK_LIST], T[BK_LIST], 0, st>>>(A);
+  kb_solid2mushy<<<E->total[BK_S2M], T[BK_S2M], 0, st>>>(A);
   kb_active_count<<<E->total[BK_ACOUNT], T[BK_ACOUNT], 0, st>>>(A);
   kb_scan_blocks<<<E->total[BK_SCAN], T[BK_SCAN], 0, st>>>(A);
   kb_active_scatter<<<E->total[BK_ASCATTER], T[BK_ASCATTER], 0, st>>>(A);
+  kb_reset_rows<<<E->total[BK_RESET_ROWS], T[BK_RESET_ROWS], 0, st>>>(A);
   kb_gather<<<E->total[BK_GATHER], T[BK_GATHER], 0, st>>>(A);
   kb_lists_count<<<E->total[BK_LCOUNT], T[BK_LCOUNT], 0, st>>>(A);
   kb_scan_pairs<<<E->total[BK_SCANP], T[BK_SCANP], 0, st>>>(A);
@@ -2412,6 +2408,7 @@ int batch_capture(CafeBatchEngine *E) {
   kb_rows_finalize<<<E->total[BK_FINAL], T[BK_FINAL], 0, st>>>(A);
   kb_writeback<<<E->total[BK_WB], T[BK_WB], 0, st>>>(A);
   kb_mushy2solid<<<E->total[BK_M2S], T[BK_M2S], 0, st>>>(A);
+  kb_report<<<E->total[BK_REPORT], T[BK_REPORT], 0, st>>>(A);
   cudaMemcpyAsync(E->hReport, E->dReport, 2 * (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st);
   cudaGraph_t g = nullptr;
   cudaError_t le = cudaGetLastError();
@@ -2602,7 +2599,6 @@ int cafe_internal_batch_engine_step(CafeBatchEngine *E, int *phase, long long *s
     x.K = s->K;
     x.act_chunks = s->act_chunks;
     x.allow_fast = s->event_scan ? 0 : 1;
-    x.nblk_act = s->nblk_act;
     x.nblk_pos = s->nblk_pos;
     if (!E->hR_valid[r] || std::memcmp(&x, &E->hR[r], sizeof x) != 0) {
       E->hR[r] = x;

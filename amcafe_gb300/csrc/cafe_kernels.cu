@@ -28,10 +28,9 @@
 #define CAFE_DENSE_THREADS 256
 #define CAFE_CELLS_PER_THREAD 8
 #define CAFE_CELLS_PER_BLOCK (CAFE_DENSE_THREADS * CAFE_CELLS_PER_THREAD)
-// The active-set compaction takes `chunks` (1..4) 8-cell chunks per thread:
-// more per thread on very large grids, where nearly every chunk is decided
-// from its state bytes and the number of blocks dominates; one per thread
-// otherwise, where the cell-by-cell tests inside the pool box set the pace.
+// The active-set compaction takes `chunks` (1..4) 8-cell chunks per thread: one,
+// so that the cell-by-cell tests inside the pool box spread over the GPU, unless a
+// batch's autotuner finds more to be faster (many realisations fill the GPU).
 #define CAFE_ACT_MAX_CHUNKS 4
 #define CAFE_LOOP_THREADS 512
 #ifdef CAFE_DETAIL_CYCLES
@@ -136,8 +135,8 @@ __global__ void k_melt(CafeDev D, CafeConsts K, const CafeStepParams *__restrict
 // is equivalent to the reference's collect-then-apply: the test reads only
 // "neighbour == liquid", which this pass never changes. Liquid cells can only
 // be (a) cells listed by the previous step's write-back, (b) cells of the
-// previous step's pool box, (c) cells of this step's pool box; the box kernel
-// covers (b) and (c) dilated by one cell, the list kernel (a).
+// previous step's pool box, (c) cells of this step's pool box; k_solid2mushy
+// covers these, the dense kernel every cell (after an upload or restore).
 __global__ void k_solid2mushy_dense(CafeDev D, CafeConsts K) {
   long long base = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * CAFE_CELLS_PER_THREAD;
   for (int c = 0; c < CAFE_CELLS_PER_THREAD; ++c) {
@@ -154,32 +153,117 @@ __global__ void k_solid2mushy_dense(CafeDev D, CafeConsts K) {
   }
 }
 
-// ConvertSolid1(1) over this step's pool box (which = 0) or the previous one
-// (1), each dilated by one cell, read from the step parameters in device memory.
-__device__ __forceinline__ void d_solid2mushy_pbox(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, int which, const int cafe_bid, const int cafe_nblk) {
-  const int *lo = which ? Pp->plo : Pp->lo, *hi = which ? Pp->phi : Pp->hi;
-  int x0 = lo[0], x1 = hi[0], y0 = lo[1], y1 = hi[1], z0 = lo[2], z1 = hi[2];
-  if (which && !(x1 > x0 && y1 > y0 && z1 > z0)) return;  // no previous box
-  x0 = max(x0 - 1, 0); y0 = max(y0 - 1, 0); z0 = max(z0 - 1, 0);
-  x1 = min(x1 + 1, K.nx); y1 = min(y1 + 1, K.ny); z1 = min(z1 + 1, K.nz);
-  if (x1 <= x0 || y1 <= y0 || z1 <= z0) return;
-  long long bx = x1 - x0, by = y1 - y0, nbox = bx * by * (z1 - z0);
-  for (long long t = cafe_bid * (long long)blockDim.x + threadIdx.x; t < nbox;
-       t += (long long)cafe_nblk * blockDim.x) {
-    int i = x0 + (int)(t % bx);
-    long long r = t / bx;
-    int j = y0 + (int)(r % by), k = z0 + (int)(r / by);
-    long long idx = (long long)K.nxy * k + (long long)K.nx * j + i;
-    if (D.state[idx] != 3) continue;
-    long long nb[26];
-    int n = cafe_moore(K, i, j, k, nb);
-    bool liq = false;
-    for (int a = 0; a < n && !liq; ++a) liq = (D.state[nb[a]] == 1);
-    if (liq) D.state[idx] = 2;
+// Eight bytes a[i .. i+7] as one word for any i (a is 8-byte aligned and padded).
+__device__ __forceinline__ unsigned long long cafe_load8(const uint8_t *a, long long i) {
+  const unsigned long long *w = (const unsigned long long *)(a + (i & ~7LL));
+  const int sh = (int)(i & 7) * 8;
+  unsigned long long v = w[0];
+  if (sh) v = (v >> sh) | (w[1] << (64 - sh));
+  return v;
+}
+// The lowest bits of the eight bytes of w (each 0 or 1) as a mask, bit c for byte c.
+__device__ __forceinline__ uint32_t cafe_gather8(unsigned long long w) {
+  return (uint32_t)((w * 0x0102040810204080ULL) >> 56);
+}
+
+// ConvertSolid1(1) for the eight cells i0..i0+7 of row (j, k): the states of the
+// 3 x 3 rows around them as words (a state is 0..3: solid has both low bits,
+// liquid the lowest only), the liquid cells of the nine rows as one mask, and
+// its three-wide window. Cells past the row's end are masked out.
+__device__ __forceinline__ void cafe_chunk_solid2mushy(const CafeDev &D, const CafeConsts &K, int i0, int j, int k) {
+  const int n = min(8, K.nx - i0);
+  const uint32_t valid = (1u << n) - 1u;
+  const long long base = (long long)K.nxy * k + (long long)K.nx * j + i0;
+  const unsigned long long w0 = cafe_load8(D.state, base);
+  const uint32_t solid = cafe_gather8(w0 & (w0 >> 1) & 0x0101010101010101ULL) & valid;
+  if (!solid) return;
+  uint32_t liq = 0;  // bit x: cell i0 - 1 + x of some row
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int y = j + r % 3 - 1, z = k + r / 3 - 1;
+    if (y < 0 || y >= K.ny || z < 0 || z >= K.nz) continue;
+    const long long rb = (long long)K.nxy * z + (long long)K.nx * y + i0;
+    const unsigned long long w = cafe_load8(D.state, rb);
+    liq |= (cafe_gather8(w & ~(w >> 1) & 0x0101010101010101ULL) & valid) << 1;
+    if (i0 > 0 && D.state[rb - 1] == 1) liq |= 1u;
+    if (i0 + 8 < K.nx && D.state[rb + 8] == 1) liq |= 1u << 9;
+  }
+  uint32_t hit = solid & ((liq | (liq << 1) | (liq >> 1)) >> 1);
+  for (; hit; hit &= hit - 1) D.state[base + __ffs(hit) - 1] = 2;
+}
+
+// ConvertSolid1(1) where liquid cells can be: this step's pool box and the
+// previous one, each dilated by one cell (as one box when that is no larger),
+// in chunks of eight cells, and around the cells that the previous step listed.
+// Eight cells per thread: the cell-by-cell form (26 loads for every solid cell,
+// two boxes and the list in launches of their own) took 98 us a step on
+// 1024x1024x256 cells, bound by its dependent loads.
+__device__ __forceinline__ void d_solid2mushy(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, const int cafe_bid, const int cafe_nblk) {
+  int lo[2][3], hi[2][3];
+  long long cnt[2] = {0, 0}, vol[2] = {0, 0};
+  const bool prev = Pp->phi[0] > Pp->plo[0] && Pp->phi[1] > Pp->plo[1] && Pp->phi[2] > Pp->plo[2];
+  const int nmax[3] = {K.nx, K.ny, K.nz};
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      lo[b][a] = max((b ? Pp->plo[a] : Pp->lo[a]) - 1, 0);
+      hi[b][a] = min((b ? Pp->phi[a] : Pp->hi[a]) + 1, nmax[a]);
+    }
+    vol[b] = (long long)max(hi[b][0] - lo[b][0], 0) * max(hi[b][1] - lo[b][1], 0) * max(hi[b][2] - lo[b][2], 0);
+  }
+  if (!prev) vol[1] = 0;
+  if (vol[0] > 0 && vol[1] > 0) {
+    int ul[3], uh[3];
+    long long uv = 1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      ul[a] = min(lo[0][a], lo[1][a]);
+      uh[a] = max(hi[0][a], hi[1][a]);
+      uv *= uh[a] - ul[a];
+    }
+    if (uv <= vol[0] + vol[1]) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        lo[0][a] = ul[a];
+        hi[0][a] = uh[a];
+      }
+      vol[1] = 0;
+    }
+  }
+  int cx[2];
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    lo[b][0] &= ~7;
+    cx[b] = (hi[b][0] - lo[b][0] + 7) >> 3;
+    if (vol[b] > 0) cnt[b] = (long long)cx[b] * (hi[b][1] - lo[b][1]) * (hi[b][2] - lo[b][2]);
+  }
+  const long long total = cnt[0] + cnt[1] + D.ctr[CTR_NLIQ];
+  for (long long t = cafe_bid * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)cafe_nblk * blockDim.x) {
+    if (t < cnt[0] + cnt[1]) {
+      const int b = t < cnt[0] ? 0 : 1;
+      const unsigned int u = (unsigned int)(b ? t - cnt[0] : t), nxc = b ? cx[1] : cx[0];
+      const unsigned int ny = b ? hi[1][1] - lo[1][1] : hi[0][1] - lo[0][1];
+      const unsigned int r = u / nxc, z = r / ny;
+      cafe_chunk_solid2mushy(D, K, (b ? lo[1][0] : lo[0][0]) + 8 * (int)(u - r * nxc),
+                             (b ? lo[1][1] : lo[0][1]) + (int)(r - z * ny), (b ? lo[1][2] : lo[0][2]) + (int)z);
+    } else {
+      const long long idx = D.liq[t - cnt[0] - cnt[1]];
+      if (D.state[idx] != 1) continue;
+      int i, j, k;
+      cafe_cell_xyz(K, idx, i, j, k);
+#pragma unroll
+      for (int d = 0; d < 27; ++d) {
+        const int x = i + d % 3 - 1, y = j + d / 3 % 3 - 1, z = k + d / 9 - 1;
+        if (x < 0 || x >= K.nx || y < 0 || y >= K.ny || z < 0 || z >= K.nz) continue;
+        const long long nb = (long long)K.nxy * z + (long long)K.nx * y + x;
+        if (D.state[nb] == 3) D.state[nb] = 2;
+      }
+    }
   }
 }
-__global__ void k_solid2mushy_pbox(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, int which) {
-  d_solid2mushy_pbox(D, K, Pp, which, blockIdx.x, gridDim.x);
+__global__ void k_solid2mushy(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp) {
+  d_solid2mushy(D, K, Pp, blockIdx.x, gridDim.x);
 }
 
 // The step parameters into device memory (kernel arguments are copied at
@@ -187,77 +271,48 @@ __global__ void k_solid2mushy_pbox(CafeDev D, CafeConsts K, const CafeStepParams
 __global__ void k_put_params(CafeStepParams *Pd, CafeStepParams P) { *Pd = P; }
 
 
-__device__ __forceinline__ void d_solid2mushy_list(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
-  int n = D.ctr[CTR_NLIQ];
-  for (int t = cafe_bid * blockDim.x + threadIdx.x; t < n; t += cafe_nblk * blockDim.x) {
-    long long idx = D.liq[t];
-    if (D.state[idx] != 1) continue;
-    int i, j, k;
-    cafe_cell_xyz(K, idx, i, j, k);
-    long long nb[26];
-    int m = cafe_moore(K, i, j, k, nb);
-    for (int a = 0; a < m; ++a)
-      if (D.state[nb[a]] == 3) D.state[nb[a]] = 2;
-  }
-}
-__global__ void k_solid2mushy_list(CafeDev D, CafeConsts K) {
-  d_solid2mushy_list(D, K, blockIdx.x, gridDim.x);
-}
-
 // ------------------------------------------------------------------ active set
-__device__ __forceinline__ bool cafe_is_active(const CafeDev &D, const CafeConsts &K,
-                                               const CafeStepParams &P, long long idx) {
-  uint8_t s = D.state[idx];
-  if (s == 2) return true;
-  int i, j, k;
-  cafe_cell_xyz(K, idx, i, j, k);
-  int hot = cafe_hot(D, K, P, i, j, k);
-  if (!hot) return s == 1;  // undercooled liquid; a cell below the liquidus is active only as such
-  // a cell at/above the liquidus is active when a neighbour is mushy or undercooled liquid
-  for (int dz = -1; dz <= 1; ++dz) {
-    int z = k + dz;
-    if (z < 0 || z >= K.nz) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      int y = j + dy;
-      if (y < 0 || y >= K.ny) continue;
-      for (int dx = -1; dx <= 1; ++dx) {
-        int x = i + dx;
-        if (x < 0 || x >= K.nx || (dx == 0 && dy == 0 && dz == 0)) continue;
-        uint8_t t = D.state[(long long)K.nxy * z + (long long)K.nx * y + x];
-        if (t == 2) return true;
-        if (t == 1 && !cafe_hot(D, K, P, x, y, z)) return true;
-      }
+// Box that can hold active cells this step: the mushy and liquid cells left by
+// the previous step (k_writeback), this and the previous pool box, widened by
+// one cell. Every active cell is mushy, liquid, or at/above the liquidus
+// (inside the pool box); a cell turns mushy this step only next to a liquid
+// cell (ConvertSolid1(1)), and liquid cells are those left by the previous
+// step or melted in the pool box; new layers bring solid and powder cells
+// only. In chunks of eight cells along x (x0 a multiple of 8), whose order is
+// the order of their cells. (Whole z planes instead, 62 M cells a step on
+// 1024x1024x256, made the compaction 130 us.)
+struct CafeBox {
+  int x0, y0, z0, nxc, ny;
+  long long n;  // chunks
+};
+__device__ __forceinline__ CafeBox cafe_active_box(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ P) {
+  const bool cur = P->hi[0] > P->lo[0] && P->hi[1] > P->lo[1] && P->hi[2] > P->lo[2];
+  const bool prev = P->phi[0] > P->plo[0] && P->phi[1] > P->plo[1] && P->phi[2] > P->plo[2];
+  const int nmax[3] = {K.nx, K.ny, K.nz};
+  int lo[3], hi[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = D.ctr[CTR_BOX + a];
+    hi[a] = D.ctr[CTR_BOX + 3 + a];
+    if (cur) {
+      lo[a] = min(lo[a], P->lo[a]);
+      hi[a] = max(hi[a], P->hi[a] - 1);
     }
+    if (prev) {
+      lo[a] = min(lo[a], P->plo[a]);
+      hi[a] = max(hi[a], P->phi[a] - 1);
+    }
+    lo[a] = max(lo[a] - 1, 0);
+    hi[a] = min(hi[a] + 1, nmax[a] - 1);
   }
-  return false;
-}
-
-// Cell-index range that can hold active cells this step: the z planes of the
-// mushy and liquid cells left by the previous step (k_writeback) and of this
-// and the previous pool box, widened by one plane. Every active cell is mushy,
-// liquid, or at/above the liquidus (inside the pool box); a cell turns mushy
-// this step only next to a liquid cell (ConvertSolid1(1)), and liquid cells
-// are those left by the previous step or melted in the pool box; new layers
-// bring solid and powder cells only.
-__device__ __forceinline__ void cafe_active_range(const CafeDev &D, const CafeConsts &K, const CafeStepParams &P,
-                                                  long long &r0, long long &r1) {
-  int zlo = D.ctr[CTR_ZLO], zhi = D.ctr[CTR_ZHI];
-  if (P.hi[0] > P.lo[0] && P.hi[1] > P.lo[1] && P.hi[2] > P.lo[2]) {
-    zlo = min(zlo, P.lo[2]);
-    zhi = max(zhi, P.hi[2] - 1);
-  }
-  if (P.phi[0] > P.plo[0] && P.phi[1] > P.plo[1] && P.phi[2] > P.plo[2]) {
-    zlo = min(zlo, P.plo[2]);
-    zhi = max(zhi, P.phi[2] - 1);
-  }
-  zlo = max(zlo - 1, 0);
-  zhi = min(zhi + 1, K.nz - 1);
-  if (zhi < zlo) {
-    r0 = r1 = 0;
-    return;
-  }
-  r0 = (long long)zlo * K.nxy;
-  r1 = (long long)(zhi + 1) * K.nxy;
+  CafeBox b;
+  b.x0 = lo[0] & ~7;
+  b.y0 = lo[1];
+  b.z0 = lo[2];
+  b.nxc = (hi[0] - b.x0 + 8) >> 3;
+  b.ny = hi[1] - lo[1] + 1;
+  b.n = hi[0] < lo[0] || hi[1] < lo[1] || hi[2] < lo[2] ? 0 : (long long)b.nxc * b.ny * (hi[2] - lo[2] + 1);
+  return b;
 }
 
 // Flags of the eight state bytes of w (bit c for byte c): the byte is 1
@@ -272,25 +327,35 @@ __device__ __forceinline__ uint32_t cafe_liq_or_mushy8(unsigned long long w) {
   return (uint32_t)((a * 0x0102040810204080ULL) >> 56);
 }
 
-// Activity flags of the eight cells i0..i0+7 of row (j, k), i0 and nx multiples
-// of 8: cafe_is_active for each. The chunk's own classes come first: when no
-// cell of the chunk is at or above the liquidus, each is active exactly when
-// liquid or mushy. Otherwise the states of the 3 x 3 rows around the chunk over
-// i0-1..i0+8 (an aligned 64-bit word and two bytes per row) and the classes of
-// their liquid cells are loaded, all before any test, so that no load waits on
-// another's outcome. A neighbour "emits" when it is mushy or liquid below the
-// liquidus; a cell at or above the liquidus is active when mushy or when an
-// emitter lies among its 26 neighbours, i.e. in the three-wide window of the
-// nine rows' emitter masks (the cell itself, at or above the liquidus, emits
-// only if mushy, and then it is active anyway).
-__device__ __forceinline__ uint32_t cafe_chunk_active_rows(const CafeDev &D, const CafeConsts &K,
-                                                           const CafeStepParams &P, int i0, int j, int k) {
+// Activity flags of the eight cells i0..i0+7 of row (j, k), i0 a multiple of 8
+// (bit c for cell i0 + c; cells past the row's end are not active). A cell that
+// cannot be at or above the liquidus (outside the pool box, or not below the
+// laser plane) is active exactly when it is liquid or mushy, so a chunk outside
+// the hot region is decided from its state bytes, loaded as one word. In the
+// hot region the chunk's own classes come next: when no cell of it is at or
+// above the liquidus, the same holds. Otherwise the states of the 3 x 3 rows
+// around the chunk over i0-1..i0+8 (a word and two bytes per row) and the
+// classes of their liquid cells are loaded, all before any test, so that no
+// load waits on another's outcome. A neighbour "emits" when it is mushy or
+// liquid below the liquidus; a cell at or above the liquidus is active when
+// mushy or when an emitter lies among its 26 neighbours, i.e. in the
+// three-wide window of the nine rows' emitter masks (the cell itself, at or
+// above the liquidus, emits only if mushy, and then it is active anyway).
+__device__ __forceinline__ uint32_t cafe_chunk_active(const CafeDev &D, const CafeConsts &K, const CafeStepParams &P,
+                                                      int i0, int j, int k) {
+  const int n = min(8, K.nx - i0);
+  const uint32_t valid = (1u << n) - 1u;
+  const unsigned long long wown = cafe_load8(D.state, (long long)K.nxy * k + (long long)K.nx * j + i0);
+  const uint32_t own_lm = cafe_liq_or_mushy8(wown) & valid;
+  // (with any_hot_full, T0 or tS reaches the liquidus and no class is cold)
+  if (!P.any_hot_full && (k >= P.kabove || k < P.lo[2] || k >= P.hi[2] || j < P.lo[1] || j >= P.hi[1] ||
+                          i0 + 7 < P.lo[0] || i0 >= P.hi[0]))
+    return own_lm;
   const uint32_t hotmask = (K.hot_cls[0] ? 1u : 0u) | (K.hot_cls[1] ? 2u : 0u) | (K.hot_cls[2] ? 4u : 0u);
-  const unsigned long long wown = *(const unsigned long long *)(D.state + (long long)K.nxy * k + (long long)K.nx * j + i0);
   uint32_t own_hot = 0;  // bit c: cell i0 + c at or above the liquidus
 #pragma unroll
-  for (int c = 0; c < 8; ++c) own_hot |= ((hotmask >> cafe_cls(D, P, i0 + c, j, k)) & 1u) << c;
-  const uint32_t own_lm = cafe_liq_or_mushy8(wown);
+  for (int c = 0; c < 8; ++c)
+    if (c < n) own_hot |= ((hotmask >> cafe_cls(D, P, i0 + c, j, k)) & 1u) << c;
   if (own_hot == 0) return own_lm;
   uint32_t own_mushy = 0;
 #pragma unroll
@@ -301,13 +366,14 @@ __device__ __forceinline__ uint32_t cafe_chunk_active_rows(const CafeDev &D, con
     const int y = j + r % 3 - 1, z = k + r / 3 - 1;
     const bool rowin = y >= 0 && y < K.ny && z >= 0 && z < K.nz;
     const long long rb = (long long)K.nxy * (rowin ? z : 0) + (long long)K.nx * (rowin ? y : 0);
-    const unsigned long long w = rowin ? *(const unsigned long long *)(D.state + rb + i0) : 0ULL;
+    const unsigned long long w = rowin ? cafe_load8(D.state, rb + i0) : 0ULL;
     const unsigned int sl = (rowin && i0 > 0) ? D.state[rb + i0 - 1] : 0u;
     const unsigned int sr = (rowin && i0 + 8 < K.nx) ? D.state[rb + i0 + 8] : 0u;
     uint32_t e = 0;
 #pragma unroll
     for (int x = 0; x < 10; ++x) {
-      const unsigned int s = x == 0 ? sl : (x == 9 ? sr : (unsigned int)(w >> (8 * (x - 1))) & 0xffu);
+      const unsigned int s =
+          x == 0 ? sl : (x == 9 ? sr : (x - 1 < n ? (unsigned int)(w >> (8 * (x - 1))) & 0xffu : 0u));
       // the class of a liquid neighbour
       const int c = s == 1u ? cafe_cls(D, P, i0 - 1 + x, y, z) : 1;
       const bool hot = (hotmask >> c) & 1u;
@@ -317,107 +383,47 @@ __device__ __forceinline__ uint32_t cafe_chunk_active_rows(const CafeDev &D, con
   }
   // cell i0 + c is bit c + 1 of the window
   const uint32_t nb = (win >> 1) & 0xffu;
-  return ((~own_hot & own_lm) | (own_hot & (own_mushy | nb))) & 0xffu;
+  return ((~own_hot & own_lm) | (own_hot & (own_mushy | nb))) & valid;
 }
 
-// Activity flags of the 8-cell chunk i0..i0+7 of row (j0, k0) (bit c for
-// cell i0 + c). A cell that cannot be at or above the liquidus (outside the
-// pool box, or not below the laser plane) is active exactly when it is liquid
-// or mushy, so a chunk outside the hot region is decided from its state bytes,
-// loaded as one 64-bit word; other chunks take the 3 x 3-row test.
-__device__ __forceinline__ uint32_t cafe_chunk_active_row(const CafeDev &D, const CafeConsts &K,
-                                                          const CafeStepParams &P, long long base, int i0,
-                                                          int j0, int k0) {
-  // (with any_hot_full, T0 or tS reaches the liquidus and no class is cold)
-  const bool cold = !P.any_hot_full && (k0 >= P.kabove || k0 < P.lo[2] || k0 >= P.hi[2] || j0 < P.lo[1] ||
-                                        j0 >= P.hi[1] || i0 + 7 < P.lo[0] || i0 >= P.hi[0]);
-  if (cold) return cafe_liq_or_mushy8(*(const unsigned long long *)(D.state + base));
-  return cafe_chunk_active_rows(D, K, P, i0, j0, k0);
-}
-
-// Activity flags of the CAFE_CELLS_PER_THREAD (8) cells from `base` (bit c
-// for cell base + c) for any grid: a chunk lying in one row is decided as in
-// cafe_chunk_active_row, others cell by cell.
-__device__ __forceinline__ uint32_t cafe_chunk_active(const CafeDev &D, const CafeConsts &K,
-                                                      const CafeStepParams &P, long long base) {
-  static_assert(CAFE_CELLS_PER_THREAD == 8, "one 64-bit word of states per thread");
-  uint32_t flags = 0;
-  if (base + 8 <= K.N) {
-    int i0, j0, k0, i1, j1, k1;
-    cafe_cell_xyz(K, base, i0, j0, k0);
-    cafe_cell_xyz(K, base + 7, i1, j1, k1);
-    if (j0 == j1 && k0 == k1 && (K.nx & 7) == 0) return cafe_chunk_active_row(D, K, P, base, i0, j0, k0);
-    bool cold = false;
-    if (!P.any_hot_full && j0 == j1 && k0 == k1)
-      cold = k0 >= P.kabove || k0 < P.lo[2] || k0 >= P.hi[2] || j0 < P.lo[1] || j0 >= P.hi[1] || i1 < P.lo[0] ||
-             i0 >= P.hi[0];
-    if (cold && (base & 7) == 0) return cafe_liq_or_mushy8(*(const unsigned long long *)(D.state + base));
-  }
-  for (int c = 0; c < CAFE_CELLS_PER_THREAD; ++c) {
-    long long idx = base + c;
-    if (idx < K.N && cafe_is_active(D, K, P, idx)) flags |= 1u << c;
-  }
-  return flags;
-}
-
-// Activity flags of this thread's `chunks` chunks (bit 8 c + j for cell
-// base + 8 c + j), base a multiple of 8. With nx a multiple of 8 every chunk
-// lies in one row: the cell coordinates are formed once and stepped from
-// chunk to chunk.
-__device__ __forceinline__ uint32_t cafe_thread_active(const CafeDev &D, const CafeConsts &K,
-                                                       const CafeStepParams &P, long long base, int chunks,
-                                                       long long r0, long long r1) {
-  uint32_t f = 0;
-  if (base >= r1 || base + 8LL * chunks <= r0) return 0;  // no plane that can hold active cells
-  if ((K.nx & 7) == 0 && base + 8LL * chunks <= K.N) {
-    int i, j, k;
-    cafe_cell_xyz(K, base, i, j, k);
+// A thread's `chunks` consecutive chunks of the box, from chunk t on: f(c, i0, j,
+// k) for each (coordinates formed once, then stepped).
+template <class F>
+__device__ __forceinline__ void cafe_for_chunks(const CafeBox &b, long long t, int chunks, F f) {
+  if (t >= b.n) return;
+  const unsigned int u = (unsigned int)t, r = u / (unsigned int)b.nxc, z = r / (unsigned int)b.ny;
+  int xc = (int)(u - r * b.nxc), y = (int)(r - z * b.ny), k = b.z0 + (int)z;
 #pragma unroll
-    for (int c = 0; c < CAFE_ACT_MAX_CHUNKS; ++c)
-      if (c < chunks) {
-        f |= cafe_chunk_active_row(D, K, P, base + 8 * c, i, j, k) << (8 * c);
-        i += 8;
-        if (i == K.nx) {
-          i = 0;
-          if (++j == K.ny) {
-            j = 0;
-            ++k;
-          }
-        }
+  for (int c = 0; c < CAFE_ACT_MAX_CHUNKS; ++c) {
+    if (c >= chunks || t + c >= b.n) break;
+    f(c, b.x0 + 8 * xc, b.y0 + y, k);
+    if (++xc == b.nxc) {
+      xc = 0;
+      if (++y == b.ny) {
+        y = 0;
+        ++k;
       }
-  } else {
-#pragma unroll
-    for (int c = 0; c < CAFE_ACT_MAX_CHUNKS; ++c)
-      if (c < chunks) f |= cafe_chunk_active(D, K, P, base + 8 * c) << (8 * c);
+    }
   }
-  // cells of the range's edge chunks that lie outside it: keep [r0 - base, r1 - base)
-  const long long lo = r0 - base, hi = r1 - base;
-  if (lo > 0) f &= lo >= 32 ? 0u : ~((1u << lo) - 1u);
-  if (hi < 32) f &= hi <= 0 ? 0u : (1u << hi) - 1u;
-  return f;
 }
 
 // The compaction runs over "virtual blocks" of CAFE_DENSE_THREADS threads x
-// `chunks` 8-cell chunks (nvb of them cover the grid); a persistent grid
-// strides over them, writes a zero count for those outside the active range
-// (cafe_active_range) without touching their cells, and counts the rest.
-__device__ __forceinline__ void d_active_count(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, int chunks, long long nvb, const int cafe_bid, const int cafe_nblk) {
+// `chunks` chunks of the box; a persistent grid strides over them.
+__device__ __forceinline__ long long cafe_box_vblocks(const CafeBox &b, int chunks) {
+  const long long per = (long long)CAFE_DENSE_THREADS * chunks;
+  return (b.n + per - 1) / per;
+}
+__device__ __forceinline__ void d_active_count(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, int chunks, const int cafe_bid, const int cafe_nblk) {
   const CafeStepParams P = *Pp;
   __shared__ int wsum[CAFE_DENSE_THREADS / 32];
-  long long r0, r1;
-  cafe_active_range(D, K, P, r0, r1);
-  const long long per_vb = (long long)CAFE_DENSE_THREADS * CAFE_CELLS_PER_THREAD * chunks;
+  const CafeBox B = cafe_active_box(D, K, Pp);
+  const long long nvb = cafe_box_vblocks(B, chunks);
   for (long long vb = cafe_bid; vb < nvb; vb += cafe_nblk) {
-    long long b0 = vb * per_vb;
-    if (b0 >= r1 || b0 + per_vb <= r0) {
-      if (threadIdx.x == 0) D.blk[vb] = 0;
-      continue;
-    }
-    long long base = b0 + (long long)threadIdx.x * (CAFE_CELLS_PER_THREAD * chunks);
-    const uint32_t f = cafe_thread_active(D, K, P, base, chunks, r0, r1);
+    uint32_t f = 0;
+    cafe_for_chunks(B, (vb * CAFE_DENSE_THREADS + threadIdx.x) * chunks, chunks,
+                    [&](int c, int i0, int j, int k) { f |= cafe_chunk_active(D, K, P, i0, j, k) << (8 * c); });
     D.act_flags[vb * CAFE_DENSE_THREADS + threadIdx.x] = f;
-    int cnt = __popc(f);
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    const int cnt = __reduce_add_sync(0xffffffffu, __popc(f));
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cnt;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -428,8 +434,8 @@ __device__ __forceinline__ void d_active_count(const CafeDev &D, const CafeConst
     __syncthreads();
   }
 }
-__global__ void k_active_count(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, int chunks, long long nvb) {
-  d_active_count(D, K, Pp, chunks, nvb, blockIdx.x, gridDim.x);
+__global__ void k_active_count(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, int chunks) {
+  d_active_count(D, K, Pp, chunks, blockIdx.x, gridDim.x);
 }
 
 // Exclusive scan over the block of one value per thread (blockDim.x a multiple
@@ -460,8 +466,11 @@ __device__ __forceinline__ long long cafe_block_excl_scan(long long v, long long
   return ws[w] + incl - v;
 }
 
-// Exclusive scan of n block counts in place; writes the total to *total.
-__device__ __forceinline__ void d_scan_blocks(int32_t *blk, long long n, int *total, const int cafe_bid, const int cafe_nblk) {
+// Exclusive scan of the compaction's block counts in place; the total is the
+// active-list length.
+__device__ __forceinline__ void d_scan_blocks(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, int chunks) {
+  int32_t *blk = D.blk;
+  const long long n = cafe_box_vblocks(cafe_active_box(D, K, Pp), chunks);
   __shared__ long long ws[33];
   // each thread's segment is a multiple of four counts, so that its groups of
   // four are aligned 16-byte loads and stores (a warp's lanes read segments
@@ -485,7 +494,7 @@ __device__ __forceinline__ void d_scan_blocks(int32_t *blk, long long n, int *to
   }
   long long tot;
   long long acc = cafe_block_excl_scan(s, ws, tot);
-  if (threadIdx.x == 0) *total = (int)tot;
+  if (threadIdx.x == 0) D.ctr[CTR_NA] = (int)tot;
   for (long long b = b0; b < b1; b += 16) {
     int4 v[4];
 #pragma unroll
@@ -518,20 +527,15 @@ __device__ __forceinline__ void d_scan_blocks(int32_t *blk, long long n, int *to
     }
   }
 }
-__global__ void __launch_bounds__(1024) k_scan_blocks(int32_t *blk, long long n, int *total) {
-  d_scan_blocks(blk, n, total, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(1024) k_scan_blocks(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, int chunks) {
+  d_scan_blocks(D, K, Pp, chunks);
 }
 
-__device__ __forceinline__ void d_active_scatter(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, int chunks, long long nvb, const int cafe_bid, const int cafe_nblk) {
-  const CafeStepParams P = *Pp;
+__device__ __forceinline__ void d_active_scatter(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, int chunks, const int cafe_bid, const int cafe_nblk) {
   __shared__ int wsum[CAFE_DENSE_THREADS / 32];
-  long long r0, r1;
-  cafe_active_range(D, K, P, r0, r1);
-  const long long per_vb = (long long)CAFE_DENSE_THREADS * CAFE_CELLS_PER_THREAD * chunks;
-  long long vb_lo = r0 / per_vb, vb_hi = r1 > 0 ? (r1 - 1) / per_vb : -1;
-  if (vb_hi >= nvb) vb_hi = nvb - 1;
-  for (long long vb = vb_lo + cafe_bid; vb <= vb_hi; vb += cafe_nblk) {
-  long long base = vb * per_vb + (long long)threadIdx.x * (CAFE_CELLS_PER_THREAD * chunks);
+  const CafeBox B = cafe_active_box(D, K, Pp);
+  const long long nvb = cafe_box_vblocks(B, chunks);
+  for (long long vb = cafe_bid; vb < nvb; vb += cafe_nblk) {
   const uint32_t flags = D.act_flags[vb * CAFE_DENSE_THREADS + threadIdx.x];  // from k_active_count
   const int cnt = __popc(flags);
   // block-exclusive scan of per-thread counts
@@ -554,22 +558,43 @@ __device__ __forceinline__ void d_active_scatter(const CafeDev &D, const CafeCon
   }
   __syncthreads();
   long long pos = (long long)D.blk[vb] + wsum[w] + (incl - cnt);
-  for (int c = 0; c < CAFE_CELLS_PER_THREAD * chunks; ++c) {
-    if (!(flags >> c & 1u)) continue;
-    long long idx = base + c;
-    if (pos < D.act_cap) {
-      D.act[pos] = (int32_t)idx;
-      D.pos_of[idx] = (int32_t)pos;
-    } else {
-      atomicOr(D.err, CAFE_ERR_ACTIVE_CAP);
-    }
-    ++pos;
-  }
+  if (flags)
+    cafe_for_chunks(B, (vb * CAFE_DENSE_THREADS + threadIdx.x) * chunks, chunks, [&](int c, int i0, int j, int k) {
+      const long long base = (long long)K.nxy * k + (long long)K.nx * j + i0;
+      for (uint32_t m = (flags >> (8 * c)) & 0xffu; m; m &= m - 1) {
+        const long long idx = base + __ffs(m) - 1;
+        if (pos < D.act_cap) {
+          D.act[pos] = (int32_t)idx;
+          D.pos_of[idx] = (int32_t)pos;
+        } else {
+          atomicOr(D.err, CAFE_ERR_ACTIVE_CAP);
+        }
+        ++pos;
+      }
+    });
   __syncthreads();  // wsum is reused by the next virtual block
   }
 }
-__global__ void k_active_scatter(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, int chunks, long long nvb) {
-  d_active_scatter(D, K, Pp, chunks, nvb, blockIdx.x, gridDim.x);
+__global__ void k_active_scatter(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp, int chunks) {
+  d_active_scatter(D, K, Pp, chunks, blockIdx.x, gridDim.x);
+}
+
+// Counters of the step from the gather on (one thread, before the row set-up and
+// after k_solid2mushy and the compaction read last step's): the active box, rebuilt
+// by k_writeback, and the row set-up's.
+__device__ __forceinline__ void d_reset_rows(const CafeDev &D, const CafeConsts &K) {
+  for (int a = 0; a < 3; ++a) {
+    D.ctr[CTR_BOX + a] = 0x7fffffff;
+    D.ctr[CTR_BOX + 3 + a] = -1;
+  }
+  D.row_mag[0] = D.row_mag[1] = 0ULL;  // formed by k_rows_order and k_children
+  D.row_mag[2] = ~0ULL;
+  D.row_mag[3] = 0ULL;
+  // the row set-up's counters; a per-cell field grows rows with their own velocities
+  D.ctr[CTR_SLOW] = K.easm ? 1 : 0;
+  D.ctr[CTR_NPAIRS] = D.ctr[CTR_NDUE] = D.ctr[CTR_NKEY] = 0;
+  for (int d = 0; d < CAFE_CHILD_DEPTH; ++d) D.ctr[CTR_NCHILD + d] = 0;
+  D.ctr[CTR_NLIQ] = 0;  // listed again by k_writeback (k_solid2mushy has read it)
 }
 
 // ------------------------------------------------------------------ gather
@@ -583,18 +608,6 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
   int na = D.ctr[CTR_NA];
   if (na > D.act_cap) na = (int)D.act_cap;
   uint32_t seed = cafe_minstd_seed((uint64_t)(uint32_t)(30 * P.tInd + (int)K.seed1));
-  if (cafe_bid == 0 && threadIdx.x == 0) {  // rebuilt by k_writeback for the next step
-    D.ctr[CTR_ZLO] = 0x7fffffff;
-    D.ctr[CTR_ZHI] = -1;
-    D.row_mag[0] = D.row_mag[1] = 0ULL;  // formed by k_rows_order and k_children
-    D.row_mag[2] = ~0ULL;
-    D.row_mag[3] = 0ULL;
-    // the row set-up's counters; a per-cell field grows rows with their own velocities
-    D.ctr[CTR_SLOW] = K.easm ? 1 : 0;
-    D.ctr[CTR_NPAIRS] = D.ctr[CTR_NDUE] = D.ctr[CTR_NKEY] = 0;
-    for (int d = 0; d < CAFE_CHILD_DEPTH; ++d) D.ctr[CTR_NCHILD + d] = 0;
-    D.ctr[CTR_NLIQ] = 0;  // listed again by k_writeback (k_solid2mushy_list has read it)
-  }
   for (int p = cafe_bid * blockDim.x + threadIdx.x; p < na; p += cafe_nblk * blockDim.x) {
     long long idx = D.act[p];
     int i, j, k;
@@ -641,6 +654,7 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
   }
 }
 __global__ void k_gather(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) d_reset_rows(D, K);
   d_gather(D, K, Pp, blockIdx.x, gridDim.x);
 }
 
@@ -865,13 +879,17 @@ __global__ void k_rows_finalize(CafeDev D, CafeConsts K) {
 __device__ __forceinline__ void d_writeback(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
   int na = D.ctr[CTR_NA];
   if (na > D.act_cap) na = (int)D.act_cap;
-  int zlo = 0x7fffffff, zhi = -1;
+  int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-1, -1, -1};
   for (int p = cafe_bid * blockDim.x + threadIdx.x; p < na; p += cafe_nblk * blockDim.x) {
     long long idx = D.act[p];
     if (D.a_state[p] == 1 || D.a_state[p] == 2) {
-      int k = (int)(idx / K.nxy);
-      zlo = min(zlo, k);
-      zhi = max(zhi, k);
+      int c[3];
+      cafe_cell_xyz(K, idx, c[0], c[1], c[2]);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        lo[a] = min(lo[a], c[a]);
+        hi[a] = max(hi[a], c[a]);
+      }
     }
     D.state[idx] = D.a_state[p];
     D.gid[idx] = D.a_gid[p];
@@ -885,13 +903,21 @@ __device__ __forceinline__ void d_writeback(const CafeDev &D, const CafeConsts &
       D.liq[t] = (int32_t)idx;  // t < na <= act_cap = liq capacity
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    zlo = min(zlo, __shfl_down_sync(0xffffffffu, zlo, o));
-    zhi = max(zhi, __shfl_down_sync(0xffffffffu, zhi, o));
+  __shared__ int box[6];
+  if (threadIdx.x < 6) box[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : -1;
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
+    if ((threadIdx.x & 31) == 0 && h >= 0) {
+      atomicMin(&box[a], l);
+      atomicMax(&box[3 + a], h);
+    }
   }
-  if ((threadIdx.x & 31) == 0 && zhi >= 0) {
-    atomicMin(&D.ctr[CTR_ZLO], zlo);
-    atomicMax(&D.ctr[CTR_ZHI], zhi);
+  __syncthreads();
+  if (threadIdx.x < 3 && box[3] >= 0) {
+    atomicMin(&D.ctr[CTR_BOX + threadIdx.x], box[threadIdx.x]);
+    atomicMax(&D.ctr[CTR_BOX + 3 + threadIdx.x], box[3 + threadIdx.x]);
   }
 }
 __global__ void k_writeback(CafeDev D, CafeConsts K) {
