@@ -154,9 +154,10 @@ struct CafeDev {
   int32_t *act;
   long long act_cap;
   uint8_t *a_state, *a_cls, *a_cold;
+  uint8_t *a_kind;  // bit 0: mushy, bit 1: ... with a liquid neighbour and none at the liquidus
   // a_nbr: 26 neighbour positions by direction (ascending cell index; direction
   // s and 25 - s are opposite), -1 = not active or outside the grid
-  int32_t *a_gid, *a_liq, *a_frow, *a_nbr;
+  int32_t *a_gid, *a_frow, *a_nbr;
   double *a_ext, *a_cx, *a_cy, *a_cz, *a_ruq;
   double *a_nuc;  // nucleation probability per position (Gaussian undercooling only)
   // mushy list (vs2ind) and frontier rows

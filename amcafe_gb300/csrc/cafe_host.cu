@@ -866,7 +866,7 @@ int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
   {
     PhaseScope ps(s, CAFE_PH_GATHER);
     k_gather<<<gb, 256, 0, st>>>(D, K, Pp);
-    int nbp = (int)s->nblk_pos;
+    const int nbp = (int)std::min<long long>(s->nblk_pos, (long long)s->gsm * 4);  // (persistent)
     k_lists_count<<<nbp, CAFE_DENSE_THREADS, 0, st>>>(D);
     k_scan_pairs<<<1, 1024, 0, st>>>(D.blk, s->nblk_pos, D.ctr + CTR_NA, D.ctr + CTR_NVS2, D.ctr + CTR_NROWS);
     k_lists_scatter<<<nbp, CAFE_DENSE_THREADS, 0, st>>>(D);
@@ -1186,7 +1186,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
       (rc = dalloc(&D.cth, 4 * (size_t)D.grain_cap, o)) || (rc = dalloc(&D.rot, 9 * (size_t)D.grain_cap, o)) ||
       (rc = dalloc(&D.act, acap, o)) || (rc = dalloc(&D.a_state, acap + 4, o)) || (rc = dalloc(&D.a_cls, acap + 4, o)) ||
       (rc = dalloc(&D.a_cold, acap + 4, o)) || (rc = dalloc(&D.a_gid, acap, o)) ||
-      (rc = dalloc(&D.a_liq, acap, o)) || (rc = dalloc(&D.a_frow, acap, o)) ||
+      (rc = dalloc(&D.a_kind, acap + 8, o)) || (rc = dalloc(&D.a_frow, acap, o)) ||
       (rc = dalloc(&D.a_nbr, (size_t)acap * CAFE_NSLOT, o)) || (rc = dalloc(&D.a_ext, acap, o)) ||
       (rc = dalloc(&D.a_cx, acap, o)) || (rc = dalloc(&D.a_cy, acap, o)) || (rc = dalloc(&D.a_cz, acap, o)) ||
       (rc = dalloc(&D.a_ruq, acap, o)) || (rc = dalloc(&D.vs2, acap, o)) || (rc = dalloc(&D.row_pos, nrow, o)) ||
@@ -2344,7 +2344,7 @@ long long batch_blocks(const cafe_sim *s, int kind, int loop_blocks) {
     case BK_PREP: case BK_ORDER: case BK_FINAL: return g * 4;
     case BK_ACOUNT: case BK_ASCATTER: return std::max<long long>(1, std::min<long long>(s->nblk_act, g * 8));
     case BK_GATHER: case BK_GEO: case BK_WB: case BK_M2S: return g * 8;
-    case BK_LCOUNT: case BK_LSCATTER: return std::max<long long>(1, s->nblk_pos);
+    case BK_LCOUNT: case BK_LSCATTER: return std::max<long long>(1, std::min<long long>(s->nblk_pos, g * 4));
     default: return 1;  // resets, scans, the report
   }
 }

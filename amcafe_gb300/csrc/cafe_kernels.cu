@@ -600,7 +600,7 @@ __device__ __forceinline__ void d_reset_rows(const CafeDev &D, const CafeConsts 
 // ------------------------------------------------------------------ gather
 // Per active position: copies of the cell data, temperature class, neighbour
 // positions by direction (CAFE_NSLOT, in ascending index order; -1 = not active
-// or outside the grid), liquid-neighbour count,
+// or outside the grid), kind (a_kind),
 // all-neighbours-below-liquidus flag and the ruq offset (VoxelsCA.C:380:
 // ruq[p] = (U_p - .5) dX / 100, U_p the p-th uniform of minstd(30 tInd + seed1)).
 __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, const int cafe_bid, const int cafe_nblk) {
@@ -608,49 +608,70 @@ __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, 
   int na = D.ctr[CTR_NA];
   if (na > D.act_cap) na = (int)D.act_cap;
   uint32_t seed = cafe_minstd_seed((uint64_t)(uint32_t)(30 * P.tInd + (int)K.seed1));
-  for (int p = cafe_bid * blockDim.x + threadIdx.x; p < na; p += cafe_nblk * blockDim.x) {
-    long long idx = D.act[p];
-    int i, j, k;
-    cafe_cell_xyz(K, idx, i, j, k);
-    D.a_state[p] = D.state[idx];
-    D.a_gid[p] = D.gid[idx];
-    D.a_ext[p] = D.ext[idx];
-    D.a_cx[p] = D.cx[idx];
-    D.a_cy[p] = D.cy[idx];
-    D.a_cz[p] = D.cz[idx];
-    D.a_cls[p] = (uint8_t)cafe_cls(D, P, i, j, k);
-    if (K.easm) {
-      // VoxelsCA.C:405: T >= tL ? 0 : Avel pow(tL - T, nvel)
-      double T = D.temp[idx];
-      D.a_vh[p] = T >= K.tL ? 0.0 : K.Avel * crm_pow_int(K.tL - T, K.nvel_i);
+  // A warp takes 32 positions: their copies with a position per lane, then their
+  // neighbours with a direction per lane, one position after another (a
+  // position's 26 neighbours loaded by one thread took 28 us for 36 thousand,
+  // waiting on each load in turn).
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int warps = (cafe_nblk * blockDim.x) >> 5;
+  const uint32_t pw = cafe_minstd_pow(2 * lane);  // the stream's step to lane's position from the warp's first
+  const int d27 = lane < 13 ? lane : lane + 1;    // direction of this lane (CAFE_NSLOT of them)
+  const int dx = d27 % 3 - 1, dy = d27 / 3 % 3 - 1, dz = d27 / 9 - 1;
+  for (int w = (cafe_bid * blockDim.x + threadIdx.x) >> 5; w * 32 < na; w += warps) {
+    const int p0 = w * 32, p = p0 + lane, n = min(32, na - p0);
+    int i = 0, j = 0, k = 0;
+    uint8_t st = 0;
+    if (lane < n) {
+      const long long idx = D.act[p];
+      cafe_cell_xyz(K, idx, i, j, k);
+      st = D.state[idx];
+      D.a_state[p] = st;
+      D.a_gid[p] = D.gid[idx];
+      D.a_ext[p] = D.ext[idx];
+      D.a_cx[p] = D.cx[idx];
+      D.a_cy[p] = D.cy[idx];
+      D.a_cz[p] = D.cz[idx];
+      D.a_cls[p] = (uint8_t)cafe_cls(D, P, i, j, k);
+      if (K.easm) {
+        // VoxelsCA.C:405: T >= tL ? 0 : Avel pow(tL - T, nvel)
+        double T = D.temp[idx];
+        D.a_vh[p] = T >= K.tL ? 0.0 : K.Avel * crm_pow_int(K.tL - T, K.nvel_i);
+      }
+      D.a_frow[p] = -1;
+      D.a_ev[p] = 0;
+      if (K.nuc_gauss) D.a_nuc[p] = cafe_nuc_rate(D, K, p);
+      // the p-th uniform of the stream: outputs 2 p + 1 and 2 p + 2
+      const uint32_t x1 = (uint32_t)(((uint64_t)cafe_minstd_skip(seed, 2ULL * p0 + 1) * pw) % CAFE_MINSTD_M);
+      const double U = cafe_canonical(x1, cafe_minstd_next(x1));
+      D.a_ruq[p] = (U - .5) * K.ruq_dx / 100.;
     }
-    int liq = 0, cold = 1;
-#pragma unroll 1
-    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-      for (int dyx = 0; dyx < 9; ++dyx) {
-        const int dy = dyx / 3 - 1, dx = dyx % 3 - 1;
-        if (dz == 0 && dyx == 4) continue;
-        const int d27 = (dz + 1) * 9 + dyx, a = d27 - (d27 > 13 ? 1 : 0);
-        const int x = i + dx, y = j + dy, z = k + dz;
-        int q = -1;
+    bool liq = false, cold = false;
+#pragma unroll 4
+    for (int t = 0; t < n; ++t) {
+      const int x = __shfl_sync(FULL, i, t) + dx, y = __shfl_sync(FULL, j, t) + dy, z = __shfl_sync(FULL, k, t) + dz;
+      int q = -1;
+      bool l = false, h = false;
+      if (lane < CAFE_NSLOT) {
         if (x >= 0 && x < K.nx && y >= 0 && y < K.ny && z >= 0 && z < K.nz) {
           const long long nb = (long long)K.nxy * z + (long long)K.nx * y + x;
           q = D.pos_of[nb];
-          if (q >= 0) {
-            if (D.state[nb] == 1) ++liq;
-            if (cafe_hot(D, K, P, x, y, z)) cold = 0;
-          }
+          l = q >= 0 && D.state[nb] == 1;
+          h = q >= 0 && cafe_hot(D, K, P, x, y, z);
         }
-        D.a_nbr[(long long)p * CAFE_NSLOT + a] = q;
+        D.a_nbr[(long long)(p0 + t) * CAFE_NSLOT + lane] = q;
       }
-    D.a_liq[p] = liq;
-    D.a_cold[p] = (uint8_t)cold;
-    D.a_frow[p] = -1;
-    D.a_ev[p] = 0;
-    if (K.nuc_gauss) D.a_nuc[p] = cafe_nuc_rate(D, K, p);
-    double U = cafe_uniform_at(seed, (uint64_t)p);
-    D.a_ruq[p] = (U - .5) * K.ruq_dx / 100.;
+      const uint32_t bl = __ballot_sync(FULL, l), bh = __ballot_sync(FULL, h);
+      if (lane == t) {
+        liq = bl != 0u;
+        cold = bh == 0u;
+      }
+    }
+    if (lane < n) {
+      D.a_cold[p] = cold;
+      // mushy; able to capture (VoxelsCA.C:396-397)
+      D.a_kind[p] = st == 2 ? (liq && cold ? 3 : 1) : 0;
+    }
   }
 }
 __global__ void k_gather(CafeDev D, CafeConsts K, const CafeStepParams *__restrict__ Pp) {
@@ -662,37 +683,39 @@ __global__ void k_gather(CafeDev D, CafeConsts K, const CafeStepParams *__restri
 // Two order-preserving compactions over positions: mushy positions (vs2ind,
 // VoxelsCA.C:346-353) and, among them, those with a liquid neighbour and no
 // neighbour at the liquidus (the cells that can capture, VoxelsCA.C:396-397).
+// Eight positions per thread, their kinds as one word (positions past the
+// list's end count as nothing).
+__device__ __forceinline__ unsigned long long cafe_kinds8(const CafeDev &D, long long base, int na) {
+  if (base >= na) return 0ULL;
+  unsigned long long w = *(const unsigned long long *)(D.a_kind + base);
+  if (base + 8 > na) w &= (1ULL << (8 * (na - base))) - 1ULL;
+  return w;
+}
 __device__ __forceinline__ void d_lists_count(const CafeDev &D, const int cafe_bid, const int cafe_nblk) {
   __shared__ int ws[2][CAFE_DENSE_THREADS / 32];
   int na = D.ctr[CTR_NA];
   if (na > D.act_cap) na = (int)D.act_cap;
-  long long base = ((long long)cafe_bid * blockDim.x + threadIdx.x) * CAFE_CELLS_PER_THREAD;
-  int c2 = 0, cf = 0;
-  for (int c = 0; c < CAFE_CELLS_PER_THREAD; ++c) {
-    long long p = base + c;
-    if (p >= na) break;
-    if (D.a_state[p] == 2) {
-      ++c2;
-      if (D.a_liq[p] > 0 && D.a_cold[p]) ++cf;
+  const int nvb = (na + CAFE_CELLS_PER_BLOCK - 1) / CAFE_CELLS_PER_BLOCK;
+  for (int vb = cafe_bid; vb < nvb; vb += cafe_nblk) {
+    const unsigned long long w =
+        cafe_kinds8(D, ((long long)vb * CAFE_DENSE_THREADS + threadIdx.x) * CAFE_CELLS_PER_THREAD, na);
+    const int c2 = __reduce_add_sync(0xffffffffu, __popcll(w & 0x0101010101010101ULL));
+    const int cf = __reduce_add_sync(0xffffffffu, __popcll(w & 0x0202020202020202ULL));
+    if ((threadIdx.x & 31) == 0) {
+      ws[0][threadIdx.x >> 5] = c2;
+      ws[1][threadIdx.x >> 5] = cf;
     }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    c2 += __shfl_down_sync(0xffffffffu, c2, o);
-    cf += __shfl_down_sync(0xffffffffu, cf, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    ws[0][threadIdx.x >> 5] = c2;
-    ws[1][threadIdx.x >> 5] = cf;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s2 = 0, sf = 0;
-    for (int w = 0; w < CAFE_DENSE_THREADS / 32; ++w) {
-      s2 += ws[0][w];
-      sf += ws[1][w];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int s2 = 0, sf = 0;
+      for (int q = 0; q < CAFE_DENSE_THREADS / 32; ++q) {
+        s2 += ws[0][q];
+        sf += ws[1][q];
+      }
+      D.blk[2 * vb] = s2;
+      D.blk[2 * vb + 1] = sf;
     }
-    D.blk[2 * cafe_bid] = s2;
-    D.blk[2 * cafe_bid + 1] = sf;
+    __syncthreads();
   }
 }
 __global__ void k_lists_count(CafeDev D) {
@@ -751,62 +774,59 @@ __device__ __forceinline__ void d_lists_scatter(const CafeDev &D, const int cafe
   __shared__ int ws[2][CAFE_DENSE_THREADS / 32];
   int na = D.ctr[CTR_NA];
   if (na > D.act_cap) na = (int)D.act_cap;
-  long long base = ((long long)cafe_bid * blockDim.x + threadIdx.x) * CAFE_CELLS_PER_THREAD;
-  int c2 = 0, cf = 0;
-  for (int c = 0; c < CAFE_CELLS_PER_THREAD; ++c) {
-    long long p = base + c;
-    if (p >= na) break;
-    if (D.a_state[p] == 2) {
-      ++c2;
-      if (D.a_liq[p] > 0 && D.a_cold[p]) ++cf;
-    }
-  }
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int i2 = c2, i_f = cf;
-  for (int o = 1; o < 32; o <<= 1) {
-    int v2 = __shfl_up_sync(0xffffffffu, i2, o), vf = __shfl_up_sync(0xffffffffu, i_f, o);
-    if (lane >= o) {
-      i2 += v2;
-      i_f += vf;
-    }
-  }
-  if (lane == 31) {
-    ws[0][w] = i2;
-    ws[1][w] = i_f;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int a2 = 0, af = 0;
-    for (int q = 0; q < CAFE_DENSE_THREADS / 32; ++q) {
-      int v2 = ws[0][q], vf = ws[1][q];
-      ws[0][q] = a2;
-      ws[1][q] = af;
-      a2 += v2;
-      af += vf;
-    }
-  }
-  __syncthreads();
-  long long j2 = (long long)D.blk[2 * cafe_bid] + ws[0][w] + (i2 - c2);
-  long long jf = (long long)D.blk[2 * cafe_bid + 1] + ws[1][w] + (i_f - cf);
-  for (int c = 0; c < CAFE_CELLS_PER_THREAD; ++c) {
-    long long p = base + c;
-    if (p >= na) break;
-    if (D.a_state[p] != 2) continue;
-    if (j2 < D.vs2_cap)
-      D.vs2[j2] = (int32_t)p;
-    else
-      atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
-    if (D.a_liq[p] > 0 && D.a_cold[p]) {
-      if (jf < D.row_cap) {
-        D.row_pos[jf] = (int32_t)p;
-        D.row_j[jf] = (int32_t)j2;
-        D.a_frow[p] = (int32_t)jf;
-      } else {
-        atomicOr(D.err, CAFE_ERR_ROW_CAP);
+  const int nvb = (na + CAFE_CELLS_PER_BLOCK - 1) / CAFE_CELLS_PER_BLOCK;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int vb = cafe_bid; vb < nvb; vb += cafe_nblk) {
+    const long long base = ((long long)vb * CAFE_DENSE_THREADS + threadIdx.x) * CAFE_CELLS_PER_THREAD;
+    const unsigned long long kinds = cafe_kinds8(D, base, na);
+    const int c2 = __popcll(kinds & 0x0101010101010101ULL), cf = __popcll(kinds & 0x0202020202020202ULL);
+    int i2 = c2, i_f = cf;
+    for (int o = 1; o < 32; o <<= 1) {
+      int v2 = __shfl_up_sync(0xffffffffu, i2, o), vf = __shfl_up_sync(0xffffffffu, i_f, o);
+      if (lane >= o) {
+        i2 += v2;
+        i_f += vf;
       }
-      ++jf;
     }
-    ++j2;
+    if (lane == 31) {
+      ws[0][w] = i2;
+      ws[1][w] = i_f;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int a2 = 0, af = 0;
+      for (int q = 0; q < CAFE_DENSE_THREADS / 32; ++q) {
+        int v2 = ws[0][q], vf = ws[1][q];
+        ws[0][q] = a2;
+        ws[1][q] = af;
+        a2 += v2;
+        af += vf;
+      }
+    }
+    __syncthreads();
+    long long j2 = (long long)D.blk[2 * vb] + ws[0][w] + (i2 - c2);
+    long long jf = (long long)D.blk[2 * vb + 1] + ws[1][w] + (i_f - cf);
+    for (int c = 0; c < CAFE_CELLS_PER_THREAD; ++c) {
+      const int kind = (int)(kinds >> (8 * c)) & 0xff;
+      if (!kind) continue;
+      const long long p = base + c;
+      if (j2 < D.vs2_cap)
+        D.vs2[j2] = (int32_t)p;
+      else
+        atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
+      if (kind & 2) {
+        if (jf < D.row_cap) {
+          D.row_pos[jf] = (int32_t)p;
+          D.row_j[jf] = (int32_t)j2;
+          D.a_frow[p] = (int32_t)jf;
+        } else {
+          atomicOr(D.err, CAFE_ERR_ROW_CAP);
+        }
+        ++jf;
+      }
+      ++j2;
+    }
+    __syncthreads();  // ws is reused by the next virtual block
   }
 }
 __global__ void k_lists_scatter(CafeDev D) {
@@ -859,16 +879,46 @@ __device__ __forceinline__ int cafe_exp_lb(double x) {
 // Brings every row's extent up to the end of the step (the lazily applied
 // growth of VoxelsCA.C:511-516), spread over the whole GPU, and copies it back
 // to the row cell's active-list position.
+// The growths come through shared memory, a batch at a time, so that a row's
+// chain is its additions and no load waits on it.
+#define CAFE_FINAL_BATCH 512
 __device__ __forceinline__ void d_rows_finalize(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
+  __shared__ double vd[CAFE_FINAL_BATCH];
   int nrows = D.ctr[CTR_NROWS_END];
   if (nrows > D.row_cap) nrows = (int)D.row_cap;
-  int nev = D.ctr[CTR_NEV];
+  const int nev = D.ctr[CTR_NEV];
   const bool pr = D.ctr[CTR_EVLOG] != 0;
   const int nrows0 = D.ctr[CTR_NROWS];
-  for (int k = cafe_bid * blockDim.x + threadIdx.x; k < nrows; k += cafe_nblk * blockDim.x) {
-    const int r = cafe_row_at(D, nrows0, k);
-    cafe_row_replay(D, K, r, nev, pr);
-    D.a_ext[D.row_pos[r]] = D.row_E[r];
+  for (int k0 = cafe_bid * blockDim.x; k0 < nrows; k0 += cafe_nblk * blockDim.x) {
+    const int k = k0 + threadIdx.x;
+    int r = -1, p = 0, m = 0, stop = 0;
+    double E = 0.0, v = 0.0;
+    if (k < nrows) {
+      r = cafe_row_at(D, nrows0, k);
+      p = D.row_pos[r];
+      m = D.row_m[r];
+      E = D.row_E[r];
+      if (pr) v = cafe_vh(D, K, p);
+      if (m >= nev)
+        m = 0;  // (its extent is final: nothing to apply)
+      else
+        stop = min(nev, cafe_row_death(D, r));
+    }
+    for (int e0 = 1; e0 <= nev; e0 += CAFE_FINAL_BATCH) {
+      const int n = min(CAFE_FINAL_BATCH, nev - e0 + 1);
+      __syncthreads();
+      for (int e = threadIdx.x; e < n; e += blockDim.x) vd[e] = D.ev_vd[e0 + e];
+      __syncthreads();
+      const int a = max(m + 1 - e0, 0), b = min(stop - e0 + 1, n);
+      if (pr) {
+#pragma unroll 4
+        for (int e = a; e < b; ++e) E = cafe_grow(E, v * vd[e]);
+      } else {
+#pragma unroll 4
+        for (int e = a; e < b; ++e) E = cafe_grow(E, vd[e]);
+      }
+    }
+    if (r >= 0) D.a_ext[p] = E;
   }
 }
 __global__ void k_rows_finalize(CafeDev D, CafeConsts K) {
@@ -935,10 +985,17 @@ __device__ __forceinline__ void d_mushy2solid(const CafeDev &D, const CafeConsts
     long long idx = D.act[p];
     int i, j, k;
     cafe_cell_xyz(K, idx, i, j, k);
-    long long nb[26];
-    int n = cafe_moore(K, i, j, k, nb);
+    // the two or three states around i of each neighbouring row as bytes of one
+    // word: mushy and solid (2, 3) have the second bit
+    const int x0 = i > 0 ? i - 1 : 0, n = min(i + 1, K.nx - 1) - x0 + 1;
+    const unsigned long long need = 0x020202ULL & ((1ULL << (8 * n)) - 1ULL);
     bool all = true;
-    for (int a = 0; a < n && all; ++a) all = D.state[nb[a]] >= 2;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+      const int y = j + r % 3 - 1, z = k + r / 3 - 1;
+      if (y < 0 || y >= K.ny || z < 0 || z >= K.nz) continue;
+      all = all && (cafe_load8(D.state, (long long)K.nxy * z + (long long)K.nx * y + x0) & need) == need;
+    }
     if (all) {
       D.state[idx] = 3;
       D.ext[idx] = 0.0;
