@@ -128,7 +128,7 @@ __global__ void kb_rows_prep(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_PREP);
   d_rows_prep(R.D, R.K, b, nb);
 }
-__global__ void kb_rows_geo(CafeBatchArgs B) {
+__global__ void __launch_bounds__(CAFE_QUAD_THREADS) kb_rows_geo(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_GEO);
   d_rows_geo(R.D, R.K, b, nb);
 }
@@ -139,7 +139,7 @@ __global__ void kb_rows_order(CafeBatchArgs B) {
 static_assert(CAFE_CHILD_DEPTH == 3, "one batched launch per generation");
 __global__ void __launch_bounds__(CAFE_QUAD_THREADS) kb_children(CafeBatchArgs B, int depth) {
   CAFE_BATCH_BLOCK(BK_CHILD0 + depth);
-  d_children(R.D, R.K, depth, b, nb);
+  d_children(R.D, R.K, depth, CAFE_CHILD_DEPTH, b, nb);
 }
 __global__ void __launch_bounds__(CAFE_LOOP_THREADS, 1) kb_event_loop(CafeBatchArgs B) {
   CAFE_BATCH_BLOCK(BK_LOOP);

@@ -23,8 +23,6 @@
 // and how far past the step's end (in time steps) a capture is foreseen.
 #define CAFE_CHILD_DEPTH 3
 #define CAFE_CHILD_REACH 1.1
-// Rows listed for the event loop's first window.
-#define CAFE_DUE_MAX 4096
 
 // Error bits written to CafeDev::err by device code.
 enum {
@@ -95,6 +93,7 @@ struct CafeConsts {
   double ros_q, ros_c, ros_rmin;
   double Avel;        // Grid::Avel
   int nvel_i;         // Grid::nvel (an integer when easm)
+  int all_rows;       // 1: every frontier row is evaluated (the full scan per event)
   // Gaussian-undercooling nucleation (extension keyword "nucgauss mean sd")
   int nuc_gauss;
   double nuc_mean, nuc_sd;
@@ -191,7 +190,8 @@ struct CafeDev {
   // keys of the largest |g|, the largest extent, the smallest and the largest
   // velocity of the step's rows
   double *row_E;
-  int32_t *row_m, *row_due;  // row_due: CAFE_DUE_MAX rows that can capture soon
+  int32_t *row_m, *row_due;  // row_due: the rows that may capture soon
+  float *row_glb;            // lower bound of the numerators of a row without a record
   unsigned long long *row_key, *row_mag;
   // the logged growth of each event (CTR_EVLOG: fl(v * DtMin), or DtMin) and
   // its running sum
@@ -226,8 +226,8 @@ enum {
   CTR_EASM_QHEAD,                       // next queued cell to take
   CTR_GLOG_N,                           // growth-log entries written
   CTR_GLOG_OVER,                        // 1: the growth log ran out of room
-  CTR_NDUE,                             // rows listed for the event loop's first window
-  CTR_NKEY,                             // rows with a capture candidate at the step's start
+  CTR_NDUE,                             // rows that may be due (row_due)
+  CTR_NKEY,                             // rows that are not, and have no record
   CTR_EVLOG,                            // 1: ev_vd holds DtMin, 0: fl(v * DtMin)
   CTR_NCHILD,                           // foreseen captures listed, one count per generation
   CTR_NCHILD_LAST = CTR_NCHILD + CAFE_CHILD_DEPTH - 1,

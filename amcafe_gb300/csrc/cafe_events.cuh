@@ -24,7 +24,10 @@ struct CafeChildList {
 };
 __device__ __forceinline__ int cafe_slot_child(uint32_t m) { return (int)(m >> 5) - 1; }
 
-#define CAFE_DUE_REACH 4.0  // time steps
+#define CAFE_DUE_REACH 1.5      // time steps
+#define CAFE_OUTSIDE_REACH 1.5  // ... for a row that a capture creates
+#define CAFE_SHORT_REACH 1.1    // ... to which a window may shrink
+#define CAFE_FEW_ROWS 512       // up to here every row gets its record (one wave of k_rows_geo)
 
 // Sorts the slots of row r (one per lane: liv, numerator gv, neighbour position
 // q) by g (NaN last, ties by slot) into the row's record, and forms the row's key: the order key of T + t
@@ -90,6 +93,65 @@ __device__ __forceinline__ unsigned long long cafe_row_sort_warp(const CafeDev &
   return ak;
 }
 
+// ------------------------------------------------------------------ lower bounds
+// Most rows cannot capture within the step, and their exact geometry (~600 FP64
+// instructions a slot, 64 cycles each on this GPU) would only tell that they
+// cannot. So every slot's numerator is first bounded in single precision, with
+// the folded angles of VoxelsCA.C:409-424 in closed form: g = sqrt(cos th sin ph)
+// |R^T dn|_1, cos th = max(|dx|, |dy|)/rho and sin ph = max(rho, |dz|)/r, both in
+// [1/sqrt 2, 1].
+// A row whose bound says that it is not due within CAFE_DUE_REACH time steps gets
+// no record (row_n = CAFE_NO_RECORD, row_glb its bound), only a key; the event
+// loop makes the record if the row is needed after all.
+#define CAFE_NO_RECORD 255
+// A double in single precision, truncated (no FP64 instruction); zero below the
+// normal range, NaN above 2^127.
+__device__ __forceinline__ float cafe_trunc_f32(double x) {
+  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - (1023 - 127);
+  const int f = (hi & (int)0x80000000) | ((e << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29));
+  return e <= 0 ? 0.f : (e >= 255 ? NAN : __int_as_float(f));
+}
+// Bounds of g of the slot in direction `lane` (0..25) of a cell whose centre lies
+// at c0 from its octahedron's, rotation R. The offsets are good to 3e-7 of |c0|
+// plus the cell size (truncation, one product and sum), e is over three times
+// that, and R's truncation adds as little; the quotients take the errors of both
+// operands, so that offsets that cancel only loosen the bound. NaN where an
+// operand is not finite.
+__device__ __forceinline__ void cafe_glb_slot(int lane, const float *c0, float dx, const float *R, float &lo, float &hi) {
+  const float e = 1e-6f * (fabsf(c0[0]) + fabsf(c0[1]) + fabsf(c0[2]) + 3.f * dx);
+  const int d27 = lane < 13 ? lane : lane + 1;
+  const float a = c0[0] + (float)(d27 % 3 - 1) * dx, b = c0[1] + (float)(d27 / 3 % 3 - 1) * dx,
+              c = c0[2] + (float)(d27 / 9 - 1) * dx;
+  const float rho2 = a * a + b * b, r2 = rho2 + c * c, rho = sqrtf(rho2);
+  const float ct = fmaxf(0.7071f, (fmaxf(fabsf(a), fabsf(b)) - e) / (rho + 1.5f * e));
+  const float sp = fmaxf(0.7071f, (fmaxf(rho, fabsf(c)) - 1.5f * e) / (sqrtf(r2) + 2.f * e));
+  const float l0 = R[0] * a + R[3] * b + R[6] * c, l1 = R[1] * a + R[4] * b + R[7] * c,
+              l2 = R[2] * a + R[5] * b + R[8] * c;
+  const float l = fabsf(l0) + fabsf(l1) + fabsf(l2);
+  lo = sqrtf(ct * sp) * fmaxf(l - 8.f * e, 0.f) * (1.f - 1e-5f);
+  hi = (l + 8.f * e) * (1.f + 1e-5f);
+  if (!(r2 < 1e30f) || !(l < 1e30f) || !(e > 1e-20f)) lo = hi = NAN;  // (fmaxf drops a NaN operand)
+}
+// The offsets c0 of a cell (si, sj, sk) from octahedron centre cs.
+__device__ __forceinline__ void cafe_glb_centre(const CafeConsts &K, int si, int sj, int sk, const double *cs, float *c0) {
+  double dn[3];
+  cafe_geo_dn(K, si, sj, sk, cs, dn);
+  for (int a = 0; a < 3; ++a) c0[a] = cafe_trunc_f32(dn[a]);
+}
+// Smallest lower and largest upper bound over the slots `liv` of a warp; any NaN gives NaN.
+__device__ __forceinline__ void cafe_glb_range(bool liv, float &lo, float &hi) {
+  const unsigned FULL = 0xffffffffu;
+  const bool nan = __any_sync(FULL, liv && !(lo >= 0.f));
+  lo = __uint_as_float(__reduce_min_sync(FULL, liv ? __float_as_uint(lo) : 0x7f800000u));
+  hi = __uint_as_float(__reduce_max_sync(FULL, liv ? __float_as_uint(hi) : 0u));
+  if (nan) lo = hi = NAN;
+}
+// Lower bound of a row's capture time from the bound of its g.
+__device__ __forceinline__ double cafe_lb_time(float glb, double E, double v) {
+  const double t = ((double)glb - E) / v;
+  return t - fabs(t) * 0x1p-40;
+}
+
 // The captured cell's grain, centre and extent as the capture just stored
 // them, handed to the fill through shared memory.
 struct CafeNewCell {
@@ -99,45 +161,30 @@ struct CafeNewCell {
 // Per-slot partial results passed between the four warps of cafe_row_fill_quad.
 struct CafeQuadScratch {
   double cth[32], sph[32], l[32], d1I[32], dI2[32], d1J[32], dJ3[32], dr[32];
+  CafeNewCell nc;
 };
 #define CAFE_QUAD_THREADS 128
-__device__ __forceinline__ void cafe_bar_quad() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void cafe_bar_quad(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
-// Fills row r for position p, the cell just captured (nc), at time T with warps
-// 0-3 of the block together (all 128 threads must call it): every liquid
-// neighbour slot gets its numerator g and capture result (extent, centre), and
-// the record is sorted. A warp issues one FP64 instruction per ~64 cycles
-// whatever its active lanes, so the independent chains of each slot's geometry
-// run in different warps, lane s of each warp on slot s. First stage:
+// Geometry of up to 32 slots with four warps of the block together (all 128
+// threads call it, with a barrier `bar` of their own): lane t of every warp holds
+// slot t (work: the neighbour (ci, cj, ck) of cell (si, sj, sk) with centre cs and
+// rotation Rg). A warp issues one FP64 instruction per ~64 cycles whatever its
+// active lanes, so the independent chains of a slot run in different warps. First
+// stage:
 //   warp 0: cos th and the cell distance l; warp 1: sin ph;
 //   warp 2: |R^T dn|_1 and the projection on edge p0-p1;
 //   warp 3: the projection on edge p0-p2.
-// Second stage, after one barrier: warp 0 forms g and sorts; warp 2 the extent
-// and warp 3 the centre a capture from this row gives. The return value (the
-// order key of the row's largest |g|) is valid in warp 0.
-__device__ __noinline__ unsigned long long cafe_row_fill_quad(const CafeDev &D, const CafeConsts &K, long long r, int p,
-                                                              double T, CafeQuadScratch &S, const CafeNewCell &nc,
-                                                              const CafeChildList &C) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int gp = nc.gid;
-  const bool grain_ok = gp >= 1 && gp <= D.grain_cap;
-  bool liv = false;
-  int q = -1;
-  double dn[3] = {0.0, 0.0, 0.0}, cs[3] = {0.0, 0.0, 0.0};
-  int ci = 0, cj = 0, ck = 0, si = 0, sj = 0, sk = 0;
-  if (lane < CAFE_NSLOT) {
-    q = D.a_nbr[(long long)p * CAFE_NSLOT + lane];
-    liv = q >= 0 && D.a_state[q] == 1;
-  }
-  const bool work = liv && grain_ok;
+// Second stage, after one barrier: warp 0 forms g (returned in warp 0), warp 2 the
+// extent and warp 3 the centre a capture through the slot gives (into o).
+__device__ __forceinline__ double cafe_geo_quad(const CafeConsts &K, bool work, int ci, int cj, int ck, int si, int sj,
+                                                int sk, const double *cs, const double *Rg, CafeQuadScratch &S, int bar,
+                                                double *o) {
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 3;
   double R[9], loc[3], dr = 0.0, pk[3][3];
   int s0i = 0;
   if (work) {
-    cafe_cell_xyz(K, D.act[q], ci, cj, ck);
-    cafe_cell_xyz(K, D.act[p], si, sj, sk);
-    cs[0] = nc.c[0];
-    cs[1] = nc.c[1];
-    cs[2] = nc.c[2];
+    double dn[3];
     cafe_geo_dn(K, ci, cj, ck, cs, dn);
     if (w == 0) {
       S.cth[lane] = cafe_geo_costh(dn);
@@ -145,7 +192,6 @@ __device__ __noinline__ unsigned long long cafe_row_fill_quad(const CafeDev &D, 
     } else if (w == 1) {
       S.sph[lane] = cafe_geo_sinph(dn);
     } else {
-      const double *Rg = D.rot + 9LL * (gp - 1);
       for (int a = 0; a < 9; ++a) R[a] = Rg[a];
       dr = cafe_geo_loc(R, dn, loc);
       s0i = cafe_geo_corners(loc, dr, pk);
@@ -157,15 +203,11 @@ __device__ __noinline__ unsigned long long cafe_row_fill_quad(const CafeDev &D, 
       }
     }
   }
-  cafe_bar_quad();
-  unsigned long long ak = 0ULL;
-  if (w == 0) {
-    double gv = liv ? NAN : 0.0;  // a capturing cell without a grain never captures
-    if (work) gv = crm_pow_half(S.cth[lane] * S.sph[lane]) * S.dr[lane];
-    ak = cafe_row_sort_warp(D, r, liv, gv, q, nc.ext, cafe_vh(D, K, p), T, gp, D.a_ruq[p], C, true);
-  } else if (w >= 2 && work) {
+  cafe_bar_quad(bar);
+  if (!work) return 0.0;
+  if (w == 0) return crm_pow_half(S.cth[lane] * S.sph[lane]) * S.dr[lane];
+  if (w >= 2) {
     double Lmud = cafe_geo_lmud(K, S.l[lane], S.d1I[lane], S.dI2[lane], S.d1J[lane], S.dJ3[lane]);
-    double *o = D.row_geo + (r * CAFE_NSLOT + lane) * 4;
     if (w == 2) {
       double f = crm_pow_half(S.cth[lane] * S.sph[lane]);
       o[0] = f * Lmud * 1.0;
@@ -177,7 +219,37 @@ __device__ __noinline__ unsigned long long cafe_row_fill_quad(const CafeDev &D, 
       o[3] = cn[2];
     }
   }
-  return ak;
+  return 0.0;
+}
+
+// Makes the record of row r, position p, cell nc, at time T with four warps
+// (cafe_geo_quad): every slot whose neighbour was liquid at the step's start gets
+// its numerator and capture result, and warp 0 sorts. The return value (the order
+// key of the row's largest |g|) is valid in warp 0.
+__device__ __noinline__ unsigned long long cafe_row_fill_quad(const CafeDev &D, const CafeConsts &K, long long r, int p,
+                                                              double T, CafeQuadScratch &S, const CafeNewCell &nc,
+                                                              const CafeChildList &C, int bar = 1) {
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 3;
+  const int gp = nc.gid;
+  const bool grain_ok = gp >= 1 && gp <= D.grain_cap;
+  bool liv = false;
+  int q = -1;
+  if (lane < CAFE_NSLOT) {
+    q = D.a_nbr[(long long)p * CAFE_NSLOT + lane];
+    liv = q >= 0 && (D.a_state[q] == 1 || D.a_ev[q] != 0);
+  }
+  const bool work = liv && grain_ok;
+  int ci = 0, cj = 0, ck = 0, si = 0, sj = 0, sk = 0;
+  if (work) {
+    cafe_cell_xyz(K, D.act[q], ci, cj, ck);
+    cafe_cell_xyz(K, D.act[p], si, sj, sk);
+  }
+  const double gq = cafe_geo_quad(K, work, ci, cj, ck, si, sj, sk, nc.c, D.rot + 9LL * (grain_ok ? gp - 1 : 0), S, bar,
+                                  D.row_geo + (r * CAFE_NSLOT + lane) * 4);
+  if (w != 0) return 0ULL;
+  // (a capturing cell without a grain never captures)
+  return cafe_row_sort_warp(D, r, liv, work ? gq : (liv ? NAN : 0.0), q, nc.ext, cafe_vh(D, K, p), T, gp, D.a_ruq[p], C,
+                            true);
 }
 
 // ------------------------------------------------------------------ candidates
@@ -241,6 +313,20 @@ __device__ __forceinline__ int cafe_row_next(const CafeDev &D, int r, int k) {
 // so the first look nearly always ends it.
 #define CAFE_ALIVE 0x7fffffff
 __device__ __forceinline__ int cafe_row_death(const CafeDev &D, int r) {
+  if (D.row_n[r] == CAFE_NO_RECORD) {
+    const int32_t *nb = D.a_nbr + (long long)D.row_pos[r] * CAFE_NSLOT;
+    bool liq = false;
+#pragma unroll
+    for (int s = 0; s < CAFE_NSLOT; ++s) {
+      const int q = nb[s];
+      liq |= q >= 0 && D.a_state[q] == 1;
+    }
+    if (liq) return CAFE_ALIVE;
+    int d = 0;
+    for (int s = 0; s < CAFE_NSLOT; ++s)
+      if (nb[s] >= 0) d = max(d, D.a_ev[nb[s]]);
+    return d;
+  }
   const CafeSlot *rec = D.row_slot + (long long)r * CAFE_NSLOT;
   int d = 0;
   for (int k = (int)D.row_n[r] - 1; k >= 0; --k) {
@@ -345,93 +431,177 @@ __device__ __forceinline__ bool cafe_v_ordinary(double v) { return v > 0x1p-100 
 // ------------------------------------------------------------------ row kernels
 // Frontier rows of the step, in three passes so that the capture geometry,
 // the expensive part, runs with one (row, slot) pair per lane:
-// k_rows_prep (one warp per row) finds each row's liquid neighbours, sets the
-// row's extent and growth watermark, and lists the pairs that need geometry;
-// k_rows_geo evaluates the listed pairs; k_rows_order (one warp per row) sorts
-// each row's record. CTR_SLOW: bit 0 some row grows with another velocity, bit 1
-// some row has a velocity or extent that only the full scan handles.
+// k_rows_prep (eight rows per warp) sets the row's extent and growth watermark, bounds
+// its numerators and, when it may be due, lists it and its (row, slot) pairs;
+// k_rows_geo evaluates the listed pairs, 32 at a time by four warps; k_rows_order (one warp per listed row)
+// sorts the records. CTR_SLOW: bit 0 some row grows with another velocity, bit 1
+// some row has a velocity or extent that only the full scan handles. row_mag: the
+// magnitudes that bound the keys' rounding, the largest |g| and extent, the
+// smallest and the largest velocity over the rows (order keys). Geometry of every
+// slot of every row instead took 145 us a step, its sort 26 (512x256x128).
+#define CAFE_PREP_ROWS 8
 __device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
   int nrows = D.ctr[CTR_NROWS];
   if (nrows > D.row_cap) nrows = (int)D.row_cap;
+  // A warp takes CAFE_PREP_ROWS rows: what is one value per row with a row per
+  // lane, then the slots with a direction per lane, one row after another.
   const int warps = (cafe_nblk * blockDim.x) >> 5;
-  const int w = (cafe_bid * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
-  for (int r = w; r < nrows; r += warps) {
-    int p = D.row_pos[r];
-    int gp = D.a_gid[p];
-    bool grain_ok = gp >= 1 && gp <= D.grain_cap;
-    bool liv = false;
-    if (lane < CAFE_NSLOT) {
-      const int q = D.a_nbr[(long long)p * CAFE_NSLOT + lane];
-      liv = q >= 0 && D.a_state[q] == 1;
-    }
-    if (liv && !grain_ok) D.row_slot[(long long)r * CAFE_NSLOT + lane].g = NAN;  // never captures
-    uint32_t work = __ballot_sync(FULL, liv && grain_ok);
-    int base = 0;
-    if (lane == 0 && work) base = atomicAdd(&D.ctr[CTR_NPAIRS], __popc(work));
-    base = __shfl_sync(FULL, base, 0);
-    if (work >> lane & 1u) D.row_pairs[base + __popc(work & ((1u << lane) - 1u))] = r * 32 + lane;
-    if (lane == 0) {
-      const double E = D.a_ext[p];
+  __shared__ unsigned int mag[4];  // high words of the magnitudes' order keys
+  if (threadIdx.x < 4) mag[threadIdx.x] = threadIdx.x == 2 ? 0xffffffffu : 0u;
+  __syncthreads();
+  int nkey = 0;  // rows without a record that may be candidates
+  const double lim = K.DelT * CAFE_DUE_REACH, V1 = K.vhat_cls[1], rV1 = 1.0 / V1;
+  const float dx = (float)K.dx[0];
+  const bool all = K.all_rows || nrows <= CAFE_FEW_ROWS;
+  for (int w = (cafe_bid * blockDim.x + threadIdx.x) >> 5; w * CAFE_PREP_ROWS < nrows; w += warps) {
+    const int r0 = w * CAFE_PREP_ROWS, n = min(CAFE_PREP_ROWS, nrows - r0);
+    int p = 0, gp = 0;
+    float c0[3] = {0.f, 0.f, 0.f}, gmax = 0.f;
+    double E = 0.0, v = 1.0;
+    if (lane < n) {
+      const int r = r0 + lane;
+      p = D.row_pos[r];
+      gp = D.a_gid[p];
+      if (gp < 1 || gp > D.grain_cap) gp = 0;
+      E = D.a_ext[p];
+      v = cafe_vh(D, K, p);
+      int si, sj, sk;
+      cafe_cell_xyz(K, D.act[p], si, sj, sk);
+      const double cs[3] = {D.a_cx[p], D.a_cy[p], D.a_cz[p]};
+      cafe_glb_centre(K, si, sj, sk, cs, c0);
       D.row_E[r] = E;
       D.row_m[r] = 0;
-      const double v = cafe_vh(D, K, p);
       const int bad = (cafe_v_ordinary(v) && fabs(E) != INFINITY) ? 0 : 2;
       const int slow = bad | (D.a_cls[p] != 1 ? 1 : 0);
       if (slow) atomicOr(&D.ctr[CTR_SLOW], slow);
     }
+    float lo = NAN;  // this lane's row
+    uint32_t liq = 0u;
+    for (int t = 0; t < n; ++t) {
+      const int pt = __shfl_sync(FULL, p, t), gt = __shfl_sync(FULL, gp, t);
+      float ct[3];
+      for (int a = 0; a < 3; ++a) ct[a] = __shfl_sync(FULL, c0[a], t);
+      bool liv = false;
+      if (lane < CAFE_NSLOT) {
+        const int q = D.a_nbr[(long long)pt * CAFE_NSLOT + lane];
+        liv = q >= 0 && D.a_state[q] == 1;
+      }
+      float l = 0.f, h = 0.f;
+      if (gt) {
+        const double *Rg = D.rot + 9LL * (gt - 1);
+        float R[9];
+        for (int a = 0; a < 9; ++a) R[a] = cafe_trunc_f32(Rg[a]);
+        if (liv) cafe_glb_slot(lane, ct, dx, R, l, h);
+        cafe_glb_range(liv, l, h);
+        gmax = fmaxf(gmax, h);  // (fmaxf drops NaN: such a row's times are NaN)
+      }
+      const uint32_t bl = __ballot_sync(FULL, liv);
+      if (lane == t) {
+        lo = gt ? l : NAN;
+        liq = bl;
+      }
+    }
+    // the rows that may be due are listed with their pairs
+    double tl = ((double)lo - E) * (v == V1 ? rV1 : 1.0 / v);
+    tl -= fabs(tl) * 0x1p-40;
+    const bool due = lane < n && (all || !gp || !(tl > lim));
+    const uint32_t work = due && gp ? liq : 0u;
+    const uint32_t bd = __ballot_sync(FULL, due);
+    int cnt = __popc(work), incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += u;
+    }
+    int base = 0, ib = 0;
+    if (lane == 31 && incl) base = atomicAdd(&D.ctr[CTR_NPAIRS], incl);
+    if (lane == 0 && bd) ib = atomicAdd(&D.ctr[CTR_NDUE], __popc(bd));
+    base = __shfl_sync(FULL, base, 31) + incl - cnt;
+    ib = __shfl_sync(FULL, ib, 0);
+    if (lane < n) {
+      const int r = r0 + lane;
+      if (due) {
+        D.row_due[ib + __popc(bd & ((1u << lane) - 1u))] = r;
+        for (uint32_t m = work; m; m &= m - 1) D.row_pairs[base++] = r * 32 + __ffs(m) - 1;
+        if (!gp)  // never captures
+          for (uint32_t m = liq; m; m &= m - 1) D.row_slot[(long long)r * CAFE_NSLOT + __ffs(m) - 1].g = NAN;
+      } else {
+        D.row_n[r] = CAFE_NO_RECORD;
+        D.row_glb[r] = lo;
+        D.row_key[r] = cafe_key(tl);
+      }
+    }
+    nkey += n - __popc(bd);
+    // magnitudes, rounded outwards to the keys' high words
+    const bool in = lane < n;
+    const uint32_t ekey = in && !cafe_is_nan(E) ? (uint32_t)(cafe_key(fabs(E)) >> 32) + 1u : 0u;  // NaN extents occur (the reference's 0/0)
+    const uint32_t vkey = (uint32_t)(cafe_key(v) >> 32);
+    const uint32_t e1 = __reduce_max_sync(FULL, ekey), v0 = __reduce_min_sync(FULL, in ? vkey : 0xffffffffu),
+                   v1 = __reduce_max_sync(FULL, in ? vkey + 1u : 0u);
+    if (lane == 0) {
+      if (gmax > 0.f) atomicMax(&mag[0], (uint32_t)(cafe_key((double)gmax) >> 32) + 1u);
+      atomicMax(&mag[1], e1);
+      atomicMin(&mag[2], v0);
+      atomicMax(&mag[3], v1);
+    }
   }
+  __syncthreads();
+  if (threadIdx.x < 4 && mag[2] != 0xffffffffu) {
+    const unsigned long long k = (unsigned long long)mag[threadIdx.x] << 32;
+    if (threadIdx.x == 2)
+      atomicMin(&D.row_mag[2], k);
+    else
+      atomicMax(&D.row_mag[threadIdx.x], k);
+  }
+  if (lane == 0 && nkey) atomicAdd(&D.ctr[CTR_NKEY], nkey);
 }
 __global__ void k_rows_prep(CafeDev D, CafeConsts K) {
   d_rows_prep(D, K, blockIdx.x, gridDim.x);
 }
 
 __device__ __forceinline__ void d_rows_geo(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
+  __shared__ CafeQuadScratch Q;
+  const int lane = threadIdx.x & 31;
   int n = D.ctr[CTR_NPAIRS];
   const long long cap = D.row_cap * CAFE_NSLOT;
   if (n > cap) n = (int)cap;
-  for (int i = cafe_bid * blockDim.x + threadIdx.x; i < n; i += cafe_nblk * blockDim.x) {
-    int v = D.row_pairs[i];
-    int r = v >> 5, sl = v & 31;
-    int p = D.row_pos[r];
-    int q = D.a_nbr[(long long)p * CAFE_NSLOT + sl];
-    const double *Rg = D.rot + 9LL * (D.a_gid[p] - 1);
-    double Rm[9];
-    for (int a = 0; a < 9; ++a) Rm[a] = Rg[a];
-    int i0, j0, k0, si, sj, sk;
-    cafe_cell_xyz(K, D.act[q], i0, j0, k0);
-    cafe_cell_xyz(K, D.act[p], si, sj, sk);
-    double cs[3] = {D.a_cx[p], D.a_cy[p], D.a_cz[p]};
-    double g, e, cn[3];
-    cafe_capture_geometry(K, i0, j0, k0, si, sj, sk, cs, Rm, &g, &e, cn);
-    long long o = (long long)r * CAFE_NSLOT + sl;
-    D.row_slot[o].g = g;  // by slot; k_rows_order sorts the record in place
-    double *og = D.row_geo + o * 4;
-    og[0] = e;
-    og[1] = cn[0];
-    og[2] = cn[1];
-    og[3] = cn[2];
+  for (int i0 = cafe_bid * 32; i0 < n; i0 += cafe_nblk * 32) {
+    const bool work = i0 + lane < n;
+    int ci = 0, cj = 0, ck = 0, si = 0, sj = 0, sk = 0;
+    double cs[3] = {0.0, 0.0, 0.0};
+    const double *Rg = D.rot;
+    long long o = 0;
+    if (work) {
+      const int v = D.row_pairs[i0 + lane], r = v >> 5, sl = v & 31, p = D.row_pos[r];
+      cafe_cell_xyz(K, D.act[p], si, sj, sk);
+      const int d27 = sl < 13 ? sl : sl + 1;
+      ci = si + d27 % 3 - 1;
+      cj = sj + d27 / 3 % 3 - 1;
+      ck = sk + d27 / 9 - 1;
+      Rg = D.rot + 9LL * (D.a_gid[p] - 1);
+      cs[0] = D.a_cx[p];
+      cs[1] = D.a_cy[p];
+      cs[2] = D.a_cz[p];
+      o = (long long)r * CAFE_NSLOT + sl;
+    }
+    const double g = cafe_geo_quad(K, work, ci, cj, ck, si, sj, sk, cs, Rg, Q, 1, D.row_geo + o * 4);
+    if (work && threadIdx.x < 32) D.row_slot[o].g = g;  // by slot; k_rows_order sorts the record in place
+    __syncthreads();  // the scratch is used again
   }
 }
-__global__ void k_rows_geo(CafeDev D, CafeConsts K) {
+__global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_rows_geo(CafeDev D, CafeConsts K) {
   d_rows_geo(D, K, blockIdx.x, gridDim.x);
 }
 
-// Also the magnitudes that bound the keys' rounding: the largest |g| and
-// extent, the smallest and the largest velocity over the rows (order keys, in row_mag).
 __device__ __forceinline__ void d_rows_order(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
-  int nrows = D.ctr[CTR_NROWS];
-  if (nrows > D.row_cap) nrows = (int)D.row_cap;
+  const int n = D.ctr[CTR_NDUE];
   const int warps = (cafe_nblk * blockDim.x) >> 5;
-  const int w = (cafe_bid * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  unsigned long long gk = 0ULL, ek = 0ULL, vk = CAFE_KEY_NONE, xk = 0ULL;
+  unsigned long long gk = 0ULL;
   const CafeChildList C = {&D.ctr[CTR_NCHILD], 0, D.ch_cap, K.DelT * CAFE_CHILD_REACH};
-  const unsigned long long due = cafe_key(K.DelT * CAFE_DUE_REACH);
-  int nkey = 0;  // (lane 0) rows with a candidate
-  for (int r = w; r < nrows; r += warps) {
-    int p = D.row_pos[r];
+  for (int i = (cafe_bid * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const int r = D.row_due[i], p = D.row_pos[r];
     int q = -1;
     bool liv = false;
     double gv = 0.0;
@@ -441,41 +611,20 @@ __device__ __forceinline__ void d_rows_order(const CafeDev &D, const CafeConsts 
       if (liv) gv = D.row_slot[(long long)r * CAFE_NSLOT + lane].g;
     }
     __syncwarp();  // the record is read before it is written in order
-    const double E = D.row_E[r], v = cafe_vh(D, K, p);
-    const unsigned long long ak = cafe_row_sort_warp(D, r, liv, gv, q, E, v, 0.0, D.a_gid[p], D.a_ruq[p], C, false);
-    gk = max(gk, ak);
-    __syncwarp();
-    if (!cafe_is_nan(E)) ek = max(ek, cafe_key(fabs(E)));  // NaN extents occur (the reference's 0/0)
-    // rows that can capture soon are listed for the event loop's first window
-    if (lane == 0) {
-      const unsigned long long key = D.row_key[r];
-      if (key != CAFE_KEY_NONE) ++nkey;
-      if (key <= due) {
-        const int i = atomicAdd(&D.ctr[CTR_NDUE], 1);
-        if (i < CAFE_DUE_MAX) D.row_due[i] = r;
-      }
-    }
-    vk = min(vk, cafe_key(v));
-    xk = max(xk, cafe_key(v));
+    gk = max(gk, cafe_row_sort_warp(D, r, liv, gv, q, D.row_E[r], cafe_vh(D, K, p), 0.0, D.a_gid[p], D.a_ruq[p], C, false));
   }
-  if (lane == 0 && w < nrows) {
-    atomicMax(&D.row_mag[0], gk);
-    atomicMax(&D.row_mag[1], ek);
-    atomicMin(&D.row_mag[2], vk);
-    atomicMax(&D.row_mag[3], xk);
-    if (nkey) atomicAdd(&D.ctr[CTR_NKEY], nkey);
-  }
+  if (lane == 0 && gk) atomicMax(&D.row_mag[0], gk);
 }
 __global__ void k_rows_order(CafeDev D, CafeConsts K) {
   d_rows_order(D, K, blockIdx.x, gridDim.x);
 }
 
 // The rows of foreseen captures, one per block of four warps: generation `depth`
-// lists the next one (in CTR_NCHILD + depth + 1) up to CAFE_CHILD_DEPTH. An
+// lists the next one (in CTR_NCHILD + depth + 1) up to ndepth <= CAFE_CHILD_DEPTH. An
 // event's chain of dependent captures within one step is rarely longer; a row
 // that is not foreseen is filled by the event loop itself.
 #define CAFE_CHILD_BLOCKS_PER_SM 4
-__device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K, int depth, const int cafe_bid, const int cafe_nblk) {
+__device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K, int depth, int ndepth, const int cafe_bid, const int cafe_nblk) {
   __shared__ CafeQuadScratch Q;
   __shared__ CafeNewCell nc;
   int off = 0, n = 0;
@@ -485,7 +634,8 @@ __device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K
   }
   const int last = off + n;
   const CafeChildList C = {&D.ctr[CTR_NCHILD + min(depth + 1, CAFE_CHILD_DEPTH - 1)], last,
-                           depth + 1 < CAFE_CHILD_DEPTH ? D.ch_cap : last, K.DelT * CAFE_CHILD_REACH};
+                           depth + 1 < ndepth ? D.ch_cap : last, K.DelT * CAFE_CHILD_REACH};
+  const int lane = threadIdx.x & 31;
   for (int i = off + cafe_bid; i < last; i += cafe_nblk) {
     const long long id = D.row_cap + i;
     const int p = D.row_pos[id];
@@ -496,13 +646,44 @@ __device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K
       nc.gid = D.ch_gid[i];
     }
     __syncthreads();
-    const unsigned long long gk = cafe_row_fill_quad(D, K, id, p, D.ch_T[i], Q, nc, C);
+    // (every warp evaluates the bound)
+    const double T = D.ch_T[i], v = cafe_vh(D, K, p);
+    bool liv = false;
+    if (lane < CAFE_NSLOT) {
+      const int q = D.a_nbr[(long long)p * CAFE_NSLOT + lane];
+      liv = q >= 0 && D.a_state[q] == 1;
+    }
+    bool due = true;
+    double tl = 0.0;
+    float lo = 0.f, hi = 0.f;
+    if (nc.gid >= 1 && nc.gid <= D.grain_cap) {
+      int si, sj, sk;
+      cafe_cell_xyz(K, D.act[p], si, sj, sk);
+      const double *Rg = D.rot + 9LL * (nc.gid - 1);
+      float R[9], c0[3];
+      for (int a = 0; a < 9; ++a) R[a] = cafe_trunc_f32(Rg[a]);
+      const float dx = (float)K.dx[0];
+      cafe_glb_centre(K, si, sj, sk, nc.c, c0);
+      if (liv) cafe_glb_slot(lane, c0, dx, R, lo, hi);
+      cafe_glb_range(liv, lo, hi);
+      tl = cafe_lb_time(lo, nc.ext, v);
+      due = K.all_rows || !(T + tl > K.DelT * CAFE_DUE_REACH) || !cafe_v_ordinary(v);
+    }
+    unsigned long long gk = 0ULL;
+    if (due) {
+      gk = cafe_row_fill_quad(D, K, id, p, T, Q, nc, C);
+    } else if (threadIdx.x == 0) {
+      D.row_n[id] = CAFE_NO_RECORD;
+      D.row_glb[id] = lo;
+      if (hi > 0.f) gk = cafe_key((double)hi);
+    }
+    __syncthreads();  // (every warp has read ch_T)
     if (threadIdx.x == 0) {
       D.row_key[id] = CAFE_KEY_NONE;  // until the row exists
       D.row_m[id] = CAFE_M_DONE;  // (set when it leaves the resident set)
+      D.ch_T[i] = tl;  // from here on: the bound of the time from its capture to its first
       atomicMax(&D.row_mag[0], gk);
       if (!cafe_is_nan(nc.ext)) atomicMax(&D.row_mag[1], cafe_key(fabs(nc.ext)));
-      const double v = cafe_vh(D, K, p);
       if (cafe_v_ordinary(v)) {
         atomicMin(&D.row_mag[2], cafe_key(v));
         atomicMax(&D.row_mag[3], cafe_key(v));
@@ -511,8 +692,8 @@ __device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_children(const __grid_constant__ CafeDev D, const __grid_constant__ CafeConsts K, int depth) {
-  d_children(D, K, depth, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_children(const __grid_constant__ CafeDev D, const __grid_constant__ CafeConsts K, int depth, int ndepth) {
+  d_children(D, K, depth, ndepth, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------------ event loop
@@ -548,7 +729,8 @@ __global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_children(const __grid_con
 // window. Rows with another velocity than the step's class-1 velocity switch the
 // step to per-row velocities (PR); a velocity that is not positive and finite,
 // or a window that does not fit, to the full scan of every row per event.
-#define CAFE_RES_MAX 768  // resident rows
+#define CAFE_RES_MAX 640  // resident rows
+#define CAFE_QUADS 4  // groups of four warps that fill rows side by side
 #define CAFE_RES_TARGET 320  // rows an opened window aims at: one per thread with room for the step's new rows
 #define CAFE_OPEN_TRIES 48   // windows in a row without an event before the step takes the full scan
 #define CAFE_WARPS (CAFE_LOOP_THREADS / 32)
@@ -591,9 +773,11 @@ struct CafeResident {
   double wd[CAFE_WARPS];
   unsigned long long wk[CAFE_WARPS], wrk[CAFE_WARPS], thr[32];  // full keys of the close ones
   int hist[32];
-  int top, nfree, newslot, overflow, sink[32];
+  int top, nfree, newslot, overflow, nfill, sink[32];
   uint32_t klim[2];  // [e & 1]: a smallest key below it needs no further test at event e
   unsigned long long kw;    // rows with keys at or below it are resident
+  double slack;             // rounding bound of the keys
+  int outside;              // the row created by this event stays outside the set
   double wlim, dsum_cap;    // latest safe T + t; the window holds while dsum <= dsum_cap and ev <= ev_cap
   int ev_cap, all;          // all: every row with a candidate is resident
   CafeCand red[CAFE_WARPS];
@@ -745,9 +929,27 @@ __device__ __noinline__ void cafe_load_resident(const CafeDev &D, const CafeCons
   }
 }
 
+// The record of row r, made by the four warps that call it together (its cell's
+// grain, centre and extent are in the active list).
+__device__ __forceinline__ void cafe_make_record(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeQuadScratch *Q, int r) {
+  const int quad = threadIdx.x >> 7, p = D.row_pos[r];
+  CafeNewCell &nc = Q[quad].nc;
+  if ((threadIdx.x & 127) == 0) {
+    nc.gid = D.a_gid[p];
+    nc.ext = D.row_E[r];
+    nc.c[0] = D.a_cx[p];
+    nc.c[1] = D.a_cy[p];
+    nc.c[2] = D.a_cz[p];
+  }
+  cafe_bar_quad(1 + quad);
+  const CafeChildList none = {nullptr, 0, 0, 0.0};
+  cafe_row_fill_quad(D, K, r, p, L.tinc, Q[quad], nc, none, 1 + quad);
+  cafe_bar_quad(1 + quad);  // (the scratch is used again)
+}
+
 // Opens the window: the earliest rows by key become resident.
 template <bool PR>
-__device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev, int tries) {
+__device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, CafeQuadScratch *Q, int ev, int tries) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   const unsigned FULL = 0xffffffffu;
@@ -755,11 +957,13 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
   cafe_res_flush<PR>(D, K, L, S, ev, true);
   __syncthreads();
-  // the first window takes its rows from the list of those that are due
+  // the first window takes its rows from the list of those that may be due
   // soon (k_rows_order), later ones from all rows of the step
-  const bool first = ev == 0 && tries == 1 && D.ctr[CTR_NDUE] <= CAFE_DUE_MAX;
+  const bool first = ev == 0 && tries == 1;
   const int nrows0 = L.nrows0, nrows = first ? D.ctr[CTR_NDUE] : L.nrows;
   auto row_at = [&](int k) -> int { return first ? D.row_due[k] : cafe_row_at(D, nrows0, k); };
+  // (a row without a record has to be filled: it counts for twenty)
+  auto weight = [&](int r) -> int { return D.row_n[r] == CAFE_NO_RECORD ? 20 : 1; };
   unsigned long long mn = CAFE_KEY_NONE;
   int cnt = 0;
   for (int r0 = tid; r0 < nrows; r0 += 8 * NT) {
@@ -769,7 +973,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       mn = min(mn, kk[u]);
-      cnt += kk[u] != CAFE_KEY_NONE;
+      if (kk[u] != CAFE_KEY_NONE) cnt += weight(row_at(r0 + u * NT));
     }
   }
   int src;
@@ -780,6 +984,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     S.wi[warp] = cnt;
   }
   if (tid < 32) S.hist[tid] = 0;
+  if (tid == 0) S.nfill = 0;  // (rows in the first bin)
   for (int i = tid; i < CAFE_RES_MAX; i += NT) {
     S.g[i] = NAN;
     S.q[i] = S.r[i] = -1;
@@ -789,7 +994,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   mn = cafe_warp_min_key(lane < NW ? S.wk[lane] : CAFE_KEY_NONE, src);
   cnt = __reduce_add_sync(FULL, lane < NW ? S.wi[lane] : 0);
   // the rows that are not listed have keys above this bound
-  const unsigned long long kdue = first && D.ctr[CTR_NKEY] > cnt ? cafe_key(K.DelT * CAFE_DUE_REACH) : CAFE_KEY_NONE - 1;
+  const unsigned long long kdue = first && D.ctr[CTR_NKEY] > 0 ? cafe_key(K.DelT * CAFE_DUE_REACH) : CAFE_KEY_NONE - 1;
   const bool all = cnt <= CAFE_RES_TARGET;
   // rounding bound of the keys for the next 4096 events and 64 DelT of growth
   const double dcap = L.dsum + 64.0 * K.DelT;
@@ -808,14 +1013,16 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     __syncthreads();
     const unsigned long long last = S.thr[31];
     for (int r = tid; r < nrows; r += NT) {
-      const unsigned long long k = D.row_key[row_at(r)];
+      const int rr = row_at(r);
+      const unsigned long long k = D.row_key[rr];
       if (k > last) continue;
       int lo = 0, hi = 31;  // first threshold at or above the key
       while (lo < hi) {
         const int md = (lo + hi) >> 1;
         if (k <= S.thr[md]) hi = md; else lo = md + 1;
       }
-      atomicAdd(&S.hist[lo], 1);
+      atomicAdd(&S.hist[lo], weight(rr));
+      if (lo == 0) atomicAdd(&S.nfill, 1);
     }
     __syncthreads();
     int h = S.hist[lane];
@@ -826,8 +1033,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     const uint32_t fits = __ballot_sync(FULL, h <= CAFE_RES_TARGET);
     // the counts ascend: the last threshold that fits the target, else the first if it fits at all
     pick = fits ? 31 - __clz(fits) : 0;
-    const int n0 = __shfl_sync(FULL, h, 0);
-    if (tid == 0) S.overflow = !fits && n0 > CAFE_RES_MAX - 64;
+    if (tid == 0) S.overflow = !fits && S.nfill > CAFE_RES_MAX - 64;
   }
   const unsigned long long kw = min(kdue, all ? CAFE_KEY_NONE - 1 : S.thr[pick]);
   const bool every = kw == CAFE_KEY_NONE - 1;
@@ -842,6 +1048,8 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     S.ev_cap = ev + 4096;
     S.dsum_cap = dcap;
     S.wlim = every ? INFINITY : cafe_unkey(kw) - slack;
+    S.slack = slack;
+    S.nfill = 0;
     L.opens++;
     S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, L.dsum);
   }
@@ -851,9 +1059,15 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     const int r = row_at(k);
     if (D.row_key[r] <= kw) {
       const int i = atomicAdd(&S.top, 1);
-      if (i < CAFE_RES_MAX) S.r[i] = r;
+      if (i < CAFE_RES_MAX) {
+        S.r[i] = r;
+        if (D.row_n[r] == CAFE_NO_RECORD) S.free[atomicAdd(&S.nfill, 1)] = (unsigned short)i;
+      }
     }
   }
+  __syncthreads();
+  // the records that were not made, four rows at a time
+  for (int j = warp >> 2; j < S.nfill; j += CAFE_QUADS) cafe_make_record(D, K, L, Q, S.r[S.free[j]]);
   __syncthreads();
   {
     const int top = S.top;
@@ -892,7 +1106,7 @@ __device__ __noinline__ void cafe_select_exact(const CafeDev &D, const CafeConst
 // A negative event may clamp a small extent at zero (VoxelsCA.C:515),
 // which breaks the key bound of a row outside the set: the rows whose
 // extrapolated extent comes near zero are brought up to date with a new key
-// (true: one of them may be due before the window's end).
+// (true: one of them may be due within the step).
 template <bool PR>
 __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -907,7 +1121,7 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
   const double g0 = vsp + vd;
   const double need = PR ? (g0 >= 0.0 ? margin - g0 * L.vmin : margin - g0 * L.vmax) : margin - g0;
   const long long thr0 = need > 0.0 ? crm_bits(need * (1.0 + 0x1p-40)) : 0;
-  bool again = false;
+  unsigned long long near = CAFE_KEY_NONE;  // smallest new key
   const int nrows = L.nrows, nrows0 = L.nrows0;
   for (int k0 = tid; k0 < nrows; k0 += 8 * NT) {
     int rr[8], mm[8];
@@ -942,23 +1156,36 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
     const double En = cafe_row_replayed<PR>(D, r, ev, v, stop);
     D.row_E[r] = En;
     D.row_m[r] = stop < ev ? CAFE_M_DONE : ev;  // (a row that stopped growing keeps its extent)
-    const int k = cafe_row_next(D, r, D.row_k[r]);
-    D.row_k[r] = (uint8_t)k;
-    if (k < D.row_n[r]) {
-      const double t = (D.row_slot[(long long)r * CAFE_NSLOT + k].g - En) / v;
-      const unsigned long long key = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
-      D.row_key[r] = key;
-      again = again || key <= S.kw;
+    double t = NAN;
+    if (D.row_n[r] == CAFE_NO_RECORD) {
+      t = cafe_lb_time(D.row_glb[r], En, v);
+    } else {
+      const int k = cafe_row_next(D, r, D.row_k[r]);
+      D.row_k[r] = (uint8_t)k;
+      if (k < D.row_n[r]) t = (D.row_slot[(long long)r * CAFE_NSLOT + k].g - En) / v;
     }
+    const unsigned long long key = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
+    D.row_key[r] = key;
+    if (key < near) near = key;
     }
   }
-  return __syncthreads_or(again);
+  // one of them due within the step: a new window; else the window ends before it
+  if (__syncthreads_or(near <= cafe_key(K.DelT * CAFE_SHORT_REACH))) return true;
+  if (near < S.kw) atomicMin(&S.kw, near);
+  __syncthreads();
+  if (tid == 0 && S.kw < CAFE_KEY_NONE - 1) {
+    S.all = 0;
+    S.wlim = fmin(S.wlim, cafe_unkey(S.kw) - S.slack);
+    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, L.dsum);
+  }
+  __syncthreads();
+  return false;
 }
 
 // The captured cell's own row when it was not foreseen, or found no room in the
 // resident set (true: open a new window).
 template <bool PR>
-__device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, CafeQuadScratch &Q, int ev, int icap) {
+__device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, CafeQuadScratch *Q, int ev, int icap) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   const unsigned FULL = 0xffffffffu;
@@ -978,7 +1205,7 @@ __device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K,
   __syncthreads();
   if (warp < CAFE_QUAD_THREADS / 32) {
     const CafeChildList none = {nullptr, 0, 0, 0.0};
-    const unsigned long long gk = cafe_row_fill_quad(D, K, nr, icap, L.tinc, Q, L.nc, none);
+    const unsigned long long gk = cafe_row_fill_quad(D, K, nr, icap, L.tinc, Q[0], L.nc, none);
     if (tid == 0) {
       D.row_E[nr] = L.nc.ext;
       if (gk != 0ULL) L.gmax = fmax(L.gmax, cafe_unkey(gk));
@@ -1002,7 +1229,7 @@ __device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K,
 // scan (every row's extent and place are then in the row arrays).
 template <bool PR>
 __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const CafeConsts &K, long long max_events,
-                                                     CafeLoop &L, CafeResident &S, CafeQuadScratch &Q,
+                                                     CafeLoop &L, CafeResident &S, CafeQuadScratch *Q,
                                                      const CafeDev &sD, const CafeConsts &sK) {
   const unsigned FULL = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1023,7 +1250,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       // ---- open the window: the earliest rows by key
       need_open = false;
       ++tries;
-      cafe_window_open<PR>(sD, sK, L, S, ev, tries);
+      cafe_window_open<PR>(sD, sK, L, S, Q, ev, tries);
       if (tid == 0) {
         const long long t1 = clock64();
         L.cyc[3] += t1 - t0;
@@ -1170,7 +1397,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       const bool nuc = L.unext[ev & 1] < cafe_nuc_rate_at(D, K, icap);
       const bool foreseen = child >= 0 && !nuc;
       if (foreseen) {
-        cn = D.row_n[child];
+        cn = D.row_n[child];  // (the record's entries are not valid when there is none)
         if (lane < CAFE_NSLOT) cr = D.row_slot[(long long)child * CAFE_NSLOT + lane];
       }
       if (lane >= CAFE_NSLOT && lane < 30) gx = D.row_geo[((long long)wr * CAFE_NSLOT + (wm & 31u)) * 4 + lane - 26];
@@ -1179,8 +1406,9 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       const int cls = D.a_cls[icap];
       const double vq = PR ? cafe_vh(D, K, icap) : V;
       // level 2: which of its neighbours (all but the captured ones) are left
+      const bool rec = foreseen && cn != CAFE_NO_RECORD;
       bool left = false;
-      if (foreseen) {
+      if (rec) {
         left = lane < cn && D.a_ev[cr.q] == 0;
       } else if (lane < CAFE_NSLOT) {
         const int q = D.a_nbr[(long long)icap * CAFE_NSLOT + lane];
@@ -1191,7 +1419,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       const int row = foreseen ? child : cnr;
       // the captured cell's own row: a foreseen one enters the resident set at once
       int ci = -1;
-      if (grows && foreseen && room) {
+      if (grows && rec && room) {
         const int nf = S.nfree, tp = S.top;
         __syncwarp();
         if (nf > 0) {
@@ -1231,6 +1459,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         if (lane < 30) {
           gd[icap] = gx;
           *sd = gx;
+          if (lane == 26 && foreseen && !rec) D.row_E[child] = gx;
           if (lane == 26 && fabs(gx) == INFINITY) L.sw = 1;  // its times need the full scan
         } else if (lane == 30) {
           D.a_gid[icap] = gcap;
@@ -1247,7 +1476,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
           L.done = 1;
         }
         L.newrow = grows && room ? row : -1;
-        L.fill = !foreseen;
+        L.fill = !rec;
         S.newslot = ci;
         if (grows) {
           if (room) {
@@ -1292,6 +1521,20 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       L.dsum = dsum;
       D.ev_vs[ev] = vs;
       if (cafe_is_neg(dt)) L.negdt++;
+      // a foreseen row that is not due within the step stays outside the set, and
+      // the window ends before its key
+      int out = 0;
+      if (child >= 0 && !nuc && D.row_n[child] == CAFE_NO_RECORD) {
+        const double kc = tinc + D.ch_T[child - (int)D.row_cap];
+        if (kc > K.DelT * CAFE_OUTSIDE_REACH) {
+          out = 1;
+          D.row_key[child] = cafe_key(kc);
+          S.kw = min(S.kw, cafe_key(kc));
+          S.wlim = fmin(S.wlim, kc - S.slack);
+          S.all = 0;
+        }
+      }
+      S.outside = out;
       S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, tinc, dsum);
     } else if (tid == CAFE_DRAW_WARP * 32) {
       // the next event's draw (VoxelsCA.C:483; two engine outputs per event)
@@ -1311,9 +1554,13 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         int x = 0;  // (kept, so that the loads are)
         if (lane < CAFE_NSLOT) {
           if (c2 >= 0) {
-            const int n2 = D.row_n[c2];
-            const CafeSlot cs = D.row_slot[(long long)c2 * CAFE_NSLOT + lane];
-            x = D.a_ev[cs.q] + (int)cs.m + __double2hiint(cs.g) + (int)cs.rk + n2;
+            if (D.row_n[c2] != CAFE_NO_RECORD) {
+              const CafeSlot cs = D.row_slot[(long long)c2 * CAFE_NSLOT + lane];
+              x = D.a_ev[cs.q] + (int)cs.m + __double2hiint(cs.g) + (int)cs.rk;
+            } else {
+              x = D.a_nbr[(long long)q2 * CAFE_NSLOT + lane];
+              if (x >= 0) x = D.a_state[x];
+            }
           }
         } else if (lane < 30) {
           x = __double2hiint(D.row_geo[((long long)r2 * CAFE_NSLOT + (S.wm[s2] & 31u)) * 4 + lane - 26]);
@@ -1361,7 +1608,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     }
     // ---- events with more to do than the row that was foreseen
     if (cafe_is_neg(L.vd) && cafe_negative_event<PR>(sD, sK, L, S, ev)) need_open = true;
-    if (L.newrow >= 0 && born < 0) {
+    if (L.newrow >= 0 && born < 0 && !S.outside) {
       if (cafe_new_row<PR>(sD, sK, L, S, Q, ev, icap)) need_open = true;
       if (tid == 0) {
         const long long t1 = clock64();
@@ -1386,12 +1633,17 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
 // The reference's scan of every row per event: from the start (mode 2), or where
 // the resident loop stopped with L.sw.
 __device__ __noinline__ void cafe_events_scan(const CafeDev &D, const CafeConsts &K, long long max_events, CafeLoop &L,
-                                              CafeResident &S, CafeQuadScratch &Q, int mode) {
+                                              CafeResident &S, CafeQuadScratch *Q, int mode) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   if (L.done || !(mode == 2 || L.sw)) return;
   {
-    // extents are kept current from here on
+    // every row needs its record, and extents are kept current from here on
+    for (int k = warp >> 2; k < L.nrows; k += CAFE_QUADS) {
+      const int r = cafe_row_at(D, L.nrows0, k);
+      if (D.row_n[r] == CAFE_NO_RECORD) cafe_make_record(D, K, L, Q, r);
+    }
+    __syncthreads();
     const int e0 = L.ev;
     for (int k = tid; k < L.nrows; k += NT) {
       const int r = cafe_row_at(D, L.nrows0, k);
@@ -1511,7 +1763,7 @@ __device__ __noinline__ void cafe_events_scan(const CafeDev &D, const CafeConsts
           D.row_new[r - L.nrows0] = r;
         }
         const CafeChildList none = {nullptr, 0, 0, 0.0};
-        cafe_row_fill_quad(D, K, r, icap, L.tinc, Q, L.nc, none);
+        cafe_row_fill_quad(D, K, r, icap, L.tinc, Q[0], L.nc, none);
         if (tid == 0) L.nrows = r + 1;
       } else if (tid == 0) {
         atomicOr(D.err, CAFE_ERR_ROW_CAP);
@@ -1525,7 +1777,7 @@ __device__ __noinline__ void cafe_events_scan(const CafeDev &D, const CafeConsts
 __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, long long max_events, int allow_fast, const int cafe_bid, const int cafe_nblk) {
   __shared__ CafeLoop L;
   __shared__ CafeResident S;
-  __shared__ CafeQuadScratch Q;
+  __shared__ CafeQuadScratch Q[CAFE_QUADS];
   __shared__ CafeDev sD;
   __shared__ CafeConsts sK;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -871,11 +871,14 @@ int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
     k_scan_pairs<<<1, 1024, 0, st>>>(D.blk, s->nblk_pos, D.ctr + CTR_NA, D.ctr + CTR_NVS2, D.ctr + CTR_NROWS);
     k_lists_scatter<<<nbp, CAFE_DENSE_THREADS, 0, st>>>(D);
     k_rows_prep<<<s->gsm * 4, 256, 0, st>>>(D, K);
-    k_rows_geo<<<s->gsm * 8, 256, 0, st>>>(D, K);
+    k_rows_geo<<<s->gsm * 4, CAFE_QUAD_THREADS, 0, st>>>(D, K);
     k_rows_order<<<s->gsm * 4, 256, 0, st>>>(D, K);
-    for (int d = 0; d < CAFE_CHILD_DEPTH; ++d)
-      k_children<<<s->gsm * CAFE_CHILD_BLOCKS_PER_SM, CAFE_QUAD_THREADS, 0, st>>>(D, K, d);
-    LAUNCHED(CAFE_PH_GATHER, 7 + CAFE_CHILD_DEPTH);
+    // two generations of foreseen captures: a third one costs a launch of ~28 us
+    // and saves the event loop less (76 cycles an event against ~250)
+    const int ndepth = 2;
+    for (int d = 0; d < ndepth; ++d)
+      k_children<<<s->gsm * CAFE_CHILD_BLOCKS_PER_SM, CAFE_QUAD_THREADS, 0, st>>>(D, K, d, ndepth);
+    LAUNCHED(CAFE_PH_GATHER, 7 + ndepth);
   }
   {
     PhaseScope ps(s, CAFE_PH_EVENTS);
@@ -1091,6 +1094,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
   K.tmodel = g.EASM_Flag == 1 ? 1 : (g.rosenthal ? 2 : 0);
   K.easm = K.tmodel != 0;
   K.Avel = g.Avel;
+  K.all_rows = s->event_scan != 0;
   K.nvel_i = 0;
   {
     const double pi = 3.14159265358979323846;
@@ -1196,7 +1200,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
       (rc = dalloc(&D.row_new, D.row_cap, o)) || (rc = dalloc(&D.ch_src, D.ch_cap, o)) ||
       (rc = dalloc(&D.ch_gid, D.ch_cap, o)) || (rc = dalloc(&D.ch_T, D.ch_cap, o)) ||
       (rc = dalloc(&D.row_pairs, (size_t)D.row_cap * CAFE_NSLOT, o)) || (rc = dalloc(&D.blk, D.blk_cap, o)) ||
-      (rc = dalloc(&D.row_E, nrow, o)) || (rc = dalloc(&D.row_m, nrow, o)) || (rc = dalloc(&D.row_due, CAFE_DUE_MAX, o)) ||
+      (rc = dalloc(&D.row_E, nrow, o)) || (rc = dalloc(&D.row_m, nrow, o)) || (rc = dalloc(&D.row_due, D.row_cap, o)) || (rc = dalloc(&D.row_glb, nrow, o)) ||
       (rc = dalloc(&D.row_key, nrow, o)) || (rc = dalloc(&D.row_mag, 4, o)) ||
       (rc = dalloc(&D.ev_vd, D.ev_cap, o)) || (rc = dalloc(&D.ev_vs, D.ev_cap, o)) || (K.nuc_gauss && (rc = dalloc(&D.a_nuc, acap, o))) ||
       (rc = dalloc(&D.ctr, CTR_COUNT, o)) || (rc = dalloc(&D.err, 1, o)) || (rc = dalloc(&D.stat, STAT_COUNT, o)) ||
@@ -2328,7 +2332,7 @@ struct CafeBatchEngine {
 namespace {
 
 const int kBatchThreads[BK_COUNT] = {32, 256, 256, CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 32, 256,
-                                     CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256, 256, 256,
+                                     CAFE_DENSE_THREADS, 1024, CAFE_DENSE_THREADS, 256, CAFE_QUAD_THREADS, 256,
                                      CAFE_QUAD_THREADS, CAFE_QUAD_THREADS, CAFE_QUAD_THREADS,
                                      CAFE_LOOP_THREADS, 256, 256, 256, 32};
 
@@ -2343,7 +2347,8 @@ long long batch_blocks(const cafe_sim *s, int kind, int loop_blocks) {
     case BK_CHILD0: case BK_CHILD1: case BK_CHILD2: return g * CAFE_CHILD_BLOCKS_PER_SM;
     case BK_PREP: case BK_ORDER: case BK_FINAL: return g * 4;
     case BK_ACOUNT: case BK_ASCATTER: return std::max<long long>(1, std::min<long long>(s->nblk_act, g * 8));
-    case BK_GATHER: case BK_GEO: case BK_WB: case BK_M2S: return g * 8;
+    case BK_GEO: return g * 4;
+    case BK_GATHER: case BK_WB: case BK_M2S: return g * 8;
     case BK_LCOUNT: case BK_LSCATTER: return std::max<long long>(1, std::min<long long>(s->nblk_pos, g * 4));
     default: return 1;  // resets, scans, the report
   }
