@@ -72,6 +72,7 @@ struct CafeConsts {
   double hLX0, hLX1;  // LX/2
   double a1[6];       // TempField::a1 (TempField.C:69-76)
   double bmDX0;       // DelT * bmV
+  float ra1[6];       // reciprocals of a1 (k_melt)
   double tL, tS, T0, xi;
   double Tcls[3];     // temperature per class: 0 = T0 (above laser plane), 1 = tS, 2 = xi
   double vhat_cls[3]; // growth velocity per class (VoxelsCA.C:405), host libm pow

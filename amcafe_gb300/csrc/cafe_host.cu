@@ -799,7 +799,7 @@ int launch_melt(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
     if (s->K.easm)
       k_melt_easm<<<grid_blocks(nbox, 256, s), 256, 0, s->stream>>>(s->D, s->K, P);
     else
-      k_melt<<<graph ? s->gsm * 16 : grid_blocks(nbox, 256, s), 256, 0, s->stream>>>(s->D, s->K, Pp);
+      k_melt<<<s->gsm * 4, 256, 0, s->stream>>>(s->D, s->K, Pp);
     LAUNCHED(CAFE_PH_MELT, 1);
   }
   CUDA_TRY(cudaGetLastError());
@@ -1071,6 +1071,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
   K.a1[4] = K.a1[1];
   K.a1[5] = K.a1[2];
   K.bmDX0 = s->DelT * g.bmV;
+  for (int a = 0; a < 6; ++a) K.ra1[a] = (float)(1.0 / K.a1[a]);
   K.tL = g.tL;
   K.tS = g.tS;
   K.T0 = g.T0;
@@ -2342,7 +2343,7 @@ long long batch_blocks(const cafe_sim *s, int kind, int loop_blocks) {
   const long long g = s->gsm;
   switch (kind) {
     case BK_LOOP: return loop_blocks;
-    case BK_MELT: return g * 16;
+    case BK_MELT: return g * 4;
     case BK_S2M: return g * 8;
     case BK_CHILD0: case BK_CHILD1: case BK_CHILD2: return g * CAFE_CHILD_BLOCKS_PER_SM;
     case BK_PREP: case BK_ORDER: case BK_FINAL: return g * 4;

@@ -96,32 +96,70 @@ __device__ __forceinline__ int cafe_moore(const CafeConsts &K, int i, int j, int
 }
 
 // ------------------------------------------------------------------ K: melt
-// Over the box where T may reach the liquidus: SetLiquid3 and BuildjID.
+// Over the box where T may reach the liquidus: SetLiquid3 and BuildjID, a warp
+// per row of the box. A cell's class is a test of two or three quotients against
+// one, so single precision decides all cells but those near the pool's
+// surface, which take the FP64 evaluation: with it for every cell the pass was
+// bound by FP64 issue (three divisions a cell; 88 us a step for the rotated pool
+// of the 1024x1024x256 deck).
 __device__ __forceinline__ void d_melt(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, const int cafe_bid, const int cafe_nblk) {
   const CafeStepParams P = *Pp;
-  int bx = P.hi[0] - P.lo[0], by = P.hi[1] - P.lo[1], bz = P.hi[2] - P.lo[2];
-  long long nbox = (long long)bx * by * bz;
-  long long iz1 = (long long)P.ilaserLoc * K.nxy;
+  const int bx = P.hi[0] - P.lo[0], by = P.hi[1] - P.lo[1], bz = P.hi[2] - P.lo[2];
+  const int lane = threadIdx.x & 31, warps = (cafe_nblk * blockDim.x) >> 5;
+  const long long iz1 = (long long)P.ilaserLoc * K.nxy;
   int any = 0;
-  for (long long t = cafe_bid * (long long)blockDim.x + threadIdx.x; t < nbox;
-       t += (long long)cafe_nblk * blockDim.x) {
-    int i = P.lo[0] + (int)(t % bx);
-    long long r = t / bx;
-    int j = P.lo[1] + (int)(r % by);
-    int k = P.lo[2] + (int)(r / by);
-    int c = cafe_temp_class_exact(K, P, i, j, k);
-    D.tcls[t] = (uint8_t)c;
-    long long idx = (long long)K.nxy * k + (long long)K.nx * j + i;
-    if (K.gt_cls[c]) D.buildj[idx] = 1;
-    if (K.hot_cls[c]) {
-      any = 1;
-      if (idx < K.nxy) {
-        D.state[idx] = 2;
-      } else if (idx < iz1) {
-        D.state[idx] = 1;
-        D.gid[idx] = 0;
+  const float fux = (float)(P.cg * K.dx[0]), fwx = (float)(-P.sg * K.dx[0]);
+  const float i1 = K.ra1[1], i2 = K.ra1[2], i3 = K.ra1[3], i4 = K.ra1[4], i5 = K.ra1[5];
+  const float imax = fmaxf(fmaxf(fmaxf(fabsf(i1), fabsf(i2)), fmaxf(fabsf(i3), fabsf(i4))), fabsf(i5));
+  const float front = (float)K.bmDX0;
+  // (the sign of dirp r0 is that of the factors unless the product underflows)
+  const bool ok = imax < 1e30f && (P.dirp == 0.0 || fabs(P.dirp) > 1e-200) && !P.any_hot_full;
+  const float sd = P.dirp > 0.0 ? 1.f : (P.dirp < 0.0 ? -1.f : 0.f);
+  for (int row = (cafe_bid * blockDim.x + threadIdx.x) >> 5; row < by * bz; row += warps) {
+    const int j = P.lo[1] + row % by, k = P.lo[2] + row / by;
+    const double zp = ((double)k + .5) * K.dx[2], y0 = ((double)j + .5) * K.dx[1];
+    const double X = ((double)P.lo[0] + .5) * K.dx[0] - K.hLX0, Y = y0 - K.hLX1;
+    const float u0 = (float)(P.cg * X + P.sg * Y + K.hLX0 - P.lx), w0 = (float)(-P.sg * X + P.cg * Y + K.hLX1 - P.ly);
+    const float r2 = (float)(zp - P.lz);
+    const bool above = zp > P.lz;
+    // coordinates relative to the laser, in error by at most eu (roundings to single
+    // precision of the row's first and along it), quotients by eq
+    const float eu = 0x1p-21f * (fabsf(u0) + fabsf(w0) + fabsf(r2) + (fabsf(fux) + fabsf(fwx)) * (float)bx);
+    const float eq = eu * imax, amb = 16.f * eq + 1e-5f;
+    const bool usable = ok && eq < 0.01f;
+    const long long base = (long long)K.nxy * k + (long long)K.nx * j + P.lo[0];
+    for (int x = lane; x < bx; x += 32) {
+      int c = -1;
+      if (above) {
+        c = 0;
+      } else if (usable) {
+        const float u = u0 + fux * (float)x, w = w0 + fwx * (float)x;
+        const float du = sd * u;
+        if (fabsf(u) > 2.f * eu || sd == 0.f) {
+          const bool ahead = du > 0.f;
+          const float q1 = w * (ahead ? i1 : i4), q2 = r2 * (ahead ? i2 : i5), q0 = ahead ? 0.f : u * i3;
+          const float d = q0 * q0 + q1 * q1 + q2 * q2;
+          if (d > 1.f + amb || (ahead && fabsf(u) > front + 2.f * eu))
+            c = 1;
+          else if (d < 1.f - amb && (!ahead || fabsf(u) < front - 2.f * eu))
+            c = 2;
+        }
       }
-      D.ext[idx] = 0.0;
+      const int i = P.lo[0] + x;
+      if (c < 0) c = cafe_temp_class_exact(K, P, i, j, k);
+      D.tcls[(long long)row * bx + x] = (uint8_t)c;
+      const long long idx = base + x;
+      if (K.gt_cls[c]) D.buildj[idx] = 1;
+      if (K.hot_cls[c]) {
+        any = 1;
+        if (idx < K.nxy) {
+          D.state[idx] = 2;
+        } else if (idx < iz1) {
+          D.state[idx] = 1;
+          D.gid[idx] = 0;
+        }
+        D.ext[idx] = 0.0;
+      }
     }
   }
   if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(&D.ctr[CTR_HOT], 1);
