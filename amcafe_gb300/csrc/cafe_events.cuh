@@ -738,7 +738,8 @@ __global__ void __launch_bounds__(CAFE_QUAD_THREADS) k_children(const __grid_con
 #define CAFE_CLOCK_WARP (CAFE_LOOP_THREADS / 32 - 2)   // capture time and clock
 #define CAFE_DRAW_WARP (CAFE_LOOP_THREADS / 32 - 3)    // nucleation draws
 #define CAFE_AHEAD_WARP (CAFE_LOOP_THREADS / 32 - 4)   // loads the likely next events' data ahead
-static_assert(CAFE_CAP_WARP >= 8, "warps 0-3 fill rows");
+#define CAFE_CELL_WARP (CAFE_LOOP_THREADS / 32 - 5)    // the captured cell's state
+static_assert(CAFE_CELL_WARP >= 8, "warps 0-3 fill rows");
 // Row of the k-th frontier row of the step: the rows present at its start, then
 // the rows that captures created, in their order (row_new).
 __device__ __forceinline__ int cafe_row_at(const CafeDev &D, int nrows0, int k) {
@@ -767,11 +768,12 @@ struct CafeResident {
   unsigned char k[CAFE_RES_MAX];     // ... and its place in the record
   unsigned char flag[CAFE_RES_MAX];  // CAFE_RF_*
   unsigned short free[CAFE_RES_MAX];
-  // each warp's smallest candidate: key, index, row, position, slot, g - E
+  // each warp's smallest candidate: key, index, row, position, slot, g - E, tie-break
   uint32_t wh[CAFE_WARPS], wm[CAFE_WARPS];
   int wi[CAFE_WARPS], wr[CAFE_WARPS], wq[CAFE_WARPS], wf[CAFE_WARPS];
   double wd[CAFE_WARPS];
-  unsigned long long wk[CAFE_WARPS], wrk[CAFE_WARPS], thr[32];  // full keys of the close ones
+  unsigned long long wrk[CAFE_WARPS];
+  unsigned long long wk[CAFE_WARPS], thr[32];  // (opening a window)
   int hist[32];
   int top, nfree, newslot, overflow, nfill, sink[32];
   uint32_t klim[2];  // [e & 1]: a smallest key below it needs no further test at event e
@@ -1243,12 +1245,26 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
   if (tid == 0) S.top = 0;
   __syncthreads();
   long long t0 = clock64();
-  const double rV = 1.0 / V;
-  int cnv = L.nvs2, cnr = L.nrows;  // (capturing warp) list and row counts
+  const double rV = 1.0 / V, kout = K.DelT * CAFE_OUTSIDE_REACH;
+  int cnv = L.nvs2, cnr = L.nrows;  // (capturing warps) list and row counts
+  // this thread's smallest and second smallest keys; whether they are known
+  uint32_t bk = 0xffffffffu, b2 = 0xffffffffu;
+  double bd = 0.0;
+  int bi = -1;
+  bool have = false;
+  auto consider = [&](int i, double d) {  // (g is NaN where no row is)
+    const uint32_t k = cafe_key32(PR ? __float_as_int((float)d * S.rv[i]) : __double2hiint(d), XM);
+    b2 = min(b2, max(k, bk));
+    if (k < bk) {
+      bk = k;
+      bd = d;
+      bi = i;
+    }
+  };
   while (true) {
     if (need_open) {
       // ---- open the window: the earliest rows by key
-      need_open = false;
+      need_open = have = false;
       ++tries;
       cafe_window_open<PR>(sD, sK, L, S, Q, ev, tries);
       if (tid == 0) {
@@ -1263,21 +1279,10 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       }
     }
     // ---- select: the smallest (g - E) / v over the resident rows
-    uint32_t bk = 0xffffffffu, b2 = 0xffffffffu;  // this thread's smallest and second smallest keys
-    double bd = 0.0;
-    int bi = -1;
-    {
+    if (!have) {
+      bk = b2 = 0xffffffffu;
       const int top = S.top;
-      for (int i = tid; i < top; i += NT) {  // (g is NaN where no row is)
-        const double d = S.g[i] - S.E[i];
-        const uint32_t k = cafe_key32(PR ? __float_as_int((float)d * S.rv[i]) : __double2hiint(d), XM);
-        b2 = min(b2, max(k, bk));
-        if (k < bk) {
-          bk = k;
-          bd = d;
-          bi = i;
-        }
-      }
+      for (int i = tid; i < top; i += NT) consider(i, S.g[i] - S.E[i]);
     }
     {
       const uint32_t wmin = __reduce_min_sync(FULL, bk);
@@ -1310,7 +1315,6 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
           S.wh[warp] = wmin;
           S.wf[warp] = hard;
           S.wd[warp] = bd;
-          S.wk[warp] = kf;
           S.wrk[warp] = S.rk[bi];
           S.wi[warp] = bi;
           S.wr[warp] = S.r[bi];
@@ -1330,7 +1334,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     if (!exact) {
       if (wcl & (wcl - 1u)) {  // several warps' candidates are close: likewise among them
         const bool c = wcl >> lane & 1u;
-        const unsigned long long kf = c ? S.wk[lane] : CAFE_KEY_NONE;
+        const unsigned long long kf = c ? cafe_key_canon(S.wd[lane]) : CAFE_KEY_NONE;
         const unsigned long long k1 = cafe_warp_min_key(kf, src);
         const unsigned long long rf = kf == k1 ? S.wrk[lane] : CAFE_KEY_NONE;
         const unsigned long long r1 = cafe_warp_min_key(rf, src);
@@ -1383,11 +1387,11 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     }
     // ---- apply the event
     const int icap = wq, child = cafe_slot_child(wm);
+    double kc = 0.0, dta = 0.0;  // (clock thread) the outside row's key, |dt|
     if (warp == CAFE_CAP_WARP) {
-      // level 1: the foreseen row's record (lane = place); the capture result of
-      // this slot (lanes 26-29: extent and centre, computed when the row was
-      // filled) and the grain
-      int gcap = 0, cn = 0;
+      // the captured cell's row. Level 1: the foreseen row's record (lane = place)
+      // and its cell's extent, computed when the capturing row was filled
+      int cn = 0;
       double gx = 0.0;
       CafeSlot cr;
       cr.g = NAN;
@@ -1399,12 +1403,12 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       if (foreseen) {
         cn = D.row_n[child];  // (the record's entries are not valid when there is none)
         if (lane < CAFE_NSLOT) cr = D.row_slot[(long long)child * CAFE_NSLOT + lane];
+        if (lane == CAFE_NSLOT) gx = D.row_geo[((long long)wr * CAFE_NSLOT + (wm & 31u)) * 4];
       }
-      if (lane >= CAFE_NSLOT && lane < 30) gx = D.row_geo[((long long)wr * CAFE_NSLOT + (wm & 31u)) * 4 + lane - 26];
-      if (lane == 30) gcap = D.a_gid[D.row_pos[wr]];
       const bool cold = D.a_cold[icap] != 0;
       const int cls = D.a_cls[icap];
       const double vq = PR ? cafe_vh(D, K, icap) : V;
+      const int nf = S.nfree, tp = S.top;
       // level 2: which of its neighbours (all but the captured ones) are left
       const bool rec = foreseen && cn != CAFE_NO_RECORD;
       bool left = false;
@@ -1417,64 +1421,34 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       const uint32_t clive = __ballot_sync(FULL, left);
       const bool grows = clive != 0u && cold, room = cnr < D.row_cap;
       const int row = foreseen ? child : cnr;
-      // the captured cell's own row: a foreseen one enters the resident set at once
-      int ci = -1;
-      if (grows && rec && room) {
-        const int nf = S.nfree, tp = S.top;
-        __syncwarp();
-        if (nf > 0) {
-          ci = S.free[nf - 1];
-          if (lane == 0) S.nfree = nf - 1;
-        } else if (tp < CAFE_RES_MAX) {
-          ci = tp;
-          if (lane == 0) S.top = tp + 1;
-        }
-        const int k1 = __ffs(clive) - 1;
-        const double g2 = __shfl_sync(FULL, cr.g, k1 + 1);
-        if (ci >= 0) {
-          if (lane == k1) {
-            const unsigned long long d2 = k1 + 1 < cn ? cafe_key_canon(g2) - cafe_key_canon(cr.g) : CAFE_KEY_NONE;
-            S.g[ci] = cr.g;
-            S.q[ci] = cr.q;
-            S.m[ci] = cr.m;
-            S.rk[ci] = cr.rk;
-            S.k[ci] = (unsigned char)k1;
-            S.flag[ci] = d2 < (1ULL << 33) ? CAFE_RF_NEAR : 0;
-            S.r[ci] = child;
-            if (PR) {
-              S.v[ci] = vq;
-              S.rv[ci] = 1.0f / (float)vq;
-            }
+      // a foreseen row enters the resident set at once
+      const bool enter = grows && rec && room && (nf > 0 || tp < CAFE_RES_MAX);
+      const int ci = !enter ? -1 : nf > 0 ? (int)S.free[nf - 1] : tp;
+      const int k1 = __ffs(clive | 0x80000000u) - 1;
+      const double g2 = __shfl_sync(FULL, cr.g, (k1 + 1) & 31);
+      if (enter) {
+        if (lane == k1) {
+          const unsigned long long d2 = k1 + 1 < cn ? cafe_key_canon(g2) - cafe_key_canon(cr.g) : CAFE_KEY_NONE;
+          S.g[ci] = cr.g;
+          S.q[ci] = cr.q;
+          S.m[ci] = cr.m;
+          S.rk[ci] = cr.rk;
+          S.k[ci] = (unsigned char)k1;
+          S.flag[ci] = d2 < (1ULL << 33) ? CAFE_RF_NEAR : 0;
+          S.r[ci] = child;
+          if (PR) {
+            S.v[ci] = vq;
+            S.rv[ci] = 1.0f / (float)vq;
           }
-          if (lane == 26) S.E[ci] = gx;
+        }
+        if (lane == CAFE_NSLOT) S.E[ci] = gx;
+        if (lane == 30) {
+          if (nf > 0) S.nfree = nf - 1;
+          else S.top = tp + 1;
         }
       }
-      // the captured cell (VoxelsCA.C:483-505 and 518-605)
-      if (nuc) {
-        if (lane == 0) cafe_nucleate(sD, sK, L, icap);
-      } else if (lane >= 26) {
-        // (one store each: the destination by lane)
-        double *gd = lane == 26 ? D.a_ext : lane == 27 ? D.a_cx : lane == 28 ? D.a_cy : D.a_cz;
-        double *sd = lane == 26 ? &L.nc.ext : &L.nc.c[(lane - 27) & 3];
-        if (lane < 30) {
-          gd[icap] = gx;
-          *sd = gx;
-          if (lane == 26 && foreseen && !rec) D.row_E[child] = gx;
-          if (lane == 26 && fabs(gx) == INFINITY) L.sw = 1;  // its times need the full scan
-        } else if (lane == 30) {
-          D.a_gid[icap] = gcap;
-          L.nc.gid = gcap;
-        }
-      }
+      if (lane == CAFE_NSLOT && foreseen && !rec) D.row_E[child] = gx;
       if (lane == 31) {
-        D.a_state[icap] = 2;
-        D.a_ev[icap] = ev;
-        if (cnv < D.vs2_cap) {
-          D.vs2[cnv] = icap;
-        } else {
-          atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
-          L.done = 1;
-        }
         L.newrow = grows && room ? row : -1;
         L.fill = !rec;
         S.newslot = ci;
@@ -1504,38 +1478,59 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       }
       cnv += 1;
       cnr += grows && room;
+    } else if (warp == CAFE_CELL_WARP) {
+      // the captured cell (VoxelsCA.C:483-505 and 518-605): the capture result of
+      // this slot (lanes 26-29: extent and centre), the grain
+      if (lane == 31) {
+        D.a_state[icap] = 2;
+        D.a_ev[icap] = ev;
+        if (cnv < D.vs2_cap) {
+          D.vs2[cnv] = icap;
+        } else {
+          atomicOr(D.err, CAFE_ERR_MUSHY_CAP);
+          L.done = 1;
+        }
+      }
+      cnv += 1;
+      if (L.unext[ev & 1] < cafe_nuc_rate_at(D, K, icap)) {
+        if (lane == 0) cafe_nucleate(sD, sK, L, icap);
+      } else if (lane >= CAFE_NSLOT && lane < 30) {
+        const double gx = D.row_geo[((long long)wr * CAFE_NSLOT + (wm & 31u)) * 4 + lane - 26];
+        // (one store each: the destination by lane)
+        double *gd = lane == 26 ? D.a_ext : lane == 27 ? D.a_cx : lane == 28 ? D.a_cy : D.a_cz;
+        double *sd = lane == 26 ? &L.nc.ext : &L.nc.c[(lane - 27) & 3];
+        gd[icap] = gx;
+        *sd = gx;
+        if (lane == 26 && fabs(gx) == INFINITY) L.sw = 1;  // its times need the full scan
+      } else if (lane == 30) {
+        D.a_gid[icap] = L.nc.gid = D.a_gid[D.row_pos[wr]];
+      }
     } else if (tid == CAFE_CLOCK_WARP * 32) {
       // the capture time, the clock (VoxelsCA.C:381, 483-516) and the growth log
       const bool nuc = L.unext[ev & 1] < cafe_nuc_rate_at(D, K, icap);
+      int cn = 0;
+      if (child >= 0) {
+        cn = D.row_n[child];
+        kc = D.ch_T[child - (int)D.row_cap];
+      }
       const double t = exact ? wc.t : (PR ? wd / S.v[win] : cafe_div_by(wd, V, rV));
       const double dt = nuc ? 0.0 : t;
       const double vd = PR ? dt : (nuc ? 0.0 : V * dt);
       const double tinc = L.tinc + dt;
       L.vd = vd;
+      D.ev_vd[ev] = vd;
       L.tinc = tinc;
       // while (vSind2 != countS && tinc < DelT): an event always lengthens the list
       if (cafe_is_nan(tinc) || !(cafe_key(tinc) < cafe_key(K.DelT))) L.done = 1;
-      D.ev_vd[ev] = vd;
-      const double vs = L.vs + vd, dsum = L.dsum + fabs(dt);
+      const double vs = L.vs + vd;
       L.vs = vs;
-      L.dsum = dsum;
       D.ev_vs[ev] = vs;
       if (cafe_is_neg(dt)) L.negdt++;
+      dta = fabs(dt);
       // a foreseen row that is not due within the step stays outside the set, and
       // the window ends before its key
-      int out = 0;
-      if (child >= 0 && !nuc && D.row_n[child] == CAFE_NO_RECORD) {
-        const double kc = tinc + D.ch_T[child - (int)D.row_cap];
-        if (kc > K.DelT * CAFE_OUTSIDE_REACH) {
-          out = 1;
-          D.row_key[child] = cafe_key(kc);
-          S.kw = min(S.kw, cafe_key(kc));
-          S.wlim = fmin(S.wlim, kc - S.slack);
-          S.all = 0;
-        }
-      }
-      S.outside = out;
-      S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, tinc, dsum);
+      kc = tinc + kc;
+      S.outside = child >= 0 && !nuc && cn == CAFE_NO_RECORD && kc > kout;
     } else if (tid == CAFE_DRAW_WARP * 32) {
       // the next event's draw (VoxelsCA.C:483; two engine outputs per event)
       cafe_uniform_stream st;
@@ -1580,26 +1575,44 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         if (S.q[i] == icap) cafe_res_first(D, S, i, S.r[i], S.k[i] + 1);
     }
     __syncthreads();
-    // ---- grow (VoxelsCA.C:511-516); a row that lost its last slot leaves
+    // ---- grow (VoxelsCA.C:511-516), and the next event's smallest candidates; a
+    // row that lost its last slot leaves
     const int born = S.newslot;
     {
       const double vd = L.vd;
       const int top = S.top;
+      bk = b2 = 0xffffffffu;
       for (int i = tid; i < top; i += NT) {
+        double E = S.E[i];
         // (a row created by this event grows from the next one on)
-        if (i == born || S.r[i] < 0) continue;
-        const double E = cafe_grow(S.E[i], PR ? S.v[i] * vd : vd);
-        S.E[i] = E;
-        if (S.flag[i] & CAFE_RF_DYING) {
-          const int r = S.r[i];
-          D.row_E[r] = E;
-          D.row_m[r] = ev;
-          D.row_key[r] = CAFE_KEY_NONE;
-          S.flag[i] = 0;
-          S.r[i] = -1;
-          S.free[atomicAdd(&S.nfree, 1)] = (unsigned short)i;
+        if (i != born && S.r[i] >= 0) {
+          E = cafe_grow(E, PR ? S.v[i] * vd : vd);
+          S.E[i] = E;
+          if (S.flag[i] & CAFE_RF_DYING) {
+            const int r = S.r[i];
+            D.row_E[r] = E;
+            D.row_m[r] = ev;
+            D.row_key[r] = CAFE_KEY_NONE;
+            S.flag[i] = 0;
+            S.r[i] = -1;
+            S.free[atomicAdd(&S.nfree, 1)] = (unsigned short)i;
+          }
         }
+        consider(i, S.g[i] - E);
       }
+      have = true;
+    }
+    if (tid == CAFE_CLOCK_WARP * 32) {
+      // the window's limit for the next event
+      const double dsum = L.dsum + dta;
+      L.dsum = dsum;
+      if (S.outside) {
+        D.row_key[child] = cafe_key(kc);
+        S.kw = min(S.kw, cafe_key(kc));
+        S.wlim = fmin(S.wlim, kc - S.slack);
+        S.all = 0;
+      }
+      S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, dsum);
     }
     if (tid == 0) {
       const long long t1 = clock64();
@@ -1607,13 +1620,18 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       t0 = t1;
     }
     // ---- events with more to do than the row that was foreseen
-    if (cafe_is_neg(L.vd) && cafe_negative_event<PR>(sD, sK, L, S, ev)) need_open = true;
-    if (L.newrow >= 0 && born < 0 && !S.outside) {
-      if (cafe_new_row<PR>(sD, sK, L, S, Q, ev, icap)) need_open = true;
-      if (tid == 0) {
-        const long long t1 = clock64();
-        L.cyc[2] += t1 - t0;
-        t0 = t1;
+    const bool neg = cafe_is_neg(L.vd), fresh = L.newrow >= 0 && born < 0 && !S.outside;
+    if (neg || fresh) {
+      __syncthreads();
+      have = false;
+      if (neg && cafe_negative_event<PR>(sD, sK, L, S, ev)) need_open = true;
+      if (fresh) {
+        if (cafe_new_row<PR>(sD, sK, L, S, Q, ev, icap)) need_open = true;
+        if (tid == 0) {
+          const long long t1 = clock64();
+          L.cyc[2] += t1 - t0;
+          t0 = t1;
+        }
       }
     }
     if (L.done || L.sw) break;
