@@ -870,6 +870,12 @@ template <bool PR>
 constexpr __host__ __device__ uint32_t cafe_ktiny() { return 0x80000000u | (PR ? 0x0d800000u : (1023u - 900u) << 20); }
 template <bool PR>
 constexpr __host__ __device__ int cafe_xm() { return PR ? 0x7f800000 : 0x7ff00000; }
+// The largest key that is close to the smallest one, k.
+template <bool PR>
+__device__ __forceinline__ uint32_t cafe_close_key(uint32_t k) {
+  const uint32_t t = k + cafe_kc<PR>(), mag = k & 0x80000000u ? k : ~k;
+  return mag <= cafe_ktiny<PR>() ? max(t, cafe_ktiny<PR>()) : t;
+}
 
 // The largest key that a winner at clock T may have and be the global one.
 template <bool PR>
@@ -1237,7 +1243,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_LOOP_THREADS / 32;
   const double V = K.vhat_cls[1];
-  constexpr uint32_t KC = cafe_kc<PR>(), KTINY = cafe_ktiny<PR>();
+  constexpr uint32_t KTINY = cafe_ktiny<PR>();
   constexpr int XM = cafe_xm<PR>();
   int ev = 0;
   int tries = 0;  // windows opened since the last event
@@ -1286,7 +1292,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     }
     {
       const uint32_t wmin = __reduce_min_sync(FULL, bk);
-      const uint32_t thr = wmin + KC;
+      const uint32_t thr = cafe_close_key<PR>(wmin);
       const uint32_t cl = wmin == 0xffffffffu ? 0u : __ballot_sync(FULL, bk <= thr);
       if (cl == 0u) {
         if (lane == 0) S.wh[warp] = wmin;
@@ -1299,6 +1305,9 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         if (bk <= thr) {
           const int ed = (__double2hiint(bd) >> 20) & 0x7ff, eg = (__double2hiint(S.g[bi]) >> 20) & 0x7ff;
           hard = S.flag[bi] || ed > eg + 20 || b2 <= thr;
+          // a tiny g - E is decided here only when it is zero, so that the time is,
+          // and g is ordinary, so that the row's next slot is not tiny as well
+          if (bk <= KTINY && ~bk <= KTINY) hard = hard || PR || bd != 0.0 || eg < 400;
           kf = cafe_key_canon(bd);
         }
         if (cl & (cl - 1u)) {
@@ -1327,10 +1336,10 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     const uint32_t wkey = lane < NW ? S.wh[lane] : 0xffffffffu;
     const uint32_t kmin = __reduce_min_sync(FULL, wkey);
     const bool inside = kmin < S.klim[(ev + 1) & 1];
-    const uint32_t wcl = __ballot_sync(FULL, wkey <= kmin + KC && wkey != 0xffffffffu);
-    const uint32_t kmag = kmin & 0x80000000u ? kmin : ~kmin;  // key of the magnitude
+    const uint32_t kthr = cafe_close_key<PR>(kmin);
+    const uint32_t wcl = __ballot_sync(FULL, wkey <= kthr && wkey != 0xffffffffu);
     int src = __ffs(wcl | 0x80000000u) - 1;
-    bool exact = !inside || kmag <= KTINY;
+    bool exact = !inside;
     if (!exact) {
       if (wcl & (wcl - 1u)) {  // several warps' candidates are close: likewise among them
         const bool c = wcl >> lane & 1u;
@@ -1357,7 +1366,6 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         continue;
       }
       // exact candidates of the close rows, the reference's order among them
-      const uint32_t kthr = kmag > KTINY ? kmin + KC : max(kmin + KC, KTINY);
       if (kmin != 0xffffffffu) cafe_select_exact<PR>(sD, sK, S, kthr);
       wc = kmin != 0xffffffffu ? S.red[0] : cafe_cand_none();
       __syncthreads();
