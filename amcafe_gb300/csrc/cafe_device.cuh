@@ -192,6 +192,7 @@ struct CafeDev {
   // velocity of the step's rows
   double *row_E;
   int32_t *row_m, *row_due;  // row_due: the rows that may capture soon
+  uint32_t *row_low;         // per group of CAFE_PREP_ROWS rows: the smallest extent's high word, 0 once one was brought up to date
   float *row_glb;            // lower bound of the numerators of a row without a record
   unsigned long long *row_key, *row_mag;
   // the logged growth of each event (CTR_EVLOG: fl(v * DtMin), or DtMin) and

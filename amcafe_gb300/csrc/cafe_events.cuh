@@ -414,7 +414,15 @@ __device__ __forceinline__ double cafe_row_replayed(const CafeDev &D, int r, int
     stop = m;
     return E;
   }
-  for (int k = m + 1; k <= stop; ++k) E = cafe_grow(E, PR ? v * D.ev_vd[k] : D.ev_vd[k]);
+  // (the sums are a serial chain: its terms are loaded eight at a time)
+  for (int k = m + 1; k <= stop; k += 8) {
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = D.ev_vd[min(k + u, stop)];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k + u <= stop) E = cafe_grow(E, PR ? v * x[u] : x[u]);
+  }
   return E;
 }
 __device__ __forceinline__ void cafe_row_replay(const CafeDev &D, const CafeConsts &K, int r, int upto, bool pr) {
@@ -537,6 +545,8 @@ __device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &
     const bool in = lane < n;
     const uint32_t ekey = in && !cafe_is_nan(E) ? (uint32_t)(cafe_key(fabs(E)) >> 32) + 1u : 0u;  // NaN extents occur (the reference's 0/0)
     const uint32_t vkey = (uint32_t)(cafe_key(v) >> 32);
+    const uint32_t elow = __reduce_min_sync(FULL, in ? (uint32_t)__double2hiint(E) : 0xffffffffu);
+    if (lane == 0) D.row_low[w] = elow;
     const uint32_t e1 = __reduce_max_sync(FULL, ekey), v0 = __reduce_min_sync(FULL, in ? vkey : 0xffffffffu),
                    v1 = __reduce_max_sync(FULL, in ? vkey + 1u : 0u);
     if (lane == 0) {
@@ -748,7 +758,7 @@ __device__ __forceinline__ int cafe_row_at(const CafeDev &D, int nrows0, int k) 
 
 struct CafeLoop {
   // the loop's scalars (VoxelsCA.C:381-610)
-  double tinc, dt, vd, vs, vmin, vmax, dsum, gmax, emax;
+  double tinc, dt, vd, vs, rV, vmin, vmax, dsum, gmax, emax;
   double unext[2];  // unext[e & 1]: event e's draw
   int fill, nvs2, countS, nrows0, nrows, ngrain, done, nuc, ev, sw, na, newrow, slow;
   uint32_t rng;
@@ -877,13 +887,24 @@ __device__ __forceinline__ uint32_t cafe_close_key(uint32_t k) {
   return mag <= cafe_ktiny<PR>() ? max(t, cafe_ktiny<PR>()) : t;
 }
 
-// The largest key that a winner at clock T may have and be the global one.
+// The largest key that a winner at clock T may have and be the global one; Vf:
+// the common velocity, rounded down. Every event's limit is on its chain, and a
+// double-precision operation costs as much as ten others: one subtraction and one
+// conversion, then single precision rounded towards earlier.
 template <bool PR>
-__device__ __forceinline__ uint32_t cafe_window_limit(const CafeResident &S, double V, double DelT, int ev, double T, double dsum) {
-    if (!S.all && !(ev < S.ev_cap && dsum <= S.dsum_cap)) return 0u;
-    double lim = fmin(S.wlim - T, 0x1.e847fp19) * (PR ? 1.0 : V);  // 0x1.e847fp19 < 1e6
-    lim = lim - fabs(lim) * 0x1p-18;
-    return PR ? cafe_key32(__float_as_int((float)lim), cafe_xm<PR>()) : cafe_key32(__double2hiint(lim), cafe_xm<PR>());
+__device__ __forceinline__ uint32_t cafe_window_limit(const CafeResident &S, float Vf, int ev, double T, double dsum) {
+  if (!S.all && !(ev < S.ev_cap && (unsigned long long)crm_bits(dsum) <= (unsigned long long)crm_bits(S.dsum_cap))) return 0u;
+  double lim = S.wlim - T;
+  if (cafe_key(lim) > cafe_key(0x1.e847fp19)) lim = 0x1.e847fp19;  // 0x1.e847fp19 < 1e6
+  float f = __double2float_rd(lim);
+  if (!PR) f = __fmul_rd(f, Vf);
+  f = __fmaf_rd(-fabsf(f), 0x1p-17f, f);
+  const int b = __float_as_int(f), e = b >> 23 & 0xff;
+  if (e == 255) return 0u;  // (below the range)
+  if (PR) return cafe_key32(b, 0x7f800000);
+  // as the high word of a double, towards earlier; beyond single precision's range: the nearest bound
+  if (e == 0) return b < 0 ? cafe_key32((int)0xb8100000, 0x7ff00000) : 0x80000000u;
+  return cafe_key32((b & (int)0x80000000) | ((e + 896) << 20 | (b & 0x7fffff) >> 3) + (b < 0 ? 1 : 0), 0x7ff00000);
 }
 
 // The loop's rare parts, out of line: an event's chain pays for every
@@ -903,6 +924,7 @@ __device__ __noinline__ void cafe_res_flush(const CafeDev &D, const CafeConsts &
     if (r < 0) continue;
     D.row_E[r] = S.E[i];
     D.row_m[r] = ev;
+    if (r < L.nrows0) D.row_low[r / CAFE_PREP_ROWS] = 0u;
     D.row_k[r] = S.k[i];
     if (keys) {
       const double t = (S.g[i] - S.E[i]) / (PR ? S.v[i] : V);
@@ -962,6 +984,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   const unsigned FULL = 0xffffffffu;
   const double V = K.vhat_cls[1];
+  const float Vf = __double2float_rd(V);
   (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
   cafe_res_flush<PR>(D, K, L, S, ev, true);
   __syncthreads();
@@ -1059,7 +1082,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     S.slack = slack;
     S.nfill = 0;
     L.opens++;
-    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, L.dsum);
+    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, Vf, ev, L.tinc, L.dsum);
   }
   __syncthreads();
   if (S.overflow) return;
@@ -1114,14 +1137,22 @@ __device__ __noinline__ void cafe_select_exact(const CafeDev &D, const CafeConst
 // A negative event may clamp a small extent at zero (VoxelsCA.C:515),
 // which breaks the key bound of a row outside the set: the rows whose
 // extrapolated extent comes near zero are brought up to date with a new key
-// (true: one of them may be due within the step).
+// (true: one of them may be due within the step). A few rows of thousands: those
+// of the groups whose smallest extent (row_low) is below the threshold or that
+// hold a row brought up to date before, and the step's new rows, are listed in
+// shared memory and take a thread each.
 template <bool PR>
-__device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
-  const unsigned FULL = 0xffffffffu;
-  const double V = K.vhat_cls[1];
-  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
+__device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, CafeQuadScratch *Q, int ev) {
+  const int tid = threadIdx.x;
+  constexpr int NT = CAFE_LOOP_THREADS;
+  constexpr int CAP = (int)(sizeof(CafeQuadScratch) * CAFE_QUADS / sizeof(int));
+  int *list = (int *)Q;  // (no record is being made)
+  const double V = K.vhat_cls[1], rV = L.rV;
+  const float Vf = __double2float_rd(V);
+  const int nrows = L.nrows, nrows0 = L.nrows0, groups = (nrows0 + CAFE_PREP_ROWS - 1) / CAFE_PREP_ROWS;
+  uint32_t lo[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) lo[u] = tid + u * NT < groups ? D.row_low[tid + u * NT] : 0xffffffffu;
   const double vd = L.vd, vsp = D.ev_vs[ev - 1], vx = PR ? L.vmax : V;
   const double margin = (double)(ev + 16) * 0x1p-48 * (L.emax + L.gmax + vx * L.dsum + 1e-300);
   // rows that still hold the step's first extents (row_m 0, nearly all) have
@@ -1129,53 +1160,51 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
   const double g0 = vsp + vd;
   const double need = PR ? (g0 >= 0.0 ? margin - g0 * L.vmin : margin - g0 * L.vmax) : margin - g0;
   const long long thr0 = need > 0.0 ? crm_bits(need * (1.0 + 0x1p-40)) : 0;
+  const uint32_t thi = (uint32_t)(thr0 >> 32);
+  if (tid == 0) S.nfill = 0;
+  __syncthreads();
+  auto expand = [&](int g) {
+    const int n = min(CAFE_PREP_ROWS, nrows0 - g * CAFE_PREP_ROWS), b = atomicAdd(&S.nfill, n);
+    for (int u = 0; u < n && b + u < CAP; ++u) list[b + u] = g * CAFE_PREP_ROWS + u;
+  };
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (lo[u] <= thi) expand(tid + u * NT);
+  for (int g = tid + 4 * NT; g < groups; g += NT)
+    if (D.row_low[g] <= thi) expand(g);
+  __syncthreads();
+  const int nl = S.nfill, nnew = nrows - nrows0;
+  const bool listed = nl <= CAP;  // else: every row
+  const int n = listed ? nl + nnew : nrows;
   unsigned long long near = CAFE_KEY_NONE;  // smallest new key
-  const int nrows = L.nrows, nrows0 = L.nrows0;
-  for (int k0 = tid; k0 < nrows; k0 += 8 * NT) {
-    int rr[8], mm[8];
-    uint32_t todo = 0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) rr[u] = k0 + u * NT < nrows ? cafe_row_at(D, nrows0, k0 + u * NT) : -1;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) mm[u] = rr[u] >= 0 ? D.row_m[rr[u]] : ev;
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (mm[u] < ev && (mm[u] != 0 || thr0 > 0)) todo |= 1u << u;
-    if (todo) {
-      long long eb[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) eb[u] = todo >> u & 1u ? crm_bits(D.row_E[rr[u]]) : 0;
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (mm[u] == 0 && eb[u] >= thr0) todo &= ~(1u << u);  // (NaN too: it never captures)
-    }
-    for (; todo; todo &= todo - 1) {
-    int r = 0, m = 0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (u == __ffs(todo) - 1) {
-        r = rr[u];
-        m = mm[u];
-      }
+  for (int k = tid; k < n; k += NT) {
+    const int r = !listed ? cafe_row_at(D, nrows0, k) : k < nl ? list[k] : D.row_new[k - nl];
+    const int m = D.row_m[r];
+    const double E = D.row_E[r];
+    if (m >= ev || (m == 0 && crm_bits(E) >= thr0)) continue;  // (NaN too: it never captures)
     const double v = PR ? cafe_vh(D, K, D.row_pos[r]) : V;
     const double gr = (vsp - D.ev_vs[m]) + vd;
-    if (D.row_E[r] + (PR ? v * gr : gr) >= margin) continue;
+    if (E + (PR ? v * gr : gr) >= margin) continue;
     int stop;
     const double En = cafe_row_replayed<PR>(D, r, ev, v, stop);
     D.row_E[r] = En;
     D.row_m[r] = stop < ev ? CAFE_M_DONE : ev;  // (a row that stopped growing keeps its extent)
+    if (r < nrows0) D.row_low[r / CAFE_PREP_ROWS] = 0u;
     double t = NAN;
     if (D.row_n[r] == CAFE_NO_RECORD) {
-      t = cafe_lb_time(D.row_glb[r], En, v);
+      t = ((double)D.row_glb[r] - En) * (PR ? 1.0 / v : rV);
+      t -= fabs(t) * 0x1p-40;
     } else {
-      const int k = cafe_row_next(D, r, D.row_k[r]);
-      D.row_k[r] = (uint8_t)k;
-      if (k < D.row_n[r]) t = (D.row_slot[(long long)r * CAFE_NSLOT + k].g - En) / v;
+      const int kn = cafe_row_next(D, r, D.row_k[r]);
+      D.row_k[r] = (uint8_t)kn;
+      if (kn < D.row_n[r]) {
+        const double d = D.row_slot[(long long)r * CAFE_NSLOT + kn].g - En;
+        t = PR ? d / v : cafe_div_by(d, V, rV);
+      }
     }
     const unsigned long long key = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
     D.row_key[r] = key;
     if (key < near) near = key;
-    }
   }
   // one of them due within the step: a new window; else the window ends before it
   if (__syncthreads_or(near <= cafe_key(K.DelT * CAFE_SHORT_REACH))) return true;
@@ -1184,7 +1213,7 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
   if (tid == 0 && S.kw < CAFE_KEY_NONE - 1) {
     S.all = 0;
     S.wlim = fmin(S.wlim, cafe_unkey(S.kw) - S.slack);
-    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, L.dsum);
+    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, Vf, ev, L.tinc, L.dsum);
   }
   __syncthreads();
   return false;
@@ -1251,7 +1280,8 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
   if (tid == 0) S.top = 0;
   __syncthreads();
   long long t0 = clock64();
-  const double rV = 1.0 / V, kout = K.DelT * CAFE_OUTSIDE_REACH;
+  const float Vf = __double2float_rd(V);
+  const double rV = L.rV, kout = K.DelT * CAFE_OUTSIDE_REACH;
   int cnv = L.nvs2, cnr = L.nrows;  // (capturing warps) list and row counts
   // this thread's smallest and second smallest keys; whether they are known
   uint32_t bk = 0xffffffffu, b2 = 0xffffffffu;
@@ -1358,7 +1388,6 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     const int win = S.wi[src];
     int wr = S.wr[src], wq = S.wq[src];
     uint32_t wm = S.wm[src];
-    CafeCand wc = cafe_cand_none();
     if (exact) {
       if (!S.all && !inside) {  // beyond the window (or nothing in it)
         __syncthreads();
@@ -1367,16 +1396,16 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       }
       // exact candidates of the close rows, the reference's order among them
       if (kmin != 0xffffffffu) cafe_select_exact<PR>(sD, sK, S, kthr);
-      wc = kmin != 0xffffffffu ? S.red[0] : cafe_cand_none();
+      const bool none = kmin == 0xffffffffu || S.red[0].j < 0 || !(S.red[0].tk < CAFE_KEY_1E6);
+      wr = S.red[0].r;
+      wq = S.red[0].q;
+      wm = S.red[0].m;
       __syncthreads();
-      if (wc.j < 0 || !(wc.tk < CAFE_KEY_1E6)) {  // no candidate is left
+      if (none) {  // no candidate is left
         if (tid == 0) L.done = 1;
         __syncthreads();
         break;
       }
-      wr = wc.r;
-      wq = wc.q;
-      wm = wc.m;
     }
     if (ev >= max_events) {
       if (tid == 0) {
@@ -1521,7 +1550,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         cn = D.row_n[child];
         kc = D.ch_T[child - (int)D.row_cap];
       }
-      const double t = exact ? wc.t : (PR ? wd / S.v[win] : cafe_div_by(wd, V, rV));
+      const double t = exact ? S.red[0].t : (PR ? wd / S.v[win] : cafe_div_by(wd, V, rV));
       const double dt = nuc ? 0.0 : t;
       const double vd = PR ? dt : (nuc ? 0.0 : V * dt);
       const double tinc = L.tinc + dt;
@@ -1615,12 +1644,15 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       const double dsum = L.dsum + dta;
       L.dsum = dsum;
       if (S.outside) {
-        D.row_key[child] = cafe_key(kc);
-        S.kw = min(S.kw, cafe_key(kc));
-        S.wlim = fmin(S.wlim, kc - S.slack);
+        const unsigned long long key = cafe_key(kc);
+        D.row_key[child] = key;
+        if (key < S.kw) {
+          S.kw = key;
+          S.wlim = kc - S.slack;
+        }
         S.all = 0;
       }
-      S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, V, K.DelT, ev, L.tinc, dsum);
+      S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, Vf, ev, L.tinc, dsum);
     }
     if (tid == 0) {
       const long long t1 = clock64();
@@ -1632,7 +1664,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
     if (neg || fresh) {
       __syncthreads();
       have = false;
-      if (neg && cafe_negative_event<PR>(sD, sK, L, S, ev)) need_open = true;
+      if (neg && cafe_negative_event<PR>(sD, sK, L, S, Q, ev)) need_open = true;
       if (fresh) {
         if (cafe_new_row<PR>(sD, sK, L, S, Q, ev, icap)) need_open = true;
         if (tid == 0) {
@@ -1809,8 +1841,8 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_LOOP_THREADS / 32;
   if (cafe_bid != 0) return;  // event_fill_helper's second block: the loop leaves it nothing to do
-  if (tid == 32) sD = D;
-  if (tid == 64) sK = K;
+  for (int i = tid; i < (int)(sizeof(CafeDev) / 4); i += NT) ((uint32_t *)&sD)[i] = ((const uint32_t *)&D)[i];
+  for (int i = tid; i < (int)(sizeof(CafeConsts) / 4); i += NT) ((uint32_t *)&sK)[i] = ((const uint32_t *)&K)[i];
   if (tid == 0) {
     L.na = D.ctr[CTR_NA];
     L.nvs2 = D.ctr[CTR_NVS2];
@@ -1823,6 +1855,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
     L.unext[1] = cafe_uniform_next(&st);  // the first event's draw; later draws are made one event ahead
     L.rng = st.x;
     L.sdloc = K.seed0 + 32u * (unsigned int)tInd + 64u * (unsigned int)L.ngrain;
+    L.rV = 1.0 / K.vhat_cls[1];
     L.tinc = L.dsum = L.vd = L.dt = L.vs = 0.0;
     L.gmax = D.row_mag[0] ? cafe_unkey(D.row_mag[0]) : 0.0;
     L.emax = D.row_mag[1] ? cafe_unkey(D.row_mag[1]) : 0.0;

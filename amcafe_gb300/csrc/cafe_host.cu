@@ -1202,6 +1202,7 @@ int cafe_sim_create(const char *deck_path, const cafe_options *opt, cafe_sim **o
       (rc = dalloc(&D.ch_gid, D.ch_cap, o)) || (rc = dalloc(&D.ch_T, D.ch_cap, o)) ||
       (rc = dalloc(&D.row_pairs, (size_t)D.row_cap * CAFE_NSLOT, o)) || (rc = dalloc(&D.blk, D.blk_cap, o)) ||
       (rc = dalloc(&D.row_E, nrow, o)) || (rc = dalloc(&D.row_m, nrow, o)) || (rc = dalloc(&D.row_due, D.row_cap, o)) || (rc = dalloc(&D.row_glb, nrow, o)) ||
+      (rc = dalloc(&D.row_low, nrow, o)) ||
       (rc = dalloc(&D.row_key, nrow, o)) || (rc = dalloc(&D.row_mag, 4, o)) ||
       (rc = dalloc(&D.ev_vd, D.ev_cap, o)) || (rc = dalloc(&D.ev_vs, D.ev_cap, o)) || (K.nuc_gauss && (rc = dalloc(&D.a_nuc, acap, o))) ||
       (rc = dalloc(&D.ctr, CTR_COUNT, o)) || (rc = dalloc(&D.err, 1, o)) || (rc = dalloc(&D.stat, STAT_COUNT, o)) ||
