@@ -984,7 +984,6 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   const unsigned FULL = 0xffffffffu;
   const double V = K.vhat_cls[1];
-  const float Vf = __double2float_rd(V);
   (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
   cafe_res_flush<PR>(D, K, L, S, ev, true);
   __syncthreads();
@@ -1024,15 +1023,17 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   __syncthreads();
   mn = cafe_warp_min_key(lane < NW ? S.wk[lane] : CAFE_KEY_NONE, src);
   cnt = __reduce_add_sync(FULL, lane < NW ? S.wi[lane] : 0);
-  // the rows that are not listed have keys above this bound
-  const unsigned long long kdue = first && D.ctr[CTR_NKEY] > 0 ? cafe_key(K.DelT * CAFE_DUE_REACH) : CAFE_KEY_NONE - 1;
   const bool all = cnt <= CAFE_RES_TARGET;
   // rounding bound of the keys for the next 4096 events and 64 DelT of growth
-  const double dcap = L.dsum + 64.0 * K.DelT;
-  const double base = (mn == CAFE_KEY_NONE ? 0.0 : cafe_unkey(mn));
-  const double slack = (double)(ev + 4096 + 16) * 0x1p-47 *
-                       (fabs(base) + 64.0 * K.DelT + fabs(L.tinc) + 2.0 * dcap +
-                        (L.gmax + L.emax) / (PR ? L.vmin : V) + 1e-300);
+  // (by one warp: a double-precision operation of all sixteen takes 256 cycles)
+  double dcap = 0.0, base = 0.0, slack = 0.0;
+  if (warp == 0) {
+    dcap = L.dsum + 64.0 * K.DelT;
+    base = (mn == CAFE_KEY_NONE ? 0.0 : cafe_unkey(mn));
+    slack = (double)(ev + 4096 + 16) * 0x1p-47 *
+            (fabs(base) + 64.0 * K.DelT + fabs(L.tinc) + 2.0 * dcap +
+             (L.gmax + L.emax) * (PR ? 1.0 / L.vmin : L.rV) * (1.0 + 0x1p-40) + 1e-300);
+  }
   int pick = 31;
   if (!all) {
     if (tid < 32) {
@@ -1066,9 +1067,11 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     pick = fits ? 31 - __clz(fits) : 0;
     if (tid == 0) S.overflow = !fits && S.nfill > CAFE_RES_MAX - 64;
   }
-  const unsigned long long kw = min(kdue, all ? CAFE_KEY_NONE - 1 : S.thr[pick]);
-  const bool every = kw == CAFE_KEY_NONE - 1;
   if (tid == 0) {
+    // the rows that are not listed have keys above the listed ones' reach
+    const unsigned long long kdue = first && D.ctr[CTR_NKEY] > 0 ? cafe_key(K.DelT * CAFE_DUE_REACH) : CAFE_KEY_NONE - 1;
+    const unsigned long long kw = min(kdue, all ? CAFE_KEY_NONE - 1 : S.thr[pick]);
+    const bool every = kw == CAFE_KEY_NONE - 1;
     if (all) S.overflow = 0;
     if (!every && !(cafe_unkey(kw) < 1e300)) S.overflow = 1;
     if (!(slack < 1e300) || tries >= CAFE_OPEN_TRIES) S.overflow = 1;
@@ -1082,10 +1085,11 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
     S.slack = slack;
     S.nfill = 0;
     L.opens++;
-    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, Vf, ev, L.tinc, L.dsum);
+    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, __double2float_rd(V), ev, L.tinc, L.dsum);
   }
   __syncthreads();
   if (S.overflow) return;
+  const unsigned long long kw = S.kw;
   for (int k = tid; k < nrows; k += NT) {
     const int r = row_at(k);
     if (D.row_key[r] <= kw) {
@@ -1148,21 +1152,27 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
   constexpr int CAP = (int)(sizeof(CafeQuadScratch) * CAFE_QUADS / sizeof(int));
   int *list = (int *)Q;  // (no record is being made)
   const double V = K.vhat_cls[1], rV = L.rV;
-  const float Vf = __double2float_rd(V);
   const int nrows = L.nrows, nrows0 = L.nrows0, groups = (nrows0 + CAFE_PREP_ROWS - 1) / CAFE_PREP_ROWS;
   uint32_t lo[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) lo[u] = tid + u * NT < groups ? D.row_low[tid + u * NT] : 0xffffffffu;
-  const double vd = L.vd, vsp = D.ev_vs[ev - 1], vx = PR ? L.vmax : V;
-  const double margin = (double)(ev + 16) * 0x1p-48 * (L.emax + L.gmax + vx * L.dsum + 1e-300);
-  // rows that still hold the step's first extents (row_m 0, nearly all) have
-  // grown by the whole running sum: they are decided by one threshold
-  const double g0 = vsp + vd;
-  const double need = PR ? (g0 >= 0.0 ? margin - g0 * L.vmin : margin - g0 * L.vmax) : margin - g0;
-  const long long thr0 = need > 0.0 ? crm_bits(need * (1.0 + 0x1p-40)) : 0;
-  const uint32_t thi = (uint32_t)(thr0 >> 32);
-  if (tid == 0) S.nfill = 0;
+  const double vd = L.vd;
+  if (tid == 0) {  // (one warp's double-precision work, not sixteen's)
+    const double vsp = D.ev_vs[ev - 1], vx = PR ? L.vmax : V;
+    const double margin = (double)(ev + 16) * 0x1p-48 * (L.emax + L.gmax + vx * L.dsum + 1e-300);
+    // rows that still hold the step's first extents (row_m 0, nearly all) have
+    // grown by the whole running sum: they are decided by one threshold
+    const double g0 = vsp + vd;
+    const double need = PR ? (g0 >= 0.0 ? margin - g0 * L.vmin : margin - g0 * L.vmax) : margin - g0;
+    S.thr[0] = need > 0.0 ? (unsigned long long)crm_bits(need * (1.0 + 0x1p-40)) : 0ULL;
+    S.thr[1] = (unsigned long long)crm_bits(margin);
+    S.thr[2] = (unsigned long long)crm_bits(vsp);
+    S.thr[3] = cafe_key(K.DelT * CAFE_SHORT_REACH);
+    S.nfill = 0;
+  }
   __syncthreads();
+  const long long thr0 = (long long)S.thr[0];
+  const uint32_t thi = (uint32_t)(S.thr[0] >> 32);
   auto expand = [&](int g) {
     const int n = min(CAFE_PREP_ROWS, nrows0 - g * CAFE_PREP_ROWS), b = atomicAdd(&S.nfill, n);
     for (int u = 0; u < n && b + u < CAP; ++u) list[b + u] = g * CAFE_PREP_ROWS + u;
@@ -1176,6 +1186,7 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
   const int nl = S.nfill, nnew = nrows - nrows0;
   const bool listed = nl <= CAP;  // else: every row
   const int n = listed ? nl + nnew : nrows;
+  const double margin = crm_from_bits((long long)S.thr[1]), vsp = crm_from_bits((long long)S.thr[2]);
   unsigned long long near = CAFE_KEY_NONE;  // smallest new key
   for (int k = tid; k < n; k += NT) {
     const int r = !listed ? cafe_row_at(D, nrows0, k) : k < nl ? list[k] : D.row_new[k - nl];
@@ -1207,13 +1218,13 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
     if (key < near) near = key;
   }
   // one of them due within the step: a new window; else the window ends before it
-  if (__syncthreads_or(near <= cafe_key(K.DelT * CAFE_SHORT_REACH))) return true;
+  if (__syncthreads_or(near <= S.thr[3])) return true;
   if (near < S.kw) atomicMin(&S.kw, near);
   __syncthreads();
   if (tid == 0 && S.kw < CAFE_KEY_NONE - 1) {
     S.all = 0;
     S.wlim = fmin(S.wlim, cafe_unkey(S.kw) - S.slack);
-    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, Vf, ev, L.tinc, L.dsum);
+    S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, __double2float_rd(V), ev, L.tinc, L.dsum);
   }
   __syncthreads();
   return false;
