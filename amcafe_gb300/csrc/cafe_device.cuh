@@ -15,6 +15,7 @@
 #define CAFE_DEVICE_CUH
 #include <stdint.h>
 
+#include "cafe_bounds.h"
 #include "cafe_crmath.h"
 #include "cafe_rng.h"
 
@@ -336,9 +337,9 @@ __device__ __forceinline__ void cafe_rot_from_cth(const double *c, double *R) {
 // which the reference evaluates with identical expressions at the two places.
 //
 // The computation is split into parts with no data dependence between them
-// (the th and ph chains, the two point-line projections) so that the event
-// loop can run them in different warps; cafe_capture_geometry runs them all in
-// one thread. Every part is the same expression sequence wherever it runs.
+// (the th and ph chains, the two point-line projections), so that several
+// warps can share one evaluation. Every part is the same expression sequence
+// wherever it runs.
 __device__ __forceinline__ void cafe_geo_dn(const CafeConsts &K, int ci, int cj, int ck, const double *cs,
                                             double *dn) {
   dn[0] = ((double)ci + .5) * K.dx[0] - cs[0];
@@ -497,26 +498,6 @@ __device__ __forceinline__ void cafe_geo_centre(const double *R, const double *c
   cen[1] = cs[1] + g1;
   cen[2] = cs[2] + g2;
 }
-__device__ __noinline__ void cafe_capture_geometry(const CafeConsts &K, int ci, int cj, int ck,
-                                                   int si, int sj, int sk, const double *cs,
-                                                   const double *R, double *g_out,
-                                                   double *ext_out, double *cen_out) {
-  double l = cafe_geo_l(K, ci, cj, ck, si, sj, sk);
-  double dn[3], loc[3];
-  cafe_geo_dn(K, ci, cj, ck, cs, dn);
-  double dr = cafe_geo_loc(R, dn, loc);
-  double f = crm_pow_half(cafe_geo_costh(dn) * cafe_geo_sinph(dn));
-  *g_out = f * dr;
-  double pk[3][3];
-  int s0i = cafe_geo_corners(loc, dr, pk);
-  double d1I, dI2, d1J, dJ3;
-  cafe_geo_edge(loc, pk[0], pk[1], &d1I, &dI2);
-  cafe_geo_edge(loc, pk[0], pk[2], &d1J, &dJ3);
-  double Lmud = cafe_geo_lmud(K, l, d1I, dI2, d1J, dJ3);
-  *ext_out = f * Lmud * 1.0;
-  cafe_geo_centre(R, cs, pk[0], s0i, Lmud, cen_out);
-}
-
 // One orientation of SampleOrientation::GenerateSamples (SampleOrientation.C:
 // 124-161) for a single sample with engine seed `seed`.
 __device__ __noinline__ void cafe_sample_orientation(const CafeConsts &K, unsigned int seed,

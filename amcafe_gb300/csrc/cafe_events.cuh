@@ -96,42 +96,12 @@ __device__ __forceinline__ unsigned long long cafe_row_sort_warp(const CafeDev &
 // ------------------------------------------------------------------ lower bounds
 // Most rows cannot capture within the step, and their exact geometry (~600 FP64
 // instructions a slot, 64 cycles each on this GPU) would only tell that they
-// cannot. So every slot's numerator is first bounded in single precision, with
-// the folded angles of VoxelsCA.C:409-424 in closed form: g = sqrt(cos th sin ph)
-// |R^T dn|_1, cos th = max(|dx|, |dy|)/rho and sin ph = max(rho, |dz|)/r, both in
-// [1/sqrt 2, 1].
+// cannot. So every slot's numerator is first bounded in single precision
+// (cafe_glb_slot).
 // A row whose bound says that it is not due within CAFE_DUE_REACH time steps gets
 // no record (row_n = CAFE_NO_RECORD, row_glb its bound), only a key; the event
 // loop makes the record if the row is needed after all.
 #define CAFE_NO_RECORD 255
-// A double in single precision, truncated (no FP64 instruction); zero below the
-// normal range, NaN above 2^127.
-__device__ __forceinline__ float cafe_trunc_f32(double x) {
-  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - (1023 - 127);
-  const int f = (hi & (int)0x80000000) | ((e << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29));
-  return e <= 0 ? 0.f : (e >= 255 ? NAN : __int_as_float(f));
-}
-// Bounds of g of the slot in direction `lane` (0..25) of a cell whose centre lies
-// at c0 from its octahedron's, rotation R. The offsets are good to 3e-7 of |c0|
-// plus the cell size (truncation, one product and sum), e is over three times
-// that, and R's truncation adds as little; the quotients take the errors of both
-// operands, so that offsets that cancel only loosen the bound. NaN where an
-// operand is not finite.
-__device__ __forceinline__ void cafe_glb_slot(int lane, const float *c0, float dx, const float *R, float &lo, float &hi) {
-  const float e = 1e-6f * (fabsf(c0[0]) + fabsf(c0[1]) + fabsf(c0[2]) + 3.f * dx);
-  const int d27 = lane < 13 ? lane : lane + 1;
-  const float a = c0[0] + (float)(d27 % 3 - 1) * dx, b = c0[1] + (float)(d27 / 3 % 3 - 1) * dx,
-              c = c0[2] + (float)(d27 / 9 - 1) * dx;
-  const float rho2 = a * a + b * b, r2 = rho2 + c * c, rho = sqrtf(rho2);
-  const float ct = fmaxf(0.7071f, (fmaxf(fabsf(a), fabsf(b)) - e) / (rho + 1.5f * e));
-  const float sp = fmaxf(0.7071f, (fmaxf(rho, fabsf(c)) - 1.5f * e) / (sqrtf(r2) + 2.f * e));
-  const float l0 = R[0] * a + R[3] * b + R[6] * c, l1 = R[1] * a + R[4] * b + R[7] * c,
-              l2 = R[2] * a + R[5] * b + R[8] * c;
-  const float l = fabsf(l0) + fabsf(l1) + fabsf(l2);
-  lo = sqrtf(ct * sp) * fmaxf(l - 8.f * e, 0.f) * (1.f - 1e-5f);
-  hi = (l + 8.f * e) * (1.f + 1e-5f);
-  if (!(r2 < 1e30f) || !(l < 1e30f) || !(e > 1e-20f)) lo = hi = NAN;  // (fmaxf drops a NaN operand)
-}
 // The offsets c0 of a cell (si, sj, sk) from octahedron centre cs.
 __device__ __forceinline__ void cafe_glb_centre(const CafeConsts &K, int si, int sj, int sk, const double *cs, float *c0) {
   double dn[3];
@@ -383,19 +353,6 @@ __device__ __noinline__ void cafe_row_best(const CafeDev &D, int r, double E, do
 // log holds fl(v * DtMin) when the step's rows share one velocity (v NaN here),
 // else DtMin, which each row multiplies by its own velocity.
 #define CAFE_M_DONE 0x7fffffff  // row_m of a row whose extent is kept current elsewhere
-
-// a / v for 0 < v normal, y = 1/v correctly rounded: two corrections of a * y by
-// the exact remainder (Markstein, IBM J. Res. Dev. 34(1), 1990: with a correctly
-// rounded reciprocal the last one rounds the quotient correctly from a faithful
-// one). Operands near the ends of the exponent range take the division.
-__device__ __forceinline__ double cafe_div_by(double a, double v, double y) {
-  const int ea = (int)((crm_bits(a) >> 52) & 0x7ff), ev = (int)((crm_bits(v) >> 52) & 0x7ff);
-  if (ea < 200 || ea > 1800 || ev < 800 || ev > 1200 || (crm_bits(v) & 0xfffffffffffffLL) == 0xfffffffffffffLL)
-    return a / v;
-  double q = a * y;
-  q = fma(fma(-q, v, a), y, q);
-  return fma(fma(-q, v, a), y, q);
-}
 
 // One event's growth of an extent (VoxelsCA.C:511-516).
 __device__ __forceinline__ double cafe_grow(double E, double vd) {
@@ -806,11 +763,6 @@ __device__ __forceinline__ unsigned long long cafe_warp_min_key(unsigned long lo
   src = __ffs(__ballot_sync(0xffffffffu, hi == mh && lo == ml)) - 1;
   return ((unsigned long long)mh << 32) | ml;
 }
-// Order key of the high word of a double, or of a float (exponent mask xm);
-// 0xffffffff for inf and NaN.
-__device__ __forceinline__ uint32_t cafe_key32(int hi, int xm) {
-  return (hi & xm) == xm ? 0xffffffffu : (uint32_t)(hi ^ ((hi >> 31) | (int)0x80000000));
-}
 
 // Place k of the record of row r, resident index i, becomes its first slot;
 // place n: none is left.
@@ -888,23 +840,13 @@ __device__ __forceinline__ uint32_t cafe_close_key(uint32_t k) {
 }
 
 // The largest key that a winner at clock T may have and be the global one; Vf:
-// the common velocity, rounded down. Every event's limit is on its chain, and a
-// double-precision operation costs as much as ten others: one subtraction and one
-// conversion, then single precision rounded towards earlier.
+// the common velocity, rounded down.
 template <bool PR>
 __device__ __forceinline__ uint32_t cafe_window_limit(const CafeResident &S, float Vf, int ev, double T, double dsum) {
   if (!S.all && !(ev < S.ev_cap && (unsigned long long)crm_bits(dsum) <= (unsigned long long)crm_bits(S.dsum_cap))) return 0u;
   double lim = S.wlim - T;
   if (cafe_key(lim) > cafe_key(0x1.e847fp19)) lim = 0x1.e847fp19;  // 0x1.e847fp19 < 1e6
-  float f = __double2float_rd(lim);
-  if (!PR) f = __fmul_rd(f, Vf);
-  f = __fmaf_rd(-fabsf(f), 0x1p-17f, f);
-  const int b = __float_as_int(f), e = b >> 23 & 0xff;
-  if (e == 255) return 0u;  // (below the range)
-  if (PR) return cafe_key32(b, 0x7f800000);
-  // as the high word of a double, towards earlier; beyond single precision's range: the nearest bound
-  if (e == 0) return b < 0 ? cafe_key32((int)0xb8100000, 0x7ff00000) : 0x80000000u;
-  return cafe_key32((b & (int)0x80000000) | ((e + 896) << 20 | (b & 0x7fffff) >> 3) + (b < 0 ? 1 : 0), 0x7ff00000);
+  return cafe_limit_key(lim, Vf, PR);
 }
 
 // The loop's rare parts, out of line: an event's chain pays for every
@@ -914,12 +856,8 @@ __device__ __forceinline__ uint32_t cafe_window_limit(const CafeResident &S, flo
 // Every resident's extent, place and (keys) key back to the row arrays.
 template <bool PR>
 __device__ __noinline__ void cafe_res_flush(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, int ev, bool keys) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
-  const unsigned FULL = 0xffffffffu;
   const double V = K.vhat_cls[1];
-  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
-  for (int i = tid; i < S.top; i += NT) {
+  for (int i = threadIdx.x; i < S.top; i += CAFE_LOOP_THREADS) {
     const int r = S.r[i];
     if (r < 0) continue;
     D.row_E[r] = S.E[i];
@@ -984,7 +922,6 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   const unsigned FULL = 0xffffffffu;
   const double V = K.vhat_cls[1];
-  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
   cafe_res_flush<PR>(D, K, L, S, ev, true);
   __syncthreads();
   // the first window takes its rows from the list of those that may be due
@@ -1117,9 +1054,7 @@ template <bool PR>
 __device__ __noinline__ void cafe_select_exact(const CafeDev &D, const CafeConsts &K, CafeResident &S, uint32_t kthr) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
-  const unsigned FULL = 0xffffffffu;
   const double V = K.vhat_cls[1];
-  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
   CafeCand wc = cafe_cand_none();
   const int top = S.top;
   for (int i = tid; i < top; i += NT) {
@@ -1234,11 +1169,9 @@ __device__ __noinline__ bool cafe_negative_event(const CafeDev &D, const CafeCon
 // resident set (true: open a new window).
 template <bool PR>
 __device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K, CafeLoop &L, CafeResident &S, CafeQuadScratch *Q, int ev, int icap) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
-  const unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  constexpr int NT = CAFE_LOOP_THREADS;
   const double V = K.vhat_cls[1];
-  (void)lane, (void)warp, (void)FULL, (void)V, (void)NT, (void)NW;
   const int nr = L.newrow;
   if (!L.fill) {
     if (tid == 0) {
@@ -1849,8 +1782,8 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
   __shared__ CafeQuadScratch Q[CAFE_QUADS];
   __shared__ CafeDev sD;
   __shared__ CafeConsts sK;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_LOOP_THREADS / 32;
+  const int tid = threadIdx.x;
+  constexpr int NT = CAFE_LOOP_THREADS;
   if (cafe_bid != 0) return;  // event_fill_helper's second block: the loop leaves it nothing to do
   for (int i = tid; i < (int)(sizeof(CafeDev) / 4); i += NT) ((uint32_t *)&sD)[i] = ((const uint32_t *)&D)[i];
   for (int i = tid; i < (int)(sizeof(CafeConsts) / 4); i += NT) ((uint32_t *)&sK)[i] = ((const uint32_t *)&K)[i];

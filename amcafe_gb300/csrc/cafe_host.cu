@@ -843,7 +843,6 @@ int end_of_scan(cafe_sim *s, const int *hot_known = nullptr) {
 int launch_voxels(cafe_sim *s, bool graph, const CafeStepParams *Pp) {
   CafeDev &D = s->D;
   const CafeConsts &K = s->K;
-  const CafeStepParams &P = s->P;
   cudaStream_t st = s->stream;
   int nb = (int)s->nblk;
   {

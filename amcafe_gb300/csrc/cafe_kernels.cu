@@ -12,10 +12,14 @@
 //   k_gather        per-position copies, neighbour positions (VoxelsCA.C:
 //                   283-335), ruq offsets (VoxelsCA.C:380) by RNG jump-ahead
 //   k_lists_*       vs2ind (mushy positions in order) and frontier rows
-//   k_rows_*        capture-time numerators per (frontier cell, liquid
-//                   neighbour), sorted per cell
-//   k_event_loop    the sequential capture/nucleation loop (VoxelsCA.C:
-//                   381-610), one thread block
+//   k_rows_*        (cafe_events.cuh) bounds on the rows' capture times; for
+//                   the rows that may capture soon the numerators per liquid
+//                   neighbour, sorted per cell
+//   k_children      (cafe_events.cuh) rows of the cells that those rows will
+//                   capture within the step, two generations ahead
+//   k_event_loop    (cafe_events.cuh) the sequential capture/nucleation loop
+//                   (VoxelsCA.C:381-610), one thread block
+//   k_rows_finalize growth of the rows the loop left aside (VoxelsCA.C:511-516)
 //   k_writeback     VoxelsCA.C:633-643
 //   k_mushy2solid   ConvertSolid1(0) (VoxelsCA.C:739-758), in place
 // All FP64 arithmetic follows the reference's expression order; the file is
@@ -33,20 +37,8 @@
 // batch's autotuner finds more to be faster (many realisations fill the GPU).
 #define CAFE_ACT_MAX_CHUNKS 4
 #define CAFE_LOOP_THREADS 512
-#ifdef CAFE_DETAIL_CYCLES
-// clock read ordered with the surrounding memory operations and barriers
-__device__ __forceinline__ long long cafe_clock_ordered() {
-  long long t;
-  asm volatile("mov.u64 %0, %%clock64;" : "=l"(t)::"memory");
-  return t;
-}
-#endif
 
 // ------------------------------------------------------------------ helpers
-// Hint: bring the line holding *a into this SM's L1 (no effect on results).
-__device__ __forceinline__ void cafe_prefetch_l1(const void *a) {
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
-}
 // Growth velocity of active position p (VoxelsCA.C:405): per temperature class
 // with the analytic field, per cell with the EASM field.
 __device__ __forceinline__ double cafe_vh(const CafeDev &D, const CafeConsts &K, int p) {
@@ -108,43 +100,15 @@ __device__ __forceinline__ void d_melt(const CafeDev &D, const CafeConsts &K, co
   const int lane = threadIdx.x & 31, warps = (cafe_nblk * blockDim.x) >> 5;
   const long long iz1 = (long long)P.ilaserLoc * K.nxy;
   int any = 0;
-  const float fux = (float)(P.cg * K.dx[0]), fwx = (float)(-P.sg * K.dx[0]);
-  const float i1 = K.ra1[1], i2 = K.ra1[2], i3 = K.ra1[3], i4 = K.ra1[4], i5 = K.ra1[5];
-  const float imax = fmaxf(fmaxf(fmaxf(fabsf(i1), fabsf(i2)), fmaxf(fabsf(i3), fabsf(i4))), fabsf(i5));
-  const float front = (float)K.bmDX0;
-  // (the sign of dirp r0 is that of the factors unless the product underflows)
-  const bool ok = imax < 1e30f && (P.dirp == 0.0 || fabs(P.dirp) > 1e-200) && !P.any_hot_full;
-  const float sd = P.dirp > 0.0 ? 1.f : (P.dirp < 0.0 ? -1.f : 0.f);
+  const CafeClassStep C = cafe_class_step(K.ra1, K.bmDX0, P.dirp, P.cg, P.sg, K.dx[0], P.any_hot_full != 0);
   for (int row = (cafe_bid * blockDim.x + threadIdx.x) >> 5; row < by * bz; row += warps) {
     const int j = P.lo[1] + row % by, k = P.lo[2] + row / by;
     const double zp = ((double)k + .5) * K.dx[2], y0 = ((double)j + .5) * K.dx[1];
     const double X = ((double)P.lo[0] + .5) * K.dx[0] - K.hLX0, Y = y0 - K.hLX1;
-    const float u0 = (float)(P.cg * X + P.sg * Y + K.hLX0 - P.lx), w0 = (float)(-P.sg * X + P.cg * Y + K.hLX1 - P.ly);
-    const float r2 = (float)(zp - P.lz);
-    const bool above = zp > P.lz;
-    // coordinates relative to the laser, in error by at most eu (roundings to single
-    // precision of the row's first and along it), quotients by eq
-    const float eu = 0x1p-21f * (fabsf(u0) + fabsf(w0) + fabsf(r2) + (fabsf(fux) + fabsf(fwx)) * (float)bx);
-    const float eq = eu * imax, amb = 16.f * eq + 1e-5f;
-    const bool usable = ok && eq < 0.01f;
+    const CafeClassRow W = cafe_class_row(C, P.cg, P.sg, K.hLX0, K.hLX1, P.lx, P.ly, P.lz, X, Y, zp, bx);
     const long long base = (long long)K.nxy * k + (long long)K.nx * j + P.lo[0];
     for (int x = lane; x < bx; x += 32) {
-      int c = -1;
-      if (above) {
-        c = 0;
-      } else if (usable) {
-        const float u = u0 + fux * (float)x, w = w0 + fwx * (float)x;
-        const float du = sd * u;
-        if (fabsf(u) > 2.f * eu || sd == 0.f) {
-          const bool ahead = du > 0.f;
-          const float q1 = w * (ahead ? i1 : i4), q2 = r2 * (ahead ? i2 : i5), q0 = ahead ? 0.f : u * i3;
-          const float d = q0 * q0 + q1 * q1 + q2 * q2;
-          if (d > 1.f + amb || (ahead && fabsf(u) > front + 2.f * eu))
-            c = 1;
-          else if (d < 1.f - amb && (!ahead || fabsf(u) < front - 2.f * eu))
-            c = 2;
-        }
-      }
+      int c = cafe_class_fast(C, W, x);
       const int i = P.lo[0] + x;
       if (c < 0) c = cafe_temp_class_exact(K, P, i, j, k);
       D.tcls[(long long)row * bx + x] = (uint8_t)c;
@@ -901,17 +865,6 @@ __device__ __forceinline__ bool cafe_is_neg(double x) {
   long long b = crm_bits(x);
   return b < 0 && (b & CRM_ABS_MASK) != 0 && (b & CRM_ABS_MASK) <= CRM_BITS_INF;
 }
-// e with |x| < 2^e (a large value for inf and NaN)
-__device__ __forceinline__ int cafe_exp_ub(double x) {
-  int f = (int)((crm_bits(x) >> 52) & 0x7ff);
-  return f == 0x7ff ? 4096 : (f == 0 ? -1022 : f - 1022);
-}
-// e with |x| >= 2^e for a normal x (a small value for zero and subnormals)
-__device__ __forceinline__ int cafe_exp_lb(double x) {
-  int f = (int)((crm_bits(x) >> 52) & 0x7ff);
-  return f == 0 ? -4096 : f - 1023;
-}
-
 #include "cafe_events.cuh"
 
 // Brings every row's extent up to the end of the step (the lazily applied
