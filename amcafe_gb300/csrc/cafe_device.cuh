@@ -17,6 +17,7 @@
 
 #include "cafe_bounds.h"
 #include "cafe_crmath.h"
+#include "cafe_intmath.h"
 #include "cafe_rng.h"
 
 #define CAFE_NSLOT 26
@@ -285,11 +286,11 @@ __device__ __forceinline__ double cafe_rosenthal_T(const CafeConsts &K, const Ca
   double xp = P.cg * (x0 - K.hLX0) + P.sg * (y0 - K.hLX1) + K.hLX0;
   double yp = -P.sg * (x0 - K.hLX0) + P.cg * (y0 - K.hLX1) + K.hLX1;
   double r0 = xp - P.lx, r1 = yp - P.ly, r2 = zp - P.lz;
-  double R = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
+  double R = crm_sqrt_int(r0 * r0 + r1 * r1 + r2 * r2);
   if (R < K.ros_rmin) R = K.ros_rmin;
   double sd = P.dirp > 0 ? 1.0 : (P.dirp < 0 ? -1.0 : 0.0);
   double xi = sd * r0;
-  return K.T0 + K.ros_q / R * crm_exp(-(K.ros_c * (R + xi)));
+  return K.T0 + crm_div_int(K.ros_q, R) * crm_exp_int(-(K.ros_c * (R + xi)));
 }
 
 __device__ __forceinline__ void cafe_cell_xyz(const CafeConsts &K, long long idx, int &i, int &j,

@@ -1383,27 +1383,43 @@ __device__ __forceinline__ void cafe_easm_materials(double T, double M[4]) {
   M[0] = cP;
   M[1] = k;
   M[2] = rho;
-  M[3] = k / (rho * cP);
+  M[3] = crm_div_int(k, rho * cP);
+}
+// What an integral's nodes share: C of Temp_Fun_G, the material's M[3], the
+// squared distances across and below.
+struct CafeEasmPoint {
+  double C, M3, dy2, dz2;
+};
+__device__ __forceinline__ CafeEasmPoint cafe_easm_point(const CafeEasm &E, double R1, double R2, double Ly, double Lz,
+                                                         double T) {
+  const double eta = 0.56, pi = 3.14159265358979323846;
+  double M[4];
+  cafe_easm_materials(T, M);
+  const double dy = R1 - Ly, dz = fabs(R2 - Lz);
+  CafeEasmPoint p;
+  p.C = crm_div_int(eta * E.Q, pi * M[2] * M[0] * crm_sqrt_int(4 * pi * M[3]));
+  p.M3 = M[3];
+  p.dy2 = dy * dy;
+  p.dz2 = dz * dz;
+  return p;
+}
+// Term i of the rule. The field is bound by FP64 issue: with floating-point
+// divisions and exp a node took ~110 FP64 instructions, with the integer ones
+// (cafe_intmath.h, the same bits) ten.
+__device__ __forceinline__ double cafe_easm_node(const CafeEasm &E, const CafeEasmPoint &p, int i, double Lx, double R0) {
+  const double sigma = 50.0e-6;
+  const double m = 2 * p.M3 * E.tx[i], d = m + sigma * sigma, dx = R0 - Lx;
+  // (4 M3 tx + 2 sigma^2 and 4 M3 tx are exactly 2 d and 2 m)
+  const crm_recip rd = crm_reciprocal(d);
+  const double a = crm_quotient(p.C * E.r[i], rd, d, 0);
+  const double arg = -crm_quotient(dx * dx + p.dy2, rd, d, 1) - crm_quotient(p.dz2, crm_reciprocal(m), m, 1);
+  return E.qw[i] * (a * crm_exp_int(arg));
 }
 __device__ __forceinline__ double cafe_easm_integral(const CafeEasm &E, const double *Lx, double R0, double R1,
                                                      double R2, double Ly, double Lz, double T) {
-  const double sigma = 50.0e-6, eta = 0.56, pi = 3.14159265358979323846;
-  double M[4];
-  cafe_easm_materials(T, M);
-  double C = eta * E.Q / (pi * M[2] * M[0] * sqrt(4 * pi * M[3]));
-  double sig2 = sigma * sigma;
-  double dy = R1 - Ly, dz = fabs(R2 - Lz);
-  double dy2 = dy * dy, dz2 = dz * dz;
+  const CafeEasmPoint p = cafe_easm_point(E, R1, R2, Ly, Lz, T);
   double s = 0.0;
-  for (int i = 0; i < CAFE_EASM_NODES; ++i) {
-    double tx = E.tx[i];
-    double dx = R0 - Lx[i];
-    double a = C * E.r[i] / (2 * M[3] * tx + sig2);
-    double arg = -1 * (dx * dx + dy2) / (4 * M[3] * tx + 2 * sig2) - dz2 / (4 * M[3] * tx);
-    // exp(arg) is exactly 0 below -745.2, and so is this term
-    double f = arg < -745.2 ? a * 0.0 : a * crm_exp(arg);
-    s += E.qw[i] * f;
-  }
+  for (int i = 0; i < CAFE_EASM_NODES; ++i) s += cafe_easm_node(E, p, i, Lx[i], R0);
   return 300 + s;
 }
 __global__ void k_set_int(int *p, int v) { *p = v; }
@@ -1570,23 +1586,8 @@ __global__ void k_easm(CafeDev D, CafeConsts K, CafeStepParams P, CafeEasm E, lo
 __device__ __forceinline__ double cafe_easm_integral_warp(const CafeEasm &E, const double *Lx, double R0, double R1,
                                                           double R2, double Ly, double Lz, double T, int lane) {
   const unsigned FULL = 0xffffffffu;
-  const double sigma = 50.0e-6, eta = 0.56, pi = 3.14159265358979323846;
-  double M[4];
-  cafe_easm_materials(T, M);
-  double C = eta * E.Q / (pi * M[2] * M[0] * sqrt(4 * pi * M[3]));
-  double sig2 = sigma * sigma;
-  double dy = R1 - Ly, dz = fabs(R2 - Lz);
-  double dy2 = dy * dy, dz2 = dz * dz;
-  double p = 0.0;
-  if (lane < CAFE_EASM_NODES) {
-    int i = lane;
-    double tx = E.tx[i];
-    double dx = R0 - Lx[i];
-    double a = C * E.r[i] / (2 * M[3] * tx + sig2);
-    double arg = -1 * (dx * dx + dy2) / (4 * M[3] * tx + 2 * sig2) - dz2 / (4 * M[3] * tx);
-    double f = arg < -745.2 ? a * 0.0 : a * crm_exp(arg);
-    p = E.qw[i] * f;
-  }
+  const CafeEasmPoint pt = cafe_easm_point(E, R1, R2, Ly, Lz, T);
+  const double p = lane < CAFE_EASM_NODES ? cafe_easm_node(E, pt, lane, Lx[lane], R0) : 0.0;
   double s = 0.0;
 #pragma unroll
   for (int i = 0; i < CAFE_EASM_NODES; ++i) s += __shfl_sync(FULL, p, i);

@@ -83,6 +83,22 @@ def main():
         h, l = split(1 / mpmath.factorial(n))
         out.append("#define CRM_INV_FACT%s_HI %s" % (name, hx(h)))
         out.append("#define CRM_INV_FACT%s_LO %s" % (name, hx(l)))
+    # exp in integers: 2^(-j/128) / 2 as 64 + 32 bits, truncated; constants with
+    # the number of fraction bits in their names (CRM_LOG2E_95: the 32 bits that
+    # follow those of CRM_LOG2E_63)
+    rows = []
+    for j in range(128):
+        v = int(mpmath.floor(mpmath.ldexp(mpmath.power(2, -mpmath.mpf(j) / 128), 95)))
+        rows.append("  {0x%xULL, 0x%xULL}," % (v >> 32, v & 0xffffffff))
+    out.append("CRM_TABLE_DECL(unsigned long long, crm_exp2n_tab, [128][2]) = {")
+    out += rows
+    out.append("};")
+    v = int(mpmath.floor(mpmath.ldexp(1 / mpmath.log(2), 95)))
+    out.append("#define CRM_LOG2E_63 0x%xULL" % (v >> 32))
+    out.append("#define CRM_LOG2E_95 0x%xULL" % (v & 0xffffffff))
+    out.append("#define CRM_LN2_64 0x%xULL" % int(mpmath.floor(mpmath.ldexp(mpmath.log(2), 64))))
+    for n, bits in ((120, 38), (720, 40), (5040, 42)):
+        out.append("#define CRM_R%d_%d 0x%xU" % (n, bits, int(mpmath.nint(mpmath.ldexp(mpmath.mpf(1) / n, bits)))))
     out.append("#endif")
     print("\n".join(out))
 

@@ -1,0 +1,25 @@
+// Test-only wrapper exposing the host side of amcafe_gb300/csrc/cafe_intmath.h
+// beside the floating-point functions. Built by tests/test_intmath.py.
+#include "../../amcafe_gb300/csrc/cafe_intmath.h"
+
+extern "C" void ic_eval(int fn, long n, const double *x, const double *y, double *got, double *want) {
+  for (long i = 0; i < n; ++i) {
+    switch (fn) {
+      case 0:
+        got[i] = crm_exp_int(x[i]);
+        want[i] = crm_exp(x[i]);
+        break;
+      case 1:
+        got[i] = crm_div_int(x[i], y[i]);
+        want[i] = x[i] / y[i];
+        break;
+      case 2:
+        got[i] = crm_quotient(x[i], crm_reciprocal(y[i]), y[i], 1);
+        want[i] = x[i] / (2 * y[i]);
+        break;
+      default:
+        got[i] = crm_sqrt_int(x[i]);
+        want[i] = sqrt(x[i]);
+    }
+  }
+}

@@ -1,0 +1,88 @@
+"""cafe_intmath.h (exp, division, square root in integers) returns the bits of the
+floating-point functions, inside its ranges and outside (CPU only)."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+D = ctypes.POINTER(ctypes.c_double)
+
+
+@pytest.fixture(scope="module")
+def ic(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("ic") / "ic.so")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fPIC", "-shared",
+                    os.path.join(HERE, "native", "intmath_check.cpp"), "-o", so], check=True)
+    return ctypes.CDLL(so)
+
+
+def _same(ic, fn, x, y=None):
+    x = np.ascontiguousarray(x, np.float64)
+    y = x if y is None else np.ascontiguousarray(y, np.float64)
+    got, want = np.empty_like(x), np.empty_like(x)
+    ic.ic_eval(fn, ctypes.c_long(len(x)), *(a.ctypes.data_as(D) for a in (x, y, got, want)))
+    bad = (got.view(np.int64) != want.view(np.int64)) & ~(np.isnan(got) & np.isnan(want))
+    assert not bad.any(), (x[bad][:4], y[bad][:4], got[bad][:4], want[bad][:4])
+
+
+EDGES = np.array([0.0, np.inf, np.nan, 5e-324, 2.2250738585072014e-308, 1.7976931348623157e308, 1.0, 2.0, 0.5,
+                  np.nextafter(1.0, 0), np.nextafter(1.0, 2), np.nextafter(2.0, 0), 4.0, np.nextafter(4.0, 0)])
+
+
+def _around(v, n=40):
+    out = [v]
+    for s in (-np.inf, np.inf):
+        w = v
+        for _ in range(n):
+            w = np.nextafter(w, s)
+            out.append(w)
+    return np.array(out)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "scales", "steps", "limits"])
+def test_exp(ic, kind):
+    g, n = np.random.default_rng(5), 300000
+    if kind == "uniform":
+        x = -g.uniform(0, 760, n)
+    elif kind == "scales":
+        x = -(2.0 ** g.uniform(-60, 11, n))
+    elif kind == "steps":  # at and beside the table's steps and the powers of two
+        k = g.integers(1, 128 * 1020, n) * (np.log(2) / 128)
+        x = -k * (1 + g.integers(-3, 4, n) * 2.0 ** -52)
+    else:
+        x = np.concatenate([_around(-v) for v in (707.0, 745.2, 2.0 ** -40, 1.0, np.log(2), 708.4, 709.8)] +
+                           [EDGES, -EDGES, g.uniform(0, 720, 1000)])
+    _same(ic, 0, x)
+
+
+def _numbers(g, n, emax):
+    m = 1 + g.integers(0, 2 ** 52, n) * 2.0 ** -52
+    k = n // 3  # significands near the ends
+    m[:k] = np.where(g.integers(0, 2, k), 1 + g.integers(0, 4, k) * 2.0 ** -52, 2 - g.integers(1, 5, k) * 2.0 ** -52)
+    g.shuffle(m)
+    with np.errstate(all="ignore"):
+        return m * 2.0 ** g.integers(-emax, emax, n).astype(float)
+
+
+@pytest.mark.parametrize("fn", [1, 2])
+@pytest.mark.parametrize("emax", [3, 400, 1020])
+def test_division(ic, fn, emax):
+    g, n = np.random.default_rng(emax), 300000
+    a, b = _numbers(g, n, emax) * g.choice([-1, 1], n), _numbers(g, n, emax)
+    b[::97] *= -1
+    _same(ic, fn, a, b)
+    e = np.concatenate([EDGES, -EDGES])
+    _same(ic, fn, np.repeat(e, len(e)), np.tile(e, len(e)))
+
+
+@pytest.mark.parametrize("emax", [3, 400, 1020])
+def test_sqrt(ic, emax):
+    g, n = np.random.default_rng(emax), 300000
+    x = _numbers(g, n, emax)
+    _same(ic, 3, x)
+    with np.errstate(all="ignore"):  # squares and their neighbours
+        s = (x * 2.0 ** 26 % 2 ** 26) ** 2
+    _same(ic, 3, np.concatenate([s, np.nextafter(s, 0), np.nextafter(s, np.inf), EDGES, -EDGES]))
