@@ -17,6 +17,18 @@ extern "C" void ic_eval(int fn, long n, const double *x, const double *y, double
         got[i] = crm_quotient(x[i], crm_reciprocal(y[i]), y[i], 1);
         want[i] = x[i] / (2 * y[i]);
         break;
+      case 4:
+        got[i] = crm_atan2(x[i], y[i]);
+        want[i] = crm_atan2_acc(x[i], y[i]);
+        break;
+      case 5:
+        got[i] = crm_sin(x[i]);
+        want[i] = crm_sin_acc(x[i]);
+        break;
+      case 6:
+        got[i] = crm_cos(x[i]);
+        want[i] = crm_cos_acc(x[i]);
+        break;
       default:
         got[i] = crm_sqrt_int(x[i]);
         want[i] = sqrt(x[i]);

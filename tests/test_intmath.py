@@ -1,5 +1,6 @@
 """cafe_intmath.h (exp, division, square root in integers) returns the bits of the
-floating-point functions, inside its ranges and outside (CPU only)."""
+floating-point functions, inside its ranges and outside, and cafe_crmath.h's fast
+paths those of its double-double paths (CPU only)."""
 import ctypes
 import os
 import subprocess
@@ -86,3 +87,21 @@ def test_sqrt(ic, emax):
     with np.errstate(all="ignore"):  # squares and their neighbours
         s = (x * 2.0 ** 26 % 2 ** 26) ** 2
     _same(ic, 3, np.concatenate([s, np.nextafter(s, 0), np.nextafter(s, np.inf), EDGES, -EDGES]))
+
+
+@pytest.mark.parametrize("kind", ["uniform", "scales", "midpoints"])
+def test_fast_paths(ic, kind):
+    """arctangent, sine and cosine at arguments where the series' terms are largest"""
+    g, n = np.random.default_rng(2), 400000
+    y, x = g.uniform(0, 1, n), g.uniform(0, 1, n)
+    t = g.uniform(0, np.pi / 2, n)
+    if kind == "scales":
+        y *= 2.0 ** g.uniform(-60, 0, n)
+        t = np.where(g.integers(0, 2, n), np.pi / 2 - t * 2.0 ** g.uniform(-50, 0, n), t * 2.0 ** g.uniform(-50, 0, n))
+    elif kind == "midpoints":  # between the tables' points
+        y = x * (g.integers(0, 64, n) + 0.5) / 64 * (1 + g.uniform(-1, 1, n) * 1e-3)
+        t = (g.integers(0, 201, n) + 0.5) / 128 * (1 + g.uniform(-1, 1, n) * 1e-3)
+    _same(ic, 4, y, x)
+    _same(ic, 4, x, y)
+    _same(ic, 5, t)
+    _same(ic, 6, t)
