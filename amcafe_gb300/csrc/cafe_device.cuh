@@ -340,7 +340,9 @@ __device__ __forceinline__ void cafe_rot_from_cth(const double *c, double *R) {
 // The computation is split into parts with no data dependence between them
 // (the th and ph chains, the two point-line projections), so that several
 // warps can share one evaluation. Every part is the same expression sequence
-// wherever it runs.
+// wherever it runs; its functions are the integer ones (cafe_intmath.h), bit for
+// bit those of the floating-point sequences, which a warp of their own took 17k
+// cycles for.
 __device__ __forceinline__ void cafe_geo_dn(const CafeConsts &K, int ci, int cj, int ck, const double *cs,
                                             double *dn) {
   dn[0] = ((double)ci + .5) * K.dx[0] - cs[0];
@@ -350,22 +352,22 @@ __device__ __forceinline__ void cafe_geo_dn(const CafeConsts &K, int ci, int cj,
 // cos(th), th = atan2(|dy|,|dx|) folded at pi/4
 __device__ __forceinline__ double cafe_geo_costh(const double *dn) {
   const double pi4 = 3.14159265358979323846 / 4.0, pi2 = 3.14159265358979323846 / 2.0;
-  double th = crm_atan2(fabs(dn[1]), fabs(dn[0]));
+  double th = crm_atan2_int(fabs(dn[1]), fabs(dn[0]));
   th = th > pi4 ? pi2 - th : th;
-  return crm_cos(th);
+  return crm_cos_int(th);
 }
 // sin(ph), ph = atan2(sqrt(dx^2+dy^2),|dz|) folded at pi/4
 __device__ __forceinline__ double cafe_geo_sinph(const double *dn) {
   const double pi4 = 3.14159265358979323846 / 4.0, pi2 = 3.14159265358979323846 / 2.0;
-  double ph = crm_atan2(crm_pow_half(dn[0] * dn[0] + dn[1] * dn[1]), fabs(dn[2]));
+  double ph = crm_atan2_int(crm_pow_half_int(dn[0] * dn[0] + dn[1] * dn[1]), fabs(dn[2]));
   ph = ph < pi4 ? pi2 - ph : ph;
-  return crm_sin(ph);
+  return crm_sin_int(ph);
 }
 // distance between the capturing and the captured cell centres
 __device__ __forceinline__ double cafe_geo_l(const CafeConsts &K, int ci, int cj, int ck, int si, int sj,
                                              int sk) {
   double q0 = (ci - si) * K.dx[0], q1 = (cj - sj) * K.dx[1], q2 = (ck - sk) * K.dx[2];
-  return crm_pow_half(q0 * q0 + q1 * q1 + q2 * q2);
+  return crm_pow_half_int(q0 * q0 + q1 * q1 + q2 * q2);
 }
 // dn in the crystal frame, R^T dn, and its 1-norm
 __device__ __forceinline__ double cafe_geo_loc(const double *R, const double *dn, double *loc) {
@@ -454,10 +456,11 @@ __device__ __forceinline__ int cafe_geo_corners(const double *loc, double dr, do
 __device__ __forceinline__ void cafe_project(const double *A, const double *x0, const double *x1,
                                              double *xp) {
   double e0 = x1[0] - x0[0], e1 = x1[1] - x0[1], e2 = x1[2] - x0[2];
-  double snorm = crm_pow_half(e0 * e0 + e1 * e1 + e2 * e2);
-  double n0 = e0 / snorm, n1 = e1 / snorm, n2 = e2 / snorm;
+  double snorm = crm_pow_half_int(e0 * e0 + e1 * e1 + e2 * e2);
+  const crm_recip rs = crm_reciprocal(snorm);
+  double n0 = crm_quotient(e0, rs, snorm, 0), n1 = crm_quotient(e1, rs, snorm, 0), n2 = crm_quotient(e2, rs, snorm, 0);
   double d = -(n0 * A[0] + n1 * A[1] + n2 * A[2]);
-  double t = (-d - n0 * x0[0] - n1 * x0[1] - n2 * x0[2]) / (n0 * e0 + n1 * e1 + n2 * e2);
+  double t = crm_div_int(-d - n0 * x0[0] - n1 * x0[1] - n2 * x0[2], n0 * e0 + n1 * e1 + n2 * e2);
   xp[0] = x0[0] + e0 * t;
   xp[1] = x0[1] + e1 * t;
   xp[2] = x0[2] + e2 * t;
@@ -470,9 +473,9 @@ __device__ __forceinline__ void cafe_geo_edge(const double *loc, const double *p
   cafe_project(loc, p0, p1, x);
   double e0, e1, e2;
   e0 = p0[0] - x[0]; e1 = p0[1] - x[1]; e2 = p0[2] - x[2];
-  *d0 = crm_pow_half(e0 * e0 + e1 * e1 + e2 * e2);
+  *d0 = crm_pow_half_int(e0 * e0 + e1 * e1 + e2 * e2);
   e0 = p1[0] - x[0]; e1 = p1[1] - x[1]; e2 = p1[2] - x[2];
-  *d1 = crm_pow_half(e0 * e0 + e1 * e1 + e2 * e2);
+  *d1 = crm_pow_half_int(e0 * e0 + e1 * e1 + e2 * e2);
 }
 // Half-diagonal Lmud of the new octahedron (VoxelsCA.C:578-582).
 __device__ __forceinline__ double cafe_geo_lmud(const CafeConsts &K, double l, double d1I, double dI2,

@@ -175,11 +175,11 @@ __device__ __forceinline__ double cafe_geo_quad(const CafeConsts &K, bool work, 
   }
   cafe_bar_quad(bar);
   if (!work) return 0.0;
-  if (w == 0) return crm_pow_half(S.cth[lane] * S.sph[lane]) * S.dr[lane];
+  if (w == 0) return crm_pow_half_int(S.cth[lane] * S.sph[lane]) * S.dr[lane];
   if (w >= 2) {
     double Lmud = cafe_geo_lmud(K, S.l[lane], S.d1I[lane], S.dI2[lane], S.d1J[lane], S.dJ3[lane]);
     if (w == 2) {
-      double f = crm_pow_half(S.cth[lane] * S.sph[lane]);
+      double f = crm_pow_half_int(S.cth[lane] * S.sph[lane]);
       o[0] = f * Lmud * 1.0;
     } else {
       double cn[3];

@@ -99,6 +99,32 @@ def main():
     out.append("#define CRM_LN2_64 0x%xULL" % int(mpmath.floor(mpmath.ldexp(mpmath.log(2), 64))))
     for n, bits in ((120, 38), (720, 40), (5040, 42)):
         out.append("#define CRM_R%d_%d 0x%xU" % (n, bits, int(mpmath.nint(mpmath.ldexp(mpmath.mpf(1) / n, bits)))))
+    # atan, cos in integers: atan(k/64), cos(j/128) with 63 + 32 fraction bits,
+    # sin(j/128) with 64; constants as above
+    def fix(v, bits):
+        return int(mpmath.floor(mpmath.ldexp(v, bits)))
+
+    rows = []
+    for k in range(65):
+        v = fix(mpmath.atan(mpmath.mpf(k) / 64), 95)
+        rows.append("  {0x%xULL, 0x%xULL}," % (v >> 32, v & 0xffffffff))
+    out.append("CRM_TABLE_DECL(unsigned long long, crm_atani_tab, [65][2]) = {")
+    out += rows
+    out.append("};")
+    rows = []
+    for j in range(102):
+        v = fix(mpmath.cos(mpmath.mpf(j) / 128), 95)
+        rows.append("  {0x%xULL, 0x%xULL, 0x%xULL}," % (v >> 32, v & 0xffffffff, fix(mpmath.sin(mpmath.mpf(j) / 128), 64)))
+    out.append("CRM_TABLE_DECL(unsigned long long, crm_cosi_tab, [102][3]) = {")
+    out += rows
+    out.append("};")
+    v = fix(pio2, 95)
+    out.append("#define CRM_PIO2_63 0x%xULL" % (v >> 32))
+    out.append("#define CRM_PIO2_95 0x%xULL" % (v & 0xffffffff))
+    for n, bits in ((3, 65), (5, 64), (6, 64), (24, 64)):
+        out.append("#define CRM_R%d_%d 0x%xULL" % (n, bits, fix(mpmath.mpf(1) / n, bits)))
+    for n, bits in ((7, 34), (9, 32), (11, 35), (720, 41), (5040, 44)):
+        out.append("#define CRM_R%d_%d 0x%xU" % (n, bits, int(mpmath.nint(mpmath.ldexp(mpmath.mpf(1) / n, bits)))))
     out.append("#endif")
     print("\n".join(out))
 

@@ -29,6 +29,22 @@ extern "C" void ic_eval(int fn, long n, const double *x, const double *y, double
         got[i] = crm_cos(x[i]);
         want[i] = crm_cos_acc(x[i]);
         break;
+      case 7:
+        got[i] = crm_atan2_int(x[i], y[i]);
+        want[i] = crm_atan2(x[i], y[i]);
+        break;
+      case 8:
+        got[i] = crm_cos_int(x[i]);
+        want[i] = crm_cos(x[i]);
+        break;
+      case 9:
+        got[i] = crm_sin_int(x[i]);
+        want[i] = crm_sin(x[i]);
+        break;
+      case 10:
+        got[i] = crm_pow_half_int(x[i]);
+        want[i] = crm_pow_half(x[i]);
+        break;
       default:
         got[i] = crm_sqrt_int(x[i]);
         want[i] = sqrt(x[i]);

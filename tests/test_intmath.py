@@ -1,4 +1,4 @@
-"""cafe_intmath.h (exp, division, square root in integers) returns the bits of the
+"""cafe_intmath.h (exp, atan2, cos, sin, division, square root in integers) returns the bits of the
 floating-point functions, inside its ranges and outside, and cafe_crmath.h's fast
 paths those of its double-double paths (CPU only)."""
 import ctypes
@@ -105,3 +105,30 @@ def test_fast_paths(ic, kind):
     _same(ic, 4, x, y)
     _same(ic, 5, t)
     _same(ic, 6, t)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "scales", "steps", "exponents", "edges"])
+def test_angles(ic, kind):
+    """atan2 of non-negative arguments, cos on [0, pi/4] and sin on [pi/4, pi/2], and beyond"""
+    g, n = np.random.default_rng(8), 300000
+    y, x, t = g.uniform(0, 1, n), g.uniform(0, 1, n), g.uniform(0, np.pi / 4, n)
+    if kind == "scales":
+        y *= 2.0 ** g.uniform(-60, 0, n)
+        t *= 2.0 ** g.uniform(-50, 0, n)
+    elif kind == "steps":  # at, beside and between the tables' points
+        d = 1 + g.integers(-2, 3, n) * 2.0 ** -52
+        y = x * (g.integers(0, 129, n) / 128) * d
+        t = g.integers(0, 202, n) / 256 * d
+    elif kind == "exponents":
+        e = g.integers(-1000, 1000, n).astype(float)
+        y, x = y * 2.0 ** e, x * 2.0 ** (e + g.integers(-8, 9, n))
+    elif kind == "edges":
+        e = np.concatenate([EDGES, _around(1 / 128), _around(2.0 ** -37)])
+        y, x = np.repeat(e, len(e)), np.tile(e, len(e))
+        t = np.concatenate([EDGES, -EDGES, _around(np.pi / 4), _around(2.0 ** -27), np.pi / 2 - _around(np.pi / 4)])
+    _same(ic, 7, y, x)
+    _same(ic, 7, x, y)
+    _same(ic, 8, t)
+    _same(ic, 9, t)
+    _same(ic, 9, np.pi / 2 - t)
+    _same(ic, 10, np.concatenate([y, -y]))
