@@ -25,7 +25,10 @@ Printed keys beyond the common contract:
              (CUDA events on the engine's stream), against the measured HBM
              copy bandwidth;
   event_cycles  SM cycles per capture/nucleation event of the timed steps,
-             by section of the event loop (its own clock64 counters);
+             by section of the event loop (its own clock64 counters): `winner`
+             the selection and negative events, `capture` the capture, clock
+             and growth, `fill_and_next_selection` the rows of cells that were
+             not foreseen, `merge` the windows opened;
   cpu_baseline  the CPU oracle (a single-threaded restatement of the
              reference) resumed from the GPU state at the start of the timed
              window, for a bounded wall-clock sample.
