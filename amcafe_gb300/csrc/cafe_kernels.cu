@@ -282,7 +282,8 @@ __global__ void k_put_params(CafeStepParams *Pd, CafeStepParams P) { *Pd = P; }
 // step or melted in the pool box; new layers bring solid and powder cells
 // only. In chunks of eight cells along x (x0 a multiple of 8), whose order is
 // the order of their cells. (Whole z planes instead, 62 M cells a step on
-// 1024x1024x256, made the compaction 130 us.)
+// 1024x1024x256, made the compaction 130 us by instruction issue; the box's cells
+// take 22, bound by the latency of their loads.)
 struct CafeBox {
   int x0, y0, z0, nxc, ny;
   long long n;  // chunks
@@ -605,6 +606,9 @@ __device__ __forceinline__ void d_reset_rows(const CafeDev &D, const CafeConsts 
 // or outside the grid), kind (a_kind),
 // all-neighbours-below-liquidus flag and the ruq offset (VoxelsCA.C:380:
 // ruq[p] = (U_p - .5) dX / 100, U_p the p-th uniform of minstd(30 tInd + seed1)).
+// A warp takes 32 positions: one value per position a lane each, then a position's
+// 26 neighbours a lane each, bound by the latency of the scattered loads. With a
+// thread per position it and the lists took 36 us more on 1024x1024x256.
 __device__ __forceinline__ void d_gather(const CafeDev &D, const CafeConsts &K, const CafeStepParams *__restrict__ Pp, const int cafe_bid, const int cafe_nblk) {
   const CafeStepParams P = *Pp;
   int na = D.ctr[CTR_NA];
@@ -871,7 +875,8 @@ __device__ __forceinline__ bool cafe_is_neg(double x) {
 // growth of VoxelsCA.C:511-516), spread over the whole GPU, and copies it back
 // to the row cell's active-list position.
 // The growths come through shared memory, a batch at a time, so that a row's
-// chain is its additions and no load waits on it.
+// chain is its additions (64 cycles each, up to a hundred a step: 20 us) and no
+// load waits on it.
 #define CAFE_FINAL_BATCH 512
 __device__ __forceinline__ void d_rows_finalize(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
   __shared__ double vd[CAFE_FINAL_BATCH];
@@ -967,7 +972,9 @@ __global__ void k_writeback(CafeDev D, CafeConsts K) {
 
 // ConvertSolid1(0): mushy cells whose neighbours are all mushy or solid become
 // solid with zero extent. Every mushy cell is in this step's active list. In
-// place is equivalent to collect-then-apply: 2 -> 3 keeps "neighbour >= 2".
+// place is equivalent to collect-then-apply: 2 -> 3 keeps "neighbour >= 2". A row of
+// three neighbours is read as a word; bound by load latency (7 us; byte by byte
+// through a local array 11).
 __device__ __forceinline__ void d_mushy2solid(const CafeDev &D, const CafeConsts &K, const int cafe_bid, const int cafe_nblk) {
   int na = D.ctr[CTR_NA];
   if (na > D.act_cap) na = (int)D.act_cap;
@@ -1677,7 +1684,9 @@ __global__ void k_easm_long(CafeDev D, CafeConsts K, CafeStepParams P, CafeEasm 
 // The Rosenthal field (extension) over cells [0, ncell): temp, BuildjID as
 // AnalyticTempCurr sets it (TempField.C:180-185), the box of the cells at or
 // above the liquidus and the "some cell below the liquidus" flag, in the slots
-// the EASM field uses.
+// the EASM field uses. Bound by FP64 issue: the distance's root, the division and
+// exp in integers (cafe_intmath.h) took the field from 0.19 to 0.09 ms a step on
+// 256x128x64 cells.
 __global__ void k_rosenthal(CafeDev D, CafeConsts K, CafeStepParams P, long long ncell) {
   __shared__ int s_box[6], s_cold;
   if (threadIdx.x < 3) {
