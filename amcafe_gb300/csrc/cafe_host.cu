@@ -614,18 +614,35 @@ int upload_site_grid(cafe_sim *s, const std::vector<double> &xyz, const HostSite
                      CafeSiteGrid &dv, std::vector<void *> &tmp) {
   double *dxyz;
   int32_t *dstart, *didx;
+  float4 *dnear;
   CUDA_TRY(cudaMalloc((void **)&dxyz, std::max<size_t>(1, xyz.size()) * sizeof(double)));
   tmp.push_back(dxyz);
   CUDA_TRY(cudaMalloc((void **)&dstart, G.start.size() * sizeof(int32_t)));
   tmp.push_back(dstart);
   CUDA_TRY(cudaMalloc((void **)&didx, std::max<size_t>(1, G.idx.size()) * sizeof(int32_t)));
   tmp.push_back(didx);
+  // the sites in bucket order and single precision, for the kernels' first pass
+  std::vector<float4> near(std::max<size_t>(1, G.idx.size()));
+  double top = 0.0;
+  for (size_t t = 0; t < G.idx.size(); ++t) {
+    const double *x = &xyz[3 * (size_t)G.idx[t]];
+    float w;
+    memcpy(&w, &G.idx[t], sizeof w);
+    near[t] = make_float4((float)x[0], (float)x[1], (float)x[2], w);
+    for (int a = 0; a < 3; ++a) top = std::max(top, std::fabs(x[a]));
+  }
+  for (int a = 0; a < 3; ++a) top = std::max(top, std::max(std::fabs(G.lo[a]), std::fabs(G.lo[a] + G.nb[a] * G.h)));
+  CUDA_TRY(cudaMalloc((void **)&dnear, near.size() * sizeof(float4)));
+  tmp.push_back(dnear);
+  CUDA_TRY(cudaMemcpyAsync(dnear, near.data(), near.size() * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(cudaMemcpyAsync(dxyz, xyz.data(), xyz.size() * sizeof(double), cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(cudaMemcpyAsync(dstart, G.start.data(), G.start.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(cudaMemcpyAsync(didx, G.idx.data(), G.idx.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s->stream));
   dv.xyz = dxyz;
   dv.start = dstart;
   dv.idx = didx;
+  dv.near = dnear;
+  dv.top = (float)top * (1.f + 1e-6f);
   for (int a = 0; a < 3; ++a) {
     dv.lo[a] = G.lo[a];
     dv.nb[a] = G.nb[a];

@@ -36,3 +36,13 @@ def test_ragged_grids(tmp_path, nx, ny, nz, theta):
     path = tmp_path / "ragged.in"
     path.write_text(DECK % (nx, ny, nz, -20e-6, theta))
     run_and_compare(str(path), 0, 3, tmp_path)
+
+
+@pytest.mark.parametrize("mu,lrate", [("1e-6", "1e-6"), ("2e-4", ".0009"), (".2", ".1")])
+@pytest.mark.parametrize("nx,ny,nz", [(33, 9, 12), (130, 8, 12), (20, 21, 40)])
+def test_grain_densities(tmp_path, nx, ny, nz, mu, lrate):
+    """from one grain for the whole baseplate to more grains than cells"""
+    path = tmp_path / "ragged.in"
+    text = DECK % (nx, ny, nz, -20e-6, 0.7)
+    path.write_text(text.replace("mu .006", "mu " + mu).replace("lrate .0009", "lrate " + lrate))
+    run_and_compare(str(path), 0, 5, tmp_path)
