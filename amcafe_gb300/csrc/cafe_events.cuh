@@ -29,6 +29,11 @@ __device__ __forceinline__ int cafe_slot_child(uint32_t m) { return (int)(m >> 5
 #define CAFE_SHORT_REACH 1.1    // ... to which a window may shrink
 #define CAFE_FEW_ROWS 512       // up to here every row gets its record (one wave of k_rows_geo)
 
+// The extent that a row's growth starts from, for the bounds of its capture time: the
+// first event lifts a negative one (a host program's state may hold such) to zero
+// (VoxelsCA.C:515), so it grows by no more than from there.
+__device__ __forceinline__ double cafe_lifted(double E) { return E < 0.0 ? 0.0 : E; }
+
 // Sorts the slots of row r (one per lane: liv, numerator gv, neighbour position
 // q) by g (NaN last, ties by slot) into the row's record, and forms the row's key: the order key of T + t
 // for its first candidate, a lower bound of the row's absolute capture time
@@ -52,7 +57,7 @@ __device__ __forceinline__ unsigned long long cafe_row_sort_warp(const CafeDev &
   double t = NAN;
   uint32_t child = 0;
   if (liv) {
-    t = (gv - E) / v;
+    t = (gv - cafe_lifted(E)) / v;
     if (C.off < C.cap && T + t < C.tmax) {
       const int i = C.off + atomicAdd(C.n, 1);
       if (i < C.cap) {
@@ -471,7 +476,7 @@ __device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &
       }
     }
     // the rows that may be due are listed with their pairs
-    double tl = ((double)lo - E) * (v == V1 ? rV1 : 1.0 / v);
+    double tl = ((double)lo - cafe_lifted(E)) * (v == V1 ? rV1 : 1.0 / v);
     tl -= fabs(tl) * 0x1p-40;
     const bool due = lane < n && (all || !gp || !(tl > lim));
     const uint32_t work = due && gp ? liq : 0u;
@@ -504,7 +509,9 @@ __device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &
     const bool in = lane < n;
     const uint32_t ekey = in && !cafe_is_nan(E) ? (uint32_t)(cafe_key(fabs(E)) >> 32) + 1u : 0u;  // NaN extents occur (the reference's 0/0)
     const uint32_t vkey = (uint32_t)(cafe_key(v) >> 32);
-    const uint32_t elow = __reduce_min_sync(FULL, in ? (uint32_t)__double2hiint(E) : 0xffffffffu);
+    // (a sign, that of -0.0 too, counts as the smallest; NaN never captures)
+    const uint32_t elow =
+        __reduce_min_sync(FULL, in && !cafe_is_nan(E) ? (uint32_t)max(__double2hiint(E), 0) : 0xffffffffu);
     if (lane == 0) D.row_low[w] = elow;
     const uint32_t e1 = __reduce_max_sync(FULL, ekey), v0 = __reduce_min_sync(FULL, in ? vkey : 0xffffffffu),
                    v1 = __reduce_max_sync(FULL, in ? vkey + 1u : 0u);
@@ -868,7 +875,7 @@ __device__ __noinline__ void cafe_res_flush(const CafeDev &D, const CafeConsts &
     if (r < L.nrows0) D.row_low[r / CAFE_PREP_ROWS] = 0u;
     D.row_k[r] = S.k[i];
     if (keys) {
-      const double t = (S.g[i] - S.E[i]) / (PR ? S.v[i] : V);
+      const double t = (S.g[i] - cafe_lifted(S.E[i])) / (PR ? S.v[i] : V);
       D.row_key[r] = cafe_is_nan(t) ? CAFE_KEY_NONE : cafe_key(L.tinc + t);
     }
   }

@@ -75,3 +75,59 @@ def test_wide_fronts(tmp_path, nx, ny, nz, rear, half, turn, growth, extra, step
     path.write_text(WIDE % (nx, ny, nz, rear, half, turn, growth, extra))
     s = _same(str(path), steps)
     assert s["events"] > 0
+
+
+# a track's developed front: over a thousand rows, most of them outside the window
+FRONT = """dx 2.5e-6
+nX 256 128 64
+bmV 1.0
+bmP 200.0
+bmDelT %g
+r 2e-4
+lT %g
+bpH %g
+tL 1609
+tS 1531.5
+meltparam 16.31e-6 425.5e-6 55.11e-6 55.11e-6
+bhatch 100e-6
+mu 1.25e-4
+lrate 1.25e-4
+patternID 2
+outint 1000000
+offset 0.0 0.0 0.0
+gridsize 6.4e-4 3.2e-4
+gridtheta 0.0
+dendritegrowth2 1e-5 2.0
+%s
+"""
+
+
+@pytest.mark.parametrize("value", [-0.0, -1e-7])
+@pytest.mark.parametrize("field,spin", [((5e-6, 30e-6, 100e-6, "seed 7"), 40),
+                                        ((5e-6, 50e-6, 10e-6, "rosenthal 0.35 20.0 5e-6"), 60)])
+def test_uploaded_extents_with_a_sign(tmp_path, value, field, spin):
+    """Half of the mushy cells' extents -0.0 or below zero beside some that are
+    overdue: the negative events that these bring clamp the others at zero."""
+    from amcafe_gb300 import Simulation
+
+    path = tmp_path / "front.in"
+    path.write_text(FRONT % field)
+    out = []
+    for scan in (0, 1):
+        with Simulation(str(path), event_scan=scan) as sim:
+            sim.InitializeVoxels()
+            sim.begin()
+            sim.run(spin)
+            st, cth, s0 = sim.state(), sim.ctheta(), sim.stats()
+            m = np.flatnonzero(st["vState"] == 2)
+            u = np.random.default_rng(3).random(m.size)
+            st["extents"][m[u < 0.5]] = value
+            st["extents"][m[u > 0.97]] += 3e-6
+            sim.upload_state(st["gID"], st["vState"], st["extents"], st["centroid"], cth)
+            sim.run(4)
+            s1 = sim.stats()
+            out.append(dict(sim.state(), ctheta=sim.ctheta(), **{
+                k: s1[k] - s0[k] for k in ("events", "nucleations", "negative_dt", "sum_rows")}))
+    assert out[0]["negative_dt"] > 0
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k], equal_nan=np.asarray(out[0][k]).dtype.kind == "f"), k
