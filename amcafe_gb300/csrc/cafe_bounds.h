@@ -61,8 +61,10 @@ CRM_HD float cafe_trunc_f32(double x) {
 // /rho and sin ph = max(rho, |dz|)/r, both in [1/sqrt 2, 1]. The offsets are good
 // to 3e-7 of |c0| plus the cell size (truncation, one product and sum), e is over
 // three times that, and R's truncation adds as little; the quotients take the
-// errors of both operands, so that offsets that cancel only loosen the bound. NaN
-// where an operand is not finite.
+// errors of both operands, so that offsets that cancel only loosen the bound. R need
+// not be a rotation (the axis of an uploaded orientation may have any length): the
+// errors of R^T dn grow with its largest entry, those of a rotation's are below one.
+// NaN where an operand is not finite.
 CRM_HD void cafe_glb_slot(int dir, const float *c0, float dx, const float *R, float &lo, float &hi) {
   const float e = 1e-6f * (fabsf(c0[0]) + fabsf(c0[1]) + fabsf(c0[2]) + 3.f * dx);
   const int d27 = dir < 13 ? dir : dir + 1;
@@ -74,8 +76,11 @@ CRM_HD void cafe_glb_slot(int dir, const float *c0, float dx, const float *R, fl
   const float l0 = R[0] * a + R[3] * b + R[6] * c, l1 = R[1] * a + R[4] * b + R[7] * c,
               l2 = R[2] * a + R[5] * b + R[8] * c;
   const float l = fabsf(l0) + fabsf(l1) + fabsf(l2);
-  lo = sqrtf(ct * sp) * fmaxf(l - 8.f * e, 0.f) * (1.f - 1e-5f);
-  hi = (l + 8.f * e) * (1.f + 1e-5f);
+  float rm = 1.f;
+  for (int k = 0; k < 9; ++k) rm = fmaxf(rm, fabsf(R[k]));
+  const float el = 8.f * e * rm;
+  lo = sqrtf(ct * sp) * fmaxf(l - el, 0.f) * (1.f - 1e-5f);
+  hi = (l + el) * (1.f + 1e-5f);
   if (!(r2 < 1e30f) || !(l < 1e30f) || !(e > 1e-20f)) lo = hi = cafe_f32_from_bits(0x7fc00000);  // (fmaxf drops a NaN operand)
 }
 

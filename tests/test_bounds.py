@@ -53,6 +53,32 @@ def test_numerator_bounds(bc, dx, kind):
     assert np.isnan(lo[:2]).all() and np.isnan(hi[:2]).all()
 
 
+@pytest.mark.parametrize("length", [0.1, 2.0, 5.0, 40.0, 1e6])
+def test_numerator_bounds_of_axes_of_any_length(bc, length):
+    """cTheta as a host program uploads it need not hold a unit axis: the matrix that
+    SampleOrientation's formula makes of it is then no rotation, its entries up to length^2."""
+    n, g, dx = 40000, np.random.default_rng(9), 2.5e-6
+    a = g.normal(size=(n, 3))
+    a *= length / np.linalg.norm(a, axis=1, keepdims=True)
+    w = g.uniform(0, np.pi, n)
+    K = np.zeros((n, 3, 3))
+    K[:, 0, 1], K[:, 0, 2], K[:, 1, 2] = -a[:, 2], a[:, 1], -a[:, 0]
+    K -= K.transpose(0, 2, 1)
+    R = (np.cos(w)[:, None, None] * np.eye(3) + (1 - np.cos(w))[:, None, None] * a[:, :, None] * a[:, None, :] +
+         np.sin(w)[:, None, None] * K)
+    # the numerator in the direction that cancels most: a neighbour's offset that R^T nearly loses
+    c = g.uniform(-1.0, 1.0, (n, 3)) * dx
+    d = (np.arange(n) % 26).astype(np.int32)
+    d27 = np.where(d < 13, d, d + 1)
+    off = np.stack([d27 % 3 - 1, d27 // 3 % 3 - 1, d27 // 9 - 1], axis=1) * dx
+    k = n // 2
+    c[:k] = a[:k] / length * g.uniform(-1, 1, (k, 1)) * 1e-3 * dx + np.cross(a[:k] / length, g.normal(size=(k, 3))) * dx - off[:k]
+    R, c = np.ascontiguousarray(R.reshape(n, 9)), np.ascontiguousarray(c)
+    lo, hi, ex = np.empty(n, np.float32), np.empty(n, np.float32), np.empty(n)
+    bc.bc_glb(ctypes.c_long(n), ctypes.c_double(dx), _p(c, D), _p(R, D), _p(d, I), _p(lo, F), _p(hi, F), _p(ex, D))
+    assert np.all(lo <= ex) and np.all(ex <= hi)
+
+
 @pytest.mark.parametrize("theta", [0.0, 0.7, np.pi / 2, -2.0])
 @pytest.mark.parametrize("dirp", [1.0, -1.0, 0.0, 1e-250])
 @pytest.mark.parametrize("n", [1, 31, 33, 257])
