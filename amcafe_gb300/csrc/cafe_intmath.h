@@ -157,7 +157,7 @@ CRM_HD double crm_quotient(double a, const crm_recip &R, double b, int k) {
 CRM_HD double crm_div_int(double a, double b) { return crm_quotient(a, crm_reciprocal(b), b, 0); }
 
 // ------------------------------------------------------------------ square root
-// Single-precision 1/sqrt(x), a relative 2^-21 at least.
+// Single-precision 1/sqrt(x). CUDA states 2 ulp for rsqrtf, a relative 2^-22.
 CRM_HD float crm_rsqrt_f32(float x) {
 #ifdef __CUDA_ARCH__
   return rsqrtf(x);
@@ -165,28 +165,35 @@ CRM_HD float crm_rsqrt_f32(float x) {
   return 1.0f / sqrtf(x);
 #endif
 }
-// sqrt(x): for positive normal x a 53-bit root from the single-precision one by two
-// steps with exact remainders (errors 2^-21, 2^-42, then a unit), rounded by the
-// last remainder (a root has no ties).
+// The 53-bit root of w 2^42, w in [2^62, 2^64), to nearest (a root has no ties), from
+// f, 1/sqrt(w / 2^62) with a relative error d of 2^-21 at most: two steps with exact
+// remainders leave 1.5 d^2, then less than two units, and the last remainder decides.
+// After the first step the root is off by up to 1.5 2^-42 2^53 = 3072 units and its
+// remainder takes 67 bits; that of the root's upper 51 bits takes 63 (and does up to
+// d = 2^-20.3).
+CRM_HD uint64_t crm_root53(uint64_t w, float f) {
+  f *= 0x1p31f;
+  const uint32_t y = (uint32_t)(f < 2147483520.0f ? f : 2147483520.0f);
+  const uint64_t s0 = ((uint64_t)(uint32_t)(w >> 32) * y) >> 32;  // the root, 2^29
+  const int64_t e0 = (int64_t)(w - ((s0 * s0) << 4));
+  const uint64_t s1 = (s0 << 21) + (uint64_t)(((e0 >> 12) * (int64_t)(uint64_t)y) >> 32);  // 2^50
+  const int64_t e1 = (int64_t)((w << 38) - s1 * s1);
+  uint64_t q = (s1 << 2) + (uint64_t)(((e1 >> 30) * (int64_t)(uint64_t)y) >> 50);
+  // |q - root| < 2: two steps towards the nearest
+  for (int i = 0; i < 2; ++i) {
+    const int64_t r = (int64_t)((w << 42) - q * q);
+    q += (uint64_t)((r > (int64_t)q) - (r <= -(int64_t)q));
+  }
+  return q;
+}
+// sqrt(x), in integers for positive normal x.
 CRM_HD double crm_sqrt_int(double x) {
   const uint64_t b = (uint64_t)crm_bits(x);
   const int eb = (int)(b >> 52);  // (sign included)
   if (eb == 0 || eb >= 2047) return crm_sqrt_fp(x);
   const int odd = (eb & 1) ^ 1;  // exponent eb - 1023 odd
   const uint64_t w = ((b & CRM_MANT_MASK) | CRM_MANT_ONE) << (10 + odd);  // in [1, 4), 2^62
-  const uint32_t wh = (uint32_t)(w >> 32);
-  const float f = crm_rsqrt_f32((float)wh * 0x1p-30f) * 0x1p31f;
-  const uint32_t y = (uint32_t)(f < 2147483520.0f ? f : 2147483520.0f);
-  const uint64_t s0 = ((uint64_t)wh * y) >> 32;  // the root, 2^29
-  const int64_t e0 = (int64_t)(w - ((s0 * s0) << 4));
-  const uint64_t s1 = (s0 << 23) + (uint64_t)(((e0 >> 12) * (int64_t)(uint64_t)y) >> 30);  // 2^52
-  const int64_t e1 = (int64_t)((w << 42) - s1 * s1);
-  uint64_t q = s1 + (uint64_t)(((e1 >> 32) * (int64_t)(uint64_t)y) >> 52);
-  // |q - root| < 2: two steps towards the nearest
-  for (int i = 0; i < 2; ++i) {
-    const int64_t r = (int64_t)((w << 42) - q * q);
-    q += (uint64_t)((r > (int64_t)q) - (r <= -(int64_t)q));
-  }
+  const uint64_t q = crm_root53(w, crm_rsqrt_f32((float)(uint32_t)(w >> 32) * 0x1p-30f));
   return crm_from_bits((long long)(((uint64_t)((eb - 1023 - odd) / 2 + 1022) << 52) + q));
 }
 

@@ -51,3 +51,15 @@ extern "C" void ic_eval(int fn, long n, const double *x, const double *y, double
     }
   }
 }
+
+// sqrt(x) from a single-precision 1/sqrt that is off by a relative `off`.
+extern "C" void ic_root(long n, double off, const double *x, double *got) {
+  for (long i = 0; i < n; ++i) {
+    int e;
+    const double m = frexp(x[i], &e);  // in [1/2, 1)
+    const int odd = e & 1;
+    const uint64_t w = (uint64_t)(m * 0x1p53) << (odd ? 10 : 11);
+    const double f = 1.0 / sqrt((double)w * 0x1p-62) * (1.0 + off);
+    got[i] = ldexp((double)crm_root53(w, (float)f), (odd ? e - 1 : e - 2) / 2 - 52);
+  }
+}

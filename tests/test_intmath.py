@@ -89,6 +89,22 @@ def test_sqrt(ic, emax):
     _same(ic, 3, np.concatenate([s, np.nextafter(s, 0), np.nextafter(s, np.inf), EDGES, -EDGES]))
 
 
+@pytest.mark.parametrize("off", [-2.0 ** -21, -2.0 ** -22, 0.0, 2.0 ** -22, 2.0 ** -21])
+def test_sqrt_of_any_allowed_seed(ic, off):
+    """The device's 1/sqrt is not the host's: the root is right for any that is good to 2^-21."""
+    g, n = np.random.default_rng(4), 400000
+    x = g.uniform(1, 4, n)
+    x[: n // 4] = 4.0 - np.arange(1, n // 4 + 1) * 2.0 ** -51  # the largest remainders: just below powers of four
+    x[n // 4: n // 2] = 1.0 + np.arange(n // 4) * 2.0 ** -52
+    x = x * 4.0 ** g.integers(-500, 500, n)
+    got = np.empty(n)
+    ic.ic_root(ctypes.c_long(n), ctypes.c_double(off * (1 - 2.0 ** -2)), x.ctypes.data_as(D), got.ctypes.data_as(D))
+    assert np.array_equal(got, np.sqrt(x))
+    # the whole allowance, the rounding of f to single precision (2^-24) included
+    ic.ic_root(ctypes.c_long(n), ctypes.c_double(off + np.sign(-off) * 2.0 ** -24), x.ctypes.data_as(D), got.ctypes.data_as(D))
+    assert np.array_equal(got, np.sqrt(x))
+
+
 @pytest.mark.parametrize("kind", ["uniform", "scales", "midpoints"])
 def test_fast_paths(ic, kind):
     """arctangent, sine and cosine at arguments where the series' terms are largest"""
