@@ -58,7 +58,7 @@
 #undef CRM_TABLE_DECL
 #endif
 
-// Profiling builds count the calls that leave the fast paths.
+// Profiling builds count the calls that leave the fast paths (printed by cafe_sim_stats).
 #if defined(CAFE_DETAIL_CYCLES) && defined(__CUDACC__)
 __device__ unsigned long long crm_fallback_calls, crm_special_calls;
 #ifdef __CUDA_ARCH__

@@ -1667,9 +1667,10 @@ int cafe_sim_stats(cafe_sim *s, cafe_stats *st) {
   st->graph_captures = (unsigned long long)s->graph_captures;
   st->easm_integrals = v[STAT_EASM_INTEGRALS];
 #ifdef CAFE_DETAIL_CYCLES
-  fprintf(stderr, "cafe detail cycles:");
-  for (int c = 0; c < 32; ++c) fprintf(stderr, " %llu", v[STAT_DETAIL + c]);
-  fprintf(stderr, "\n");
+  unsigned long long left = 0, special = 0;
+  CUDA_TRY(cudaMemcpyFromSymbol(&left, crm_fallback_calls, sizeof left));
+  CUDA_TRY(cudaMemcpyFromSymbol(&special, crm_special_calls, sizeof special));
+  fprintf(stderr, "cafe: calls that left the fast paths %llu, with special arguments %llu\n", left, special);
 #endif
   return CAFE_OK;
 }
