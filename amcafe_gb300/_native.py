@@ -23,7 +23,7 @@ EXPORTS = (
     "cafe_batch_create", "cafe_batch_run", "cafe_batch_size", "cafe_batch_sim", "cafe_batch_finished",
     "cafe_batch_destroy", "cafe_sim_checkpoint", "cafe_sim_restore", "cafe_sim_set_growth_log",
     "cafe_sim_growth_log_count", "cafe_adjoint_pool", "cafe_adjoint_growth", "cafe_sim_grid",
-    "cafe_generate_samples", "cafe_batch_report", "cafe_sim_set_output",
+    "cafe_generate_samples", "cafe_batch_report", "cafe_sim_set_output", "cafe_sim_event_paths",
 )
 PHASES = ("melt", "classify", "gather", "events", "writeback", "layer")
 NPHASE = 8
@@ -77,6 +77,10 @@ class CafeStats(ctypes.Structure):
                 ("cycles_merge", ctypes.c_ulonglong)]
 
 
+class CafeEventPaths(ctypes.Structure):
+    _fields_ = [("full_scan_steps", ctypes.c_ulonglong)]
+
+
 _lib = None
 
 
@@ -112,6 +116,7 @@ def load():
         "cafe_batch_report": (I, [P, ctypes.POINTER(LL), ctypes.POINTER(LL), ctypes.c_char_p, I]),
         "cafe_sim_set_output": (I, [P, ctypes.c_char_p]),
         "cafe_sim_stats": (I, [P, ctypes.POINTER(CafeStats)]),
+        "cafe_sim_event_paths": (I, [P, ctypes.POINTER(CafeEventPaths)]),
         "cafe_sim_download_state": (I, [P, i32p, i32p, f64p, f64p, i32p]),
         "cafe_sim_download_temperature": (I, [P, f64p]),
         "cafe_sim_download_ctheta": (I, [P, f64p, LL, ctypes.POINTER(I)]),

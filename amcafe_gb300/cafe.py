@@ -25,7 +25,7 @@ import os
 
 import numpy as np
 
-from ._native import NPHASE, PHASES, CafeGrid, CafeInfo, CafeOptions, CafeStats, check, load
+from ._native import NPHASE, PHASES, CafeEventPaths, CafeGrid, CafeInfo, CafeOptions, CafeStats, check, load
 
 
 def _ptr(a, ct):
@@ -109,6 +109,12 @@ class Simulation:
         s = CafeStats()
         check(self._lib.cafe_sim_stats(self._h, ctypes.byref(s)))
         return {f: getattr(s, f) for f, _ in CafeStats._fields_}
+
+    def event_paths(self):
+        """The paths that the event loop took (cafe_sim_event_paths)."""
+        p = CafeEventPaths()
+        check(self._lib.cafe_sim_event_paths(self._h, ctypes.byref(p)))
+        return {f: getattr(p, f) for f, _ in CafeEventPaths._fields_}
 
     def state(self, out=None):
         """gID, vState, extents, centroid (x,y,z interleaved) and buildj as

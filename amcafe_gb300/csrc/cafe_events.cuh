@@ -1653,6 +1653,7 @@ __device__ __noinline__ void cafe_events_scan(const CafeDev &D, const CafeConsts
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = CAFE_LOOP_THREADS, NW = CAFE_WARPS;
   if (L.done || !(mode == 2 || L.sw)) return;
+  if (tid == 0) atomicAdd(&D.stat[STAT_FULLSCAN], 1ULL);
   {
     // every row needs its record, and extents are kept current from here on
     for (int k = warp >> 2; k < L.nrows; k += CAFE_QUADS) {

@@ -1675,6 +1675,15 @@ int cafe_sim_stats(cafe_sim *s, cafe_stats *st) {
   return CAFE_OK;
 }
 
+int cafe_sim_event_paths(cafe_sim *s, cafe_event_paths *p) {
+  if (!s || !p) return fail(CAFE_E_ARG, "null argument");
+  unsigned long long v[STAT_COUNT];
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  CUDA_TRY(cudaMemcpy(v, s->D.stat, sizeof v, cudaMemcpyDeviceToHost));
+  p->full_scan_steps = v[STAT_FULLSCAN];
+  return CAFE_OK;
+}
+
 int cafe_sim_set_timing(cafe_sim *s, int on) {
   if (!s) return fail(CAFE_E_ARG, "null handle");
   CUDA_TRY(cudaSetDevice(s->device));

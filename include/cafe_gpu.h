@@ -82,6 +82,12 @@ typedef struct {
   unsigned long long cycles_merge;     /* ... opening windows */
 } cafe_stats;
 
+/* The paths that the event loop took, summed over the handle's steps. */
+typedef struct {
+  unsigned long long full_scan_steps; /* steps with events that evaluated every frontier row: asked for
+                                         (event_scan), or where the resident window cannot be used */
+} cafe_event_paths;
+
 /* Grid::Grid (Grid.C:15-109, deck parse Grid.C:165-318) + Partition::
  * PartitionGraph2 at world size 1 (Partition.C:260-412) + BasePlate::BasePlate
  * (BasePlate.C:18-30) + TempField::TempField/InitializeAnalytic
@@ -174,6 +180,7 @@ int cafe_sim_stream(cafe_sim *sim, void **stream);
 int cafe_sim_mark(cafe_sim *sim, int slot);
 int cafe_sim_elapsed(cafe_sim *sim, int a, int b, double *ms);
 int cafe_sim_stats(cafe_sim *sim, cafe_stats *stats);
+int cafe_sim_event_paths(cafe_sim *sim, cafe_event_paths *paths);
 
 /* VoxelsCA public fields gID, vState, extents, centroidOct (x,y,z interleaved,
  * 3 per cell) and TempField::BuildjID, N = nx*ny*nz entries each; any pointer

@@ -131,3 +131,19 @@ def test_uploaded_extents_with_a_sign(tmp_path, value, field, spin):
     assert out[0]["negative_dt"] > 0
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k], equal_nan=np.asarray(out[0][k]).dtype.kind == "f"), k
+
+
+@pytest.mark.parametrize("deck,steps", [("layers_rot.in", 40), ("track_easm60.in", 0), ("track_ros.in", 0)])
+def test_no_step_falls_back_to_the_full_scan(deck, steps):
+    """Neither with one growth velocity nor with per-cell ones; with event_scan=1 every step with events does."""
+    from amcafe_gb300 import Simulation
+
+    seen = []
+    for scan in (0, 1):
+        with Simulation(os.path.join(DECKS, deck), event_scan=scan) as sim:
+            sim.InitializeVoxels()
+            sim.begin()
+            sim.run(steps)
+            seen.append((sim.event_paths()["full_scan_steps"], sim.stats()))
+    assert seen[0][0] == 0 and seen[0][1]["events"] > 0
+    assert 0 < seen[1][0] <= seen[1][1]["steps"]
