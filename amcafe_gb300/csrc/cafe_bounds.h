@@ -65,7 +65,8 @@ CRM_HD float cafe_trunc_f32(double x) {
 // not be a rotation (the axis of an uploaded orientation may have any length): the
 // errors of R^T dn grow with its largest entry, those of a rotation's are below one.
 // NaN where an operand is not finite.
-CRM_HD void cafe_glb_slot(int dir, const float *c0, float dx, const float *R, float &lo, float &hi) {
+// rm: one, or the largest magnitude in R where that is more.
+CRM_HD void cafe_glb_slot(int dir, const float *c0, float dx, const float *R, float rm, float &lo, float &hi) {
   const float e = 1e-6f * (fabsf(c0[0]) + fabsf(c0[1]) + fabsf(c0[2]) + 3.f * dx);
   const int d27 = dir < 13 ? dir : dir + 1;
   const float a = c0[0] + (float)(d27 % 3 - 1) * dx, b = c0[1] + (float)(d27 / 3 % 3 - 1) * dx,
@@ -76,12 +77,15 @@ CRM_HD void cafe_glb_slot(int dir, const float *c0, float dx, const float *R, fl
   const float l0 = R[0] * a + R[3] * b + R[6] * c, l1 = R[1] * a + R[4] * b + R[7] * c,
               l2 = R[2] * a + R[5] * b + R[8] * c;
   const float l = fabsf(l0) + fabsf(l1) + fabsf(l2);
-  float rm = 1.f;
-  for (int k = 0; k < 9; ++k) rm = fmaxf(rm, fabsf(R[k]));
   const float el = 8.f * e * rm;
   lo = sqrtf(ct * sp) * fmaxf(l - el, 0.f) * (1.f - 1e-5f);
   hi = (l + el) * (1.f + 1e-5f);
   if (!(r2 < 1e30f) || !(l < 1e30f) || !(e > 1e-20f)) lo = hi = cafe_f32_from_bits(0x7fc00000);  // (fmaxf drops a NaN operand)
+}
+CRM_HD void cafe_glb_slot(int dir, const float *c0, float dx, const float *R, float &lo, float &hi) {
+  float rm = 1.f;
+  for (int k = 0; k < 9; ++k) rm = fmaxf(rm, fabsf(R[k]));
+  cafe_glb_slot(dir, c0, dx, R, rm, lo, hi);
 }
 
 // ------------------------------------------------------------------ temperature class

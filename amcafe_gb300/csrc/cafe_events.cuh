@@ -32,7 +32,7 @@ __device__ __forceinline__ int cafe_slot_child(uint32_t m) { return (int)(m >> 5
 // The extent that a row's growth starts from, for the bounds of its capture time: the
 // first event lifts a negative one (a host program's state may hold such) to zero
 // (VoxelsCA.C:515), so it grows by no more than from there.
-__device__ __forceinline__ double cafe_lifted(double E) { return E < 0.0 ? 0.0 : E; }
+__device__ __forceinline__ double cafe_lifted(double E) { return cafe_is_neg(E) ? 0.0 : E; }
 
 // Sorts the slots of row r (one per lane: liv, numerator gv, neighbour position
 // q) by g (NaN last, ties by slot) into the row's record, and forms the row's key: the order key of T + t
@@ -112,6 +112,15 @@ __device__ __forceinline__ void cafe_glb_centre(const CafeConsts &K, int si, int
   double dn[3];
   cafe_geo_dn(K, si, sj, sk, cs, dn);
   for (int a = 0; a < 3; ++a) c0[a] = cafe_trunc_f32(dn[a]);
+}
+// The rotation Rg in single precision, the same in every lane, and its largest entry: an
+// entry a lane and shuffles, in place of nine conversions (eight operations each) in every lane.
+__device__ __forceinline__ void cafe_glb_rot(const double *Rg, float *R, float &rm) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const float x = lane < 9 ? cafe_trunc_f32(Rg[lane]) : 1.f;
+  rm = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(fabsf(x))));
+  for (int a = 0; a < 9; ++a) R[a] = __shfl_sync(FULL, x, a);
 }
 // Smallest lower and largest upper bound over the slots `liv` of a warp; any NaN gives NaN.
 __device__ __forceinline__ void cafe_glb_range(bool liv, float &lo, float &hi) {
@@ -462,10 +471,9 @@ __device__ __forceinline__ void d_rows_prep(const CafeDev &D, const CafeConsts &
       }
       float l = 0.f, h = 0.f;
       if (gt) {
-        const double *Rg = D.rot + 9LL * (gt - 1);
-        float R[9];
-        for (int a = 0; a < 9; ++a) R[a] = cafe_trunc_f32(Rg[a]);
-        if (liv) cafe_glb_slot(lane, ct, dx, R, l, h);
+        float R[9], rm;
+        cafe_glb_rot(D.rot + 9LL * (gt - 1), R, rm);
+        if (liv) cafe_glb_slot(lane, ct, dx, R, rm, l, h);
         cafe_glb_range(liv, l, h);
         gmax = fmaxf(gmax, h);  // (fmaxf drops NaN: such a row's times are NaN)
       }
@@ -636,12 +644,11 @@ __device__ __forceinline__ void d_children(const CafeDev &D, const CafeConsts &K
     if (nc.gid >= 1 && nc.gid <= D.grain_cap) {
       int si, sj, sk;
       cafe_cell_xyz(K, D.act[p], si, sj, sk);
-      const double *Rg = D.rot + 9LL * (nc.gid - 1);
-      float R[9], c0[3];
-      for (int a = 0; a < 9; ++a) R[a] = cafe_trunc_f32(Rg[a]);
+      float R[9], c0[3], rm;
+      cafe_glb_rot(D.rot + 9LL * (nc.gid - 1), R, rm);
       const float dx = (float)K.dx[0];
       cafe_glb_centre(K, si, sj, sk, nc.c, c0);
-      if (liv) cafe_glb_slot(lane, c0, dx, R, lo, hi);
+      if (liv) cafe_glb_slot(lane, c0, dx, R, rm, lo, hi);
       cafe_glb_range(liv, lo, hi);
       tl = cafe_lb_time(lo, nc.ext, v);
       due = K.all_rows || !(T + tl > K.DelT * CAFE_DUE_REACH) || !cafe_v_ordinary(v);
