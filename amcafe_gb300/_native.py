@@ -78,7 +78,8 @@ class CafeStats(ctypes.Structure):
 
 
 class CafeEventPaths(ctypes.Structure):
-    _fields_ = [("full_scan_steps", ctypes.c_ulonglong)]
+    _fields_ = [("full_scan_steps", ctypes.c_ulonglong), ("records_late", ctypes.c_ulonglong),
+                ("rows_outside", ctypes.c_ulonglong), ("rows_filled", ctypes.c_ulonglong)]
 
 
 _lib = None

@@ -245,7 +245,7 @@ enum {
 static_assert(CTR_EASM_CURSOR % 2 == 0, "64-bit cursor needs an 8-byte aligned slot");
 enum { STAT_EVENTS = 0, STAT_NUC, STAT_MAXNA, STAT_MAXROWS, STAT_STEPS, STAT_NEGDT, STAT_SUMNA, STAT_SUMROWS,
        STAT_SLOWSTEPS, STAT_EVALS, STAT_CYC_SELECT, STAT_CYC_APPLY, STAT_CYC_FILL, STAT_CYC_OTHER,
-       STAT_EASM_INTEGRALS, STAT_FULLSCAN, STAT_COUNT };
+       STAT_EASM_INTEGRALS, STAT_FULLSCAN, STAT_LATE, STAT_OUTSIDE, STAT_FILLED, STAT_COUNT };
 
 // --------------------------------------------------------------- temperature
 // TempField::AnalyticTempCurr (TempField.C:155-190) for one cell; returns the

@@ -738,6 +738,7 @@ struct CafeLoop {
   uint32_t rng;
   unsigned int sdloc;
   long long nnuc, negdt, opens, cyc[4];
+  int late, outside, filled;  // cafe_event_paths
   CafeNewCell nc;
 };
 struct CafeResident {
@@ -1056,6 +1057,7 @@ __device__ __noinline__ void cafe_window_open(const CafeDev &D, const CafeConsts
   }
   __syncthreads();
   // the records that were not made, four rows at a time
+  if (tid == 0) L.late += S.nfill;
   for (int j = warp >> 2; j < S.nfill; j += CAFE_QUADS) cafe_make_record(D, K, L, Q, S.r[S.free[j]]);
   __syncthreads();
   {
@@ -1205,6 +1207,7 @@ __device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K,
     const CafeChildList none = {nullptr, 0, 0, 0.0};
     const unsigned long long gk = cafe_row_fill_quad(D, K, nr, icap, L.tinc, Q[0], L.nc, none);
     if (tid == 0) {
+      L.filled++;
       D.row_E[nr] = L.nc.ext;
       if (gk != 0ULL) L.gmax = fmax(L.gmax, cafe_unkey(gk));
       if (!cafe_is_nan(L.nc.ext)) L.emax = fmax(L.emax, fabs(L.nc.ext));
@@ -1618,6 +1621,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
         S.all = 0;
       }
       S.klim[(ev + 1) & 1] = cafe_window_limit<PR>(S, Vf, ev, L.tinc, dsum);
+      L.outside += S.outside;
     }
     if (tid == 0) {
       const long long t1 = clock64();
@@ -1829,6 +1833,7 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
     L.vmax = D.row_mag[3] ? cafe_unkey(D.row_mag[3]) : 1.0;
     L.countS = L.na;
     L.nnuc = L.negdt = L.opens = 0;
+    L.late = L.outside = L.filled = 0;
     L.ev = L.sw = 0;
     L.newrow = -1;
     L.cyc[0] = L.cyc[1] = L.cyc[2] = L.cyc[3] = 0;
@@ -1870,6 +1875,9 @@ __device__ __forceinline__ void d_event_loop(const CafeDev &D, const CafeConsts 
     atomicAdd(&D.stat[STAT_SUMROWS], (unsigned long long)L.nrows);
     atomicAdd(&D.stat[STAT_EVALS], (unsigned long long)L.opens);
     if (mode || L.sw) atomicAdd(&D.stat[STAT_SLOWSTEPS], 1ULL);
+    if (L.late) atomicAdd(&D.stat[STAT_LATE], (unsigned long long)L.late);
+    if (L.outside) atomicAdd(&D.stat[STAT_OUTSIDE], (unsigned long long)L.outside);
+    if (L.filled) atomicAdd(&D.stat[STAT_FILLED], (unsigned long long)L.filled);
     for (int c = 0; c < 4; ++c) atomicAdd(&D.stat[STAT_CYC_SELECT + c], (unsigned long long)L.cyc[c]);
   }
 }

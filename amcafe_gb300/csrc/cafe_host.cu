@@ -1681,6 +1681,9 @@ int cafe_sim_event_paths(cafe_sim *s, cafe_event_paths *p) {
   CUDA_TRY(cudaStreamSynchronize(s->stream));
   CUDA_TRY(cudaMemcpy(v, s->D.stat, sizeof v, cudaMemcpyDeviceToHost));
   p->full_scan_steps = v[STAT_FULLSCAN];
+  p->records_late = v[STAT_LATE];
+  p->rows_outside = v[STAT_OUTSIDE];
+  p->rows_filled = v[STAT_FILLED];
   return CAFE_OK;
 }
 

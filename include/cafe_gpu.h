@@ -86,6 +86,11 @@ typedef struct {
 typedef struct {
   unsigned long long full_scan_steps; /* steps with events that evaluated every frontier row: asked for
                                          (event_scan), or where the resident window cannot be used */
+  unsigned long long records_late;    /* frontier rows whose record a reopened window made: their lower
+                                         bound had put them past the step */
+  unsigned long long rows_outside;    /* rows of foreseen captures that stayed outside the window */
+  unsigned long long rows_filled;     /* rows that the loop set up itself: captures that were not
+                                         foreseen or come due again at once, nucleations */
 } cafe_event_paths;
 
 /* Grid::Grid (Grid.C:15-109, deck parse Grid.C:165-318) + Partition::

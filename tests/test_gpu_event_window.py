@@ -102,35 +102,60 @@ dendritegrowth2 1e-5 2.0
 """
 
 
-@pytest.mark.parametrize("value", [-0.0, -1e-7])
-@pytest.mark.parametrize("field,spin", [((5e-6, 30e-6, 100e-6, "seed 7"), 40),
-                                        ((5e-6, 50e-6, 10e-6, "rosenthal 0.35 20.0 5e-6"), 60)])
-def test_uploaded_extents_with_a_sign(tmp_path, value, field, spin):
-    """Half of the mushy cells' extents -0.0 or below zero beside some that are
-    overdue: the negative events that these bring clamp the others at zero."""
+def _uploaded(path, spin, steps, extent=None):
+    """`steps` steps from a developed state whose mushy cells are in part overdue (and half
+    of them set to `extent`), by the window and by the full scan: same results. Returns the
+    window's counts over these steps."""
     from amcafe_gb300 import Simulation
 
-    path = tmp_path / "front.in"
-    path.write_text(FRONT % field)
     out = []
     for scan in (0, 1):
         with Simulation(str(path), event_scan=scan) as sim:
             sim.InitializeVoxels()
             sim.begin()
             sim.run(spin)
-            st, cth, s0 = sim.state(), sim.ctheta(), sim.stats()
+            st, cth, s0 = sim.state(), sim.ctheta(), dict(sim.stats(), **sim.event_paths())
             m = np.flatnonzero(st["vState"] == 2)
             u = np.random.default_rng(3).random(m.size)
-            st["extents"][m[u < 0.5]] = value
+            if extent is not None:
+                st["extents"][m[u < 0.5]] = extent
             st["extents"][m[u > 0.97]] += 3e-6
             sim.upload_state(st["gID"], st["vState"], st["extents"], st["centroid"], cth)
-            sim.run(4)
-            s1 = sim.stats()
-            out.append(dict(sim.state(), ctheta=sim.ctheta(), **{
-                k: s1[k] - s0[k] for k in ("events", "nucleations", "negative_dt", "sum_rows")}))
-    assert out[0]["negative_dt"] > 0
-    for k in out[0]:
-        assert np.array_equal(out[0][k], out[1][k], equal_nan=np.asarray(out[0][k]).dtype.kind == "f"), k
+            sim.run(steps)
+            s1 = dict(sim.stats(), **sim.event_paths())
+            out.append((dict(sim.state(), ctheta=sim.ctheta()), {k: s1[k] - s0[k] for k in s1}, s1["max_rows"]))
+    (a, sa, rows), (b, sb, _) = out
+    for k in ("events", "nucleations", "negative_dt", "sum_rows"):
+        assert sa[k] == sb[k], k
+    for k in a:
+        assert np.array_equal(a[k], b[k], equal_nan=a[k].dtype.kind == "f"), k
+    return dict(sa, max_rows=rows)
+
+
+@pytest.mark.parametrize("value", [-0.0, -1e-7])
+@pytest.mark.parametrize("field,spin", [((5e-6, 30e-6, 100e-6, "seed 7"), 40),
+                                        ((5e-6, 50e-6, 10e-6, "rosenthal 0.35 20.0 5e-6"), 60)])
+def test_uploaded_extents_with_a_sign(tmp_path, value, field, spin):
+    """Half of the mushy cells' extents -0.0 or below zero beside some that are
+    overdue: the negative events that these bring clamp the others at zero."""
+    path = tmp_path / "front.in"
+    path.write_text(FRONT % field)
+    s = _uploaded(path, spin, 4, value)
+    assert s["negative_dt"] > 0
+
+
+@pytest.mark.parametrize("dt", [5e-6, 1e-5, 2e-5])
+def test_every_part_of_the_window_runs(tmp_path, dt):
+    """A front on which the loop takes all its parts: bounds in place of records (more than
+    512 rows), windows (more than 640 rows) opened again within a step, records made
+    then, rows kept outside, rows set up in the loop, negative events."""
+    path = tmp_path / "front.in"
+    path.write_text(FRONT % (dt, 30e-6, 100e-6, "seed 7"))
+    s = _uploaded(path, int(2e-4 / dt), 6)
+    assert s["max_rows"] > 640 and s["full_scan_steps"] == 0
+    assert s["row_evaluations"] > s["steps"] == 6  # windows opened
+    for k in ("records_late", "rows_outside", "rows_filled", "negative_dt"):
+        assert s[k] > 0, k
 
 
 @pytest.mark.parametrize("deck,steps", [("layers_rot.in", 40), ("track_easm60.in", 0), ("track_ros.in", 0)])
