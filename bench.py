@@ -25,10 +25,10 @@ Printed keys beyond the common contract:
              (CUDA events on the engine's stream), against the measured HBM
              copy bandwidth;
   event_cycles  SM cycles per capture/nucleation event of the timed steps,
-             by section of the event loop (its own clock64 counters): `winner`
-             the selection and negative events, `capture` the capture, clock
-             and growth, `fill_and_next_selection` the rows of cells that were
-             not foreseen, `merge` the windows opened;
+             by section of the event loop (its own clock64 counters):
+             `select` the selection and negative events, `apply` the capture,
+             clock and growth, `unforeseen_rows` the rows that the loop set up
+             itself, `windows` the windows opened;
   cpu_baseline  the CPU oracle (a single-threaded restatement of the
              reference) resumed from the GPU state at the start of the timed
              window, for a bounded wall-clock sample.
@@ -874,8 +874,8 @@ def main():
             # the event loop's own clock (thread 0 of its block), SM cycles per
             # capture/nucleation event in the timed steps, by section
             "event_cycles": {sec: round((stats1["cycles_" + key] - stats0["cycles_" + key]) / max(1, ev))
-                             for sec, key in (("winner", "select"), ("capture", "apply"),
-                                              ("fill_and_next_selection", "fill"), ("merge", "merge"))},
+                             for sec, key in (("select", "select"), ("apply", "apply"),
+                                              ("unforeseen_rows", "fill"), ("windows", "merge"))},
             "phase_ms": {p: round(v[0], 3) for p, v in phases.items()},
             "wall_s_timed": wall,
             "setup_s": setup_s,
