@@ -109,8 +109,9 @@ struct CafeConsts {
 // A cell whose fixed point has not converged after CAFE_EASM_LANE_INTEGRALS
 // integrals in the lane-per-cell pass continues in the warp-per-cell pass, where an
 // integral costs several times as much (its 25 additions take a warp's time) but
-// one cell's hundred integrals end soon. On 181 x 93 x 47 cells a step takes 2.05 ms
-// with 4, 1.93 with 6, 1.87 with 8, 1.99 with 12.
+// one cell's hundred integrals end soon. A step of a single track takes, with 4, 6, 8
+// and 12: 1.74, 1.66, 1.64 and 1.93 ms on 128 x 64 x 32 cells, 2.03, 1.90, 1.82 and
+// 2.04 on 181 x 93 x 47, 4.11, 4.08, 4.12 and 4.04 on 512 x 256 x 128.
 #define CAFE_EASM_LANE_INTEGRALS 8
 struct CafeEasmItem {
   long long idx;

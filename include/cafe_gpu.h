@@ -36,9 +36,10 @@ typedef struct {
   long long grain_capacity;    /* initial grain-table capacity; 0 = automatic */
   int event_scan;              /* 0: keyed event selection (default); 1: evaluate every
                                   frontier cell at every event (the reference's scan) */
-  int event_fill_helper;       /* 1: batched launches give the event loop of each realisation a
-                                  second thread block. It is idle: new frontier rows are set up
-                                  ahead of the loop. Same results as 0 (default) */
+  int event_fill_helper;       /* accepted, without a use: new frontier rows are set up ahead of the
+                                  event loop. 1: a batch whose realisations all have it launches (and
+                                  reports) a second, idle block per event loop; a plain simulation
+                                  runs as with 0 (default). Same results */
 } cafe_options;
 
 typedef struct {
