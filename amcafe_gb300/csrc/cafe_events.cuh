@@ -30,7 +30,7 @@ __device__ __forceinline__ int cafe_slot_child(uint32_t m) { return (int)(m >> 5
 #define CAFE_FEW_ROWS 512       // up to here every row gets its record (one wave of k_rows_geo)
 
 // The extent that a row's growth starts from, for the bounds of its capture time: the
-// first event lifts a negative one (a host program's state may hold such) to zero
+// first capture lifts a negative one (a host program's state may hold such) to zero
 // (VoxelsCA.C:515), so it grows by no more than from there.
 __device__ __forceinline__ double cafe_lifted(double E) { return cafe_is_neg(E) ? 0.0 : E; }
 
@@ -368,14 +368,19 @@ __device__ __noinline__ void cafe_row_best(const CafeDev &D, int r, double E, do
 // else DtMin, which each row multiplies by its own velocity.
 #define CAFE_M_DONE 0x7fffffff  // row_m of a row whose extent is kept current elsewhere
 
-// One event's growth of an extent (VoxelsCA.C:511-516).
+// One event's growth of an extent (VoxelsCA.C:511-516): (E < 0.0) ? 0.0 : E after the
+// addition. A nucleation grows no extent (VoxelsCA.C:483-505) and logs -0, which leaves
+// every one as it is; one below zero (a host program's state may hold such) is
+// lifted by the first event that grows it. On an event's chain, hence one test of the
+// sum's high word: a NaN that an addition returns is quiet (above infinity's high
+// word), and only -0 with -0 adds up to -0.
 __device__ __forceinline__ double cafe_grow(double E, double vd) {
+  const bool grows = crm_bits(vd) != ~CRM_ABS_MASK;
   E = E + vd;
-  return cafe_is_neg(E) ? 0.0 : E;  // (E < 0.0) ? 0.0 : E
+  return grows && ((unsigned)__double2hiint(E) ^ 0x80000000u) <= 0x7ff00000u ? 0.0 : E;
 }
 // Extent of row r after the logged growth of events row_m+1 .. min(upto, its
-// last). A nucleation logs +0, which leaves an extent unchanged (extents
-// are never -0).
+// last).
 template <bool PR>
 __device__ __forceinline__ double cafe_row_replayed(const CafeDev &D, int r, int upto, double v, int &stop) {
   const int m = D.row_m[r];
@@ -1520,7 +1525,7 @@ __device__ __forceinline__ void cafe_events_resident(const CafeDev &D, const Caf
       }
       const double t = exact ? S.red[0].t : (PR ? wd / S.v[win] : cafe_div_by(wd, V, rV));
       const double dt = nuc ? 0.0 : t;
-      const double vd = PR ? dt : (nuc ? 0.0 : V * dt);
+      const double vd = nuc ? -0.0 : PR ? dt : V * dt;  // (cafe_grow)
       const double tinc = L.tinc + dt;
       L.vd = vd;
       D.ev_vd[ev] = vd;

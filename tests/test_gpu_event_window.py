@@ -172,3 +172,14 @@ def test_no_step_falls_back_to_the_full_scan(deck, steps):
             seen.append((sim.event_paths()["full_scan_steps"], sim.stats()))
     assert seen[0][0] == 0 and seen[0][1]["events"] > 0
     assert 0 < seen[1][0] <= seen[1][1]["steps"]
+
+
+@pytest.mark.parametrize("field", [(5e-6, 30e-6, 100e-6, "seed 7"), (5e-6, 50e-6, 10e-6, "rosenthal 0.35 20.0 5e-6")])
+def test_nucleations_leave_extents_below_zero(tmp_path, field):
+    """Fifteen of sixteen events nucleate: uploaded extents below zero stay as they
+    are until the first capture grows them."""
+    path = tmp_path / "front.in"
+    path.write_text((FRONT % field).replace("r 2e-4", "r 6e-2"))
+    for steps in (1, 3):
+        s = _uploaded(path, 50, steps, -1e-7)
+        assert s["nucleations"] > 0
