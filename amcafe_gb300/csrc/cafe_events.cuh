@@ -1231,7 +1231,7 @@ __device__ __noinline__ bool cafe_new_row(const CafeDev &D, const CafeConsts &K,
 }
 
 // Keyed loop over the resident set; every thread of the block calls it. Bound by the
-// chain of an event, ~6.0k cycles on 512x256x128 (36k when the winner was searched
+// chain of an event, ~6.2k cycles on 512x256x128 (36k when the winner was searched
 // among all rows and the captured cell's row made behind it), ~11 cycles an
 // instruction: hence one warp per independent part, two barriers, and the rare
 // parts out of line. Leaves
